@@ -78,6 +78,9 @@ struct RepGeom {
   int cao;
   long long p0, np;  // particle range
   long long rm_off;  // real mesh offset (elements)
+  long long tl_off;  // assignment tile offset (elements)
+  int sbn[3];        // super-bricks of the charge assignment per dimension
+  int cov_off[3];    // per axis: its cover table (see cover_entry)
   long long re_off;  // field mesh offset (records of 4 values)
   int epad[3];       // field mesh extent: mesh plus high-side ghost layers
   long long bin_off; // corner key offset: bricks of brick^3 corners

@@ -252,7 +252,12 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     if (G.np >= (1LL << kNbIndexBits))
       throw Error(1, "a replica holds more than 2^26 particles (Verlet list index limit)");
   cudaStream_t st = m_stream;
-  upload_vec(m_geom_d, m_geom, st);
+  int sms = 148;
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
   {
     std::vector<typename CplxOf<double>::type> t64(tw.size());
     for (size_t k = 0; k < tw.size(); ++k)
@@ -294,91 +299,58 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
         bp.push_back(int2{r, b});
       m_blk_pair_start.push_back(static_cast<int>(bp.size()));
     }
-    // super-bricks of the charge assignment grouped by colour: per
-    // dimension, the tile intervals [bE, bE + min(E, M - bE) + cao - 1) of
-    // the super-bricks (E = kSbEdge) on the periodic axis are coloured
-    // greedily so that intervals of one colour never intersect (modulo M);
-    // super-bricks sharing the colour triple then have disjoint tiles.  All
-    // sort bricks in spatial order feed the interpolation.
+    // super-bricks of the charge assignment and sort bricks of the
+    // interpolation, grouped by order (one launch of each per order present;
+    // replicas may differ in cao), in spatial order; cover tables of the
+    // super-bricks' tiles per (mesh, order)
     {
-      // super-brick edge: 16, unless one colour's 16^3 super-bricks (about
-      // an eighth of them) would leave SMs without a block
+      // super-brick edge: 16, unless 16^3 super-bricks would leave SMs with
+      // less than two blocks
       {
         long long n16 = 0;
         for (auto const &G : m_geom)
           n16 += static_cast<long long>(ceil_div(G.mesh[0], kSbEdge)) * ceil_div(G.mesh[1], kSbEdge) *
                  ceil_div(G.mesh[2], kSbEdge);
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess)
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        m_sb_edge = (n16 / 8 < sms) ? kSbEdgeSmall : kSbEdge;
+        m_sb_edge = (n16 < 2 * sms) ? kSbEdgeSmall : kSbEdge;
       }
-      auto colours = [](int M, int B, int P) {
-        int const nb = (M + B - 1) / B;
-        std::vector<int> s(nb), e(nb), col(nb, -1);
-        for (int b = 0; b < nb; ++b) {
-          s[b] = b * B;
-          e[b] = s[b] + std::min(B, M - s[b]) + P - 1;
-        }
-        auto hit = [&](int a, int b) {
-          if (e[a] - s[a] >= M || e[b] - s[b] >= M)
-            return true;
-          for (int k = -1; k <= 1; ++k)
-            if (s[a] < e[b] + k * M && s[b] + k * M < e[a])
-              return true;
-          return false;
-        };
-        for (int b = 0; b < nb; ++b) {
-          std::vector<char> used(nb + 1, 0);
-          for (int a = 0; a < nb; ++a)
-            if (a != b && col[a] >= 0 && hit(a, b))
-              used[col[a]] = 1;
-          int c = 0;
-          while (used[c])
-            ++c;
-          col[b] = c;
-        }
-        return col;
-      };
-      // replicas may differ in cao: one phase per (cao, colour), and the
-      // sort bricks grouped by cao (one interpolation launch per order)
-      std::vector<std::vector<int2>> phase;
-      std::vector<std::vector<int2>> bricks_of(8);
+      std::vector<std::vector<int2>> sbs_of(8), bricks_of(8);
+      std::map<std::pair<int, int>, int> cov_at; // (mesh, cao) -> table
+      std::vector<int> cov;
       nat.clear();
+      m_tiles_n = 0;
       for (int r = 0; r < R; ++r) {
-        auto const &G = m_geom[r];
-        auto const cxv = colours(G.mesh[0], m_sb_edge, G.cao);
-        auto const cyv = colours(G.mesh[1], m_sb_edge, G.cao);
-        auto const czv = colours(G.mesh[2], m_sb_edge, G.cao);
-        int const n0 = static_cast<int>(cxv.size()), n1 = static_cast<int>(cyv.size()),
-                  n2 = static_cast<int>(czv.size());
-        for (int bx = 0; bx < n0; ++bx)
-          for (int by = 0; by < n1; ++by)
-            for (int bz = 0; bz < n2; ++bz) {
-              int const p = (G.cao - 1) * 512 + cxv[bx] + 8 * (cyv[by] + 8 * czv[bz]);
-              if (static_cast<int>(phase.size()) <= p)
-                phase.resize(p + 1);
-              phase[p].push_back(int2{r, (bx * n1 + by) * n2 + bz});
-            }
+        auto &G = m_geom[r];
+        int nsb = 1;
+        long long const te = m_sb_edge + G.cao - 1;
+        for (int d = 0; d < 3; ++d) {
+          G.sbn[d] = ceil_div(G.mesh[d], m_sb_edge);
+          nsb *= G.sbn[d];
+          auto const key = std::make_pair(G.mesh[d], G.cao);
+          if (!cov_at.count(key)) {
+            cov_at[key] = static_cast<int>(cov.size());
+            cover_table(G.mesh[d], m_sb_edge, G.cao, cov);
+          }
+          G.cov_off[d] = cov_at[key];
+        }
+        G.tl_off = m_tiles_n;
+        m_tiles_n += nsb * te * te * sb_tile_z(static_cast<int>(te));
+        for (int b = 0; b < nsb; ++b)
+          sbs_of[G.cao].push_back(int2{r, b});
         for (int b = 0; b < G.nbx * G.nby * G.nbz; ++b)
           bricks_of[G.cao].push_back(int2{r, b});
       }
-      m_phase_off.assign(1, 0);
-      m_phase_cao.clear();
-      for (size_t p = 0; p < phase.size(); ++p) {
-        if (phase[p].empty())
-          continue;
-        bm.insert(bm.end(), phase[p].begin(), phase[p].end());
-        m_phase_off.push_back(static_cast<int>(bm.size()));
-        m_phase_cao.push_back(static_cast<int>(p / 512) + 1);
-      }
+      m_sb_off.assign(9, 0);
       m_brick_off.assign(9, 0);
       for (int c = 1; c <= 7; ++c) {
+        bm.insert(bm.end(), sbs_of[c].begin(), sbs_of[c].end());
+        m_sb_off[c + 1] = static_cast<int>(bm.size());
         nat.insert(nat.end(), bricks_of[c].begin(), bricks_of[c].end());
         m_brick_off[c + 1] = static_cast<int>(nat.size());
       }
-      m_brick_off[1] = 0;
+      upload_vec(m_cov, cov, st);
+      P3MX_CUDA(cudaStreamSynchronize(st)); // the table leaves scope
     }
+    upload_vec(m_geom_d, m_geom, st);
     m_n_blk_mesh = static_cast<int>(bm.size());
     m_n_bricks = static_cast<int>(nat.size());
     m_n_blk_cplx = static_cast<int>(bc.size());
@@ -396,7 +368,9 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     std::vector<Blk> zf, y, x, zi;
     m_blk_x_start.assign(1, 0);
     int maxM0 = 1, maxM1 = 1, maxM2 = 1;
+    long long all_lines = 0;
     for (auto const &G : m_geom) {
+      all_lines += static_cast<long long>(G.mesh[0]) * G.mesh[1];
       maxM0 = std::max(maxM0, G.mesh[0]);
       maxM1 = std::max(maxM1, G.mesh[1]);
       maxM2 = std::max(maxM2, G.mesh[2]);
@@ -424,18 +398,22 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       int const ldz = line_ld(M2);
       // forward z: two real lines per complex transform; FP32: as many line
       // pairs as keep four blocks within the SM's shared memory (24 lines at
-      // 256^3: forward z+y 0.102 -> 0.098 ms against 30 at three blocks)
+      // 256^3), fewer where the launch would have less than two blocks per
+      // SM (meshes up to 64)
+      auto const zf_smem = [&](int pairs) {
+        return (2 * static_cast<size_t>(pairs) * ldz + M2) * csz + 3 * M2 * sizeof(int);
+      };
       int lz = static_cast<int>(std::max<size_t>(1, cap / ldz)) * 2;
       if (m_fp32) {
         int q = 1;
-        while ((2 * static_cast<size_t>(q + 1) * ldz + M2) * csz <= 54 * 1024)
+        while (zf_smem(q + 1) <= 54 * 1024)
           ++q;
         lz = 2 * q;
       }
+      lz = std::min({lz, kZfLines, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2)});
       for (int l = 0; l < lines; l += lz)
         zf.push_back(Blk{r, l, std::min(lz, lines - l), 0});
-      smem_zf = std::max(smem_zf,
-                         (2 * static_cast<size_t>((std::min(lz, lines) + 1) / 2) * ldz + M2) * csz);
+      smem_zf = std::max(smem_zf, zf_smem((std::min(lz, lines) + 1) / 2));
       // backward z: nl lines -> nl (Ex, Ey) + ceil(nl/2) (Ez pairs) transforms.
       // FP32: as many lines as keep a block within a quarter of the SM's
       // shared memory, so that four blocks are resident (8 lines at 256^3:
@@ -542,7 +520,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_dist.ensure(3 * n * rsz);
   m_W.ensure(static_cast<size_t>(wstride<7, 4>()) * n * rsz);
   m_skey.ensure((n + 8) * sizeof(int));
-  m_rho.ensure(m_bins * rsz + 64); // + slack: bulk copies of 16-byte aligned supersets
+  m_tiles.ensure(static_cast<size_t>(m_tiles_n) * rsz);
   m_E.ensure(4 * m_ebins * rsz);
   encode_field_maps(st);
   m_ck.ensure(m_cplx * csz);
@@ -690,40 +668,26 @@ void Engine::encode_field_maps(cudaStream_t st) {
 }
 
 namespace {
-// One colour launch of the charge assignment; `chained` launches it as a
-// programmatic dependent of the previous colour (see k_p3m_assign_sb).
-template <typename Real, int P, int E>
-void launch_assign_e(bool chained, int cnt, cudaStream_t st, RepGeom const *geom, int2 const *tab,
-                     int const *start, Real const *W, int const *s_key, unsigned const *qmax_bits,
-                     Real *rho, int *err, int ncomp, long long comp_w, long long comp_rho,
-                     int comp_q) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp));
-  cfg.blockDim = dim3(32 * kSbWarps);
-  cfg.dynamicSmemBytes = sb_smem<Real, P, E>();
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = chained ? 1 : 0;
-  auto const kern = ncomp > 1 ? k_p3m_assign_sb<Real, P, E, true> : k_p3m_assign_sb<Real, P, E, false>;
-  P3MX_CUDA(cudaLaunchKernelEx(&cfg, kern, geom, tab, cnt, start, W, s_key, qmax_bits, rho, err,
-                               comp_w, comp_rho, comp_q));
-}
-// ... with the engine's super-brick edge (16 or 8); ncomp charge sets
-// (records, meshes and |q| maxima comp_w / comp_rho / comp_q apart)
+// The charge assignment of cnt super-bricks of edge E (16 or 8); ncomp charge
+// sets (records, tiles and |q| maxima comp_w / comp_tile / comp_q apart).
 template <typename Real, int P>
-void launch_assign(int edge, bool chained, int cnt, cudaStream_t st, RepGeom const *geom,
-                   int2 const *tab, int const *start, Real const *W, int const *s_key,
-                   unsigned const *qmax_bits, Real *rho, int *err, int ncomp = 1,
-                   long long comp_w = 0, long long comp_rho = 0, int comp_q = 0) {
+void launch_assign(int edge, int cnt, cudaStream_t st, RepGeom const *geom, int2 const *tab,
+                   int const *start, Real const *W, int const *s_key, unsigned const *qmax_bits,
+                   Real *tiles, int *err, int ncomp = 1, long long comp_w = 0,
+                   long long comp_tile = 0, int comp_q = 0) {
+  auto go = [&](auto kern, size_t smem) {
+    kern<<<dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp)), 32 * kSbWarps, smem,
+           st>>>(geom, tab, cnt, start, W, s_key, qmax_bits, tiles, err, comp_w, comp_tile,
+                 comp_q);
+  };
   if (edge == kSbEdgeSmall)
-    launch_assign_e<Real, P, kSbEdgeSmall>(chained, cnt, st, geom, tab, start, W, s_key, qmax_bits,
-                                           rho, err, ncomp, comp_w, comp_rho, comp_q);
+    go(ncomp > 1 ? k_p3m_assign_sb<Real, P, kSbEdgeSmall, true>
+                 : k_p3m_assign_sb<Real, P, kSbEdgeSmall, false>,
+       sb_smem<Real, P, kSbEdgeSmall>());
   else
-    launch_assign_e<Real, P, kSbEdge>(chained, cnt, st, geom, tab, start, W, s_key, qmax_bits, rho,
-                                      err, ncomp, comp_w, comp_rho, comp_q);
+    go(ncomp > 1 ? k_p3m_assign_sb<Real, P, kSbEdge, true>
+                 : k_p3m_assign_sb<Real, P, kSbEdge, false>,
+       sb_smem<Real, P, kSbEdge>());
 }
 
 // Persistent grid of the back-interpolation pipeline: resident blocks per
@@ -790,28 +754,23 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   } else {
     P3MX_CUDA(cudaMemsetAsync(m_start.p, 0, (m_nkeys + 1) * sizeof(int), st));
   }
-  // 2. charge assignment: one block per super-brick, colour by colour
-  P3MX_CUDA(cudaMemsetAsync(m_rho.p, 0, m_bins * sizeof(Real), st));
-  {
-    bool chained = false; // the first colour waits for the mesh memset normally
-    for (size_t p = 0; p + 1 < m_phase_off.size(); ++p) {
-      int const cnt = m_phase_off[p + 1] - m_phase_off[p];
-      if (cnt == 0)
-        continue;
-      int2 const *tab = m_blk_mesh.as<int2>() + m_phase_off[p];
-      P3MX_CAO_DISPATCH_R(m_phase_cao[p], (launch_assign<Real, P>(m_sb_edge, chained, cnt, st, geom, tab,
-                                                       m_start.as<int>(), m_W.as<Real>(),
-                                                       m_skey.as<int>(), qmax_bits,
-                                                       m_rho.as<Real>(), m_kerr.as<int>())));
-      chained = true;
-      ++m_launches;
-    }
+  // 2. charge assignment: one block per super-brick, its tile stored whole
+  for (int c = 1; c <= 7; ++c) {
+    int const cnt = m_sb_off[c + 1] - m_sb_off[c];
+    if (cnt == 0)
+      continue;
+    int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
+    P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, geom, tab, m_start.as<int>(),
+                                                   m_W.as<Real>(), m_skey.as<int>(), qmax_bits,
+                                                   m_tiles.as<Real>(), m_kerr.as<int>())));
+    ++m_launches;
   }
   mark("p3m_assign", st);
   // 3. forward FFT z (r2c) and y
   C const *tw = m_tw.as<C>();
-  k_fft_z_fwd<Real><<<m_n_blk_zf, 256, m_smem_zf, st>>>(geom, m_blk_zf.as<Blk>(), m_rho.as<Real>(),
-                                                        m_ck.as<C>(), tw, m_kerr.as<int>());
+  k_fft_z_fwd<Real><<<m_n_blk_zf, 256, m_smem_zf, st>>>(geom, m_blk_zf.as<Blk>(),
+                                                        m_tiles.as<Real>(), 0, m_cov.as<int>(),
+                                                        m_sb_edge, m_ck.as<C>(), 0, tw);
   ++m_launches;
   launch_fft_y<Real>(m_ck.p, 0, 1, false, st);
   mark("fft_fwd_zy", st);
@@ -1330,18 +1289,24 @@ std::vector<double> Engine::mesh_copy(int r, cudaStream_t st) {
   auto const &G = m_geom[r];
   long long const ms = static_cast<long long>(G.mesh[0]) * G.mesh[1] * G.mesh[2];
   std::vector<double> out(ms);
-  if (m_fp32) {
-    std::vector<float> t(ms);
-    P3MX_CUDA(cudaMemcpyAsync(t.data(), m_rho.as<float>() + G.rm_off, ms * sizeof(float),
-                              cudaMemcpyDeviceToHost, st));
+  // the mesh is the sum of the assignment's tiles
+  auto sum = [&](auto zero) {
+    using Real = decltype(zero);
+    m_rho.ensure(ms * sizeof(Real));
+    k_tiles_to_mesh<Real><<<ceil_div(ms, 256), 256, 0, st>>>(
+        m_geom_d.as<RepGeom>(), r, m_tiles.as<Real>(), m_cov.as<int>(), m_sb_edge,
+        m_rho.as<Real>());
+    ++m_launches;
+    std::vector<Real> t(ms);
+    P3MX_CUDA(cudaMemcpyAsync(t.data(), m_rho.p, ms * sizeof(Real), cudaMemcpyDeviceToHost, st));
     P3MX_CUDA(cudaStreamSynchronize(st));
     for (long long k = 0; k < ms; ++k)
       out[k] = t[k];
-  } else {
-    P3MX_CUDA(cudaMemcpyAsync(out.data(), m_rho.as<double>() + G.rm_off, ms * sizeof(double),
-                              cudaMemcpyDeviceToHost, st));
-    P3MX_CUDA(cudaStreamSynchronize(st));
-  }
+  };
+  if (m_fp32)
+    sum(0.0f);
+  else
+    sum(0.0);
   return out;
 }
 

@@ -189,15 +189,16 @@ private:
   long long m_ncorner = 0; // corner keys (bricks x brick^3)
   int m_n_bricks = 0; // sort bricks of all replicas (interpolation blocks)
   int m_sb_edge = 16; // super-brick edge of the charge assignment (16, or 8 for small meshes)
-  std::vector<int> m_phase_off; // assignment super-brick table offsets per (cao, colour) phase
-  std::vector<int> m_phase_cao; // the cao of each phase
+  long long m_tiles_n = 0;   // values of the assignment's stored tiles
+  std::vector<int> m_sb_off; // assignment super-brick table offsets per cao (index cao .. cao+1)
   std::vector<int> m_brick_off; // interpolation brick table offsets per cao (index cao .. cao+1)
   int m_ntypes = 1;
   std::vector<PairIA> m_ia;
 
   // tables
   DevBuf m_geom_d, m_rep_of, m_tw, m_ia_d;
-  DevBuf m_blk_mesh; // super-bricks of the charge assignment, grouped by colour
+  DevBuf m_blk_mesh; // super-bricks of the charge assignment, grouped by order
+  DevBuf m_cov;      // cover tables of the assignment's tiles
   DevBuf m_blk_cplx, m_blk_census, m_blk_pair;
   DevBuf m_blk_brick; // all bricks in spatial order (interpolation)
   DevBuf m_blk_zf, m_blk_y, m_blk_x, m_blk_zi;
@@ -214,7 +215,8 @@ private:
   // p3m
   DevBuf m_key, m_bkey, m_slot, m_cnt, m_start, m_perm, m_scan_tiles;
   DevBuf m_dist, m_W, m_skey;
-  DevBuf m_rho, m_ck, m_field, m_E, m_ginf;
+  DevBuf m_rho; // charge mesh of one replica (mesh_copy only)
+  DevBuf m_tiles, m_ck, m_field, m_E, m_ginf;
   DevBuf m_tmap; // per replica: tensor map of its field mesh (interpolation tiles)
   DevBuf m_part_x, m_part_census, m_sums_x, m_sums_census, m_dipole;
   bool m_ginf_valid = false;

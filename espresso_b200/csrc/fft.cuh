@@ -15,6 +15,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "p3m_kernels.cuh"
 
 namespace p3mx {
 
@@ -402,55 +403,28 @@ __device__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
   return src;
 }
 
-// Copy the contiguous global range [src, src + count) to shared memory with
-// one bulk copy (TMA engine) when its 16-byte aligned superset fits in the
-// `room` bytes at `area`.  Returns the shared-memory copy of src, or nullptr
-// when the range does not fit (nothing copied; the decision is uniform over
-// the block).  Called by all threads of the block; the copy has landed when
-// it returns.  A wait that runs out sets *err and `failed` (the caller
-// returns).  The aligned superset may reach up to 15 bytes past the range:
-// the buffer behind src is allocated with that slack.
-template <typename T>
-__device__ inline const T *bulk_stage(const T *src, long long count, unsigned char *area,
-                                      size_t room, unsigned long long *bar, int *err,
-                                      bool &failed) {
-  uintptr_t const g0 = reinterpret_cast<uintptr_t>(src) & ~uintptr_t(15);
-  uintptr_t const g1 = (reinterpret_cast<uintptr_t>(src + count) + 15) & ~uintptr_t(15);
-  unsigned const pad = (16u - (smem_u32(area) & 15u)) & 15u;
-  size_t const bytes = g1 - g0;
-  if (pad + bytes > room || bytes >= (1u << 20))
-    return nullptr;
-  unsigned char *dst = area + pad;
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_arrive_expect_tx(bar, static_cast<unsigned>(bytes));
-    bulk_g2s(dst, reinterpret_cast<const void *>(g0), static_cast<unsigned>(bytes), bar);
-  }
-  __syncthreads(); // barrier initialised before anyone waits on it
-  bool const ok = mbar_wait(bar, 0);
-  if (__syncthreads_or(!ok)) {
-    if (threadIdx.x == 0) {
-      atomicExch(err, 1);
-      mbar_wait(bar, 0); // second bounded wait for the copy in flight
-    }
-    failed = true;
-    return nullptr;
-  }
-  return reinterpret_cast<const T *>(dst + (reinterpret_cast<uintptr_t>(src) - g0));
-}
-
 // ---- pass z, forward: real lines -> complex half lines -----------------
 // Two real lines per complex transform: Z = x0 + i x1, then
 // X0[k] = (Z[k] + conj Z[n-k]) / 2 and X1[k] = -i (Z[k] - conj Z[n-k]) / 2.
 // bk.b real lines per block (an odd last line is paired with zeros).
-// Shared memory: 2 x ceil(bk.b/2) staged lines of line_ld(n), twiddles (n).
+// The charge mesh exists only as the assignment's tiles: the block sums, for
+// every (x, y) line, the 1 to 4 tile rows that cover it (contiguous along z),
+// first each point's own super-brick (four points per load), then the points
+// in a halo of the previous one along z.
+// blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
+// Shared memory: 2 x bk.b/2 staged lines of line_ld(n), twiddles (n), the
+// halo points' z and offsets (3 n ints).  Meshes are even, so is bk.b.
+constexpr int kZfLines = 64; // most real lines per block
 template <typename Real>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
 k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
-            const Real *__restrict__ rmesh, typename CplxOf<Real>::type *__restrict__ cmesh,
-            const typename CplxOf<Real>::type *__restrict__ twtab, int *__restrict__ err) {
+            const Real *__restrict__ tiles, long long tile_stride, const int *__restrict__ cov,
+            int E, typename CplxOf<Real>::type *__restrict__ cmesh, long long c_stride,
+            const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ long long s_bx[kZfLines][3];
+  __shared__ int s_by[kZfLines][3];
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
   int const n = G.mesh[2];
@@ -460,26 +434,60 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = a + np * ld;
   C *tw = b + np * ld;
+  int *zc = reinterpret_cast<int *>(tw + n);
+  tiles += blockIdx.y * tile_stride + G.tl_off;
+  cmesh += blockIdx.y * c_stride;
   load_twiddles(tw, twtab, G.plan[2]);
   long long const line0 = bk.a;
-  const Real *src = rmesh + G.rm_off + line0 * n;
-  // the block's nl real lines are one contiguous range of the mesh: stage it
-  // in b (the FFT scratch) with one bulk copy when it fits there
-  __shared__ __align__(8) unsigned long long bar;
-  bool failed = false;
-  const Real *sv = bulk_stage(src, static_cast<long long>(nl) * n,
-                              reinterpret_cast<unsigned char *>(b), np * ld * sizeof(C), &bar,
-                              err, failed);
-  if (failed)
-    return;
-  if (sv == nullptr)
-    sv = src;
+  int const nh = cov[G.cov_off[2] + 3 * n];
+  {
+    TileMap const tm(G, E);
+    int const M0 = G.mesh[0], M1 = G.mesh[1];
+    const int *cz = cov + G.cov_off[2];
+    for (int t = threadIdx.x; t < nh; t += blockDim.x) {
+      int const z = cz[3 * n + 1 + t];
+      zc[t] = z;
+      zc[n + t] = tm.z(cz[n + z]);
+      zc[2 * n + t] = tm.z(cz[2 * n + z]);
+    }
+    for (int t = threadIdx.x; t < 3 * nl; t += blockDim.x) {
+      int const l = t / 3, j = t - 3 * l;
+      int const x = static_cast<int>((line0 + l) / M1), y = static_cast<int>((line0 + l) % M1);
+      s_bx[l][j] = tm.x(cov[G.cov_off[0] + j * M0 + x]);
+      s_by[l][j] = tm.y(cov[G.cov_off[1] + j * M1 + y]);
+    }
+  }
+  __syncthreads();
   // real line l, element k -> real or imaginary part of slot l/2
   Real *ar = reinterpret_cast<Real *>(a);
-  // odd count: the last slot's imaginary part is line nl, all zeros
-  for_lines(nl + (nl & 1), n, [&](int l, int k) {
-    ar[2 * ((l >> 1) * ld + pix(k)) + (l & 1)] = (l < nl) ? sv[l * n + k] : Real(0);
-  });
+  using R4 = typename Real4Of<Real>::type;
+  int const tz = sb_tile_z(E + G.cao - 1);
+  int const g4 = (n + 3) >> 2, total = nl * g4;
+  float const rg4 = 1.0f / static_cast<float>(g4);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    int const l = qdiv(t, g4, rg4), k = 4 * (t - l * g4);
+    // E is a multiple of 4: the four points lie in one super-brick (rows are
+    // padded, so the last group may reach past the mesh)
+    R4 const v = tile_rows<R4>(tiles, s_bx[l], s_by[l], (k / E) * tz + k % E);
+    Real *o = ar + 2 * ((l >> 1) * ld + pix(k)) + (l & 1);
+    o[0] = v.x;
+    o[2] = v.y;
+    if (k + 2 < n) {
+      o[4] = v.z;
+      o[6] = v.w;
+    }
+  }
+  __syncthreads();
+  float const rnh = 1.0f / static_cast<float>(max(nh, 1));
+#pragma unroll 2
+  for (int t = threadIdx.x; t < nl * nh; t += blockDim.x) {
+    int const l = qdiv(t, nh, rnh), h = t - l * nh;
+    Real v = tile_rows<Real>(tiles, s_bx[l], s_by[l], zc[n + h]);
+    if (zc[2 * n + h] >= 0)
+      v += tile_rows<Real>(tiles, s_bx[l], s_by[l], zc[2 * n + h]);
+    ar[2 * ((l >> 1) * ld + pix(zc[h])) + (l & 1)] += v;
+  }
   __syncthreads();
   C *res = fft_lines<C>(a, b, np, ld, G.plan[2], tw, false);
   int const H = n / 2 + 1;

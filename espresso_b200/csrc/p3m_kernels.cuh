@@ -5,6 +5,9 @@
 
 #include "common.cuh"
 
+#include <algorithm>
+#include <vector>
+
 namespace p3mx {
 
 // Fold into [0, L) like algorithm/periodic_fold.hpp:72-89 (repeated shifts);
@@ -208,16 +211,16 @@ struct TileStrides {
 // (x, y) stencil rows (one row per lane, the P z points of a row unrolled)
 // and adds q wx wy wz into a shared-memory tile of (E + P - 1)^3
 // points, in fixed point; the tile is then added to the mesh.  E = 16, or 8
-// when the 16^3 super-bricks of one colour would not give every SM a block
-// (small meshes: more, smaller tiles with a larger halo share).  Tiles of
-// neighbouring super-bricks overlap by P - 1 points, so super-bricks are
-// coloured (greedy interval colouring per dimension: tiles of one colour
-// never overlap, modulo the mesh) and launched colour by colour: the plain
-// read-add-write of a tile is race-free and the colour order fixes the
-// order of the FP adds, so the mesh is bitwise reproducible.  The colour
-// launches are chained by programmatic dependent launch: a colour fills its
-// tiles while the previous one drains, and waits (griddepcontrol.wait) only
-// before its read-add-write of the mesh.
+// when the 16^3 super-bricks would not give every SM two blocks (small
+// meshes: more, smaller tiles with a larger halo share).  Tiles of
+// neighbouring super-bricks overlap by P - 1 points.  Every block stores its
+// whole tile, halo included, to its own place in HBM, and the forward z pass
+// sums the tiles that cover a mesh point while it loads its lines
+// (TileMap): all super-bricks run in one launch, no mesh is zeroed and none
+// is read back and rewritten, and the sum over the (up to 8, in wrap corners
+// 27) tiles has a fixed order, so the mesh is bitwise reproducible.  The
+// tiles hold ((16 + P - 1) / 16)^3 = 2.6 mesh sizes at P = 7.  The kernel is
+// bound by the shared-memory atomics and loads of the stencil terms.
 //
 // Fixed point: a term v = q wx wy wz becomes t = rint(v S) by one FP64 FMA
 // with the magic constant 1.5 * 2^52 (the bits of the sum are those of the
@@ -322,6 +325,12 @@ template <typename Real, int P, int E> __host__ __device__ constexpr size_t sb_s
   return sb_tile_bytes<Real, P, E>() + sizeof(Real) * kSbChunk * kRecStride +
          sizeof(double) * 8 * kSbChunk + sizeof(int) * kSbChunk;
 }
+// The stored tiles of a replica, TE = E + P - 1 points per edge, z rows
+// padded to TZ values (a multiple of 4): value (lx, ly, lz) of super-brick
+// (bx, by, bz) at ((bx TE + lx) (n1 TE) + by TE + ly) (n2 TZ) + bz TZ + lz,
+// n1, n2 the super-bricks along y and z -- the rows of a mesh line's tiles
+// along z are one contiguous range.
+__host__ __device__ constexpr int sb_tile_z(int te) { return (te + 3) / 4 * 4; }
 // sort-brick runs of a super-brick: (kSbEdge / B)^2 brick columns, one
 // contiguous z run each
 constexpr int kSbMaxRuns = (kSbEdge / 4) * (kSbEdge / 4);
@@ -331,17 +340,17 @@ __global__ void __launch_bounds__(32 * kSbWarps, sizeof(Real) == 4 ? 4 : 1)
 k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, int nsb,
                 const int *__restrict__ start, const Real *__restrict__ W,
                 const int *__restrict__ s_key, const unsigned *__restrict__ qmax_bits,
-                Real *__restrict__ rho, int *__restrict__ err, long long comp_w,
-                long long comp_rho, int comp_q) {
+                Real *__restrict__ tiles, int *__restrict__ err, long long comp_w,
+                long long comp_tile, int comp_q) {
   // MC: blockIdx.y picks one of several charge sets assigned by one launch
-  // (the dipole components): its weight records, mesh and |q| maxima lie
-  // comp_w / comp_rho / comp_q elements after the previous set's. The
+  // (the dipole components): its weight records, tiles and |q| maxima lie
+  // comp_w / comp_tile / comp_q elements after the previous set's. The
   // single-set instance leaves the three pointers as kernel parameters: the
-  // offset copies cost six registers, which spill the FP32 order-7 16^3
-  // instance at its 64-register bound (0.239 -> 0.307 ms at 2^20 ions).
+  // offset copies cost six registers at the FP32 instances' 64-register
+  // bound.
   if constexpr (MC) {
     W += blockIdx.y * comp_w;
-    rho += blockIdx.y * comp_rho;
+    tiles += blockIdx.y * comp_tile;
     qmax_bits += blockIdx.y * comp_q;
   }
   using Word = typename SbWord<Real>::type;
@@ -364,7 +373,6 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_r0[kSbMaxRuns], s_r1[kSbMaxRuns];
   __shared__ int s_count;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (static_cast<int>(blockIdx.x) >= nsb)
     return; // whole block
   Word *tile = reinterpret_cast<Word *>(smem_raw);
@@ -406,8 +414,24 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   __syncthreads();
   int const count = s_count;
   float const qmax = __uint_as_float(qmax_bits[sb.x]);
-  if (count == 0 || !(qmax > 0.0f))
-    return; // nothing to add to the mesh
+  // store the tile, value(x, y, z) (lanes along z: conflict-free shared
+  // reads, row segments stored whole; the row padding is zero)
+  auto store_tile = [&](auto const &value) {
+    constexpr int TZ = sb_tile_z(TE);
+    int const rz = no2 * TZ;
+    long long const rx = static_cast<long long>(no1) * TE * rz;
+    Real *const out = tiles + G.tl_off + (o0 / E) * TE * rx +
+                      static_cast<long long>(o1 / E) * TE * rz + (o2 / E) * TZ;
+    for (int t = tid; t < TE * TE * TZ; t += NT) {
+      int const row = t / TZ, z = t - row * TZ;
+      int const x = row / TE, y = row - x * TE;
+      out[x * rx + y * rz + z] = (z < TE) ? value(x, y, z) : Real(0);
+    }
+  };
+  if (count == 0 || !(qmax > 0.0f)) {
+    store_tile([](int, int, int) { return Real(0); });
+    return;
+  }
   int es;
   {
     double const unit = static_cast<double>(qmax) * bspline_wmax<P>() * bspline_wmax<P>() *
@@ -489,80 +513,119 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   }
   __syncthreads();
   Real const inv_S = static_cast<Real>(ldexp(1.0, -es));
-  // the previous colour's read-add-write has completed and is visible
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  // add the tile to the mesh: real extent of the super-brick plus the stencil
-  int const ex0 = min(E, M0 - o0) + P - 1, ey = min(E, M1 - o1) + P - 1,
-            ez = min(E, M2 - o2) + P - 1;
-  Real *mesh = rho + G.rm_off;
-  // a tile wider than the mesh maps two tile points onto one mesh point:
-  // add such points in separate passes (one per wrap class)
-  bool const self_wrap = (ex0 > M0) || (ey > M1) || (ez > M2);
-  int const passes = self_wrap ? 8 : 1;
-  // each thread owns fixed (y, z) slots of the tile's yz plane; loop over x
-  constexpr int NS = (TE * TE + NT - 1) / NT;
-  int yzt[NS], yzg[NS], ycls[NS];
-  int const nyz = ey * ez;
-#pragma unroll
-  for (int k2 = 0; k2 < NS; ++k2) {
-    int const t = tid + NT * k2;
-    int const y = (t < nyz) ? t / ez : 0, z = (t < nyz) ? t - (t / ez) * ez : 0;
-    int gy = o1 + y, gz = o2 + z, cls = 0;
-    if (gy >= M1) { gy -= M1; cls |= 2; }
-    if (gy >= M1) gy -= M1;
-    if (gz >= M2) { gz -= M2; cls |= 4; }
-    if (gz >= M2) gz -= M2;
-    yzt[k2] = (t < nyz) ? y * SY + z : -1;
-    yzg[k2] = gy * M2 + gz;
-    ycls[k2] = cls;
-  }
-  if (!self_wrap) {
-    // every tile point maps to its own mesh point: issue the thread's mesh
-    // loads of XG x planes first, then the adds and stores
-    constexpr int XG = 8;
-#pragma unroll 1
-    for (int xg = 0; xg < ex0; xg += XG) {
-      Real old[XG][NS];
-#pragma unroll
-      for (int xx = 0; xx < XG; ++xx) {
-        int const x = xg + xx;
-        int gx = o0 + x;
-        gx -= (gx >= M0) ? M0 : 0;
-        long long const gbase = static_cast<long long>(gx) * M1 * M2;
-#pragma unroll
-        for (int k2 = 0; k2 < NS; ++k2)
-          if (x < ex0 && yzt[k2] >= 0)
-            old[xx][k2] = mesh[gbase + yzg[k2]];
-      }
-#pragma unroll
-      for (int xx = 0; xx < XG; ++xx) {
-        int const x = xg + xx;
-        int gx = o0 + x;
-        gx -= (gx >= M0) ? M0 : 0;
-        long long const gbase = static_cast<long long>(gx) * M1 * M2;
-#pragma unroll
-        for (int k2 = 0; k2 < NS; ++k2)
-          if (x < ex0 && yzt[k2] >= 0)
-            mesh[gbase + yzg[k2]] = old[xx][k2] + sb_value(tile[x * SX + yzt[k2]], inv_S);
+  store_tile([&](int x, int y, int z) { return sb_value(tile[x * SX + y * SY + z], inv_S); });
+}
+
+// Cover table of an axis of M mesh points in super-bricks of edge E, order P:
+// entry j (j < 3) of point i names the j-th super-brick b whose tile holds
+// the point (offset l: b E + l = i modulo M) as (b << 8) | l, or -1; the
+// point's own super-brick comes first.  A point lies in its own super-brick's
+// tile and maybe in the halo of the one before; the first P - 1 points of an
+// axis whose last super-brick is shorter than P - 1 also in that of the one
+// before the last.  Entry j of point i is at cov[cov_off + j M + i]; behind
+// the 3 M entries the number of points with a second cover and their list.
+inline void cover_table(int M, int E, int P, std::vector<int> &cov) {
+  size_t const at = cov.size();
+  cov.resize(at + 3 * static_cast<size_t>(M), -1);
+  std::vector<int> n(M, 0);
+  int const nb = (M + E - 1) / E;
+  for (int halo = 0; halo < 2; ++halo)
+    for (int b = 0; b < nb; ++b) {
+      int const len = std::min(E, M - b * E);
+      for (int l = halo ? len : 0; l < (halo ? len + P - 1 : len); ++l) {
+        int const i = (b * E + l) % M;
+        if (n[i] == 3)
+          throw Error(3, "assignment tiles: more than three covers of a mesh point");
+        cov[at + static_cast<size_t>(n[i]++) * M + i] = (b << 8) | l;
       }
     }
+  cov.push_back(0);
+  size_t const cnt = cov.size() - 1;
+  for (int i = 0; i < M; ++i)
+    if (n[i] > 1) {
+      ++cov[cnt];
+      cov.push_back(i);
+    }
+}
+
+// Per-axis offset contributions of cover entries in the stored tiles (-1 for
+// no entry).
+struct TileMap {
+  long long sx;
+  int te, sy, tz;
+  __device__ explicit TileMap(RepGeom const &G, int E)
+      : te(E + G.cao - 1), tz(sb_tile_z(te)) {
+    sy = G.sbn[2] * tz;
+    sx = static_cast<long long>(G.sbn[1]) * te * sy;
+  }
+  __device__ long long x(int c) const {
+    return c < 0 ? -1 : ((c >> 8) * te + (c & 255)) * sx;
+  }
+  __device__ int y(int c) const { return c < 0 ? -1 : ((c >> 8) * te + (c & 255)) * sy; }
+  __device__ int z(int c) const { return c < 0 ? -1 : (c >> 8) * tz + (c & 255); }
+};
+
+__device__ inline float tile_add(float a, float b) { return a + b; }
+__device__ inline double tile_add(double a, double b) { return a + b; }
+template <typename V> __device__ inline V tile_add(V a, V b) {
+  a.x += b.x;
+  a.y += b.y;
+  a.z += b.z;
+  a.w += b.w;
+  return a;
+}
+// Sum over the (x, y) covers of a line (offset contributions bx, by: entry 0
+// always there, 1 and 2 may be -1) of the value V (one or four points along
+// z) at z offset z.  The up to 4 loads of the first two entries are issued
+// together; a third entry occurs in wrap corners only.
+template <typename V, typename Real>
+__device__ inline V tile_rows(const Real *__restrict__ t, const long long *bx, const int *by,
+                              int z) {
+  V v[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    long long const x = bx[c >> 1];
+    int const y = by[c & 1];
+    v[c] = (c == 0 || (x >= 0 && y >= 0)) ? *reinterpret_cast<const V *>(t + (x + y + z)) : V{};
+  }
+  V s = tile_add(tile_add(v[0], v[1]), tile_add(v[2], v[3]));
+  if (bx[2] >= 0 || by[2] >= 0)
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j)
+        if ((i == 2 || j == 2) && bx[i] >= 0 && by[j] >= 0)
+          s = tile_add(s, *reinterpret_cast<const V *>(t + (bx[i] + by[j] + z)));
+  return s;
+}
+
+// The charge mesh from the stored tiles (mesh copies for parity checks; the
+// path itself sums the tiles inside the forward z pass).
+template <typename Real>
+__global__ void k_tiles_to_mesh(const RepGeom *__restrict__ reps, int r,
+                                const Real *__restrict__ tiles, const int *__restrict__ cov, int E,
+                                Real *__restrict__ rho) {
+  RepGeom const &G = reps[r];
+  int const M0 = G.mesh[0], M1 = G.mesh[1], M2 = G.mesh[2];
+  long long const local = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (local >= static_cast<long long>(M0) * M1 * M2)
     return;
+  int const z = static_cast<int>(local % M2), y = static_cast<int>((local / M2) % M1),
+            x = static_cast<int>(local / (static_cast<long long>(M1) * M2));
+  TileMap const tm(G, E);
+  long long bx[3];
+  int by[3], bz[3];
+  for (int j = 0; j < 3; ++j) {
+    bx[j] = tm.x(cov[G.cov_off[0] + j * M0 + x]);
+    by[j] = tm.y(cov[G.cov_off[1] + j * M1 + y]);
+    bz[j] = tm.z(cov[G.cov_off[2] + j * M2 + z]);
   }
-  for (int pass = 0; pass < passes; ++pass) {
-    for (int x = 0; x < ex0; ++x) {
-      int gx = o0 + x, xcls = 0;
-      if (gx >= M0) { gx -= M0; xcls = 1; }
-      if (gx >= M0) gx -= M0;
-      long long const gbase = static_cast<long long>(gx) * M1 * M2;
-#pragma unroll
-      for (int k2 = 0; k2 < NS; ++k2) {
-        if (yzt[k2] < 0 || (xcls | ycls[k2]) != pass)
-          continue;
-        mesh[gbase + yzg[k2]] += sb_value(tile[x * SX + yzt[k2]], inv_S);
-      }
-    }
-    __syncthreads();
+  Real s = tile_rows<Real>(tiles + G.tl_off, bx, by, bz[0]);
+  if (bz[1] >= 0) {
+    Real h = tile_rows<Real>(tiles + G.tl_off, bx, by, bz[1]);
+    if (bz[2] >= 0)
+      h += tile_rows<Real>(tiles + G.tl_off, bx, by, bz[2]);
+    s += h;
   }
+  rho[local] = s;
 }
 
 // Force back-interpolation (AssignForces, electrostatics/p3m.cpp:344-373) as
