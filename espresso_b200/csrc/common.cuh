@@ -63,6 +63,7 @@ struct AxisPlan {
   int nstages;
   int radix[kMaxStages];
   int tw_off; // offset of exp(-2 pi i k / n), k < n, in the twiddle table
+  int n1, n2; // n = n1 n2 with transform lengths of at most 16 (n1 = 0: none)
 };
 
 // Per-replica device descriptor (one system of the batch).

@@ -7,9 +7,9 @@
 //  2. brick binning and sort of the particles (once), weight records with
 //     q = mu_d for each component d = x, y, z, one super-brick assignment
 //     launch, one r2c z pass and one y pass over the three;
-//  3. k_fft_x_dp3m in three modes (torque fields with the energy sum, the
-//     two halves of the force-field tensor), each followed by the backward
-//     y and z passes and the back-interpolation with unit-charge weights;
+//  3. k_fft_x_dp3m (energy sum, five spectra), the backward y and z passes to
+//     the three torque fields and the six entries of the force-field tensor,
+//     and the back-interpolation of the nine with unit-charge weights;
 //  4. k_dp3m_combine: forces and torques from the nine interpolated values;
 //  5. the real-space pair kernel over the Verlet lists of the dipoles.
 // The charge engine provides steps 2-3's kernels, buffers, block tables,
@@ -101,13 +101,24 @@ public:
       P3MX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(limit)));
     };
+    auto attrs = [&](auto zero, auto two) {
+      using Real = decltype(zero);
+      constexpr bool TWO = decltype(two)::value;
+      attr(k_fft_x_dp3m<Real, true, TWO>);
+      attr(k_fft_x_dp3m<Real, false, TWO>);
+      attr(k_fft_x_dp3m_inv<Real, TWO>);
+    };
     if (E.fp32()) {
-      attr(k_fft_x_dp3m<float, true>);
-      attr(k_fft_x_dp3m<float, false>);
+      attrs(0.0f, std::true_type{});
+      attrs(0.0f, std::false_type{});
     } else {
-      attr(k_fft_x_dp3m<double, true>);
-      attr(k_fft_x_dp3m<double, false>);
+      attrs(0.0, std::true_type{});
+      attrs(0.0, std::false_type{});
     }
+    // the field spectra and three field meshes
+    E.m_field.ensure(kDipoleSpectra * E.m_cplx * csz);
+    E.m_E.ensure(3 * 4 * E.m_ebins * rsz);
+    E.encode_field_maps(st, 3);
     m_g_valid = false;
     m_phi_valid = false;
     m_M = M;
@@ -171,7 +182,6 @@ public:
     E.mark("dp_sort", st);
     // 2. the three component meshes: weight records per component, then one
     // assignment and one z pass over all three (blockIdx.y = component)
-    C const *tw = E.m_tw.as<C>();
     C *ck3 = m_ck3.as<C>();
     long long const wst = static_cast<long long>(kRecStride) * n;
     unsigned *qmax3 = m_qmax3.as<unsigned>();
@@ -195,12 +205,9 @@ public:
                                                      wst, E.m_tiles_n, 1)));
       ++E.m_launches;
     }
-    k_fft_z_fwd<Real><<<dim3(E.m_n_blk_zf, 3), 256, E.m_smem_zf, st>>>(
-        geom, E.m_blk_zf.as<Blk>(), m_tiles3.as<Real>(), E.m_tiles_n, E.m_cov.as<int>(),
-        E.m_sb_edge, ck3, E.m_cplx, tw);
-    ++E.m_launches;
+    E.launch_fft_z_fwd<Real>(m_tiles3.as<Real>(), ck3, 3, st);
     E.mark("dp_assign_fft_z", st);
-    E.launch_fft_y<Real>(ck3, E.m_cplx, 3, false, st);
+    E.launch_fft_y<Real>(ck3, E.m_cplx, y_plain(3), false, 0, st);
     // unit-charge weights of the magnetic particles (selector) for the
     // back-interpolation
     if (want_ft) {
@@ -210,51 +217,53 @@ public:
       ++E.m_launches;
     }
     E.mark("dp_fft_y_weights", st);
-    // 3. x pass per mode, backward y and z, interpolation
-    for (int mode = 0; mode < 3; ++mode) {
-      bool const ev = want_e && mode == 0;
-      if (!want_ft && !ev)
-        break;
-      if (ev) {
-        k_fft_x_dp3m<Real, true><<<E.m_n_blk_x, 256, E.m_smem_x, st>>>(
-            geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx, m_ge.as<Real>(), m_gf.as<Real>(), mode,
-            E.m_field.as<C>(), E.m_tile_x, m_part.as<double>(), tw);
-        ++E.m_launches;
-        k_dp3m_sum_rows<<<1, 32 * 1, 0, st>>>(m_part.as<double>(), E.m_n_blk_x, 1,
-                                          m_sums.as<double>() + 5);
-        ++E.m_launches;
-      } else {
-        k_fft_x_dp3m<Real, false><<<E.m_n_blk_x, 256, E.m_smem_x, st>>>(
-            geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx, m_ge.as<Real>(), m_gf.as<Real>(), mode,
-            E.m_field.as<C>(), E.m_tile_x, nullptr, tw);
-        ++E.m_launches;
-      }
-      E.mark("dp_x_pass", st);
-      if (!want_ft)
-        break;
-      E.launch_fft_y<Real>(E.m_field.p, E.m_cplx, 3, true, st);
-      k_fft_z_inv3<Real><<<E.m_n_blk_zi, 256, E.m_smem_zi, st>>>(
-          geom, E.m_blk_zi.as<Blk>(), E.m_field.as<C>(), E.m_cplx, E.m_E.as<Real>(), tw,
-          E.m_kerr.as<int>());
+    // 3. one x pass, backward y and z passes over the nine fields, one
+    // interpolation of the three field sets
+    if (!want_ft && !want_e)
+      return;
+    {
+      auto const kern =
+          want_e ? (E.m_two[0] ? k_fft_x_dp3m<Real, true, true> : k_fft_x_dp3m<Real, true, false>)
+                 : (E.m_two[0] ? k_fft_x_dp3m<Real, false, true> : k_fft_x_dp3m<Real, false, false>);
+      kern<<<E.m_n_blk_x, 256, E.m_smem_x, st>>>(geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx,
+                                                 m_ge.as<Real>(), E.m_tile_x, m_part.as<double>(),
+                                                 E.m_tw.as<C>());
       ++E.m_launches;
-      E.mark("dp_inv_yz", st);
-      double *out = m_out.as<double>() + 3 * n * mode;
-      RepGeom const *gi = m_geom_interp.as<RepGeom>();
-      for (int c = 1; n > 0 && c <= 7; ++c) {
-        int const nbr = E.m_brick_off[c + 1] - E.m_brick_off[c];
-        if (nbr == 0)
-          continue;
-        int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
-        P3MX_CAO_DISPATCH_R(c, (k_p3m_interp<Real, P><<<interp_grid<Real, P>(nbr),
-                                   32 * (1 + kInterpWarps), interp_smem<Real, P>(), st>>>(
-                                   gi, tab, nbr, E.m_start.as<int>(), E.m_perm.as<int>(),
-                                   E.m_skey.as<int>(), E.m_W.as<Real>(), E.m_E.as<Real>(),
-                                   E.m_tmap.as<CUtensorMap>(), E.d_q(), E.m_dipole.as<double>(),
-                                   out, 1, E.m_kerr.as<int>())));
+      if (want_e) {
+        k_dp3m_sum_rows<<<1, 32 * 1, 0, st>>>(m_part.as<double>(), E.m_n_blk_x, 1,
+                                              m_sums.as<double>() + 5);
         ++E.m_launches;
       }
-      E.mark("dp_interp", st);
     }
+    if (want_ft) {
+      auto const kern = E.m_two[0] ? k_fft_x_dp3m_inv<Real, true> : k_fft_x_dp3m_inv<Real, false>;
+      kern<<<5 * E.m_n_blk_x, 256, E.m_smem_x, st>>>(geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx,
+                                                     m_ge.as<Real>(), m_gf.as<Real>(),
+                                                     E.m_field.as<C>(), E.m_tile_x, E.m_tw.as<C>());
+      ++E.m_launches;
+    }
+    E.mark("dp_x_pass", st);
+    if (!want_ft)
+      return;
+    E.launch_fft_y<Real>(E.m_field.p, E.m_cplx, dp_y_pass(), true, 0, st);
+    E.launch_fft_z_inv<Real>(E.m_field.p, E.m_cplx, dp_z_pass(), 3, 0, E.m_E.p, st);
+    E.mark("dp_inv_yz", st);
+    double *out = m_out.as<double>();
+    RepGeom const *gi = m_geom_interp.as<RepGeom>();
+    for (int c = 1; n > 0 && c <= 7; ++c) {
+      int const nbr = E.m_brick_off[c + 1] - E.m_brick_off[c];
+      if (nbr == 0)
+        continue;
+      int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
+      P3MX_CAO_DISPATCH_R(c, (k_p3m_interp<Real, P><<<dim3(ceil_div(interp_grid<Real, P>(3 * nbr), 3), 3),
+                                 32 * (1 + kInterpWarps), interp_smem<Real, P>(), st>>>(
+                                 gi, tab, nbr, E.m_start.as<int>(), E.m_perm.as<int>(),
+                                 E.m_skey.as<int>(), E.m_W.as<Real>(), E.m_tmap.as<CUtensorMap>(),
+                                 1, E.d_q(), E.m_dipole.as<double>(), out, 3 * n, 1,
+                                 E.m_kerr.as<int>())));
+      ++E.m_launches;
+    }
+    E.mark("dp_interp", st);
   }
 
   // Full evaluation.  f, t: device arrays (3N) or nullptr when not wanted;

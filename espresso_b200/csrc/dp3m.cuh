@@ -233,28 +233,23 @@ __global__ void k_dp3m_sum_rows(const double *__restrict__ partials, int nblk, i
     out[k] = s;
 }
 
-// ---- x pass of the dipolar k-space operator ------------------------------
-// Per block: one ky, a tile of kz (the block table of the charge x pass).
-// In mode 0 the three forward-transformed components F_d are staged and
-// transformed along x one after another, accumulating mk = sum_d d_op_d F_d,
-// which then replaces component x in place (each block rewrites only the
-// lines it read); modes 1 and 2 load that mk.  Three output spectra are
-// formed from mk and transformed backward along x:
-//   mode 0 (torques, AssignTorques, dp3m.cpp:372-395):
-//     d_op_j G_energy mk,                                   j = x, y, z
-//   mode 1 / 2 (forces, AssignForces, dp3m.cpp:396-430):
-//     -i d_op_c d_op_d G_force mk,  (c, d) = (x,x) (x,y) (x,z) / (y,y) (y,z) (z,z)
+// ---- x passes of the dipolar k-space operator -----------------------------
+// Forward (per block: one ky, a tile of kz, the block table of the charge x
+// pass): mk = sum_d d_op_d F_d in x-transformed space from the three
+// components F_d.  d_op_y and d_op_z are constant along x, so
+//   mk = d_op_x FFT_x(F_x) + FFT_x(d_op_y F_y + d_op_z F_z):
+// two transforms; mk replaces component x in place (each block rewrites only
+// the lines it read).
 // EV: per-block partial of the k-space energy sum G_energy |mk|^2 with the
 // Hermitian weights of the half mesh (1 at kz = 0 and M/2, else 2).
-// Shared memory: 3 x tile staged lines of line_ld(M) (two FFT buffers and
-// mk), twiddles (M): the charge x pass's layout.
-template <typename Real, bool EV>
-__global__ void __launch_bounds__(256, 1)
+// Shared memory: 2 x tile staged lines of line_ld(M) (3 x unless TWO: a
+// scratch buffer), twiddles (M): the charge x pass's layout.
+template <typename Real, bool EV, bool TWO>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && TWO ? 3 : 2)
 k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              typename CplxOf<Real>::type *__restrict__ comp_hat, long long fstride,
-             const Real *__restrict__ g_e, const Real *__restrict__ g_f, int mode,
-             typename CplxOf<Real>::type *__restrict__ field0, int tile,
-             double *__restrict__ partials, const typename CplxOf<Real>::type *__restrict__ twtab) {
+             const Real *__restrict__ g_e, int tile, double *__restrict__ partials,
+             const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Blk const bk = blks[blockIdx.x];
@@ -267,63 +262,40 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = a + L;
-  C *mk = b + L;
-  C *tw = mk + L;
+  C *c = TWO ? nullptr : b + L;
+  C *tw = a + (TWO ? 2 : 3) * L;
   load_twiddles(tw, twtab, G.plan[0]);
   long long const stride_x = static_cast<long long>(M1) * G.hp;
-  long long const base = G.km_off + static_cast<long long>(y) * G.hp + kz0;
   int const tq = threadIdx.x & 15, xq = threadIdx.x >> 4;
   bool const col = tq < T;
   int const kz = kz0 + tq;
-  int const dop_y = dp_dop(y, M1), dop_z = dp_dop(kz, M2);
-  // stage T lines of src (column tq, rows x) into dst
-  auto stage = [&](const C *src, C *dst) {
-    for (int x0 = xq; x0 < M0; x0 += 64) {
-      C v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int const x = x0 + 16 * u;
-        if (col && x < M0)
-          v[u] = src[base + x * stride_x + tq];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int const x = x0 + 16 * u;
-        if (col && x < M0)
-          dst[tq * ld + pix(x)] = v[u];
-      }
+  long long const base = G.km_off + static_cast<long long>(y) * G.hp + kz;
+  Real const dop_y = static_cast<Real>(dp_dop(y, M1)), dop_z = static_cast<Real>(dp_dop(kz, M2));
+#pragma unroll 4
+  for (int x = xq; x < M0; x += 16)
+    if (col) {
+      long long const at = base + x * stride_x;
+      C const vx = comp_hat[at], vy = comp_hat[at + fstride], vz = comp_hat[at + 2 * fstride];
+      a[tq * ld + pix(x)] = vx;
+      b[tq * ld + pix(x)] = C{dop_y * vy.x + dop_z * vz.x, dop_y * vy.y + dop_z * vz.y};
     }
-  };
-  if (mode == 0) {
-    for (int d = 0; d < 3; ++d) {
-      stage(comp_hat + fstride * d, a);
-      __syncthreads();
-      C const *res = fft_lines<C>(a, b, T, ld, G.plan[0], tw, false);
-      for (int x = xq; col && x < M0; x += 16) {
-        Real const op = static_cast<Real>(d == 0 ? dp_dop(x, M0) : (d == 1 ? dop_y : dop_z));
-        C const v = res[tq * ld + pix(x)];
-        C const m = (d == 0) ? C{Real(0), Real(0)} : mk[tq * ld + pix(x)];
-        mk[tq * ld + pix(x)] = C{m.x + op * v.x, m.y + op * v.y};
-      }
-      __syncthreads();
-    }
-    // mk for the force modes, in place of component x (same thread, same
-    // point as the staging: the block's own lines only)
-    if (col)
-      for (int x = xq; x < M0; x += 16)
-        comp_hat[base + x * stride_x + tq] = mk[tq * ld + pix(x)];
-  } else {
-    stage(comp_hat, mk);
-    __syncthreads();
+  __syncthreads();
+  C *ra = fft_lines<TWO>(a, c, T, ld, G.plan[0], tw);
+  // without TWO: the buffer that the first transform left free
+  C *rb = fft_lines<TWO>(b, ra == a ? c : a, T, ld, G.plan[0], tw);
+  double acc = 0.0;
+  double const wgt = (kz == 0 || kz == M2 / 2) ? 1.0 : 2.0;
+  for (int x = xq; col && x < M0; x += 16) {
+    Real const op = static_cast<Real>(dp_dop(x, M0));
+    C const u = ra[tq * ld + pix(x)], v = rb[tq * ld + pix(x)];
+    C const m = C{op * u.x + v.x, op * u.y + v.y};
+    long long const at = base + x * stride_x;
+    comp_hat[at] = m;
+    if constexpr (EV)
+      acc += wgt * static_cast<double>(g_e[at]) *
+             (static_cast<double>(m.x) * m.x + static_cast<double>(m.y) * m.y);
   }
   if constexpr (EV) {
-    double acc = 0.0;
-    double const wgt = (kz == 0 || kz == M2 / 2) ? 1.0 : 2.0;
-    for (int x = xq; col && x < M0; x += 16) {
-      C const m = mk[tq * ld + pix(x)];
-      double const g = static_cast<double>(g_e[base + x * stride_x + tq]);
-      acc += wgt * g * (static_cast<double>(m.x) * m.x + static_cast<double>(m.y) * m.y);
-    }
     __shared__ double red[8];
     int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1)
@@ -338,29 +310,70 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       partials[blockIdx.x] = s;
     }
   }
-  for (int j = 0; j < 3; ++j) {
-    __syncthreads(); // the previous field's transform has been stored
-    for (int x = xq; col && x < M0; x += 16) {
-      int const op[3] = {dp_dop(x, M0), dop_y, dop_z};
-      C const m = mk[tq * ld + pix(x)];
-      C v;
-      if (mode == 0) {
-        Real const c = static_cast<Real>(op[j]) * g_e[base + x * stride_x + tq];
-        v = C{c * m.x, c * m.y};
-      } else {
-        int const c0 = (mode == 1) ? 0 : (j == 2 ? 2 : 1);
-        int const c1 = (mode == 1) ? j : (j == 0 ? 1 : 2);
-        Real const c = static_cast<Real>(op[c0] * op[c1]) * g_f[base + x * stride_x + tq];
-        v = C{c * m.y, -c * m.x}; // -i c mk
-      }
-      a[tq * ld + pix(x)] = v;
+}
+
+// Backward: block 5 k + o forms spectrum o of tile k from mk and transforms it
+// along x:
+//   o = 0, 1:    d_op_x^p G_energy mk,     p = 1, 0  (torques, AssignTorques,
+//                dp3m.cpp:372-395)
+//   o = 2, 3, 4: -i d_op_x^p G_force mk,   p = 2, 1, 0  (forces, AssignForces,
+//                dp3m.cpp:396-430)
+// d_op along y and z commutes with the x transform: the y and z passes apply
+// its powers (dp_y_pass, dp_z_pass), so 5 backward x transforms serve the
+// three torque fields and the six entries of the symmetric force-field tensor.
+// Shared memory: the forward pass's.
+template <typename Real, bool TWO>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && TWO ? 3 : 2)
+k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
+                 const typename CplxOf<Real>::type *__restrict__ mk_hat, long long fstride,
+                 const Real *__restrict__ g_e, const Real *__restrict__ g_f,
+                 typename CplxOf<Real>::type *__restrict__ field0, int tile,
+                 const typename CplxOf<Real>::type *__restrict__ twtab) {
+  using C = typename CplxOf<Real>::type;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  int const blk = blockIdx.x / 5, o = blockIdx.x - 5 * blk;
+  Blk const bk = blks[blk];
+  RepGeom const &G = reps[bk.rep];
+  int const M0 = G.mesh[0], M1 = G.mesh[1];
+  int const T = min(tile, G.mesh[2] / 2 + 1 - bk.b);
+  int const ld = line_ld(M0);
+  C *a = reinterpret_cast<C *>(smem_raw);
+  C *b = TWO ? nullptr : a + tile * ld;
+  C *tw = a + (TWO ? 2 : 3) * tile * ld;
+  load_twiddles(tw, twtab, G.plan[0]);
+  long long const stride_x = static_cast<long long>(M1) * G.hp;
+  int const tq = threadIdx.x & 15, xq = threadIdx.x >> 4;
+  bool const col = tq < T;
+  long long const base = G.km_off + static_cast<long long>(bk.a) * G.hp + bk.b + tq;
+  bool const tor = o < 2;
+  int const p = tor ? 1 - o : 4 - o; // power of d_op_x
+  const Real *g = tor ? g_e : g_f;
+#pragma unroll 4
+  for (int x = xq; x < M0; x += 16)
+    if (col) {
+      C const m = mk_hat[base + x * stride_x];
+      int const dx = dp_dop(x, M0);
+      Real const c = static_cast<Real>(p == 0 ? 1 : (p == 1 ? dx : dx * dx)) * g[base + x * stride_x];
+      // c mk, or -i c mk; real and imaginary parts swapped (backward)
+      a[tq * ld + pix(x)] = tor ? C{c * m.y, c * m.x} : C{-c * m.x, c * m.y};
     }
-    __syncthreads();
-    C const *fres = fft_lines<C>(a, b, T, ld, G.plan[0], tw, true);
-    if (col)
-      for (int x = xq; x < M0; x += 16)
-        field0[fstride * j + base + x * stride_x + tq] = fres[tq * ld + pix(x)];
-  }
+  __syncthreads();
+  C const *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw);
+  if (col)
+    for (int x = xq; x < M0; x += 16)
+      field0[fstride * o + base + x * stride_x] = cswap(res[tq * ld + pix(x)]);
+}
+
+// Backward y pass over the x pass's five arrays: nine fields (E_x, E_y, E_z in
+// arrays 0, 5, 6; the tensor's xx, xy, xz, yy, yz, zz in 2, 7, 8, 9, 10, 11);
+// and their backward z pass, sets (E_x, E_y, E_z), (xx, xy, xz), (yy, yz, zz).
+constexpr int kDipoleSpectra = 12;
+inline YPass dp_y_pass() {
+  return YPass{9, {0, 1, 1, 2, 3, 3, 4, 4, 4}, {0, 5, 6, 2, 7, 8, 9, 10, 11},
+               {0, 1, 0, 0, 1, 0, 2, 1, 0}};
+}
+inline ZPass dp_z_pass() {
+  return ZPass{{0, 5, 6, 2, 7, 8, 9, 10, 11}, {0, 0, 1, 0, 0, 1, 0, 1, 2}};
 }
 
 // Forces and torques from the interpolated fields (AoS, 3 per particle):

@@ -65,6 +65,13 @@ AxisPlan make_plan(int n, int tw_off) {
     if (p > 31)
       throw Error(1, "mesh size " + std::to_string(n) +
                          " has a prime factor > 31; choose a mesh with factors <= 31");
+  // two factors of at most 16 with a register transform each, the largest
+  // as small as possible (n1 >= n2)
+  for (int a = 16; a >= 2; --a)
+    if (n % a == 0 && a != 11 && a != 13 && n / a >= 2 && n / a <= a && n / a != 11 && n / a != 13) {
+      pl.n1 = a;
+      pl.n2 = n / a;
+    }
   pl.nstages = (n == 1) ? 0 : static_cast<int>(f.size());
   for (int s = 0; s < pl.nstages; ++s)
     pl.radix[s] = f[s];
@@ -281,7 +288,6 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   }
   // block tables
   size_t const csz = m_fp32 ? sizeof(float2) : sizeof(double2);
-  size_t const cap = m_fp32 ? 4096 : 2048; // complex elements per smem buffer
   {
     std::vector<int2> bm, bc, bcen, bp, nat;
     m_blk_census_start.assign(1, 0);
@@ -376,19 +382,22 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       maxM2 = std::max(maxM2, G.mesh[2]);
     }
     // staged lines are padded (line_ld); every pass also holds its axis
-    // twiddle table (n complex) in shared memory
+    // twiddle table (n complex) in shared memory.  Axes whose lines all have
+    // two-factor plans transform in place (one buffer fewer per pass)
+    for (int d = 0; d < 3; ++d) {
+      m_two[d] = true;
+      for (auto const &G : m_geom)
+        m_two[d] = m_two[d] && G.plan[d].n1 > 0;
+    }
     size_t const ldy = line_ld(maxM1), ldx = line_ld(maxM0);
-    // y pass: power-of-two lines of 32..256 transform in place (no scratch
-    // buffer)
-    bool yin = true;
-    for (auto const &G : m_geom)
-      yin = yin && fft_inplace_ok(G.mesh[1], 16, 256);
-    m_yin = yin;
-    m_tile_y = static_cast<int>(std::max<size_t>(1, std::min<size_t>(16, cap / ldy)));
-    // x pass: three line buffers (phi, field lines, scratch) of T kz columns
-    size_t const x_budget = 96 * 1024;
+    // y and x passes: tiles of up to 16 kz columns; 72 KB keep three FP32
+    // blocks of the x pass per SM at 256
+    size_t const y_budget = 72 * 1024, x_budget = m_two[0] ? 72 * 1024 : 96 * 1024;
+    size_t const y_bufs = m_two[1] ? 1 : 2, x_bufs = m_two[0] ? 2 : 3;
+    m_tile_y = static_cast<int>(
+        std::max<size_t>(1, std::min<size_t>(16, y_budget / (y_bufs * ldy * csz))));
     m_tile_x = static_cast<int>(
-        std::max<size_t>(1, std::min<size_t>(16, x_budget / (3 * ldx * csz))));
+        std::max<size_t>(1, std::min<size_t>(16, x_budget / (x_bufs * ldx * csz))));
     size_t smem_zf = 0, smem_zi = 0;
     for (int r = 0; r < R; ++r) {
       auto const &G = m_geom[r];
@@ -396,44 +405,36 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       int const H = M2 / 2 + 1;
       int const lines = M0 * M1;
       int const ldz = line_ld(M2);
-      // forward z: two real lines per complex transform; FP32: as many line
-      // pairs as keep four blocks within the SM's shared memory (24 lines at
-      // 256^3), fewer where the launch would have less than two blocks per
-      // SM (meshes up to 64)
+      // z passes: as many complex lines as give every thread of a block one
+      // transform of the smaller factor, within a quarter (FP64: half) of the
+      // SM's shared memory, and fewer where the launch would have less than
+      // two blocks per SM (meshes up to 64)
+      AxisPlan const &pz = G.plan[2];
+      bool const two = m_two[2];
+      size_t const z_budget = m_fp32 ? 54 * 1024 : 100 * 1024;
+      int const want = two ? 256 / std::min(pz.n1, pz.n2) : 256;
       auto const zf_smem = [&](int pairs) {
-        return (2 * static_cast<size_t>(pairs) * ldz + M2) * csz + 3 * M2 * sizeof(int);
+        return ((two ? 1 : 2) * static_cast<size_t>(pairs) * ldz + M2) * csz + 3 * M2 * sizeof(int);
       };
-      int lz = static_cast<int>(std::max<size_t>(1, cap / ldz)) * 2;
-      if (m_fp32) {
-        int q = 1;
-        while (zf_smem(q + 1) <= 54 * 1024)
-          ++q;
-        lz = 2 * q;
-      }
-      lz = std::min({lz, kZfLines, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2)});
+      // forward: two real lines per complex transform
+      int lz = 2;
+      while (lz / 2 < want && lz + 2 <= kZfLines && zf_smem(lz / 2 + 1) <= z_budget)
+        lz += 2;
+      lz = std::min(lz, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2));
       for (int l = 0; l < lines; l += lz)
         zf.push_back(Blk{r, l, std::min(lz, lines - l), 0});
       smem_zf = std::max(smem_zf, zf_smem((std::min(lz, lines) + 1) / 2));
-      // backward z: nl lines -> nl (Ex, Ey) + ceil(nl/2) (Ez pairs) transforms.
-      // FP32: as many lines as keep a block within a quarter of the SM's
-      // shared memory, so that four blocks are resident (8 lines at 256^3:
-      // 0.287 -> 0.271 ms for the backward y+z stage against 10 lines at
-      // three blocks per SM)
+      // backward: nl lines -> nl (Ex, Ey) + ceil(nl/2) (Ez pairs) transforms
       auto const zi_smem = [&](int nl) {
-        size_t const nc = nl + (nl + 1) / 2;
-        return (nc * ldz + z_inv_b_size(nl, M2) + M2) * csz;
+        return ((two ? 1 : 2) * static_cast<size_t>(nl + (nl + 1) / 2) * ldz + M2) * csz;
       };
-      int lzi = static_cast<int>(std::max<size_t>(1, 2 * (cap / ldz) / 3));
-      if (m_fp32) {
-        lzi = 1;
-        while (lzi < lines && zi_smem(lzi + 1) <= 54 * 1024)
-          ++lzi;
-      }
+      int lzi = 2;
+      while (3 * (lzi + 2) / 2 <= want && zi_smem(lzi + 2) <= z_budget)
+        lzi += 2;
+      lzi = std::min(lzi, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2));
       for (int l = 0; l < lines; l += lzi)
         zi.push_back(Blk{r, l, std::min(lzi, lines - l), 0});
-      int const nzi = std::min(lzi, lines);
-      size_t const nci = nzi + (nzi + 1) / 2;
-      smem_zi = std::max(smem_zi, (nci * ldz + z_inv_b_size(nzi, M2) + M2) * csz);
+      smem_zi = std::max(smem_zi, zi_smem(std::min(lzi, lines)));
       for (int xx = 0; xx < M0; ++xx)
         for (int k0 = 0; k0 < H; k0 += m_tile_y)
           y.push_back(Blk{r, xx, k0, 0});
@@ -444,8 +445,8 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     }
     m_smem_zf = smem_zf;
     m_smem_zi = smem_zi;
-    m_smem_y = ((yin ? 1 : 2) * static_cast<size_t>(m_tile_y) * ldy + maxM1) * csz;
-    m_smem_x = (3 * static_cast<size_t>(m_tile_x) * ldx + maxM0) * csz;
+    m_smem_y = (y_bufs * m_tile_y * ldy + maxM1) * csz;
+    m_smem_x = (x_bufs * m_tile_x * ldx + maxM0) * csz;
     m_n_blk_zf = static_cast<int>(zf.size());
     m_n_blk_y = static_cast<int>(y.size());
     m_n_blk_x = static_cast<int>(x.size());
@@ -483,21 +484,22 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
         aset(k_p3m_interp<double, 7>);
       }
     }
+    auto fft_attrs = [&](auto zero, auto two) {
+      using Real = decltype(zero);
+      constexpr bool TWO = decltype(two)::value;
+      attr(k_fft_z_fwd<Real, TWO>, m_smem_zf);
+      attr(k_fft_y<Real, false, TWO>, m_smem_y);
+      attr(k_fft_y<Real, true, TWO>, m_smem_y);
+      attr(k_fft_x_kspace<Real, true, TWO>, m_smem_x);
+      attr(k_fft_x_kspace<Real, false, TWO>, m_smem_x);
+      attr(k_fft_z_inv3<Real, TWO>, m_smem_zi);
+    };
     if (m_fp32) {
-      attr(k_fft_z_fwd<float>, m_smem_zf);
-      attr(k_fft_y<float, true>, m_smem_y);
-      attr(k_fft_y<float, false>, m_smem_y);
-      attr(k_fft_x_kspace<float, true>, m_smem_x);
-      attr(k_fft_x_kspace<float, false>, m_smem_x);
-      attr(k_fft_x_kspace<float, false, 3>, m_smem_x);
-      attr(k_fft_z_inv3<float>, m_smem_zi);
+      fft_attrs(0.0f, std::true_type{});
+      fft_attrs(0.0f, std::false_type{});
     } else {
-      attr(k_fft_z_fwd<double>, m_smem_zf);
-      attr(k_fft_y<double, true>, m_smem_y);
-      attr(k_fft_y<double, false>, m_smem_y);
-      attr(k_fft_x_kspace<double, true>, m_smem_x);
-      attr(k_fft_x_kspace<double, false>, m_smem_x);
-      attr(k_fft_z_inv3<double>, m_smem_zi);
+      fft_attrs(0.0, std::true_type{});
+      fft_attrs(0.0, std::false_type{});
     }
   }
   // buffers
@@ -524,7 +526,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_E.ensure(4 * m_ebins * rsz);
   encode_field_maps(st);
   m_ck.ensure(m_cplx * csz);
-  m_field.ensure(3 * m_cplx * csz);
+  m_field.ensure(kChargeSpectra * m_cplx * csz);
   m_ginf.ensure(m_cplx * rsz);
   m_part_x.ensure(static_cast<size_t>(m_n_blk_x) * 8 * sizeof(double));
   m_sums_x.ensure(static_cast<size_t>(R) * 8 * sizeof(double));
@@ -640,13 +642,16 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // One tensor map per replica over its packed, ghost-padded field mesh E (4
 // values per point): dims (4 E2, E1, E0) with E = epad, box (4 Ed, Ed, Ed)
-// with Ed = brick + cao - 1 (<= epad by construction).
-void Engine::encode_field_maps(cudaStream_t st) {
+// with Ed = brick + cao - 1 (<= epad by construction); `sets` field meshes
+// m_ebins records apart.
+void Engine::encode_field_maps(cudaStream_t st, int sets) {
   auto enc = tensor_map_encoder();
   size_t const es = m_fp32 ? sizeof(float) : sizeof(double);
-  std::vector<CUtensorMap> maps(m_geom.size());
-  for (size_t r = 0; r < m_geom.size(); ++r) {
-    RepGeom const &G = m_geom[r];
+  size_t const R = m_geom.size();
+  std::vector<CUtensorMap> maps(sets * R);
+  for (size_t m = 0; m < maps.size(); ++m) {
+    size_t const set = m / R;
+    RepGeom const &G = m_geom[m - set * R];
     cuuint32_t const Ed = static_cast<cuuint32_t>(G.brick + G.cao - 1);
     cuuint64_t const E0 = G.epad[0], E1 = G.epad[1], E2 = G.epad[2];
     if (Ed > E0 || Ed > E1 || Ed > E2 || 4 * Ed > 256)
@@ -655,9 +660,10 @@ void Engine::encode_field_maps(cudaStream_t st) {
     cuuint64_t strides[2] = {4 * E2 * es, 4 * E2 * E1 * es};
     cuuint32_t box[3] = {4 * Ed, Ed, Ed};
     cuuint32_t estr[3] = {1, 1, 1};
-    void *base = static_cast<char *>(m_E.p) + 4 * static_cast<size_t>(G.re_off) * es;
+    void *base =
+        static_cast<char *>(m_E.p) + 4 * (static_cast<size_t>(G.re_off) + set * m_ebins) * es;
     CUresult const rc =
-        enc(&maps[r], m_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+        enc(&maps[m], m_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
             3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -767,30 +773,19 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   }
   mark("p3m_assign", st);
   // 3. forward FFT z (r2c) and y
-  C const *tw = m_tw.as<C>();
-  k_fft_z_fwd<Real><<<m_n_blk_zf, 256, m_smem_zf, st>>>(geom, m_blk_zf.as<Blk>(),
-                                                        m_tiles.as<Real>(), 0, m_cov.as<int>(),
-                                                        m_sb_edge, m_ck.as<C>(), 0, tw);
-  ++m_launches;
-  launch_fft_y<Real>(m_ck.p, 0, 1, false, st);
+  launch_fft_z_fwd<Real>(m_tiles.as<Real>(), m_ck.p, 1, st);
+  launch_fft_y<Real>(m_ck.p, 0, y_plain(1), false, 0, st);
   mark("fft_fwd_zy", st);
   // 4. x pass fused with the k-space operator (+ energy/virial partials)
   bool const want_f = (f != nullptr);
   bool const want_ev = want_e || want_v;
-  if (want_ev)
-    k_fft_x_kspace<Real, true><<<m_n_blk_x, 256, m_smem_x, st>>>(
-        geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(), m_field.as<C>(), m_cplx,
-        m_tile_x, want_f ? 1 : 0, m_part_x.as<double>(), tw);
-  else if (sizeof(Real) == 4 && 3 * (m_smem_x + 1024) <= 228 * 1024)
-    // the shared memory leaves room for three blocks per SM: the instance
-    // whose registers allow them
-    k_fft_x_kspace<Real, false, 3><<<m_n_blk_x, 256, m_smem_x, st>>>(
-        geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(), m_field.as<C>(), m_cplx,
-        m_tile_x, want_f ? 1 : 0, m_part_x.as<double>(), tw);
-  else
-    k_fft_x_kspace<Real, false><<<m_n_blk_x, 256, m_smem_x, st>>>(
-        geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(), m_field.as<C>(), m_cplx,
-        m_tile_x, want_f ? 1 : 0, m_part_x.as<double>(), tw);
+  {
+    auto const kern = want_ev ? (m_two[0] ? k_fft_x_kspace<Real, true, true> : k_fft_x_kspace<Real, true, false>)
+                              : (m_two[0] ? k_fft_x_kspace<Real, false, true> : k_fft_x_kspace<Real, false, false>);
+    kern<<<m_n_blk_x, 256, m_smem_x, st>>>(geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(),
+                                           m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0,
+                                           m_part_x.as<double>(), m_tw.as<C>());
+  }
   ++m_launches;
   if (want_ev) {
     k_reduce_partials<<<ceil_div(R, 128), 128, 0, st>>>(m_part_x.as<double>(), 8,
@@ -802,10 +797,8 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   if (!want_f)
     return;
   // 5. backward FFT y (3 fields), z (c2r, 3 fields)
-  launch_fft_y<Real>(m_field.p, m_cplx, 3, true, st);
-  k_fft_z_inv3<Real><<<m_n_blk_zi, 256, m_smem_zi, st>>>(geom, m_blk_zi.as<Blk>(), m_field.as<C>(),
-                                                         m_cplx, m_E.as<Real>(), tw, m_kerr.as<int>());
-  ++m_launches;
+  launch_fft_y<Real>(m_field.p, m_cplx, y_charge(), true, 1, st);
+  launch_fft_z_inv<Real>(m_field.p, m_cplx, z_charge(), 1, 1, m_E.p, st);
   mark("fft_inv_yz", st);
   // 6. force back-interpolation
   for (int c = 1; m_n > 0 && c <= 7; ++c) {
@@ -816,8 +809,8 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     P3MX_CAO_DISPATCH_R(c, (k_p3m_interp<Real, P><<<interp_grid<Real, P>(nbr),
                                32 * (1 + kInterpWarps), interp_smem<Real, P>(), st>>>(
                                geom, tab, nbr, m_start.as<int>(), m_perm.as<int>(),
-                               m_skey.as<int>(), m_W.as<Real>(), m_E.as<Real>(),
-                               m_tmap.as<CUtensorMap>(), d_q(), m_dipole.as<double>(), f,
+                               m_skey.as<int>(), m_W.as<Real>(),
+                               m_tmap.as<CUtensorMap>(), 0, d_q(), m_dipole.as<double>(), f, 0,
                                overwrite ? 1 : 0, m_kerr.as<int>())));
     ++m_launches;
   }
@@ -1024,15 +1017,38 @@ void Engine::prepare_short_range(cudaStream_t st, bool need_spq) {
   }
 }
 
-// The y pass over nf field arrays field_stride complex elements apart, with
-// the in-place instance when every replica's y lines allow it.
+// The z, y and backward z passes with the in-place instances where every
+// replica's lines of the axis allow it.  sets: charge sets (z, tiles and
+// spectra m_tiles_n / m_cplx apart) or field sets (backward z, field meshes
+// m_ebins apart).
 template <typename Real>
-void Engine::launch_fft_y(void *c0, long long field_stride, int nf, bool inv, cudaStream_t st) {
+void Engine::launch_fft_z_fwd(const Real *tiles, void *spectra, int sets, cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
-  auto const kern = m_yin ? k_fft_y<Real, true> : k_fft_y<Real, false>;
-  kern<<<dim3(m_n_blk_y, nf), 256, m_smem_y, st>>>(m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(),
-                                                   static_cast<C *>(c0), field_stride, m_tile_y,
-                                                   inv, m_tw.as<C>());
+  auto const kern = m_two[2] ? k_fft_z_fwd<Real, true> : k_fft_z_fwd<Real, false>;
+  kern<<<dim3(m_n_blk_zf, sets), 256, m_smem_zf, st>>>(
+      m_geom_d.as<RepGeom>(), m_blk_zf.as<Blk>(), tiles, m_tiles_n, m_cov.as<int>(), m_sb_edge,
+      static_cast<C *>(spectra), m_cplx, m_tw.as<C>());
+  ++m_launches;
+}
+template <typename Real>
+void Engine::launch_fft_y(void *c0, long long field_stride, YPass const &job, bool inv, int kscale,
+                          cudaStream_t st) {
+  using C = typename CplxOf<Real>::type;
+  auto const kern = inv ? (m_two[1] ? k_fft_y<Real, true, true> : k_fft_y<Real, true, false>)
+                        : (m_two[1] ? k_fft_y<Real, false, true> : k_fft_y<Real, false, false>);
+  kern<<<m_n_blk_y * job.n, 256, m_smem_y, st>>>(
+      m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(), static_cast<C *>(c0), field_stride, job, kscale,
+      m_tile_y, m_tw.as<C>());
+  ++m_launches;
+}
+template <typename Real>
+void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp, int sets,
+                              int kscale, void *fields, cudaStream_t st) {
+  using C = typename CplxOf<Real>::type;
+  auto const kern = m_two[2] ? k_fft_z_inv3<Real, true> : k_fft_z_inv3<Real, false>;
+  kern<<<dim3(m_n_blk_zi, sets), 256, m_smem_zi, st>>>(
+      m_geom_d.as<RepGeom>(), m_blk_zi.as<Blk>(), static_cast<C *>(c0), field_stride, zp, kscale,
+      static_cast<Real *>(fields), m_ebins, m_tw.as<C>());
   ++m_launches;
 }
 

@@ -154,7 +154,13 @@ private:
   template <typename Real> void short_range_t(double *f, bool overwrite, bool want_ev,
                                               cudaStream_t st);
   template <typename Real>
-  void launch_fft_y(void *c0, long long field_stride, int nf, bool inv, cudaStream_t st);
+  void launch_fft_z_fwd(const Real *tiles, void *spectra, int sets, cudaStream_t st);
+  template <typename Real>
+  void launch_fft_y(void *c0, long long field_stride, YPass const &job, bool inv, int kscale,
+                    cudaStream_t st);
+  template <typename Real>
+  void launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp, int sets, int kscale,
+                        void *fields, cudaStream_t st);
   template <typename Real> void launch_pair(double *f, bool overwrite, bool want_ev,
                                             cudaStream_t st);
   void prepare_short_range(cudaStream_t st, bool need_spq);
@@ -165,7 +171,7 @@ private:
   void build_lists(cudaStream_t st);
   void set_list_capacity(double margin);
   void layout_lists(cudaStream_t st);
-  void encode_field_maps(cudaStream_t st);
+  void encode_field_maps(cudaStream_t st, int sets = 1);
   // want_spq: also the FP64 double4 positions (FP64 pair kernel)
   void refresh_sorted_positions(cudaStream_t st, bool want_spq = true);
   // Counting sort by key (perm: sorted position -> particle); index_order
@@ -207,7 +213,7 @@ private:
   int m_n_blk_mesh = 0, m_n_blk_cplx = 0, m_n_blk_census = 0, m_n_blk_pair = 0;
   int m_n_blk_zf = 0, m_n_blk_y = 0, m_n_blk_x = 0, m_n_blk_zi = 0;
   int m_tile_y = 16, m_tile_x = 16;
-  bool m_yin = true;  // every replica's y lines transform in place
+  bool m_two[3] = {true, true, true}; // every replica's lines of the axis have two-factor plans
   size_t m_smem_zf = 0, m_smem_y = 0, m_smem_x = 0, m_smem_zi = 0;
 
   // particles

@@ -4,18 +4,28 @@
 // (kz < M2/2+1 used, hp = padded row length).  Forward = exp(-i k x),
 // backward = exp(+i k x), both unnormalised, as the reference's FFTW
 // plans (fft/fft.cpp:682-696).  Each pass stages a tile of lines in shared
-// memory and runs Stockham autosort stages of radix 4, 2 or a generic
-// prime radix (Govindaraju et al. 2008 formulation); twiddles come from an
-// FP64-computed table rounded to the working precision.
+// memory and transforms them there; twiddles come from an FP64-computed
+// table rounded to the working precision.  Only forward transforms are
+// coded: a backward one swaps real and imaginary parts on its way into and
+// out of shared memory.
+//
+// Lengths N1 N2 with factors of at most 16 (AxisPlan n1, n2: nearly every
+// mesh up to 256) transform in place in two register steps; the others run
+// Stockham autosort stages with a second buffer (Govindaraju et al. 2008
+// formulation).
 //
 // The x pass is fused with the P3M k-space work that follows the forward
-// transform: optimal influence function, ik-differentiation (three field
-// components), k-space energy and pressure-tensor sums, and the three
-// backward x transforms -- one HBM round trip instead of five.
+// transform: optimal influence function, k-space energy and pressure-tensor
+// sums, and the backward x transforms.  The differentiation i k_d along y
+// and z commutes with the x transform, so the x pass emits two spectra only
+// (k_x phi and phi); the y pass forms and transforms k_y phi beside phi, and
+// the z pass multiplies by k_z.
 #pragma once
 
 #include "common.cuh"
 #include "p3m_kernels.cuh"
+
+#include <type_traits>
 
 namespace p3mx {
 
@@ -60,42 +70,67 @@ __device__ inline void load_twiddles(C *dst, const C *__restrict__ twtab, AxisPl
     dst[k] = src[k];
 }
 
-template <typename C> __device__ inline C ld_tw(const C *__restrict__ tw, int k, bool inv) {
-  C w = tw[k];
-  if (inv)
-    w.y = -w.y;
-  return w;
+// cos and sin of 2 pi k / n at compile time: the angle reduced to [0, pi/4]
+// in integers, then the Taylor series.
+__host__ __device__ constexpr double series_cos(double x) {
+  double t = 1.0, s = 1.0;
+  for (int i = 1; i < 12; ++i) {
+    t *= -x * x / ((2 * i - 1) * (2 * i));
+    s += t;
+  }
+  return s;
 }
+__host__ __device__ constexpr double series_sin(double x) {
+  double t = x, s = x;
+  for (int i = 1; i < 12; ++i) {
+    t *= -x * x / ((2 * i) * (2 * i + 1));
+    s += t;
+  }
+  return s;
+}
+__host__ __device__ constexpr double root_cos(int k, int n) {
+  k = ((k % n) + n) % n;
+  if (2 * k > n)
+    k = n - k;
+  // angle 2 pi k / n in [0, pi]
+  if (4 * k > n)
+    return -root_cos(n - 2 * k, 2 * n);
+  if (8 * k > n)
+    return series_sin(2.0 * kPi * (n - 4 * k) / (4.0 * n));
+  return series_cos(2.0 * kPi * k / n);
+}
+__host__ __device__ constexpr double root_sin(int k, int n) { return root_cos(4 * k - n, 4 * n); }
 
-// cos(2 pi k / 16) and sin(2 pi k / 16), k = 0..15 (exact constants of the
-// sixteenth roots of unity: 1, cos(pi/8), sqrt(1/2), sin(pi/8), 0).
-__host__ __device__ constexpr double cos16(int k) {
-  constexpr double c1 = 0.92387953251128675613, c2 = 0.70710678118654752440,
-                   c3 = 0.38268343236508977173;
-  switch (k & 15) {
-  case 0: return 1.0;
-  case 1: return c1;
-  case 2: return c2;
-  case 3: return c3;
-  case 4: return 0.0;
-  case 5: return -c3;
-  case 6: return -c2;
-  case 7: return -c1;
-  case 8: return -1.0;
-  case 9: return -c1;
-  case 10: return -c2;
-  case 11: return -c3;
-  case 12: return 0.0;
-  case 13: return c3;
-  case 14: return c2;
-  default: return c1;
+// f(integral_constant<int, I>) for I = 0 .. N-1, unrolled.
+template <int I, int N, typename F> __device__ __forceinline__ void static_for(F &&f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    static_for<I + 1, N>(f);
   }
 }
-__host__ __device__ constexpr double sin16(int k) { return cos16(k - 4); }
 
-// In-register DFT of a power-of-two length R <= 16 (radix-2 decimation in
-// time on top of the radix-4 kernel), constant twiddles.
-template <typename C, int R> __device__ __forceinline__ void dft_pow2(C *v, bool inv) {
+// v * exp(-2 pi i K / N), K and N compile-time.
+template <int K, int N, typename C> __device__ __forceinline__ C mul_root(C v) {
+  using Real = decltype(v.x);
+  constexpr int k = K % N;
+  if constexpr (k == 0) {
+    return v;
+  } else if constexpr (4 * k == N) {
+    return C{v.y, -v.x};
+  } else if constexpr (2 * k == N) {
+    return C{-v.x, -v.y};
+  } else if constexpr (4 * k == 3 * N) {
+    return C{-v.y, v.x};
+  } else {
+    constexpr Real c = static_cast<Real>(root_cos(k, N)), s = static_cast<Real>(root_sin(k, N));
+    return C{v.x * c + v.y * s, v.y * c - v.x * s};
+  }
+}
+
+// In-register forward DFT of length R, natural order in and out: 2 and 4
+// directly, odd primes from the sums and differences of mirrored inputs,
+// composites R = A B as B transforms of length A, twiddles, A of length B.
+template <typename C, int R> __device__ __forceinline__ void dft(C *v) {
   using Real = decltype(v[0].x);
   if constexpr (R == 2) {
     C const a = v[0], b = v[1];
@@ -104,87 +139,70 @@ template <typename C, int R> __device__ __forceinline__ void dft_pow2(C *v, bool
   } else if constexpr (R == 4) {
     C const s0 = cadd(v[0], v[2]), s1 = csub(v[0], v[2]);
     C const s2 = cadd(v[1], v[3]), s3 = csub(v[1], v[3]);
-    C const s3r = inv ? C{-s3.y, s3.x} : C{s3.y, -s3.x};
+    C const s3r = C{s3.y, -s3.x};
     v[0] = cadd(s0, s2);
     v[2] = csub(s0, s2);
     v[1] = cadd(s1, s3r);
     v[3] = csub(s1, s3r);
+  } else if constexpr (R % 2 == 1 && R % 3 != 0 || R == 3) {
+    constexpr int H = (R - 1) / 2;
+    C p[H], m[H];
+    static_for<0, H>([&](auto j) {
+      constexpr int J = decltype(j)::value;
+      p[J] = cadd(v[J + 1], v[R - 1 - J]);
+      m[J] = csub(v[J + 1], v[R - 1 - J]);
+    });
+    C const x0 = v[0];
+    C sum = x0;
+    static_for<0, H>([&](auto j) { sum = cadd(sum, p[decltype(j)::value]); });
+    v[0] = sum;
+    static_for<1, H + 1>([&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      C a = x0, b = C{Real(0), Real(0)};
+      static_for<0, H>([&](auto j) {
+        constexpr int J = decltype(j)::value;
+        constexpr Real c = static_cast<Real>(root_cos((J + 1) * K, R)),
+                       s = static_cast<Real>(root_sin((J + 1) * K, R));
+        a.x += c * p[J].x;
+        a.y += c * p[J].y;
+        b.x += s * m[J].x;
+        b.y += s * m[J].y;
+      });
+      // X_K = a - i b, X_{R-K} = a + i b
+      v[K] = C{a.x + b.y, a.y - b.x};
+      v[R - K] = C{a.x - b.y, a.y + b.x};
+    });
   } else {
-    constexpr int H = R / 2;
-    C e[H], o[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      e[i] = v[2 * i];
-      o[i] = v[2 * i + 1];
-    }
-    dft_pow2<C, H>(e, inv);
-    dft_pow2<C, H>(o, inv);
-#pragma unroll
-    for (int k = 0; k < H; ++k) {
-      C t;
-      if (k == 0) {
-        t = o[0];
-      } else if (2 * k == H) {
-        // exp(-+ i pi/2) = -+i
-        t = inv ? C{-o[k].y, o[k].x} : C{o[k].y, -o[k].x};
-      } else {
-        Real const wr = static_cast<Real>(cos16(k * (16 / R)));
-        Real const ws = static_cast<Real>(sin16(k * (16 / R)));
-        Real const wi = inv ? ws : -ws;
-        t = C{o[k].x * wr - o[k].y * wi, o[k].x * wi + o[k].y * wr};
-      }
-      v[k] = cadd(e[k], t);
-      v[k + H] = csub(e[k], t);
-    }
-  }
-}
-
-template <typename C, int R>
-__device__ inline void dft_small(C *v, const C *__restrict__ tw, int n, bool inv) {
-  if constexpr (R == 8 || R == 16) {
-    dft_pow2<C, R>(v, inv);
-  } else if constexpr (R == 2) {
-    C const a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  } else if constexpr (R == 4) {
-    C const s0 = cadd(v[0], v[2]), s1 = csub(v[0], v[2]);
-    C const s2 = cadd(v[1], v[3]), s3 = csub(v[1], v[3]);
-    // forward: multiply s3 by -i; backward: by +i
-    C const s3r = inv ? C{-s3.y, s3.x} : C{s3.y, -s3.x};
-    v[0] = cadd(s0, s2);
-    v[2] = csub(s0, s2);
-    v[1] = cadd(s1, s3r);
-    v[3] = csub(s1, s3r);
-  } else {
-    C out[R];
-    int const step = n / R;
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      C acc = v[0];
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        int const e = (r * m) % R;
-        acc = cadd(acc, cmul(v[r], ld_tw(tw, e * step, inv)));
-      }
-      out[m] = acc;
-    }
-#pragma unroll
-    for (int m = 0; m < R; ++m)
-      v[m] = out[m];
+    constexpr int A = R % 4 == 0 ? 4 : (R % 2 == 0 ? 2 : 3), B = R / A;
+    C y[R]; // y[k1 * B + t]
+    static_for<0, B>([&](auto tt) {
+      constexpr int T = decltype(tt)::value;
+      C w[A];
+      static_for<0, A>([&](auto mm) { w[decltype(mm)::value] = v[T + B * decltype(mm)::value]; });
+      dft<C, A>(w);
+      static_for<0, A>([&](auto kk) {
+        constexpr int K = decltype(kk)::value;
+        y[K * B + T] = mul_root<T * K, R>(w[K]);
+      });
+    });
+    static_for<0, A>([&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      dft<C, B>(y + K * B);
+      static_for<0, B>([&](auto jj) { v[K + A * decltype(jj)::value] = y[K * B + decltype(jj)::value]; });
+    });
   }
 }
 
 // Generic (runtime) radix for primes beyond the templated set.
 template <typename C>
-__device__ inline void dft_dyn(C *v, int R, const C *__restrict__ tw, int n, bool inv) {
+__device__ inline void dft_dyn(C *v, int R, const C *__restrict__ tw, int n) {
   C out[32];
   int const step = n / R;
   for (int m = 0; m < R; ++m) {
     C acc = v[0];
     for (int r = 1; r < R; ++r) {
       int const e = (r * m) % R;
-      acc = cadd(acc, cmul(v[r], ld_tw(tw, e * step, inv)));
+      acc = cadd(acc, cmul(v[r], tw[e * step]));
     }
     out[m] = acc;
   }
@@ -207,7 +225,7 @@ __device__ inline int qdiv(int a, int b, float rb) {
 // Twiddle index r*jm*tstride < n, so no modulo is needed.
 template <typename C, int R>
 __device__ inline void fft_stage_t(const C *src, C *dst, int n, int ld, int nlines, int Ns,
-                                   const C *__restrict__ tw, bool inv) {
+                                   const C *__restrict__ tw) {
   int const nb = n / R;
   int const total = nb * nlines;
   int const tstride = n / (Ns * R);
@@ -225,9 +243,9 @@ __device__ inline void fft_stage_t(const C *src, C *dst, int n, int ld, int nlin
     for (int r = 0; r < R; ++r) {
       v[r] = s[pix(j + r * nb)];
       if (r > 0 && jm != 0)
-        v[r] = cmul(v[r], ld_tw(tw, r * jm * tstride, inv));
+        v[r] = cmul(v[r], tw[r * jm * tstride]);
     }
-    dft_small<C, R>(v, tw, n, inv);
+    dft<C, R>(v);
     int const base = jq * Ns * R + jm;
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -237,7 +255,7 @@ __device__ inline void fft_stage_t(const C *src, C *dst, int n, int ld, int nlin
 
 template <typename C>
 __device__ inline void fft_stage_dyn(const C *src, C *dst, int n, int ld, int nlines, int Ns,
-                                     int R, const C *__restrict__ tw, bool inv) {
+                                     int R, const C *__restrict__ tw) {
   int const nb = n / R;
   int const total = nb * nlines;
   int const tstride = n / (Ns * R);
@@ -251,157 +269,156 @@ __device__ inline void fft_stage_dyn(const C *src, C *dst, int n, int ld, int nl
     for (int r = 0; r < R; ++r) {
       v[r] = s[pix(j + r * nb)];
       if (r > 0 && jm != 0)
-        v[r] = cmul(v[r], ld_tw(tw, r * jm * tstride, inv));
+        v[r] = cmul(v[r], tw[r * jm * tstride]);
     }
-    dft_dyn(v, R, tw, n, inv);
+    dft_dyn(v, R, tw, n);
     int const base = (j / Ns) * Ns * R + jm;
     for (int r = 0; r < R; ++r)
       d[pix(base + r * Ns)] = v[r];
   }
 }
 
-// Power-of-two line length N = N1 * N2 (N1, N2 <= 16) in two register
-// steps (n = t + N2 m, k = k1 + N1 k2):
-//   step 1, item (line, t): Y[t][k1] = w_N^(t k1) * DFT_N1 over m of x[t + N2 m],
+// Two-step transform in place, n = N1 N2 (n = t + N2 m, k = k1 + N1 k2):
+//   step 1, item (line, t): Y[t][k1] = w_n^(t k1) * DFT_N1 over m of x[t + N2 m],
 //           written in place at t + N2 k1;
-//   step 2, item (line, k1): X[k1 + N1 k2] = DFT_N2 over t of Y[t][k1],
-//           written to `b` in natural order.
-// Strides are compile-time constants; the padded layout (pix) keeps both
-// steps free of bank conflicts.  Returns b.
-template <typename C, int N1, int N2>
-__device__ C *fft_2step(C *a, C *b, int nlines, int ld, const C *__restrict__ tw, bool inv) {
-  for (int it = threadIdx.x; it < nlines * N2; it += blockDim.x) {
-    int const l = it / N2, t = it - l * N2;
+//   step 2, item (line, k1): X[k1 + N1 k2] = DFT_N2 over t of Y[t][k1]: the
+//           lines of a round are read into registers, the block
+//           synchronises, then they are written back in natural order.
+// n2 / n1 are the other factor (compile-time constants where the caller
+// passes them as such, so the strides fold).
+// opaque(): the compiler neither hoists the index arithmetic of all factors out
+// of a caller's loop nor keeps a step's 16 read addresses in registers for its
+// writes (both spill at the passes' register bounds).
+__device__ __forceinline__ int opaque(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+template <typename C, int N1>
+__device__ __forceinline__ void fft_step1(C *a, int nlines, int ld, int n2,
+                                          const C *__restrict__ tw) {
+  float const rn2 = 1.0f / static_cast<float>(n2);
+#pragma unroll 1
+  for (int it = opaque(threadIdx.x); it < nlines * n2; it += blockDim.x) {
+    int const l = qdiv(it, n2, rn2);
+    int t = it - l * n2;
     C *s = a + l * ld;
     C v[N1];
 #pragma unroll
     for (int m = 0; m < N1; ++m)
-      v[m] = s[pix(t + N2 * m)];
-    dft_pow2<C, N1>(v, inv);
+      v[m] = s[pix(t + n2 * m)];
+    dft<C, N1>(v);
 #pragma unroll
     for (int k1 = 1; k1 < N1; ++k1)
-      v[k1] = cmul(v[k1], ld_tw(tw, t * k1, inv));
+      v[k1] = cmul(v[k1], tw[t * k1]);
+    t = opaque(t);
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1)
-      s[pix(t + N2 * k1)] = v[k1];
+      s[pix(t + n2 * k1)] = v[k1];
   }
-  __syncthreads();
-  for (int it = threadIdx.x; it < nlines * N1; it += blockDim.x) {
-    int const l = it / N1, k1 = it - l * N1;
-    const C *s = a + l * ld;
-    C *d = b + l * ld;
+}
+template <typename C, int N2>
+__device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
+  int const per = blockDim.x / n1; // lines per round
+  int const tid = opaque(threadIdx.x);
+  int const lq = qdiv(tid, n1, 1.0f / static_cast<float>(n1)), k1 = tid - lq * n1;
+#pragma unroll 1
+  for (int l0 = 0; l0 < nlines; l0 += per) {
+    bool const act = lq < per && l0 + lq < nlines;
+    C *s = a + (l0 + lq) * ld;
     C v[N2];
+    if (act) {
 #pragma unroll
-    for (int t = 0; t < N2; ++t)
-      v[t] = s[pix(t + N2 * k1)];
-    dft_pow2<C, N2>(v, inv);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2)
-      d[pix(k1 + N1 * k2)] = v[k2];
-  }
-  __syncthreads();
-  return b;
-}
-
-// In-place form of fft_2step for nlines * 16 <= blockDim.x (one item per
-// thread and step): step 2 reads its column into registers, the block
-// synchronises, then every thread writes its outputs back to `a`.
-template <typename C, int N1, int N2>
-__device__ C *fft_2step_inplace(C *a, int nlines, int ld, const C *__restrict__ tw, bool inv) {
-  int const it = threadIdx.x;
-  if (it < nlines * N2) {
-    int const l = it / N2, t = it - l * N2;
-    C *s = a + l * ld;
-    C v[N1];
-#pragma unroll
-    for (int m = 0; m < N1; ++m)
-      v[m] = s[pix(t + N2 * m)];
-    dft_pow2<C, N1>(v, inv);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1)
-      v[k1] = cmul(v[k1], ld_tw(tw, t * k1, inv));
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1)
-      s[pix(t + N2 * k1)] = v[k1];
-  }
-  __syncthreads();
-  bool const act = it < nlines * N1;
-  int const l = it / N1, k1 = it - l * N1;
-  C v[N2];
-  if (act) {
-    const C *s = a + l * ld;
-#pragma unroll
-    for (int t = 0; t < N2; ++t)
-      v[t] = s[pix(t + N2 * k1)];
-    dft_pow2<C, N2>(v, inv);
-  }
-  __syncthreads();
-  if (act) {
-    C *d = a + l * ld;
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2)
-      d[pix(k1 + N1 * k2)] = v[k2];
-  }
-  __syncthreads();
-  return a;
-}
-
-// True when lines of length n transform in place (fft_lines_inplace): n a
-// power of two in 32..256 and nlines * 16 <= threads.
-__host__ __device__ inline bool fft_inplace_ok(int n, int nlines, int threads) {
-  return (n == 32 || n == 64 || n == 128 || n == 256) && nlines * 16 <= threads;
-}
-
-// In-place transform of nlines lines in `a` (requires fft_inplace_ok);
-// returns a.  A separate function from fft_lines, so that kernels that never
-// transform in place do not carry its code (and registers).
-template <typename C>
-__device__ C *fft_lines_inplace(C *a, int nlines, int ld, AxisPlan const &pl,
-                                const C *__restrict__ tw, bool inv) {
-  switch (pl.n) {
-  case 32: return fft_2step_inplace<C, 16, 2>(a, nlines, ld, tw, inv);
-  case 64: return fft_2step_inplace<C, 16, 4>(a, nlines, ld, tw, inv);
-  case 128: return fft_2step_inplace<C, 16, 8>(a, nlines, ld, tw, inv);
-  default: return fft_2step_inplace<C, 16, 16>(a, nlines, ld, tw, inv);
-  }
-}
-
-// Full transform of nlines lines in `a` (scratch `b`; element i of line l at
-// l*ld + pix(i)); tw = the axis twiddle table (shared memory).  Returns the
-// buffer holding the result.  All threads of the block must call it.
-template <typename C>
-__device__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
-                        const C *__restrict__ tw, bool inv) {
-  int const n = pl.n;
-  switch (n) {
-  case 32: return fft_2step<C, 16, 2>(a, b, nlines, ld, tw, inv);
-  case 64: return fft_2step<C, 16, 4>(a, b, nlines, ld, tw, inv);
-  case 128: return fft_2step<C, 16, 8>(a, b, nlines, ld, tw, inv);
-  case 256: return fft_2step<C, 16, 16>(a, b, nlines, ld, tw, inv);
-  default: break;
-  }
-  int Ns = 1;
-  C *src = a, *dst = b;
-  for (int s = 0; s < pl.nstages; ++s) {
-    int const R = pl.radix[s];
-    switch (R) {
-    case 2: fft_stage_t<C, 2>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 3: fft_stage_t<C, 3>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 4: fft_stage_t<C, 4>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 8: fft_stage_t<C, 8>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 16: fft_stage_t<C, 16>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 5: fft_stage_t<C, 5>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    case 7: fft_stage_t<C, 7>(src, dst, n, ld, nlines, Ns, tw, inv); break;
-    default: fft_stage_dyn<C>(src, dst, n, ld, nlines, Ns, R, tw, inv); break;
+      for (int t = 0; t < N2; ++t)
+        v[t] = s[pix(N2 * k1 + t)];
+      dft<C, N2>(v);
     }
     __syncthreads();
-    Ns *= R;
-    C *t = src;
-    src = dst;
-    dst = t;
+    if (act) {
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        s[pix(k1 + n1 * k2)] = v[k2];
+    }
   }
-  return src;
 }
+#define P3MX_FACTOR_DISPATCH(N, CALL)                                          \
+  switch (N) {                                                                 \
+  case 2: { constexpr int R = 2; CALL; } break;                                \
+  case 3: { constexpr int R = 3; CALL; } break;                                \
+  case 4: { constexpr int R = 4; CALL; } break;                                \
+  case 5: { constexpr int R = 5; CALL; } break;                                \
+  case 6: { constexpr int R = 6; CALL; } break;                                \
+  case 7: { constexpr int R = 7; CALL; } break;                                \
+  case 8: { constexpr int R = 8; CALL; } break;                                \
+  case 9: { constexpr int R = 9; CALL; } break;                                \
+  case 10: { constexpr int R = 10; CALL; } break;                              \
+  case 12: { constexpr int R = 12; CALL; } break;                              \
+  case 14: { constexpr int R = 14; CALL; } break;                              \
+  case 15: { constexpr int R = 15; CALL; } break;                              \
+  default: { constexpr int R = 16; CALL; } break;                              \
+  }
+// In-place transform of nlines lines (plan with n1, n2); the caller's block
+// of at least 16 threads synchronises before, the result is visible after.
+template <typename C>
+__device__ __forceinline__ void fft_lines_2(C *a, int nlines, int ld, AxisPlan const &pl,
+                                            const C *__restrict__ tw) {
+  if (pl.n == 256) {
+    fft_step1<C, 16>(a, nlines, ld, 16, tw);
+    __syncthreads();
+    fft_step2<C, 16>(a, nlines, ld, 16);
+  } else if (pl.n == 128) {
+    fft_step1<C, 16>(a, nlines, ld, 8, tw);
+    __syncthreads();
+    fft_step2<C, 8>(a, nlines, ld, 16);
+  } else {
+    P3MX_FACTOR_DISPATCH(pl.n1, (fft_step1<C, R>(a, nlines, ld, pl.n2, tw)))
+    __syncthreads();
+    P3MX_FACTOR_DISPATCH(pl.n2, (fft_step2<C, R>(a, nlines, ld, pl.n1)))
+  }
+  __syncthreads();
+}
+
+// Forward transform of nlines lines in `a` (element i of line l at
+// l*ld + pix(i)); tw = the axis twiddle table (shared memory).  TWO: the
+// launch's lines all have two-factor plans and transform in place (b
+// unused); otherwise `b` is a second buffer of the same size.  Returns the
+// buffer holding the result.  All threads of the block must call it.
+template <bool TWO, typename C>
+__device__ __forceinline__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
+                                        const C *__restrict__ tw) {
+  if constexpr (TWO) {
+    fft_lines_2(a, nlines, ld, pl, tw);
+    return a;
+  } else {
+    int const n = pl.n;
+    int Ns = 1;
+    C *src = a, *dst = b;
+    for (int s = 0; s < pl.nstages; ++s) {
+      int const R = pl.radix[s];
+      switch (R) {
+      case 2: fft_stage_t<C, 2>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 3: fft_stage_t<C, 3>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 4: fft_stage_t<C, 4>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 8: fft_stage_t<C, 8>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 16: fft_stage_t<C, 16>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 5: fft_stage_t<C, 5>(src, dst, n, ld, nlines, Ns, tw); break;
+      case 7: fft_stage_t<C, 7>(src, dst, n, ld, nlines, Ns, tw); break;
+      default: fft_stage_dyn<C>(src, dst, n, ld, nlines, Ns, R, tw); break;
+      }
+      __syncthreads();
+      Ns *= R;
+      C *t = src;
+      src = dst;
+      dst = t;
+    }
+    return src;
+  }
+}
+
+// Signed frequency of index i in an axis of m points, the Nyquist index as
+// zero (calc_meshift with the differential operator's convention,
+// p3m/common.hpp:248-264).
+__device__ inline int freq_dop(int i, int m) { return (i == m / 2) ? 0 : (i < m / 2 ? i : i - m); }
+template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 
 // ---- pass z, forward: real lines -> complex half lines -----------------
 // Two real lines per complex transform: Z = x0 + i x1, then
@@ -412,10 +429,11 @@ __device__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
 // first each point's own super-brick (four points per load), then the points
 // in a halo of the previous one along z.
 // blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
-// Shared memory: 2 x bk.b/2 staged lines of line_ld(n), twiddles (n), the
-// halo points' z and offsets (3 n ints).  Meshes are even, so is bk.b.
+// Shared memory: bk.b/2 staged lines of line_ld(n) (twice that unless TWO),
+// twiddles (n), the halo points' z and offsets (3 n ints).  Meshes are even,
+// so is bk.b.
 constexpr int kZfLines = 64; // most real lines per block
-template <typename Real>
+template <typename Real, bool TWO>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
 k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
             const Real *__restrict__ tiles, long long tile_stride, const int *__restrict__ cov,
@@ -432,8 +450,8 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const nl = bk.b;          // real lines in this block
   int const np = (nl + 1) >> 1; // complex lines
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = a + np * ld;
-  C *tw = b + np * ld;
+  C *b = TWO ? nullptr : a + np * ld;
+  C *tw = a + (TWO ? 1 : 2) * np * ld;
   int *zc = reinterpret_cast<int *>(tw + n);
   tiles += blockIdx.y * tile_stride + G.tl_off;
   cmesh += blockIdx.y * c_stride;
@@ -489,7 +507,7 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     ar[2 * ((l >> 1) * ld + pix(zc[h])) + (l & 1)] += v;
   }
   __syncthreads();
-  C *res = fft_lines<C>(a, b, np, ld, G.plan[2], tw, false);
+  C *res = fft_lines<TWO>(a, b, np, ld, G.plan[2], tw);
   int const H = n / 2 + 1;
   int const hp = G.hp;
   for_lines(nl, hp, [&](int l, int k) {
@@ -506,36 +524,58 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   });
 }
 
-// ---- pass y (either direction, nf field arrays via blockIdx.y) ---------
-// Shared memory: tile staged lines of line_ld(M1) (two sets unless the
-// lines transform in place), twiddles (M1).
-// INPL: every replica's lines transform in place (the host checks), so the
-// instance carries none of the out-of-place transform's code or registers.
-template <typename Real, bool INPL>
+// ---- pass y ---------------------------------------------------------------
+// Jobs of a y pass: job k transforms array src[k], times k_y^pw[k], into array
+// dst[k].  Array src[k] is read by other jobs unless dst[k] = src[k].  The
+// jobs of one tile are neighbouring blocks, so a shared source is read from
+// HBM once.
+struct YPass {
+  int n;
+  signed char src[9], dst[9], pw[9];
+};
+// nf arrays in place
+inline YPass y_plain(int nf) {
+  YPass p{};
+  p.n = nf;
+  for (int k = 0; k < nf; ++k)
+    p.src[k] = p.dst[k] = static_cast<signed char>(k);
+  return p;
+}
+// backward y pass of the charge fields: k_x phi (array 0, in place), k_y phi
+// and phi (arrays 2 and 3) from phi (array 1)
+inline YPass y_charge() { return YPass{3, {1, 1, 0}, {2, 3, 0}, {1, 0, 0}}; }
+constexpr int kChargeSpectra = 4; // arrays of the charge fields' spectra
+// TWO: every replica's y lines transform in place (the host checks).  kscale:
+// k_y in units of 2 pi / box (1) or as an integer (0).  Shared memory: tile
+// staged lines of line_ld(M1) (two sets unless TWO), twiddles (M1).
+template <typename Real, bool INV, bool TWO>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
 k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
-        typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, int tile,
-        bool inv, const typename CplxOf<Real>::type *__restrict__ twtab) {
+        typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, YPass const job,
+        int kscale, int tile, const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Blk const bk = blks[blockIdx.x];
+  int const blk = blockIdx.x / job.n, jb = blockIdx.x - blk * job.n;
+  Blk const bk = blks[blk];
   RepGeom const &G = reps[bk.rep];
-  C *cm = c0 + field_stride * blockIdx.y;
   int const M1 = G.mesh[1];
   int const H = G.mesh[2] / 2 + 1;
   int const x = bk.a, kz0 = bk.b;
   int const T = min(tile, H - kz0);
   int const ld = line_ld(M1);
-  bool const inplace = INPL || fft_inplace_ok(M1, tile, blockDim.x);
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = inplace ? nullptr : a + tile * ld;
-  C *tw = a + (inplace ? 1 : 2) * tile * ld;
+  C *b = TWO ? nullptr : a + tile * ld;
+  C *tw = a + (TWO ? 1 : 2) * tile * ld;
   load_twiddles(tw, twtab, G.plan[1]);
-  long long const rowbase = G.km_off + static_cast<long long>(x) * M1 * G.hp + kz0;
   long long const hp = G.hp;
   // 16 x 16 thread mapping (tile <= 16 columns): column tq, rows yq + 16 i
   int const tq = threadIdx.x & 15, yq = threadIdx.x >> 4;
   bool const col = tq < T;
+  long long const base = G.km_off + static_cast<long long>(x) * M1 * hp + kz0 + tq;
+  const C *src = c0 + field_stride * job.src[jb] + base;
+  C *dst = c0 + field_stride * job.dst[jb] + base;
+  int const pw = INV ? job.pw[jb] : 0;
+  Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[1]) : Real(1);
   // all of a thread's rows in flight at once (up to 16: M1 <= 256 in one
   // round)
   for (int y0 = yq; y0 < M1; y0 += 256) {
@@ -544,38 +584,42 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     for (int u = 0; u < 16; ++u) {
       int const y = y0 + 16 * u;
       if (col && y < M1)
-        v[u] = cm[rowbase + y * hp + tq];
+        v[u] = src[y * hp];
     }
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       int const y = y0 + 16 * u;
-      if (col && y < M1)
-        a[tq * ld + pix(y)] = v[u];
+      if (col && y < M1) {
+        C w = INV ? cswap(v[u]) : v[u];
+        if (INV && pw > 0) {
+          Real const k = static_cast<Real>(freq_dop(y, M1)) * ks;
+          Real const f = pw == 2 ? k * k : k;
+          w = C{f * w.x, f * w.y};
+        }
+        a[tq * ld + pix(y)] = w;
+      }
     }
   }
   __syncthreads();
-  C *res;
-  if constexpr (INPL)
-    res = fft_lines_inplace<C>(a, T, ld, G.plan[1], tw, inv);
-  else
-    res = inplace ? fft_lines_inplace<C>(a, T, ld, G.plan[1], tw, inv)
-                  : fft_lines<C>(a, b, T, ld, G.plan[1], tw, inv);
+  const C *res = fft_lines<TWO>(a, b, T, ld, G.plan[1], tw);
   if (col)
-    for (int y = yq; y < M1; y += 16)
-      cm[rowbase + y * hp + tq] = res[tq * ld + pix(y)];
+    for (int y = yq; y < M1; y += 16) {
+      C const v = res[tq * ld + pix(y)];
+      dst[y * hp] = INV ? cswap(v) : v;
+    }
 }
 
 // ---- pass x fused with the k-space operator -----------------------------
 // Per block: one ky, a tile of kz; partials[blk*8 + {E, Pxx, Pxy, Pxz, Pyy,
 // Pyz, Pzz, diag}] in FP64 (Hermitian weights 1 for kz = 0, M2/2, else 2).
-// Shared memory: 3 x tile staged lines of line_ld(M0) (phi, field lines,
-// scratch), twiddles (M0).
+// Emits two backward-x-transformed spectra: array 0 i k_x phi, array 1 i phi
+// (the y and z passes apply k_y and k_z).
+// Shared memory: 2 x tile staged lines of line_ld(M0) (phi, k_x phi; 3 x
+// unless TWO: a scratch buffer), twiddles (M0).
 // EV: energy / virial partials (a template parameter, so that the
-// forces-only instance carries none of their registers).  MINB: blocks per
-// SM the registers are sized for -- 3 pays where the shared memory of a
-// launch (small meshes) leaves room for a third block.
-template <typename Real, bool EV, int MINB = 2>
-__global__ void __launch_bounds__(256, MINB)
+// forces-only instance carries none of their registers).
+template <typename Real, bool EV, bool TWO>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && !EV && TWO ? 3 : 2)
 k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
                const typename CplxOf<Real>::type *__restrict__ rho_hat,
                const Real *__restrict__ ginf, typename CplxOf<Real>::type *__restrict__ field0,
@@ -594,8 +638,8 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = a + L;
-  C *c = b + L; // three line buffers: phi, field lines, FFT scratch
-  C *tw = c + L;
+  C *c = TWO ? nullptr : b + L;
+  C *tw = a + (TWO ? 2 : 3) * L;
   load_twiddles(tw, twtab, G.plan[0]);
   long long const stride_x = static_cast<long long>(M1) * G.hp;
   long long const base = G.km_off + static_cast<long long>(y) * G.hp + kz0;
@@ -618,23 +662,21 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
   }
   __syncthreads();
-  C *res = fft_lines<C>(a, b, T, ld, G.plan[0], tw, false);
-  C *fb = (res == a) ? b : a; // field lines go to the free buffer
+  C *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw);
+  C *fb = (res == a) ? b : a; // k_x phi goes to the free buffer
   // k-space operator
   double const wv[3] = {2.0 * kPi * G.box_i[0], 2.0 * kPi * G.box_i[1],
                         2.0 * kPi * G.box_i[2]};
   double const hai2 = (1.0 / 2.0 / G.alpha) * (1.0 / 2.0 / G.alpha);
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  // d_op (Nyquist zeroed) integer shift of index i in a mesh of size m
-  auto dop = [](int i, int m) { return (i == m / 2) ? 0 : (i < m / 2 ? i : i - m); };
-  int const kyd = dop(y, M1);
+  int const kyd = freq_dop(y, M1);
   for (int x = xq; col && x < M0; x += 16) {
     // t fastest across lanes: the influence-function reads are T-contiguous
     int const t = tq;
     int const kz = kz0 + t;
     C const rh = res[t * ld + pix(x)];
     Real const g = ginf[base + x * stride_x + t];
-    int const kxd = dop(x, M0), kzd = dop(kz, M2);
+    int const kxd = freq_dop(x, M0), kzd = freq_dop(kz, M2);
     if constexpr (EV) {
       double const wgt = (kz == 0 || kz == M2 / 2) ? 1.0 : 2.0;
       double const ek = wgt * static_cast<double>(g) *
@@ -653,8 +695,12 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
         acc[7] += ek;
       }
     }
-    // phi = G rho_hat replaces rho_hat in place (same thread, same point)
-    res[t * ld + pix(x)] = C{g * rh.x, g * rh.y};
+    // i phi and i k_x phi, real and imaginary parts swapped for the backward
+    // transforms (phi = G rho_hat replaced in place: same thread, same point)
+    Real const k = static_cast<Real>(kxd) * static_cast<Real>(wv[0]);
+    C const p = C{g * rh.x, -(g * rh.y)};
+    res[t * ld + pix(x)] = p;
+    fb[t * ld + pix(x)] = C{k * p.x, k * p.y};
   }
   if constexpr (EV) {
     // block reduction of the 8 partial sums (fixed order -> deterministic)
@@ -680,51 +726,45 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   }
   if (!want_fields)
     return;
-  // the three field components, one after another: E_d = i k_d phi, then
-  // the backward x transform of its T lines
-  int const kvec_y = kyd;
-  for (int d = 0; d < 3; ++d) {
-    __syncthreads(); // phi complete / previous component stored
-    Real const wd = static_cast<Real>(wv[d]);
-    for (int x = xq; col && x < M0; x += 16) {
-      int const t = tq;
-      int const kd = (d == 0) ? dop(x, M0) : (d == 1 ? kvec_y : dop(kz0 + t, M2));
-      Real const k = static_cast<Real>(kd) * wd;
-      C const phi = res[t * ld + pix(x)];
-      fb[t * ld + pix(x)] = C{-k * phi.y, k * phi.x};
-    }
+  __syncthreads();
+  // without TWO the scratch of the second transform is the first's buffer
+  // once that is stored
+  const C *f0 = fft_lines<TWO>(fb, c, T, ld, G.plan[0], tw);
+  if (col)
+    for (int x = xq; x < M0; x += 16)
+      field0[base + x * stride_x + tq] = cswap(f0[tq * ld + pix(x)]);
+  if constexpr (!TWO)
     __syncthreads();
-    C *fres = fft_lines<C>(fb, c, T, ld, G.plan[0], tw, true);
-    if (col)
-      for (int x = xq; x < M0; x += 16)
-        field0[field_stride * d + base + x * stride_x + tq] = fres[tq * ld + pix(x)];
-  }
+  const C *f1 = fft_lines<TWO>(res, fb, T, ld, G.plan[0], tw);
+  if (col)
+    for (int x = xq; x < M0; x += 16)
+      field0[field_stride + base + x * stride_x + tq] = cswap(f1[tq * ld + pix(x)]);
 }
 
-// ---- pass z, backward for the 3 field components -> real fields --------
-// Stride of a staged half row and size (elements) of the second buffer,
-// which holds either the FFT scratch lines or the 3 nl staged half rows.
-__host__ __device__ inline int z_inv_half_ld(int n) { return (n / 2 + 2) | 1; }
-__host__ __device__ inline int z_inv_b_size(int nl, int n) {
-  int const nc = nl + (nl + 1) / 2;
-  int const s1 = nc * line_ld(n), s2 = 3 * nl * z_inv_half_ld(n);
-  return s1 > s2 ? s1 : s2;
-}
-
+// ---- pass z, backward for 3 field components -> real fields -------------
+// Field component d of set blockIdx.y is array arr[3 set + d] times
+// k_z^pw[3 set + d].
+struct ZPass {
+  signed char arr[9], pw[9];
+};
+inline ZPass z_charge() { return ZPass{{0, 2, 3}, {0, 0, 1}}; }
 // Two real outputs per complex transform: slot l < nl carries Ex + i Ey of
 // line l, slot nl + j carries Ez of lines 2j and 2j+1.  Each half row is
 // extended by Hermitian symmetry with the imaginary parts of the k = 0 and
-// k = n/2 entries dropped (c2r semantics), so both packed outputs are real.
-// Shared memory: 2 x (nl + ceil(nl/2)) staged lines of line_ld(n),
-// twiddles (n).  FP32: four blocks per SM -- the block's load, transform and
-// store phases do not overlap, so the fourth resident block pays for the
-// spills of the 64-register bound.
-template <typename Real>
+// k = n/2 entries dropped (c2r semantics), so both packed outputs are real:
+// a thread reads entry k of the slot's two half rows and writes entries k and
+// n - k (real and imaginary parts swapped: a backward transform).
+// Set blockIdx.y writes the field mesh e_stride records further on.
+// Shared memory: nl + ceil(nl/2) staged lines of line_ld(n) (twice unless
+// TWO), twiddles (n).  FP32: four blocks per SM -- the block's load, transform
+// and store phases do not overlap, so the fourth resident block pays for the
+// 64-register bound.
+template <typename Real, bool TWO>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
 k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              const typename CplxOf<Real>::type *__restrict__ field0, long long field_stride,
-             Real *__restrict__ efield, const typename CplxOf<Real>::type *__restrict__ twtab,
-             int *__restrict__ err) {
+             ZPass const zp, int kscale, Real *__restrict__ efield, long long e_stride,
+             const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Blk const bk = blks[blockIdx.x];
@@ -736,83 +776,49 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const nz = (nl + 1) >> 1;
   int const nc = nl + nz;
   long long const line0 = bk.a;
-  // b doubles as the staging area of the 3 nl half rows (stride hl)
-  int const hl = z_inv_half_ld(n);
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = a + nc * ld;
-  C *tw = b + z_inv_b_size(nl, n);
+  C *b = TWO ? nullptr : a + nc * ld;
+  C *tw = a + (TWO ? 1 : 2) * nc * ld;
   load_twiddles(tw, twtab, G.plan[2]);
-  // stage the half rows of the 3 fields (field d, line l at
-  // sb[(d * nl + l) * hs]), then build the packed lines in a.  A field's nl
-  // rows are one contiguous range (row stride hp): one bulk copy (TMA
-  // engine) per field when the three fit in b, else plain loads (stride hl)
   const C *fsrc = field0 + G.km_off + line0 * G.hp;
-  __shared__ __align__(8) unsigned long long bar;
-  size_t const rb = static_cast<size_t>(nl) * G.hp * sizeof(C);
-  unsigned char *const bb = reinterpret_cast<unsigned char *>(b);
-  unsigned const pad = (16u - (smem_u32(bb) & 15u)) & 15u;
-  bool const bulk =
-      ((reinterpret_cast<uintptr_t>(fsrc) | static_cast<uintptr_t>(field_stride * sizeof(C))) &
-       15u) == 0 &&
-      rb % 16 == 0 && pad + 3 * rb <= z_inv_b_size(nl, n) * sizeof(C) && 3 * rb < (1u << 20);
-  C *sb = b;
-  int hs = hl;
-  if (bulk) {
-    sb = reinterpret_cast<C *>(bb + pad);
-    hs = G.hp;
-    if (threadIdx.x == 0) {
-      mbar_init(&bar, 1);
-      mbar_arrive_expect_tx(&bar, static_cast<unsigned>(3 * rb));
-      for (int d = 0; d < 3; ++d)
-        bulk_g2s(bb + pad + d * rb, fsrc + field_stride * d, static_cast<unsigned>(rb), &bar);
-    }
-    __syncthreads(); // barrier initialised before anyone waits on it
-    bool const ok = mbar_wait(&bar, 0);
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-        mbar_wait(&bar, 0); // second bounded wait for the copies in flight
-      }
-      return;
-    }
-  } else {
-    // row dl = d * nl + l of the three fields
-    for_lines(3 * nl, H, [&](int dl, int k) {
-      int const d = (dl >= 2 * nl) ? 2 : (dl >= nl ? 1 : 0), l = dl - d * nl;
-      b[dl * hl + k] = fsrc[field_stride * d + static_cast<long long>(l) * G.hp + k];
-    });
-    __syncthreads();
-  }
-  auto herm = [&](int d, int l, int k) -> C {
-    const C *row = sb + (d * nl + l) * hs;
-    if (k < H) {
-      C v = row[k];
-      if (k == 0 || 2 * k == n)
-        v.y = Real(0);
-      return v;
-    }
-    return cconj(row[n - k]);
-  };
-  for_lines(nc, n, [&](int j, int k) {
-    C X, Y;
-    if (j < nl) {
-      X = herm(0, j, k);
-      Y = herm(1, j, k);
+  int const set = 3 * blockIdx.y;
+  const C *fx = fsrc + field_stride * zp.arr[set], *fy = fsrc + field_stride * zp.arr[set + 1],
+          *fz = fsrc + field_stride * zp.arr[set + 2];
+  Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[2]) : Real(1);
+  int const px = zp.pw[set], py = zp.pw[set + 1], pz = zp.pw[set + 2];
+  float const rH = 1.0f / static_cast<float>(H);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nc * H; t += blockDim.x) {
+    int const j = qdiv(t, H, rH), k = t - j * H;
+    bool const xy = j < nl;
+    int const l0 = xy ? j : 2 * (j - nl), l1 = xy ? j : l0 + 1;
+    const C *r0 = (xy ? fx : fz) + static_cast<long long>(l0) * G.hp + k;
+    const C *r1 = (xy ? fy : fz) + static_cast<long long>(l1) * G.hp + k;
+    C X = *r0;
+    C Y = (l1 < nl) ? *r1 : C{Real(0), Real(0)};
+    int const p0 = xy ? px : pz, p1 = xy ? py : pz;
+    Real const kz = static_cast<Real>(freq_dop(k, n)) * ks;
+    Real const f0 = p0 == 0 ? Real(1) : (p0 == 2 ? kz * kz : kz);
+    Real const f1 = p1 == 0 ? Real(1) : (p1 == 2 ? kz * kz : kz);
+    X = C{f0 * X.x, f0 * X.y};
+    Y = C{f1 * Y.x, f1 * Y.y};
+    if (k == 0 || 2 * k == n) {
+      // swapped (X.x + i Y.x)
+      a[j * ld + pix(k)] = C{Y.x, X.x};
     } else {
-      int const l0 = 2 * (j - nl);
-      X = herm(2, l0, k);
-      Y = (l0 + 1 < nl) ? herm(2, l0 + 1, k) : C{Real(0), Real(0)};
+      // X + i Y at k, conj(X) + i conj(Y) at n - k, swapped
+      a[j * ld + pix(k)] = C{X.y + Y.x, X.x - Y.y};
+      a[j * ld + pix(n - k)] = C{Y.x - X.y, X.x + Y.y};
     }
-    a[j * ld + pix(k)] = C{X.x - Y.y, X.y + Y.x};
-  });
+  }
   __syncthreads();
-  C *res = fft_lines<C>(a, b, nc, ld, G.plan[2], tw, true);
+  const C *res = fft_lines<TWO>(a, b, nc, ld, G.plan[2], tw);
   // packed field mesh: one (Ex, Ey, Ez, 0) record per mesh point, so the
   // interpolation gathers one 16-byte (FP32) record per stencil point
   // (ghost-padded: every record also goes to its periodic images in the
   // high-side ghost layers of extent epad)
   using R4 = typename Real4Of<Real>::type;
-  R4 *out = reinterpret_cast<R4 *>(efield) + G.re_off;
+  R4 *out = reinterpret_cast<R4 *>(efield) + blockIdx.y * e_stride + G.re_off;
   int const M1 = G.mesh[1], M0 = G.mesh[0];
   int const P0 = G.epad[0], P1 = G.epad[1], P2 = G.epad[2];
   int const x0 = static_cast<int>(line0 / M1), y0 = static_cast<int>(line0 - static_cast<long long>(x0) * M1);
@@ -820,9 +826,9 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     C const xy = res[l * ld + pix(k)];
     C const zz = res[(nl + (l >> 1)) * ld + pix(k)];
     R4 v;
-    v.x = xy.x;
-    v.y = xy.y;
-    v.z = (l & 1) ? zz.y : zz.x;
+    v.x = xy.y; // swapped back
+    v.y = xy.x;
+    v.z = (l & 1) ? zz.x : zz.y;
     v.w = Real(0);
     int x = x0, y = y0 + l;
     while (y >= M1) {

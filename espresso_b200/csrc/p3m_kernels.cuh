@@ -685,9 +685,12 @@ __global__ void __launch_bounds__(32 * (1 + kInterpWarps), sizeof(Real) == 4 ? 2
 k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, int nbricks,
              const int *__restrict__ start, const int *__restrict__ perm,
              const int *__restrict__ s_key, const Real *__restrict__ W,
-             const Real *__restrict__ E, const CUtensorMap *__restrict__ tmaps,
+             const CUtensorMap *__restrict__ tmaps, int map_stride,
              const double *__restrict__ q, const double *__restrict__ dipole,
-             double *__restrict__ f, int overwrite, int *__restrict__ err) {
+             double *__restrict__ f, long long f_stride, int overwrite, int *__restrict__ err) {
+  // blockIdx.y: field set (tensor maps and outputs map_stride / f_stride apart)
+  tmaps += blockIdx.y * map_stride;
+  f += blockIdx.y * f_stride;
   static_assert(P <= 8, "one lane per stencil z offset");
   constexpr int R = 4;
   constexpr int WS = kRecStride;
