@@ -79,7 +79,7 @@ public:
     m_gf.ensure(E.m_cplx * rsz);
     long long const nprep = ceil_div(nn, 256);
     size_t const np = std::max<size_t>({static_cast<size_t>(E.m_n_blk_x), 5 * static_cast<size_t>(nprep),
-                                        static_cast<size_t>(E.m_n_blk_pair), size_t(kSumBlocks)});
+                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(), size_t(kSumBlocks)});
     m_part.ensure(np * sizeof(double));
     m_sums.ensure(8 * sizeof(double));
     m_flag.ensure(sizeof(int));
@@ -322,23 +322,33 @@ public:
       int const exact = accuracy > 5e-6 ? 0 : 1;
       RepGeom const *geom = E.m_geom_d.as<RepGeom>();
       // FP32-mesh mode: the pair terms in FP32 on the cell-relative offsets
+      int const lanes = E.pair_lanes();
       auto pairs = [&](auto ev, double *fo, double *part) {
         constexpr bool EV = decltype(ev)::value;
-        if (rel)
-          k_dp3m_pairs_rel<EV><<<E.m_n_blk_pair, 256, 0, st>>>(
-              geom, E.m_blk_pair.as<int2>(), E.m_spf.as<float4>(), m_smu.as<float4>(),
-              E.m_cperm.as<int>(), E.m_nb.as<int>(), E.m_nb_cnt.as<int>(), prefactor, exact, fo,
-              t, 0, part);
-        else
-          k_dp3m_pairs<EV><<<E.m_n_blk_pair, 256, 0, st>>>(
-              geom, E.m_blk_pair.as<int2>(), E.m_spq.as<double4>(), m_smu.as<double4>(),
-              E.m_cperm.as<int>(), E.m_nb.as<int>(), E.m_nb_cnt.as<int>(), prefactor, exact, fo,
-              t, 0, part);
+        auto go = [&](auto lpp) {
+          constexpr int LPP = decltype(lpp)::value;
+          if (rel)
+            k_dp3m_pairs_rel<EV, LPP><<<E.m_n_blk_pair * LPP, 256, 0, st>>>(
+                geom, E.m_blk_pair.as<int2>(), E.m_spf.as<float4>(), m_smu.as<float4>(),
+                E.m_cperm.as<int>(), E.m_nb.as<int>(), E.m_nb_cnt.as<int>(), prefactor, exact, fo,
+                t, 0, part);
+          else
+            k_dp3m_pairs<EV, LPP><<<E.m_n_blk_pair * LPP, 256, 0, st>>>(
+                geom, E.m_blk_pair.as<int2>(), E.m_spq.as<double4>(), m_smu.as<double4>(),
+                E.m_cperm.as<int>(), E.m_nb.as<int>(), E.m_nb_cnt.as<int>(), prefactor, exact, fo,
+                t, 0, part);
+        };
+        switch (lanes) {
+        case 1: go(std::integral_constant<int, 1>{}); break;
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
+        default: go(std::integral_constant<int, 8>{}); break;
+        }
         ++E.m_launches;
       };
       if (want_e) {
         pairs(std::true_type{}, want_ft ? f : nullptr, m_part.as<double>());
-        k_dp3m_sum_rows<<<1, 32 * 1, 0, st>>>(m_part.as<double>(), E.m_n_blk_pair, 1,
+        k_dp3m_sum_rows<<<1, 32 * 1, 0, st>>>(m_part.as<double>(), E.m_n_blk_pair * lanes, 1,
                                           m_sums.as<double>() + 6);
         ++E.m_launches;
       } else {

@@ -452,8 +452,42 @@ __global__ void k_dp3m_sort_mu(long long n, const int *__restrict__ perm,
 // the target accuracy is above 5e-6, else erfc itself.  The lists hold both
 // directions of every pair, so each particle sums its own force and torque
 // (no atomics, a fixed order: deterministic); the energy takes half of
-// every ordered pair.  One thread per cell-sorted particle.
-template <bool EV>
+// every ordered pair.  LPP lanes share a cell-sorted particle (whole groups
+// of 8 entries each, as k_pair_forces_rel): 16 384 dipoles fill the GPU only
+// with 8 lanes each.
+
+// Sums of the LPP lanes of a particle, its outputs (times pref; f may be
+// nullptr) and the block's energy partial.
+template <bool EV, int LPP>
+__device__ inline void dp_pairs_finish(double (&v)[6], double energy, double pref, bool active,
+                                       long long a, const int *__restrict__ perm,
+                                       double *__restrict__ f, double *__restrict__ tq,
+                                       int overwrite, double *__restrict__ partials) {
+#pragma unroll
+  for (int o = 1; o < LPP; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if (f && active && threadIdx.x % LPP == 0) {
+    int const i = perm[a];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (overwrite) {
+        f[3 * i + k] = pref * v[k];
+        tq[3 * i + k] = pref * v[3 + k];
+      } else {
+        f[3 * i + k] += pref * v[k];
+        tq[3 * i + k] += pref * v[3 + k];
+      }
+    }
+  }
+  if constexpr (EV) {
+    double const e[1] = {pref * energy};
+    block_halves<1>(e, 1, [](int) { return 0; }, partials);
+  }
+}
+
+template <bool EV, int LPP>
 __global__ void __launch_bounds__(256)
 k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
              const double4 *__restrict__ spq, const double4 *__restrict__ smu,
@@ -461,132 +495,133 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
              const int *__restrict__ nb_cnt, double pref, int exact_erfc,
              double *__restrict__ f, double *__restrict__ tq, int overwrite,
              double *__restrict__ partials) {
-  int2 const bk = blk[blockIdx.x];
+  int2 const bk = blk[blockIdx.x / LPP];
   RepGeom const &G = reps[bk.x];
-  long long const a = G.p0 + static_cast<long long>(bk.y) * blockDim.x + threadIdx.x;
+  int const sub = threadIdx.x % LPP;
+  long long const la = static_cast<long long>(bk.y) * 256 + (blockIdx.x % LPP) * (256 / LPP) +
+                       threadIdx.x / LPP;
+  bool const active = la < G.np;
+  long long const a = G.p0 + la;
   double energy = 0.0;
-  if (a < G.p0 + G.np) {
+  double s6[6] = {0, 0, 0, 0, 0, 0};
+  if (active) {
     double4 const pa = spq[a];
     double4 const ma = smu[a];
     double const alpha = G.alpha, rc = G.r_cut;
     double const coeff = 2.0 * alpha / sqrt(kPi);
     double const a2 = alpha * alpha;
-    double fx = 0, fy = 0, fz = 0, tx = 0, ty = 0, tz = 0;
     int const cw = nb_cnt[a];
-    int const cnt = nb_count(cw), cna = nb_count_a(cw);
-    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, a - G.p0);
-    int const base0 = static_cast<int>(G.p0);
+    int const ga = (nb_count_a(cw) + 7) >> 3, gt = ga + ((nb_count_b(cw) + 7) >> 3);
+    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, la);
+    int const ngroups = G.max_nb >> 3;
+    const double4 *pos = spq + G.p0, *mom = smu + G.p0;
+    auto group = [&](int v) {
+      int const grp = v < ga ? v : ngroups - 1 - (v - ga);
+      return nbp + (static_cast<long long>(grp) << 8);
+    };
     // the next partner's records are loaded while the current pair is
     // evaluated (two dependent gathers per entry otherwise serialise)
-    auto partner = [&](int k) {
-      return base0 + static_cast<int>(static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, k)]) &
-                                      kNbIndexMask);
-    };
-    int b_next = (cnt > 0) ? partner(0) : 0;
-    double4 p_next = (cnt > 0) ? spq[b_next] : pa;
-    double4 m_next = (cnt > 0) ? smu[b_next] : ma;
-    for (int k = 0; k < cnt; ++k) {
-      double4 const pb = p_next;
-      double4 const mb = m_next;
-      if (k + 1 < cnt) {
-        b_next = partner(k + 1);
-        p_next = spq[b_next];
-        m_next = smu[b_next];
+    const int *gp = (sub < gt) ? group(sub) : nbp;
+    unsigned b = (sub < gt) ? nb_index(static_cast<unsigned>(gp[0])) : 0u;
+    double4 p_next = (sub < gt) ? pos[b] : pa, m_next = (sub < gt) ? mom[b] : ma;
+    for (int v = sub; v < gt; v += LPP) {
+      const int *gn = (v + LPP < gt) ? group(v + LPP) : gp;
+      for (int u = 0; u < 8; ++u) {
+        double4 const pb = p_next;
+        double4 const mb = m_next;
+        b = nb_index(static_cast<unsigned>(u < 7 ? gp[u + 1] : gn[0]));
+        p_next = pos[b];
+        m_next = mom[b];
+        double const d0 = mi_d(pa.x - pb.x, G.box[0], G.box_i[0]);
+        double const d1 = mi_d(pa.y - pb.y, G.box[1], G.box_i[1]);
+        double const d2 = mi_d(pa.z - pb.z, G.box[2], G.box_i[2]);
+        double const r2 = d0 * d0 + d1 * d1 + d2 * d2;
+        if (!(r2 > 0.0))
+          continue;
+        double const inv_r = rsqrt(r2), r = r2 * inv_r;
+        if (!(r < rc))
+          continue;
+        double const inv_r2 = inv_r * inv_r;
+        double const ad = alpha * r;
+        double const exa = exp(-ad * ad);
+        double B;
+        if (exact_erfc) {
+          B = (erfc(ad) * inv_r + coeff * exa) * inv_r2;
+        } else {
+          double const t = rcp_newton(fma(0.3275911, ad, 1.0));
+          double const asp =
+              t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 +
+                                                                           t * 1.061405429))));
+          B = (asp * inv_r + coeff) * exa * inv_r2;
+        }
+        double const common = a2 * coeff * exa;
+        double const Cc = (3.0 * B + 2.0 * common) * inv_r2;
+        double const Dd = (5.0 * Cc + 4.0 * common * a2) * inv_r2;
+        double const mimj = ma.x * mb.x + ma.y * mb.y + ma.z * mb.z;
+        double const mir = ma.x * d0 + ma.y * d1 + ma.z * d2;
+        double const mjr = mb.x * d0 + mb.y * d1 + mb.z * d2;
+        if constexpr (EV)
+          energy += mimj * B - mir * mjr * Cc;
+        double const cd = mimj * Cc - mir * mjr * Dd;
+        double const s = mjr * Cc, q = mir * Cc;
+        s6[0] += cd * d0 + s * ma.x + q * mb.x;
+        s6[1] += cd * d1 + s * ma.y + q * mb.y;
+        s6[2] += cd * d2 + s * ma.z + q * mb.z;
+        // -mu_i x (B mu_j - s d)
+        double const w0 = s * d0 - B * mb.x, w1 = s * d1 - B * mb.y, w2 = s * d2 - B * mb.z;
+        s6[3] += ma.y * w2 - ma.z * w1;
+        s6[4] += ma.z * w0 - ma.x * w2;
+        s6[5] += ma.x * w1 - ma.y * w0;
       }
-      double const d0 = mi_d(pa.x - pb.x, G.box[0], G.box_i[0]);
-      double const d1 = mi_d(pa.y - pb.y, G.box[1], G.box_i[1]);
-      double const d2 = mi_d(pa.z - pb.z, G.box[2], G.box_i[2]);
-      double const r2 = d0 * d0 + d1 * d1 + d2 * d2;
-      double const r = sqrt(r2);
-      if (!(r < rc) || !(r > 0.0))
-        continue;
-      // one division for 1/r^2 (1/r = r / r^2) and one for the A&S t
-      double const inv_r2 = 1.0 / r2;
-      double const inv_r = r * inv_r2;
-      double const ad = alpha * r;
-      double const exa = exp(-ad * ad);
-      double B;
-      if (exact_erfc) {
-        B = (erfc(ad) * inv_r + coeff * exa) * inv_r2;
-      } else {
-        double const t = 1.0 / (1.0 + 0.3275911 * ad);
-        double const asp =
-            t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 +
-                                                                         t * 1.061405429))));
-        B = (asp * inv_r + coeff) * exa * inv_r2;
-      }
-      double const common = a2 * coeff * exa;
-      double const Cc = (3.0 * B + 2.0 * common) * inv_r2;
-      double const Dd = (5.0 * Cc + 4.0 * common * a2) * inv_r2;
-      double const mimj = ma.x * mb.x + ma.y * mb.y + ma.z * mb.z;
-      double const mir = ma.x * d0 + ma.y * d1 + ma.z * d2;
-      double const mjr = mb.x * d0 + mb.y * d1 + mb.z * d2;
-      if constexpr (EV)
-        energy += mimj * B - mir * mjr * Cc;
-      double const cd = mimj * Cc - mir * mjr * Dd;
-      fx += cd * d0 + mjr * Cc * ma.x + mir * Cc * mb.x;
-      fy += cd * d1 + mjr * Cc * ma.y + mir * Cc * mb.y;
-      fz += cd * d2 + mjr * Cc * ma.z + mir * Cc * mb.z;
-      double const s = mjr * Cc;
-      tx += -(ma.y * mb.z - ma.z * mb.y) * B + (ma.y * d2 - ma.z * d1) * s;
-      ty += -(ma.z * mb.x - ma.x * mb.z) * B + (ma.z * d0 - ma.x * d2) * s;
-      tz += -(ma.x * mb.y - ma.y * mb.x) * B + (ma.x * d1 - ma.y * d0) * s;
-    }
-    if (f) {
-      int const i = perm[a];
-      if (overwrite) {
-        f[3 * i] = pref * fx;
-        f[3 * i + 1] = pref * fy;
-        f[3 * i + 2] = pref * fz;
-        tq[3 * i] = pref * tx;
-        tq[3 * i + 1] = pref * ty;
-        tq[3 * i + 2] = pref * tz;
-      } else {
-        f[3 * i] += pref * fx;
-        f[3 * i + 1] += pref * fy;
-        f[3 * i + 2] += pref * fz;
-        tq[3 * i] += pref * tx;
-        tq[3 * i + 1] += pref * ty;
-        tq[3 * i + 2] += pref * tz;
-      }
+      gp = gn;
     }
   }
-  if constexpr (EV) {
-    __shared__ double red[8];
-    int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double v = 0.5 * pref * energy;
-    for (int o = 16; o > 0; o >>= 1)
-      v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0)
-      red[wid] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < (blockDim.x >> 5); ++w)
-        s += red[w];
-      partials[blockIdx.x] = s;
-    }
-  }
+  dp_pairs_finish<EV, LPP>(s6, energy, pref, active, a, perm, f, tq, overwrite, partials);
 }
+
+// Sum of FP32 terms in an unevaluated pair hi + lo (two-sum, Knuth: the
+// rounding error of every addition is exact and goes to lo), two sums at a
+// time: the precision of FP64 sums without six conversions and additions in
+// FP64 per pair.
+struct Sum2 {
+  f32x2 hi, lo;
+  __device__ void add(f32x2 v) {
+    f32x2 const s = add2(hi, v);
+    f32x2 const bb = sub2(s, hi);
+    f32x2 const e = add2(sub2(hi, sub2(s, bb)), sub2(v, bb));
+    hi = s;
+    lo = add2(lo, e);
+  }
+  __device__ void get(double &a, double &b) const {
+    float2 const h = up2(hi), l = up2(lo);
+    a = static_cast<double>(h.x) + static_cast<double>(l.x);
+    b = static_cast<double>(h.y) + static_cast<double>(l.y);
+  }
+};
 
 // The same pair terms for the FP32-mesh mode, in FP32 from the cell-relative
 // offsets (as k_pair_forces_rel: d = (off_a - off_b) - dc cs with dc from
 // the entry's offset code, no minimum-image arithmetic): hardware reciprocal
-// square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; each pair's force, torque and
-// energy terms summed in FP64.
-template <bool EV>
-__global__ void __launch_bounds__(256)
+// square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; each pair's force and
+// torque terms summed in FP32 pairs (Sum2), its energy in FP64.
+template <bool EV, int LPP>
+__global__ void __launch_bounds__(256, EV ? 1 : 3)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                  const float4 *__restrict__ spf, const float4 *__restrict__ smu,
                  const int *__restrict__ perm, const int *__restrict__ nb,
                  const int *__restrict__ nb_cnt, double pref, int exact_erfc,
                  double *__restrict__ f, double *__restrict__ tq, int overwrite,
                  double *__restrict__ partials) {
-  int2 const bk = blk[blockIdx.x];
+  int2 const bk = blk[blockIdx.x / LPP];
   RepGeom const &G = reps[bk.x];
-  long long const a = G.p0 + static_cast<long long>(bk.y) * blockDim.x + threadIdx.x;
+  int const sub = threadIdx.x % LPP;
+  long long const la = static_cast<long long>(bk.y) * 256 + (blockIdx.x % LPP) * (256 / LPP) +
+                       threadIdx.x / LPP;
+  bool const active = la < G.np;
+  long long const a = G.p0 + la;
   double energy = 0.0;
-  if (a < G.p0 + G.np) {
+  double s6[6] = {0, 0, 0, 0, 0, 0};
+  if (active) {
     float4 const pa = spf[a];
     float4 const ma = smu[a];
     float const alpha = static_cast<float>(G.alpha);
@@ -595,104 +630,77 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
     float const a2 = static_cast<float>(G.alpha * G.alpha);
     // exp(-(alpha r)^2) = 2^(c_exp r^2)
     float const c_exp = static_cast<float>(-G.alpha * G.alpha * 1.4426950408889634);
-    float const cs_x = static_cast<float>(G.box[0] / G.cg[0]);
-    float const cs_y = static_cast<float>(G.box[1] / G.cg[1]);
-    float const cs_z = static_cast<float>(G.box[2] / G.cg[2]);
-    double fx = 0, fy = 0, fz = 0, tx = 0, ty = 0, tz = 0;
+    float const ncs_x = -static_cast<float>(G.box[0] / G.cg[0]);
+    float const ncs_y = -0.25f * static_cast<float>(G.box[1] / G.cg[1]);
+    float const ncs_z = -0.0625f * static_cast<float>(G.box[2] / G.cg[2]);
+    Sum2 s01{0, 0}, s23{0, 0}, s45{0, 0};
     int const cw = nb_cnt[a];
-    int const cnt = nb_count(cw), cna = nb_count_a(cw);
-    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, a - G.p0);
-    long long const base0 = G.p0;
-    auto entry = [&](int k) {
-      return static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, k)]);
-    };
-    // the next partner's records are loaded while the current pair is
-    // evaluated
-    unsigned e_next = (cnt > 0) ? entry(0) : 0u;
-    float4 p_next = (cnt > 0) ? spf[base0 + (e_next & kNbIndexMask)] : pa;
-    float4 m_next = (cnt > 0) ? smu[base0 + (e_next & kNbIndexMask)] : ma;
-    for (int k = 0; k < cnt; ++k) {
-      unsigned const e = e_next;
-      float4 const pb = p_next;
-      float4 const mb = m_next;
-      if (k + 1 < cnt) {
-        e_next = entry(k + 1);
-        p_next = spf[base0 + (e_next & kNbIndexMask)];
-        m_next = smu[base0 + (e_next & kNbIndexMask)];
-      }
-      unsigned const code = e >> kNbIndexBits;
-      float const d0 = fmaf(code_axis(code, 0), -cs_x, pa.x - pb.x);
-      float const d1 = fmaf(code_axis(code, 1), -cs_y, pa.y - pb.y);
-      float const d2 = fmaf(code_axis(code, 2), -cs_z, pa.z - pb.z);
-      float const r2 = d0 * d0 + d1 * d1 + d2 * d2;
-      if (!(r2 < rc2) || !(r2 > 0.f))
-        continue;
-      float const inv_r = rsqrt_approx(r2);
-      float const inv_r2 = inv_r * inv_r;
-      float const ad = alpha * (r2 * inv_r);
-      float const exa = ex2_approx(c_exp * r2);
-      float B;
-      if (exact_erfc) {
-        B = (erfcf(ad) * inv_r + coeff * exa) * inv_r2;
-      } else {
-        float const t = rcp_r(1.f + 0.3275911f * ad);
-        float const asp =
-            t * (0.254829592f + t * (-0.284496736f + t * (1.421413741f + t * (-1.453152027f +
-                                                                           t * 1.061405429f))));
-        B = (asp * inv_r + coeff) * exa * inv_r2;
-      }
-      float const common = a2 * coeff * exa;
-      float const Cc = (3.f * B + 2.f * common) * inv_r2;
-      float const Dd = (5.f * Cc + 4.f * common * a2) * inv_r2;
-      float const mimj = ma.x * mb.x + ma.y * mb.y + ma.z * mb.z;
-      float const mir = ma.x * d0 + ma.y * d1 + ma.z * d2;
-      float const mjr = mb.x * d0 + mb.y * d1 + mb.z * d2;
-      if constexpr (EV)
-        energy += static_cast<double>(mimj * B - mir * mjr * Cc);
-      float const cd = mimj * Cc - mir * mjr * Dd;
-      fx += static_cast<double>(cd * d0 + mjr * Cc * ma.x + mir * Cc * mb.x);
-      fy += static_cast<double>(cd * d1 + mjr * Cc * ma.y + mir * Cc * mb.y);
-      fz += static_cast<double>(cd * d2 + mjr * Cc * ma.z + mir * Cc * mb.z);
-      float const s = mjr * Cc;
-      tx += static_cast<double>(-(ma.y * mb.z - ma.z * mb.y) * B + (ma.y * d2 - ma.z * d1) * s);
-      ty += static_cast<double>(-(ma.z * mb.x - ma.x * mb.z) * B + (ma.z * d0 - ma.x * d2) * s);
-      tz += static_cast<double>(-(ma.x * mb.y - ma.y * mb.x) * B + (ma.x * d1 - ma.y * d0) * s);
-    }
-    if (f) {
-      int const i = perm[a];
-      if (overwrite) {
-        f[3 * i] = pref * fx;
-        f[3 * i + 1] = pref * fy;
-        f[3 * i + 2] = pref * fz;
-        tq[3 * i] = pref * tx;
-        tq[3 * i + 1] = pref * ty;
-        tq[3 * i + 2] = pref * tz;
-      } else {
-        f[3 * i] += pref * fx;
-        f[3 * i + 1] += pref * fy;
-        f[3 * i + 2] += pref * fz;
-        tq[3 * i] += pref * tx;
-        tq[3 * i + 1] += pref * ty;
-        tq[3 * i + 2] += pref * tz;
+    int const ga = (nb_count_a(cw) + 7) >> 3, gt = ga + ((nb_count_b(cw) + 7) >> 3);
+    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, la);
+    int const ngroups = G.max_nb >> 3;
+    const float4 *pos = spf + G.p0, *mom = smu + G.p0;
+    for (int v = sub; v < gt; v += LPP) {
+      int const grp = v < ga ? v : ngroups - 1 - (v - ga);
+      const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
+      int4 const g0 = gp[0], g1 = gp[1];
+      unsigned const ent[8] = {static_cast<unsigned>(g0.x), static_cast<unsigned>(g0.y),
+                               static_cast<unsigned>(g0.z), static_cast<unsigned>(g0.w),
+                               static_cast<unsigned>(g1.x), static_cast<unsigned>(g1.y),
+                               static_cast<unsigned>(g1.z), static_cast<unsigned>(g1.w)};
+#pragma unroll
+      for (int h = 0; h < 8; h += 2) {
+        float4 pv[2], mv[2]; // four gathers in flight
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          pv[u] = pos[nb_index(ent[h + u])];
+          mv[u] = mom[nb_index(ent[h + u])];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          unsigned const e = ent[h + u];
+          float4 const pb = pv[u], mb = mv[u];
+          float const d0 = fmaf(code_axis(e, 0), ncs_x, pa.x - pb.x);
+          float const d1 = fmaf(code_axis(e, 1), ncs_y, pa.y - pb.y);
+          float const d2 = fmaf(code_axis(e, 2), ncs_z, pa.z - pb.z);
+          float const r2 = d0 * d0 + d1 * d1 + d2 * d2;
+          if (!(r2 < rc2) || !(r2 > 0.f))
+            continue;
+          float const inv_r = rsqrt_approx(r2);
+          float const inv_r2 = inv_r * inv_r;
+          float const ad = alpha * (r2 * inv_r);
+          float const exa = ex2_approx(c_exp * r2);
+          float B;
+          if (exact_erfc) {
+            B = (erfcf(ad) * inv_r + coeff * exa) * inv_r2;
+          } else {
+            float const t = rcp_r(1.f + 0.3275911f * ad);
+            float const asp =
+                t * (0.254829592f + t * (-0.284496736f + t * (1.421413741f + t * (-1.453152027f +
+                                                                               t * 1.061405429f))));
+            B = (asp * inv_r + coeff) * exa * inv_r2;
+          }
+          float const common = a2 * coeff * exa;
+          float const Cc = (3.f * B + 2.f * common) * inv_r2;
+          float const Dd = (5.f * Cc + 4.f * common * a2) * inv_r2;
+          float const mimj = ma.x * mb.x + ma.y * mb.y + ma.z * mb.z;
+          float const mir = ma.x * d0 + ma.y * d1 + ma.z * d2;
+          float const mjr = mb.x * d0 + mb.y * d1 + mb.z * d2;
+          if constexpr (EV)
+            energy += static_cast<double>(mimj * B - mir * mjr * Cc);
+          float const cd = mimj * Cc - mir * mjr * Dd;
+          float const s = mjr * Cc, q = mir * Cc;
+          float const w0 = s * d0 - B * mb.x, w1 = s * d1 - B * mb.y, w2 = s * d2 - B * mb.z;
+          s01.add(pk2(cd * d0 + s * ma.x + q * mb.x, cd * d1 + s * ma.y + q * mb.y));
+          s23.add(pk2(cd * d2 + s * ma.z + q * mb.z, ma.y * w2 - ma.z * w1));
+          s45.add(pk2(ma.z * w0 - ma.x * w2, ma.x * w1 - ma.y * w0));
+        }
       }
     }
+    s01.get(s6[0], s6[1]);
+    s23.get(s6[2], s6[3]);
+    s45.get(s6[4], s6[5]);
   }
-  if constexpr (EV) {
-    __shared__ double red[8];
-    int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double v = 0.5 * pref * energy;
-    for (int o = 16; o > 0; o >>= 1)
-      v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0)
-      red[wid] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < (blockDim.x >> 5); ++w)
-        s += red[w];
-      partials[blockIdx.x] = s;
-    }
-  }
+  dp_pairs_finish<EV, LPP>(s6, energy, pref, active, a, perm, f, tq, overwrite, partials);
 }
 
 } // namespace p3mx

@@ -132,6 +132,9 @@ template <typename T> void upload_vec(DevBuf &b, std::vector<T> const &v, cudaSt
 Engine::Engine(bool fp32) : m_fp32(fp32) {
   P3MX_CUDA(cudaStreamCreateWithFlags(&m_stream, cudaStreamNonBlocking));
   m_ia.assign(1, PairIA{0, 0, 0, 0, 0, 0, 0, 0, 0, -1.0});
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&m_sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
 Engine::~Engine() {
@@ -259,12 +262,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     if (G.np >= (1LL << kNbIndexBits))
       throw Error(1, "a replica holds more than 2^26 particles (Verlet list index limit)");
   cudaStream_t st = m_stream;
-  int sms = 148;
-  {
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess)
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
+  int const sms = m_sms;
   {
     std::vector<typename CplxOf<double>::type> t64(tw.size());
     for (size_t k = 0; k < tw.size(); ++k)
@@ -560,7 +558,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   }
   m_pos_ref.ensure(3 * n * sizeof(double));
   m_type_ref.ensure(n * sizeof(int));
-  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * 20 * sizeof(double));
+  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes() * 20 * sizeof(double));
   m_sums_pair.ensure(static_cast<size_t>(R) * 20 * sizeof(double));
   if (m_ia_d.p == nullptr)
     upload_vec(m_ia_d, m_ia, st);
@@ -593,9 +591,9 @@ void Engine::census(cudaStream_t st) {
   int const R = n_rep();
   k_census<<<m_n_blk_census, 256, 0, st>>>(m_blk_census.as<int2>(), m_geom_d.as<RepGeom>(),
                                            d_pos(), d_q(), m_part_census.as<double>()); ++m_launches;
-  k_reduce_partials<<<ceil_div(R, 128), 128, 0, st>>>(m_part_census.as<double>(), 6,
-                                                      m_blk_census_start_d.as<int>(), R,
-                                                      m_sums_census.as<double>()); ++m_launches;
+  k_reduce_partials<<<dim3(R, 6), 256, 0, st>>>(m_part_census.as<double>(), 6,
+                                                m_blk_census_start_d.as<int>(), 1,
+                                                m_sums_census.as<double>()); ++m_launches;
   m_census_h.assign(static_cast<size_t>(R) * 6, 0.0);
   P3MX_CUDA(cudaMemcpyAsync(m_census_h.data(), m_sums_census.p, R * 6 * sizeof(double),
                             cudaMemcpyDeviceToHost, st));
@@ -788,9 +786,9 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   }
   ++m_launches;
   if (want_ev) {
-    k_reduce_partials<<<ceil_div(R, 128), 128, 0, st>>>(m_part_x.as<double>(), 8,
-                                                        m_blk_x_start_d.as<int>(), R,
-                                                        m_sums_x.as<double>());
+    k_reduce_partials<<<dim3(R, 8), 256, 0, st>>>(m_part_x.as<double>(), 8,
+                                                  m_blk_x_start_d.as<int>(), 1,
+                                                  m_sums_x.as<double>());
     ++m_launches;
   }
   mark("fft_x_kspace", st);
@@ -1052,41 +1050,70 @@ void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp,
   ++m_launches;
 }
 
+// Lanes per particle of the pair kernels: lists are split over 1, 2, 4 or 8
+// lanes until the launch fills the GPU (kPairFill threads per SM).
+int Engine::pair_lanes() const {
+  int l = 1;
+  while (l < 8 && m_n * l < static_cast<long long>(m_sms) * kPairFill)
+    l *= 2;
+  return l;
+}
+
 template <typename Real>
 void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t st) {
   RepGeom const *geom = m_geom_d.as<RepGeom>();
-  size_t const smem = static_cast<size_t>(m_ntypes) * m_ntypes * sizeof(PairIA);
+  int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes();
+  auto go = [&](auto kern, auto const *pos, size_t smem) {
+    kern<<<m_n_blk_pair * lanes, 256, smem, st>>>(
+        geom, m_blk_pair.as<int2>(), pos, m_stype.as<int>(), m_cperm.as<int>(),
+        m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(), m_nb_cnt.as<int>(), f, overwrite ? 1 : 0,
+        m_part_pair.as<double>());
+    ++m_launches;
+  };
+  size_t const nt2 = static_cast<size_t>(m_ntypes) * m_ntypes;
   if constexpr (sizeof(Real) == 4) {
     // FP32-mixed: cell-relative FP32 geometry
-    if (want_ev)
-      k_pair_forces_rel<true><<<m_n_blk_pair, 256, smem, st>>>(
-          geom, m_blk_pair.as<int2>(), m_spf.as<float4>(), m_stype.as<int>(), m_cperm.as<int>(),
-          m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(), m_nb_cnt.as<int>(), f,
-          overwrite ? 1 : 0, m_part_pair.as<double>());
-    else if (m_ntypes == 1 && m_ia[0].ia_cut != -1.0 && m_ia[0].lj_offset == 0.0)
-      k_pair_forces_rel<false, true><<<m_n_blk_pair, 256, smem, st>>>(
-          geom, m_blk_pair.as<int2>(), m_spf.as<float4>(), m_stype.as<int>(), m_cperm.as<int>(),
-          m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(), m_nb_cnt.as<int>(), f,
-          overwrite ? 1 : 0, m_part_pair.as<double>());
+    const float4 *pos = m_spf.as<float4>();
+    if (want_ev) {
+      go(k_pair_forces_rel_ev, pos, nt2 * sizeof(PairIA));
+      return;
+    }
+    bool offset = false;
+    for (auto const &p : m_ia)
+      offset = offset || (p.ia_cut != -1.0 && p.lj_offset != 0.0);
+    size_t const smem = nt2 * sizeof(PairF);
+    auto mode = [&](auto m) {
+      constexpr int M = decltype(m)::value;
+      switch (lanes) {
+      case 1: go(k_pair_forces_rel<M, 1>, pos, smem); break;
+      case 2: go(k_pair_forces_rel<M, 2>, pos, smem); break;
+      case 4: go(k_pair_forces_rel<M, 4>, pos, smem); break;
+      default: go(k_pair_forces_rel<M, 8>, pos, smem); break;
+      }
+    };
+    if (offset)
+      mode(std::integral_constant<int, kPairOffset>{});
+    else if (m_ntypes == 1)
+      mode(std::integral_constant<int, kPairOneType>{});
     else
-      k_pair_forces_rel<false><<<m_n_blk_pair, 256, smem, st>>>(
-          geom, m_blk_pair.as<int2>(), m_spf.as<float4>(), m_stype.as<int>(), m_cperm.as<int>(),
-          m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(), m_nb_cnt.as<int>(), f,
-          overwrite ? 1 : 0, m_part_pair.as<double>());
-    ++m_launches;
+      mode(std::integral_constant<int, kPairTypes>{});
   } else {
     // FP64: FP64 geometry (minimum image on absolute positions)
+    const double4 *pos = m_spq.as<double4>();
+    size_t const smem = nt2 * sizeof(PairIA);
+    auto ev = [&](auto e) {
+      constexpr bool EV = decltype(e)::value;
+      switch (lanes) {
+      case 1: go(k_pair_forces<EV, 1>, pos, smem); break;
+      case 2: go(k_pair_forces<EV, 2>, pos, smem); break;
+      case 4: go(k_pair_forces<EV, 4>, pos, smem); break;
+      default: go(k_pair_forces<EV, 8>, pos, smem); break;
+      }
+    };
     if (want_ev)
-      k_pair_forces<Real, true><<<m_n_blk_pair, 256, smem, st>>>(
-          geom, m_blk_pair.as<int2>(), m_spq.as<double4>(), m_stype.as<int>(), m_cperm.as<int>(),
-          m_ia_d.as<PairIA>(), m_ntypes, m_n, m_nb.as<int>(), m_nb_cnt.as<int>(), f,
-          overwrite ? 1 : 0, m_part_pair.as<double>());
+      ev(std::true_type{});
     else
-      k_pair_forces<Real, false><<<m_n_blk_pair, 256, smem, st>>>(
-          geom, m_blk_pair.as<int2>(), m_spq.as<double4>(), m_stype.as<int>(), m_cperm.as<int>(),
-          m_ia_d.as<PairIA>(), m_ntypes, m_n, m_nb.as<int>(), m_nb_cnt.as<int>(), f,
-          overwrite ? 1 : 0, m_part_pair.as<double>());
-    ++m_launches;
+      ev(std::false_type{});
   }
 }
 
@@ -1140,9 +1167,11 @@ void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t s
   P3MX_CUDA(cudaGetLastError());
   if (want_ev && m_n > 0) {
     int const R = n_rep();
-    k_reduce_partials<<<ceil_div(R, 128), 128, 0, st>>>(m_part_pair.as<double>(), 20,
-                                                        m_blk_pair_start_d.as<int>(), R,
-                                                        m_sums_pair.as<double>()); ++m_launches;
+    bool const one = m_fp32 && !fp64_math;
+    k_reduce_partials<<<dim3(R, 20), 256, 0, st>>>(m_part_pair.as<double>(), 20,
+                                                   m_blk_pair_start_d.as<int>(),
+                                                   one ? 1 : pair_lanes(),
+                                                   m_sums_pair.as<double>()); ++m_launches;
     std::vector<double> sums(static_cast<size_t>(R) * 20);
     P3MX_CUDA(cudaMemcpyAsync(sums.data(), m_sums_pair.p, sums.size() * sizeof(double),
                               cudaMemcpyDeviceToHost, st));
@@ -1291,7 +1320,7 @@ std::vector<int> Engine::verlet_pairs(cudaStream_t st) {
       for (int k = 0; k < nb_count(cnt[a]); ++k) {
         unsigned const ent = static_cast<unsigned>(
             nbh[nb_logical(nb_base(G.nb_off, G.max_nb, a - G.p0), G.max_nb, nb_count_a(cnt[a]), k)]);
-        int const b = static_cast<int>(G.p0 + (ent & kNbIndexMask));
+        int const b = static_cast<int>(G.p0 + nb_index(ent));
         int const i = perm[a], j = perm[b];
         if (i < j) {
           pairs.push_back(i);
@@ -1468,8 +1497,7 @@ k_elc_image_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
         elc_p3m_pair(G, dl * qa * qa, d, F, E);
         for (int k = 0; k < cnt; ++k) {
           long long const b =
-              G.p0 + static_cast<long long>(static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, k)]) &
-                                            kNbIndexMask);
+              G.p0 + nb_index(static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, k)]));
           int const j = perm[b];
           double const qb = qv[j];
           if (qb == 0.0)

@@ -182,7 +182,11 @@ private:
 
   void mark(const char *name, cudaStream_t st);
 
+  // lanes per particle of the pair kernels for the current particle number
+  int pair_lanes() const;
+
   bool m_fp32;
+  int m_sms = 148;
   cudaStream_t m_stream = nullptr;
   long long m_launches = 0;
   bool m_profiling = false;

@@ -999,18 +999,29 @@ __global__ void k_census(const int2 *__restrict__ blk, const RepGeom *__restrict
   }
 }
 
-// Sum per-block partials of each replica in block order (deterministic).
-__global__ void k_reduce_partials(const double *__restrict__ partials, int width,
-                                  const int *__restrict__ blk_start, int n_rep,
-                                  double *__restrict__ out) {
-  int const r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_rep)
-    return;
-  for (int k = 0; k < width; ++k) {
-    double s = 0.0;
-    for (int b = blk_start[r]; b < blk_start[r + 1]; ++b)
-      s += partials[static_cast<long long>(b) * width + k];
-    out[static_cast<long long>(r) * width + k] = s;
+// Sum per-block partials of replica blockIdx.x, column blockIdx.y (width
+// columns; `per` rows per table block): thread t adds rows t, t + 256, ..., then
+// a fixed shuffle tree and the warps in order (deterministic; one thread per
+// replica walking all rows and columns took 70 us for 235 rows of 20).
+__global__ void __launch_bounds__(256)
+k_reduce_partials(const double *__restrict__ partials, int width,
+                  const int *__restrict__ blk_start, int per, double *__restrict__ out) {
+  int const r = blockIdx.x, k = blockIdx.y;
+  int const b0 = blk_start[r] * per, b1 = blk_start[r + 1] * per;
+  double s = 0.0;
+  for (int b = b0 + static_cast<int>(threadIdx.x); b < b1; b += 256)
+    s += partials[static_cast<long long>(b) * width + k];
+  for (int o = 16; o > 0; o >>= 1)
+    s += __shfl_down_sync(0xffffffffu, s, o);
+  __shared__ double red[8];
+  if ((threadIdx.x & 31) == 0)
+    red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w)
+      t += red[w];
+    out[static_cast<long long>(r) * width + k] = t;
   }
 }
 

@@ -139,19 +139,25 @@ __device__ inline double mi_d(double dx, double L, double Li) {
 // (cap, the per-replica capacity, a multiple of 8).  The build writes whole
 // groups with vector stores and the pair kernels read whole groups with
 // vector loads.  An entry packs the partner's index inside the replica
-// (26 bits) and its cell offset code (cell_offset_code, 6 bits).
+// (upper 26 bits) and its cell offset code (cell_offset_code, lower 6 bits:
+// one mask-and-or turns a field into an FP32 value).  The entries behind the
+// last of a group's are the particle itself with dc = 0.
 constexpr int kNbIndexBits = 26;
-constexpr unsigned kNbIndexMask = (1u << kNbIndexBits) - 1u;
+constexpr int kNbCodeBits = 6;
+__host__ __device__ constexpr unsigned nb_index(unsigned e) { return e >> kNbCodeBits; }
+__host__ __device__ constexpr unsigned nb_pack(unsigned index, int code) {
+  return (index << kNbCodeBits) | static_cast<unsigned>(code);
+}
 // Cell offset code of an entry: the partner image's cell offset dc (each
-// axis -1, 0 or +1) as three 2-bit fields dc + 1 (x lowest), in the 6 bits
-// above the index.
+// axis -1, 0 or +1) as three 2-bit fields dc + 1 (x lowest).
 __host__ __device__ constexpr int cell_offset_code(int dx, int dy, int dz) {
   return (dx + 1) | ((dy + 1) << 2) | ((dz + 1) << 4);
 }
-// dc of axis d from a code, as an FP32 value (exact: 2^23 + field, minus
-// 2^23 + 1)
-__device__ inline float code_axis(unsigned code, int d) {
-  return __uint_as_float(0x4B000000u | ((code >> (2 * d)) & 3u)) - 8388609.0f;
+// 4^d dc of axis d from an entry, as an FP32 value (exact: 2^23 + field,
+// minus 2^23 + 4^d)
+__device__ inline float code_axis(unsigned e, int d) {
+  return __uint_as_float(0x4B000000u | (e & (3u << (2 * d)))) -
+         (8388608.0f + static_cast<float>(1 << (2 * d)));
 }
 // First entry (group 0) of local particle la; group g at + g * 256.
 __host__ __device__ inline long long nb_base(long long nb_off, int cap, long long la) {
@@ -256,8 +262,7 @@ __device__ inline void verlet_build_one(long long a, const RepGeom *__restrict__
                       ((cls_a ? (na & 7) : (nb_b & 7)) != 0 ||
                        ((na + 7) >> 3) + ((nb_b + 7) >> 3) + 1 <= ngroups);
     if (room) {
-      int const ent = static_cast<int>(static_cast<unsigned>(b - G.p0) |
-                                       (static_cast<unsigned>(code) << kNbIndexBits));
+      int const ent = static_cast<int>(nb_pack(static_cast<unsigned>(b - G.p0), code));
       if (cls_a) {
         int const slot = na & 7;
         gbuf[slot] = ent;
@@ -420,7 +425,14 @@ __device__ inline void verlet_build_one(long long a, const RepGeom *__restrict__
       }
     }
   }
-  // last partial groups (entries beyond the counts are never read)
+  // last partial groups, filled up with the particle itself (zero distance:
+  // no term of a pair kernel passes its range test)
+  int const self = static_cast<int>(
+      nb_pack(static_cast<unsigned>(a - G.p0), cell_offset_code(0, 0, 0)));
+  for (int k = na & 7; k != 0 && k < 8; ++k)
+    gbuf[k] = self;
+  for (int k = nb_b & 7; k != 0 && k < 8; ++k)
+    gbuf_b[k] = self;
   if (na & 7)
     store_group(nbp + (static_cast<long long>(na >> 3) << 8), gbuf);
   if (nb_b & 7)
@@ -563,25 +575,6 @@ __device__ inline void lj_wca_sel(PairR<float> const &p, float dist, float inv_d
   }
 }
 
-// Branch-free LJ + WCA for pairs without an LJ offset (r_off = r, so the
-// LJ powers come from the same 1/r^2 as WCA's): one reciprocal square root
-// serves every term.  in_lj / in_wca select the terms by range.
-__device__ inline void lj_wca_sel_nooff(PairR<float> const &p, float dist, float inv_d2,
-                                        float &fn) {
-  {
-    float const s2 = (p.lsig * p.lsig) * inv_d2;
-    float const f6 = s2 * s2 * s2;
-    bool const in = dist < p.lcut && dist > p.lmin;
-    fn += in ? 48.f * p.leps * f6 * (f6 - 0.5f) * inv_d2 : 0.f;
-  }
-  if (p.wcut > 0.f) {
-    float const s2 = (p.wsig * p.wsig) * inv_d2;
-    float const f6 = s2 * s2 * s2;
-    bool const in = dist < p.wcut;
-    fn += in ? 48.f * p.weps * f6 * (f6 - 0.5f) * inv_d2 : 0.f;
-  }
-}
-
 // 2^x, hardware approximation (ex2.approx, relative error ~2^-22).
 __device__ inline float ex2_approx(float x) {
   float e;
@@ -609,55 +602,115 @@ __device__ inline float rsqrt_approx(float x) {
   return r;
 }
 
-// Pair kernel over the Verlet list: real-space Coulomb
-// (CoulombP3M::pair_force / pair_energy, p3m.hpp:146-180) plus LJ and WCA
-// (lj.hpp:41-60, wca.hpp:39-55).  Minimum-image difference in FP64, pair
-// arithmetic in Real, per-particle accumulation in FP64 (no atomics: each
-// particle owns its force, full list).  EV adds energies and virials: each
-// pair is seen from both ends, so per-particle sums are halved; per-block
-// FP64 partials {E_coul, E_nb, Vc[9], Vn[9]} (width 20).  Blocks map to
-// replicas through the block table so partials never straddle replicas.
-// Neighbour loads are issued two entries ahead of their use.
-// FP32-mixed real-space kernel over the same Verlet lists: positions are
-// FP32 offsets from each particle's build-time cell corner (cell_offset), the
-// list stores every partner's cell offset code, so
+// Two FP32 values in one register pair and their packed arithmetic (one
+// instruction for both, each half rounded as the scalar operation).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 up2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  return fma2(b, pk2(-1.0f, -1.0f), a); // exact product: one rounding
+}
+
+// Reciprocal in FP64 from the FP32 approximation by one third-order step
+// (y (1 + e + e^2), e = 1 - x y ~ 2^-22: relative error below 2^-52); x of
+// FP32's normal range (1 + p alpha r here).
+__device__ inline double rcp_newton(double x) {
+  double const y = static_cast<double>(rcp_r<float>(static_cast<float>(x)));
+  double const e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// LJ / WCA parameters of a type pair for the FP32 force kernel; ranges of an
+// inactive pair are empty (-1).
+struct __align__(16) PairF {
+  float lcut, lmin, lsig, le48, wcut, wsig, we48, loff;
+};
+__device__ inline PairF pair_f(PairIA const &p) {
+  bool const on = p.ia_cut != -1.0;
+  PairF r;
+  r.lcut = on ? static_cast<float>(p.lj_cut + p.lj_offset) : -1.f;
+  r.lmin = static_cast<float>(p.lj_min + p.lj_offset);
+  r.lsig = static_cast<float>(p.lj_sig);
+  r.le48 = 48.f * static_cast<float>(p.lj_eps);
+  r.wcut = on ? static_cast<float>(p.wca_cut) : -1.f;
+  r.wsig = static_cast<float>(p.wca_sig);
+  r.we48 = 48.f * static_cast<float>(p.wca_eps);
+  r.loff = static_cast<float>(p.lj_offset);
+  return r;
+}
+// Parameter modes of the FP32 force kernel: one type without LJ offset
+// (parameters in registers, the LJ powers from the Coulomb term's 1/r^2),
+// several types without offsets, LJ offsets.
+constexpr int kPairOneType = 0, kPairTypes = 1, kPairOffset = 2;
+// Threads per SM at which a pair launch counts as filling the GPU.  Below,
+// each particle's list is split over up to 8 lanes, whole groups of 8
+// entries each: 12 000 ions 25 -> 10 us, 131 072 ions are the faster the
+// fewer lanes.
+constexpr int kPairFill = 768;
+
+// Force kernel of the FP32-mixed path over the Verlet list: real-space Coulomb
+// (CoulombP3M::pair_force, p3m.hpp:146-180) plus LJ and WCA (lj.hpp:41-60,
+// wca.hpp:39-55).  Positions are FP32 offsets from each particle's build-time
+// cell corner (cell_offset), the list stores every partner's cell offset
+// code, so
 //   d = x_a - x_b' = (off_a - off_b) - dc * cs
 // is formed in FP32 from small numbers (no minimum-image arithmetic, 16-byte
-// gathers); the geometry error is about one ulp of the cell size.  Pair
-// physics as k_pair_forces; per-particle force sums are FP32 over runs of 8
-// partners and FP64 across runs.
-// NOOFF: one particle type whose LJ has no offset (the host checks), so the
-// LJ and WCA powers use the Coulomb term's 1/r^2 (lj_wca_sel_nooff).
-template <bool EV, bool NOOFF = false>
-__global__ void __launch_bounds__(256, EV ? 1 : 4)
+// gathers); the geometry error is about one ulp of the cell size.
+// LPP lanes share a particle (lane `sub` takes the list groups sub, sub + LPP,
+// ...); no atomics: each particle owns its force (full list), lane sums meet
+// in a fixed shuffle order.  Per-particle sums are FP32 over the 8 entries of
+// a group and FP64 across groups.
+// Bound by instruction issue (about 45 scalar instructions per entry and
+// three MUFU operations): the range-independent arithmetic runs on two
+// entries at a time in packed FP32, with the scalar code's roundings.
+template <int MODE, int LPP>
+__global__ void __launch_bounds__(256, 4)
 k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                   const float4 *__restrict__ spf, const int *__restrict__ stype,
                   const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
                   const int *__restrict__ nb, const int *__restrict__ nb_cnt,
-                  double *__restrict__ f, int overwrite,
-                  double *__restrict__ partials) {
-  using Real = float;
+                  double *__restrict__ f, int overwrite, double *__restrict__) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  PairIA *ia = reinterpret_cast<PairIA *>(smem_raw);
+  PairF *ia = reinterpret_cast<PairF *>(smem_raw);
   for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
-    ia[k] = ia_g[k];
-  int2 const bk = blk[blockIdx.x];
+    ia[k] = pair_f(ia_g[k]);
+  int2 const bk = blk[blockIdx.x / LPP];
   RepGeom const &G = reps[bk.x];
-  // cell sizes: the image shift of an entry is -dc cs per axis, dc from
-  // its offset code (registers, no table lookup per entry)
   float const cs_x = static_cast<float>(G.box[0] / G.cg[0]);
   float const cs_y = static_cast<float>(G.box[1] / G.cg[1]);
   float const cs_z = static_cast<float>(G.box[2] / G.cg[2]);
   __syncthreads();
-  long long const a = G.p0 + static_cast<long long>(bk.y) * blockDim.x + threadIdx.x;
-  double ev[EV ? 20 : 1];
-#pragma unroll
-  for (int k = 0; k < (EV ? 20 : 1); ++k)
-    ev[k] = 0.0;
-  bool const active = a < G.p0 + G.np;
-  // groups of 8 entries: class A first (all terms), then class B
-  // (Coulomb only); the loop runs to the warp's largest group count so that
-  // the vote on LJ stays warp-wide
+  int const sub = threadIdx.x % LPP;
+  long long const la = static_cast<long long>(bk.y) * 256 + (blockIdx.x % LPP) * (256 / LPP) +
+                       threadIdx.x / LPP;
+  bool const active = la < G.np;
+  long long const a = G.p0 + la;
+  // groups of 8 entries: class A first (all terms), then class B (Coulomb
+  // only); the loop runs to the warp's largest group count so that the vote on
+  // LJ stays warp-wide
   int na = 0, nbb = 0;
   if (active) {
     int const c = nb_cnt[a];
@@ -667,84 +720,104 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
   int const ga = (na + 7) >> 3, gt = ga + ((nbb + 7) >> 3);
   int const gmax = __reduce_max_sync(0xffffffffu, gt);
   float4 const pa = active ? spf[a] : make_float4(0.f, 0.f, 0.f, 0.f);
-  int const ta = active ? stype[a] : 0;
-  Real const rc2 = static_cast<Real>(G.r_cut * G.r_cut);
-  Real const two_a_sqrt_pi_i = static_cast<Real>(2.0 * G.alpha / sqrt(kPi));
-  Real const pref_qa = static_cast<Real>(G.prefactor) * pa.w;
+  int const ta = (MODE != kPairOneType && active) ? stype[a] * ntypes : 0;
+  float const rc2 = static_cast<float>(G.r_cut * G.r_cut);
+  float const two_a = static_cast<float>(2.0 * G.alpha / sqrt(kPi));
+  float const pref_qa = static_cast<float>(G.prefactor) * pa.w;
   // exp(-(alpha r)^2) = 2^(c_exp r^2); A&S t = 1 / (1 + p alpha r)
-  Real const c_exp = static_cast<Real>(-G.alpha * G.alpha * 1.4426950408889634);
-  Real const p_alpha = static_cast<Real>(0.3275911 * G.alpha);
-  bool const one_type = (ntypes == 1);
-  PairR<Real> const p0(ia[0]);
+  float const c_exp = static_cast<float>(-G.alpha * G.alpha * 1.4426950408889634);
+  float const p_alpha = static_cast<float>(0.3275911 * G.alpha);
+  PairF const p0 = ia[0];
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  const int *nbp = nb + nb_base(G.nb_off, G.max_nb, active ? a - G.p0 : 0);
+  const int *nbp = nb + nb_base(G.nb_off, G.max_nb, active ? la : 0);
   int const ngroups = G.max_nb >> 3;
-  long long const base0 = G.p0;
-  // the particle itself with the zero cell offset (code 13: dc = 0)
-  unsigned const self_ent = static_cast<unsigned>(active ? a - G.p0 : 0) |
-                            (static_cast<unsigned>(cell_offset_code(0, 0, 0)) << kNbIndexBits);
-  // one entry: Coulomb always, LJ / WCA when the group may hold class A
-  auto entry = [&](auto lj, unsigned e, float4 pb, float &sx, float &sy, float &sz) {
-    // d = (x_a - x_b) - dc cs (dc in {-1, 0, 1}: the FMA's product is
-    // exact, so this rounds as the sum with a stored shift would)
-    unsigned const code = e >> kNbIndexBits;
-    Real const d0 = fmaf(code_axis(code, 0), -cs_x, pa.x - pb.x);
-    Real const d1 = fmaf(code_axis(code, 1), -cs_y, pa.y - pb.y);
-    Real const d2v = fmaf(code_axis(code, 2), -cs_z, pa.z - pb.z);
-    Real const dist2 = d0 * d0 + d1 * d1 + d2v * d2v;
-    Real const inv_d = rsqrt_approx(dist2);
-    Real const dist = dist2 * inv_d;
-    bool const pos = dist2 > Real(0);
-    Real const ex = ex2_approx(c_exp * dist2);
-    Real const t = rcp_r(fmaf(p_alpha, dist, Real(1)));
-    Real const asp =
-        t * (Real(0.254829592) +
-             t * (Real(-0.284496736) +
-                  t * (Real(1.421413741) + t * (Real(-1.453152027) + t * Real(1.061405429)))));
-    Real const erfc_part_ri = asp * inv_d;
-    Real const pq = pref_qa * pb.w;
-    bool const in_c = pos && dist2 < rc2;
-    Real const fc =
-        in_c ? (pq * ex) * (erfc_part_ri + two_a_sqrt_pi_i) * (inv_d * inv_d) : Real(0);
-    Real fn = Real(0), en = Real(0);
-    if constexpr (decltype(lj)::value) {
-      if constexpr (NOOFF) {
-        lj_wca_sel_nooff(p0, dist, inv_d * inv_d, fn);
-      } else if (one_type) {
-        if (p0.active)
-          lj_wca_sel(p0, dist, inv_d, fn, en);
-      } else {
-        int const b = static_cast<int>(base0 + (e & kNbIndexMask));
-        PairR<Real> const p(ia[ta * ntypes + stype[b]]);
-        if (p.active)
-          lj_wca_sel(p, dist, inv_d, fn, en);
-      }
-      fn = pos ? fn : Real(0);
-      en = pos ? en : Real(0);
+  const float4 *pos = spf + G.p0;
+  const int *typ = stype + G.p0;
+  f32x2 const pa_xy = pk2(pa.x, pa.y), ncs_xy = pk2(-cs_x, -0.25f * cs_y);
+  float const ncs_z = -0.0625f * cs_z;
+  // two entries: Coulomb always, LJ / WCA when the group may hold class A
+  auto two = [&](auto lj, unsigned const *e, float4 const *pb, float &sx, float &sy, float &sz) {
+    float dx[2], dy[2], dz[2], r2[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      // d = (x_a - x_b) - dc cs (dc in {-1, 0, 1}: the product is exact); the
+      // y and z fields carry factors 4 and 16 that the cell sizes undo
+      f32x2 const dc = pk2(code_axis(e[u], 0), code_axis(e[u], 1));
+      float2 const xy = up2(fma2(dc, ncs_xy, sub2(pa_xy, pk2(pb[u].x, pb[u].y))));
+      dx[u] = xy.x;
+      dy[u] = xy.y;
+      dz[u] = fmaf(code_axis(e[u], 2), ncs_z, pa.z - pb[u].z);
+      r2[u] = dx[u] * dx[u] + dy[u] * dy[u] + dz[u] * dz[u];
     }
-    Real const ft = fc + fn;
-    sx += ft * d0;
-    sy += ft * d1;
-    sz += ft * d2v;
-    if constexpr (EV) {
-      Real const ec = in_c ? pq * erfc_part_ri * ex : Real(0);
-      double const dd[3] = {d0, d1, d2v};
-      ev[0] += 0.5 * double(ec);
-      ev[1] += 0.5 * double(en);
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          ev[2 + 3 * r + c] += 0.5 * double(fc) * dd[r] * dd[c];
-          ev[11 + 3 * r + c] += 0.5 * double(fn) * dd[r] * dd[c];
+    f32x2 const d2 = pk2(r2[0], r2[1]);
+    f32x2 const inv = pk2(rsqrt_approx(r2[0]), rsqrt_approx(r2[1]));
+    f32x2 const dist = mul2(d2, inv);
+    float2 const ea = up2(mul2(pk2(c_exp, c_exp), d2));
+    f32x2 const ex = pk2(ex2_approx(ea.x), ex2_approx(ea.y));
+    float2 const td = up2(fma2(pk2(p_alpha, p_alpha), dist, pk2(1.f, 1.f)));
+    f32x2 const t = pk2(rcp_r(td.x), rcp_r(td.y));
+    f32x2 poly = fma2(t, pk2(1.061405429f, 1.061405429f), pk2(-1.453152027f, -1.453152027f));
+    poly = fma2(t, poly, pk2(1.421413741f, 1.421413741f));
+    poly = fma2(t, poly, pk2(-0.284496736f, -0.284496736f));
+    poly = fma2(t, poly, pk2(0.254829592f, 0.254829592f));
+    f32x2 const er = mul2(mul2(t, poly), inv);
+    f32x2 const pq = mul2(pk2(pref_qa, pref_qa), pk2(pb[0].w, pb[1].w));
+    f32x2 const i2 = mul2(inv, inv);
+    float2 const fc = up2(mul2(mul2(mul2(pq, ex), add2(er, pk2(two_a, two_a))), i2));
+    float fcv[2] = {fc.x, fc.y};
+    float fnv[2] = {0.f, 0.f};
+    if constexpr (decltype(lj)::value) {
+      float2 const dv = up2(dist), iv = up2(inv);
+      float const dd[2] = {dv.x, dv.y}, ii[2] = {iv.x, iv.y};
+      if constexpr (MODE == kPairOneType) {
+        if (p0.le48 != 0.f) {
+          f32x2 const s2 = mul2(pk2(p0.lsig * p0.lsig, p0.lsig * p0.lsig), i2);
+          f32x2 const f6 = mul2(mul2(s2, s2), s2);
+          float2 const v = up2(mul2(mul2(mul2(pk2(p0.le48, p0.le48), f6),
+                                         add2(f6, pk2(-0.5f, -0.5f))), i2));
+          fnv[0] = (dd[0] < p0.lcut && dd[0] > p0.lmin) ? v.x : 0.f;
+          fnv[1] = (dd[1] < p0.lcut && dd[1] > p0.lmin) ? v.y : 0.f;
         }
+        if (p0.wcut > 0.f) {
+          f32x2 const s2 = mul2(pk2(p0.wsig * p0.wsig, p0.wsig * p0.wsig), i2);
+          f32x2 const f6 = mul2(mul2(s2, s2), s2);
+          float2 const v = up2(mul2(mul2(mul2(pk2(p0.we48, p0.we48), f6),
+                                         add2(f6, pk2(-0.5f, -0.5f))), i2));
+          fnv[0] += dd[0] < p0.wcut ? v.x : 0.f;
+          fnv[1] += dd[1] < p0.wcut ? v.y : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          PairF const p = ia[ta + typ[nb_index(e[u])]];
+          float const inv_d = ii[u], inv_d2 = inv_d * inv_d;
+          {
+            float const inv_off = MODE == kPairOffset ? rcp_r(dd[u] - p.loff) : inv_d;
+            float const s = p.lsig * inv_off, s2 = s * s, f6 = s2 * s2 * s2;
+            bool const in = dd[u] < p.lcut && dd[u] > p.lmin;
+            fnv[u] += in ? p.le48 * f6 * (f6 - 0.5f) * (inv_off * inv_d) : 0.f;
+          }
+          {
+            float const s = p.wsig * inv_d, s2 = s * s, f6 = s2 * s2 * s2;
+            fnv[u] += dd[u] < p.wcut ? p.we48 * f6 * (f6 - 0.5f) * inv_d2 : 0.f;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      bool const on = r2[u] > 0.f;
+      float ft = (on && r2[u] < rc2) ? fcv[u] : 0.f;
+      if constexpr (decltype(lj)::value)
+        ft += on ? fnv[u] : 0.f;
+      sx += ft * dx[u];
+      sy += ft * dy[u];
+      sz += ft * dz[u];
     }
   };
   auto group = [&](auto lj, int v) {
     // the lane's group v: class A group v, or class B group v - ga
-    bool const in_a = v < ga;
-    int const grp = in_a ? v : ngroups - 1 - (v - ga);
-    int const kn = in_a ? min(8, na - 8 * v) : min(8, nbb - 8 * (v - ga));
+    int const grp = v < ga ? v : ngroups - 1 - (v - ga);
     const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
     int4 const g0 = gp[0], g1 = gp[1];
     unsigned const ent[8] = {static_cast<unsigned>(g0.x), static_cast<unsigned>(g0.y),
@@ -754,35 +827,35 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
     float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
     for (int h = 0; h < 8; h += 4) {
-      // entries past the count stand for the particle itself (zero
-      // distance: no term passes its range test), so no lane branches on
-      // the count; the partners' positions, four gathers in flight
-      unsigned eu[4];
-      float4 pbv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        eu[u] = (h + u < kn) ? ent[h + u] : self_ent;
-        pbv[u] = spf[base0 + (eu[u] & kNbIndexMask)];
-      }
+      float4 pb[4]; // four gathers in flight
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        entry(lj, eu[u], pbv[u], sx, sy, sz);
+        pb[u] = pos[nb_index(ent[h + u])];
+      two(lj, ent + h, pb, sx, sy, sz);
+      two(lj, ent + h + 2, pb + 2, sx, sy, sz);
     }
     // FP32 sums of this group into the FP64 accumulators
     fx += static_cast<double>(sx);
     fy += static_cast<double>(sy);
     fz += static_cast<double>(sz);
   };
-  for (int v = 0; v < gmax; ++v) {
-    bool const any_a = __any_sync(0xffffffffu, active && v < ga);
-    if (active && v < gt) {
+  for (int v0 = 0; v0 < gmax; v0 += LPP) {
+    int const v = v0 + sub;
+    bool const any_a = __any_sync(0xffffffffu, v < ga);
+    if (v < gt) {
       if (any_a)
         group(std::true_type{}, v);
       else
         group(std::false_type{}, v);
     }
   }
-  if (active) {
+#pragma unroll
+  for (int o = 1; o < LPP; o <<= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, o);
+    fy += __shfl_xor_sync(0xffffffffu, fy, o);
+    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+  }
+  if (active && sub == 0) {
     int const i = perm[a];
     if (overwrite) {
       f[3 * i + 0] = fx;
@@ -794,123 +867,249 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
       f[3 * i + 2] += fz;
     }
   }
-  if constexpr (EV) {
-    __shared__ double red[20][8];
-    int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+}
+
+// Block sums of N per-thread values (FP64, fixed order) into the columns of
+// partials[blockIdx.x * width + ...]: value k goes to every column c with
+// map(c) == k, times 1/2 (each pair is seen from both ends).
+template <int N, typename Map>
+__device__ inline void block_halves(double const *ev, int width, Map const &map,
+                                    double *__restrict__ partials) {
+  __shared__ double red[N][8];
+  int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < 20; ++k) {
-      double v = ev[k];
-      for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0)
-        red[k][wid] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 20) {
-      double s = 0.0;
-      for (int w = 0; w < (blockDim.x >> 5); ++w)
-        s += red[threadIdx.x][w];
-      partials[static_cast<long long>(blockIdx.x) * 20 + threadIdx.x] = s;
-    }
+  for (int k = 0; k < N; ++k) {
+    double v = ev[k];
+    for (int o = 16; o > 0; o >>= 1)
+      v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0)
+      red[k][wid] = v;
+  }
+  __syncthreads();
+  if (static_cast<int>(threadIdx.x) < width) {
+    int const k = map(threadIdx.x);
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w)
+      s += red[k][w];
+    partials[static_cast<long long>(blockIdx.x) * width + threadIdx.x] = 0.5 * s;
+  }
+}
+// Columns {E_coul, E_nb, Vc[9], Vn[9]} (width 20) from {E_coul, E_nb, the six
+// entries xx xy xz yy yz zz of Vc, of Vn}.
+__device__ inline int ev_column(int c) {
+  if (c < 2)
+    return c;
+  int const t = (c - 2) / 9, m = (c - 2) % 9, i = min(m / 3, m % 3), j = max(m / 3, m % 3);
+  return 2 + 6 * t + (i == 0 ? j : i + j + 1);
+}
+// Energy / virial sums of one pair into ev[14] (factors fc, fn of the two
+// forces, d the pair vector).
+__device__ inline void ev_add(double *ev, double ec, double en, double fc, double fn, double d0,
+                              double d1, double d2) {
+  ev[0] += ec;
+  ev[1] += en;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    double const g = t ? fn : fc;
+    double const x = g * d0, y = g * d1, z = g * d2;
+    double *v = ev + 2 + 6 * t;
+    v[0] += x * d0;
+    v[1] += x * d1;
+    v[2] += x * d2;
+    v[3] += y * d1;
+    v[4] += y * d2;
+    v[5] += z * d2;
   }
 }
 
-template <typename Real, bool EV>
-__global__ void __launch_bounds__(256, (sizeof(Real) == 4 && !EV) ? 4 : 1)
+// The FP32-mixed pair kernel with energies and virials in FP32 arithmetic
+// (P3MX_MIXED_OBSERVABLES): one thread per particle, pairs one at a time.
+__global__ void __launch_bounds__(256)
+k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
+                     const float4 *__restrict__ spf, const int *__restrict__ stype,
+                     const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
+                     const int *__restrict__ nb, const int *__restrict__ nb_cnt,
+                     double *__restrict__ f, int overwrite, double *__restrict__ partials) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PairIA *ia = reinterpret_cast<PairIA *>(smem_raw);
+  for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
+    ia[k] = ia_g[k];
+  int2 const bk = blk[blockIdx.x];
+  RepGeom const &G = reps[bk.x];
+  float const cs_x = static_cast<float>(G.box[0] / G.cg[0]);
+  float const cs_y = static_cast<float>(G.box[1] / G.cg[1]);
+  float const cs_z = static_cast<float>(G.box[2] / G.cg[2]);
+  __syncthreads();
+  long long const a = G.p0 + static_cast<long long>(bk.y) * blockDim.x + threadIdx.x;
+  double ev[14];
+#pragma unroll
+  for (int k = 0; k < 14; ++k)
+    ev[k] = 0.0;
+  if (a < G.p0 + G.np) {
+    int const c = nb_cnt[a];
+    int const na = nb_count_a(c), cnt = nb_count(c);
+    float4 const pa = spf[a];
+    int const ta = stype[a];
+    float const rc2 = static_cast<float>(G.r_cut * G.r_cut);
+    float const two_a = static_cast<float>(2.0 * G.alpha / sqrt(kPi));
+    float const pref_qa = static_cast<float>(G.prefactor) * pa.w;
+    float const c_exp = static_cast<float>(-G.alpha * G.alpha * 1.4426950408889634);
+    float const p_alpha = static_cast<float>(0.3275911 * G.alpha);
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, a - G.p0);
+    for (int k = 0; k < cnt; ++k) {
+      unsigned const e = static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, na, k)]);
+      long long const b = G.p0 + nb_index(e);
+      float4 const pb = spf[b];
+      float const d0 = fmaf(code_axis(e, 0), -cs_x, pa.x - pb.x);
+      float const d1 = fmaf(code_axis(e, 1), -0.25f * cs_y, pa.y - pb.y);
+      float const d2 = fmaf(code_axis(e, 2), -0.0625f * cs_z, pa.z - pb.z);
+      float const r2 = d0 * d0 + d1 * d1 + d2 * d2;
+      if (!(r2 > 0.f))
+        continue;
+      float const inv_d = rsqrt_approx(r2);
+      float const dist = r2 * inv_d;
+      float const ex = ex2_approx(c_exp * r2);
+      float const t = rcp_r(fmaf(p_alpha, dist, 1.f));
+      float const asp =
+          t * (0.254829592f +
+               t * (-0.284496736f + t * (1.421413741f + t * (-1.453152027f + t * 1.061405429f))));
+      float const er = asp * inv_d;
+      float const pq = pref_qa * pb.w;
+      bool const in_c = r2 < rc2;
+      float const fc = in_c ? (pq * ex) * (er + two_a) * (inv_d * inv_d) : 0.f;
+      float const ec = in_c ? pq * er * ex : 0.f;
+      float fn = 0.f, en = 0.f;
+      PairR<float> const p(ia[ta * ntypes + stype[b]]);
+      if (p.active)
+        lj_wca_sel(p, dist, inv_d, fn, en);
+      float const ft = fc + fn;
+      fx += static_cast<double>(ft * d0);
+      fy += static_cast<double>(ft * d1);
+      fz += static_cast<double>(ft * d2);
+      ev_add(ev, ec, en, fc, fn, d0, d1, d2);
+    }
+    int const i = perm[a];
+    if (overwrite) {
+      f[3 * i + 0] = fx;
+      f[3 * i + 1] = fy;
+      f[3 * i + 2] = fz;
+    } else {
+      f[3 * i + 0] += fx;
+      f[3 * i + 1] += fy;
+      f[3 * i + 2] += fz;
+    }
+  }
+  block_halves<14>(ev, 20, [](int c) { return ev_column(c); }, partials);
+}
+
+// FP64 pair kernel: minimum-image differences of the folded positions, pair
+// arithmetic and sums in FP64; the same lists, lanes and classes as
+// k_pair_forces_rel (LJ / WCA for class A groups only).  EV adds energies and
+// virials: per-block FP64 partials {E_coul, E_nb, Vc[9], Vn[9]} (width 20).
+// Blocks map to replicas through the block table so partials never straddle
+// replicas.  Bound by the FP64 pipe: the inverse distance is one rsqrt, the
+// A&S reciprocal one FP32 seed with a third-order step.
+template <bool EV, int LPP>
+__global__ void __launch_bounds__(256, EV ? 1 : 2)
 k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
               const double4 *__restrict__ spq, const int *__restrict__ stype,
               const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
-              long long n, const int *__restrict__ nb, const int *__restrict__ nb_cnt,
-              double *__restrict__ f, int overwrite, double *__restrict__ partials) {
+              const int *__restrict__ nb, const int *__restrict__ nb_cnt, double *__restrict__ f,
+              int overwrite, double *__restrict__ partials) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PairIA *ia = reinterpret_cast<PairIA *>(smem_raw);
   for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
     ia[k] = ia_g[k];
   __syncthreads();
-  int2 const bk = blk[blockIdx.x];
+  int2 const bk = blk[blockIdx.x / LPP];
   RepGeom const &G = reps[bk.x];
-  long long const a = G.p0 + static_cast<long long>(bk.y) * blockDim.x + threadIdx.x;
-  double ev[EV ? 20 : 1];
+  int const sub = threadIdx.x % LPP;
+  long long const la = static_cast<long long>(bk.y) * 256 + (blockIdx.x % LPP) * (256 / LPP) +
+                       threadIdx.x / LPP;
+  bool const active = la < G.np;
+  long long const a = G.p0 + la;
+  double ev[EV ? 14 : 1];
 #pragma unroll
-  for (int k = 0; k < (EV ? 20 : 1); ++k)
+  for (int k = 0; k < (EV ? 14 : 1); ++k)
     ev[k] = 0.0;
-  if (a < G.p0 + G.np) {
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  if (active) {
     double4 const pa = spq[a];
-    int const ta = stype[a];
+    int const ta = stype[a] * ntypes;
     double const L0 = G.box[0], L1 = G.box[1], L2 = G.box[2];
     double const Li0 = G.box_i[0], Li1 = G.box_i[1], Li2 = G.box_i[2];
-    Real const alpha = static_cast<Real>(G.alpha);
-    Real const r_cut = static_cast<Real>(G.r_cut);
-    Real const two_a_sqrt_pi_i = static_cast<Real>(2.0 * G.alpha / sqrt(kPi));
-    Real const pref_qa = static_cast<Real>(G.prefactor * pa.w);
-    bool const one_type = (ntypes == 1);
-    PairR<Real> const p0(ia[0]);
-    double fx = 0.0, fy = 0.0, fz = 0.0;
+    double const alpha = G.alpha, r_cut = G.r_cut;
+    double const two_a = 2.0 * G.alpha / sqrt(kPi);
+    double const pref_qa = G.prefactor * pa.w;
     int const cw = nb_cnt[a];
-    int const cnt = nb_count(cw), cna = nb_count_a(cw);
-    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, a - G.p0);
-    int const base0 = static_cast<int>(G.p0);
-    int b_next =
-        (cnt > 0) ? base0 + static_cast<int>(static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, 0)]) &
-                                             kNbIndexMask)
-                  : 0;
-    double4 p_next = (cnt > 0) ? spq[b_next] : pa;
-    for (int k = 0; k < cnt; ++k) {
-      int const b = b_next;
-      double4 const pb = p_next;
-      if (k + 1 < cnt) {
-        b_next = base0 + static_cast<int>(static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, cna, k + 1)]) &
-                                          kNbIndexMask);
-        p_next = spq[b_next];
-      }
-      // geometry in FP64 (two conversions per pair instead of four)
-      double const d0 = mi_d(pa.x - pb.x, L0, Li0);
-      double const d1 = mi_d(pa.y - pb.y, L1, Li1);
-      double const d2v = mi_d(pa.z - pb.z, L2, Li2);
-      Real const dist2 = static_cast<Real>(d0 * d0 + d1 * d1 + d2v * d2v);
-      Real const inv_d = rsqrt_r(dist2);
-      Real const dist = dist2 * inv_d;
-      Real fc = Real(0), ec = Real(0);
-      Real const qb = static_cast<Real>(pb.w);
-      if (qb != Real(0) && pref_qa != Real(0) && dist < r_cut && dist > Real(0)) {
-        Real const adist = alpha * dist;
-        Real const ex = exp_r(-adist * adist);
-        Real const t = rcp_r(Real(1) + Real(0.3275911) * adist);
-        Real const asp = t * (Real(0.254829592) +
-                              t * (Real(-0.284496736) +
-                                   t * (Real(1.421413741) + t * (Real(-1.453152027) + t * Real(1.061405429)))));
-        Real const erfc_part_ri = asp * inv_d;
-        Real const pq = pref_qa * qb;
-        fc = pq * (ex * (erfc_part_ri + two_a_sqrt_pi_i) * (inv_d * inv_d));
-        if constexpr (EV)
-          ec = pq * erfc_part_ri * ex;
-      }
-      Real fn = Real(0), en = Real(0);
-      if (one_type) {
-        if (p0.active)
-          lj_wca(p0, dist, inv_d, fn, en);
-      } else {
-        PairR<Real> const p(ia[ta * ntypes + stype[b]]);
-        if (p.active)
-          lj_wca(p, dist, inv_d, fn, en);
-      }
-      double const ft = static_cast<double>(fc + fn);
-      fx += ft * d0;
-      fy += ft * d1;
-      fz += ft * d2v;
-      if constexpr (EV) {
-        double const dd[3] = {d0, d1, d2v};
-        ev[0] += 0.5 * double(ec);
-        ev[1] += 0.5 * double(en);
+    int const ga = (nb_count_a(cw) + 7) >> 3, gt = ga + ((nb_count_b(cw) + 7) >> 3);
+    const int *nbp = nb + nb_base(G.nb_off, G.max_nb, la);
+    int const ngroups = G.max_nb >> 3;
+    const double4 *pos = spq + G.p0;
+    const int *typ = stype + G.p0;
+    for (int v = sub; v < gt; v += LPP) {
+      bool const cls_a = v < ga;
+      int const grp = cls_a ? v : ngroups - 1 - (v - ga);
+      const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
+      // the next half group's positions are loaded ahead of the pairs
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+      for (int h = 0; h < 2; ++h) {
+        int4 const g = gp[h];
+        unsigned const idx[4] = {nb_index(g.x), nb_index(g.y), nb_index(g.z), nb_index(g.w)};
+        double4 pv[4];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            ev[2 + 3 * r + c] += 0.5 * double(fc) * dd[r] * dd[c];
-            ev[11 + 3 * r + c] += 0.5 * double(fn) * dd[r] * dd[c];
+        for (int u = 0; u < 4; ++u)
+          pv[u] = pos[idx[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          double4 const pb = pv[u];
+          double const d0 = mi_d(pa.x - pb.x, L0, Li0);
+          double const d1 = mi_d(pa.y - pb.y, L1, Li1);
+          double const d2 = mi_d(pa.z - pb.z, L2, Li2);
+          double const dist2 = d0 * d0 + d1 * d1 + d2 * d2;
+          if (!(dist2 > 0.0))
+            continue;
+          double const inv_d = rsqrt(dist2);
+          double const dist = dist2 * inv_d;
+          double fc = 0.0, ec = 0.0;
+          if (pb.w != 0.0 && pref_qa != 0.0 && dist < r_cut) {
+            double const adist = alpha * dist;
+            double const ex = exp(-adist * adist);
+            double const t = rcp_newton(fma(0.3275911, adist, 1.0));
+            double const asp =
+                t * (0.254829592 +
+                     t * (-0.284496736 +
+                          t * (1.421413741 + t * (-1.453152027 + t * 1.061405429))));
+            double const er = asp * inv_d;
+            double const pq = pref_qa * pb.w;
+            fc = pq * (ex * (er + two_a) * (inv_d * inv_d));
+            if constexpr (EV)
+              ec = pq * er * ex;
           }
+          double fn = 0.0, en = 0.0;
+          if (cls_a) {
+            PairR<double> const p(ia[ta + typ[idx[u]]]);
+            if (p.active)
+              lj_wca(p, dist, inv_d, fn, en);
+          }
+          double const ft = fc + fn;
+          fx += ft * d0;
+          fy += ft * d1;
+          fz += ft * d2;
+          if constexpr (EV)
+            ev_add(ev, ec, en, fc, fn, d0, d1, d2);
+        }
       }
     }
+  }
+#pragma unroll
+  for (int o = 1; o < LPP; o <<= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, o);
+    fy += __shfl_xor_sync(0xffffffffu, fy, o);
+    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+  }
+  if (active && sub == 0) {
     int const i = perm[a];
     if (overwrite) {
       f[3 * i + 0] = fx;
@@ -922,25 +1121,8 @@ k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
       f[3 * i + 2] += fz;
     }
   }
-  if constexpr (EV) {
-    __shared__ double red[20][8];
-    int const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 20; ++k) {
-      double v = ev[k];
-      for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0)
-        red[k][wid] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 20) {
-      double s = 0.0;
-      for (int w = 0; w < (blockDim.x >> 5); ++w)
-        s += red[threadIdx.x][w];
-      partials[static_cast<long long>(blockIdx.x) * 20 + threadIdx.x] = s;
-    }
-  }
+  if constexpr (EV)
+    block_halves<14>(ev, 20, [](int c) { return ev_column(c); }, partials);
 }
 
 // Largest squared displacement since the last list build, as a flag:
