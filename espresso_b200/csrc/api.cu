@@ -1116,8 +1116,7 @@ int p3mx_long_range(p3mx_handle *h, size_t n, const double *pos, const double *q
         virial9[k] = vir.empty() ? 0. : vir[k];
     if (fd)
       stage_out(h, n, f, dev, ow, st);
-    P3MX_CUDA(cudaStreamSynchronize(st));
-    check_kernels(h, st);
+    check_kernels(h, st); // synchronises
   });
 }
 
@@ -1153,8 +1152,7 @@ int p3mx_short_range(p3mx_handle *h, size_t n, const double *pos, const double *
         virial18[k] = vir.empty() ? 0. : vir[k];
     if (fd)
       stage_out(h, n, f, dev, ow, st);
-    P3MX_CUDA(cudaStreamSynchronize(st));
-    check_kernels(h, st);
+    check_kernels(h, st); // synchronises
   });
 }
 
@@ -1178,8 +1176,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
         k_elc_add<<<static_cast<unsigned>((3 * n + 255) / 256), 256, 0, st>>>(f, fo, 3 * n);
       if (f)
         stage_out(h, n, f, dev, ow, st);
-      P3MX_CUDA(cudaStreamSynchronize(st));
-      check_kernels(h, st);
+      check_kernels(h, st); // synchronises
       return;
     }
     // Forces only from host arrays, with charges and types staged by an
@@ -1206,8 +1203,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
         forces();
       }
       stage_out(h, n, f, dev, ow, st);
-      P3MX_CUDA(cudaStreamSynchronize(st));
-      check_kernels(h, st);
+      check_kernels(h, st); // synchronises
       return;
     }
     if (want_e || h->prm.epsilon != 0.)
@@ -1217,9 +1213,17 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
     if (!want_e && !want_v) {
       // forces only: real-space pairs concurrent with the k-space chain
       e.forces_all(fd, dev ? ow : true, st);
-    } else {
+    } else if (f) {
       e.long_range(fd, dev ? ow : true, want_e && !obs64, want_v && !obs64, st, &enk, &virk);
       e.short_range(fd, false, (want_e || want_v) && !obs64, st, &ens, &virs);
+      e.bond_forces(fd, st);
+    } else {
+      // observables only: no field transforms and no interpolation (the pair
+      // kernel's forces and the bond check go to the scratch buffer)
+      if (!obs64) {
+        e.long_range(nullptr, true, want_e, want_v, st, &enk, &virk);
+        e.short_range(fd, true, true, st, &ens, &virs);
+      }
       e.bond_forces(fd, st);
     }
     if (obs64 && (want_e || want_v)) {
@@ -1247,8 +1251,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
       }
     if (f)
       stage_out(h, n, f, dev, ow, st);
-    P3MX_CUDA(cudaStreamSynchronize(st));
-    check_kernels(h, st);
+    check_kernels(h, st); // synchronises
   });
 }
 

@@ -185,6 +185,31 @@ __device__ inline bool mbar_wait(unsigned long long *bar, unsigned parity) {
   return false;
 }
 
+// Programmatic dependent launch: a kernel launched by pdl_launch(chained)
+// may start while the kernel before it on the stream drains; pdl_enter, its
+// first statement, waits until that kernel has completed and its writes are
+// visible, and lets the next kernel's blocks be scheduled behind this one's.
+// Every kernel of a chain enters this way, so a wait covers all before it.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+inline void pdl_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       bool chained, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = chained ? 1 : 0;
+  P3MX_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+
 inline int ceil_div(long long a, long long b) {
   return static_cast<int>((a + b - 1) / b);
 }

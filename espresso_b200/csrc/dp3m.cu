@@ -170,15 +170,9 @@ public:
       m_g_valid = true;
     }
     // 1. brick binning and sort (shared by the three components)
-    P3MX_CUDA(cudaMemsetAsync(E.m_cnt.p, 0, (E.m_nkeys + 2) * sizeof(int), st));
     unsigned *qmax_bits = reinterpret_cast<unsigned *>(E.m_cnt.as<int>() + E.m_nkeys + 1);
     int const nb = static_cast<int>(ceil_div(n, 256));
-    k_p3m_bin<Real><<<nb, 256, 0, st>>>(geom, E.m_rep_of.as<int>(), E.d_pos(), n, E.m_key.as<int>(),
-                                        E.m_bkey.as<int>(), E.m_slot.as<int>(), E.m_cnt.as<int>(),
-                                        E.m_dist.as<Real>());
-    ++E.m_launches;
-    E.sort_keys(E.m_bkey.as<int>(), E.m_slot.as<int>(), E.m_cnt.as<int>(), E.m_start.as<int>(),
-                E.m_perm.as<int>(), E.m_nkeys, st, nullptr, false);
+    E.bin_and_sort<Real>(qmax_bits, 1, st);
     E.mark("dp_sort", st);
     // 2. the three component meshes: weight records per component, then one
     // assignment and one z pass over all three (blockIdx.y = component)
@@ -201,7 +195,7 @@ public:
       P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(E.m_sb_edge, cnt, st, geom, tab,
                                                      E.m_start.as<int>(), m_W3.as<Real>(),
                                                      E.m_skey.as<int>(), qmax3,
-                                                     m_tiles3.as<Real>(), E.m_kerr.as<int>(), 3,
+                                                     m_tiles3.as<Real>(), E.kerr(), 3,
                                                      wst, E.m_tiles_n, 1)));
       ++E.m_launches;
     }
@@ -260,7 +254,7 @@ public:
                                  gi, tab, nbr, E.m_start.as<int>(), E.m_perm.as<int>(),
                                  E.m_skey.as<int>(), E.m_W.as<Real>(), E.m_tmap.as<CUtensorMap>(),
                                  1, E.d_q(), E.m_dipole.as<double>(), out, 3 * n, 1,
-                                 E.m_kerr.as<int>())));
+                                 E.kerr())));
       ++E.m_launches;
     }
     E.mark("dp_interp", st);

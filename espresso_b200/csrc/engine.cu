@@ -10,6 +10,7 @@
 #include <atomic>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <map>
 #include <utility>
 
@@ -135,13 +136,22 @@ Engine::Engine(bool fp32) : m_fp32(fp32) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&m_sms, cudaDevAttrMultiProcessorCount, dev);
+  void *w = nullptr;
+  if (cudaHostAlloc(&w, kHostWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    throw Error(4, "pinned host allocation failed");
+  }
+  m_host_words = static_cast<int *>(w);
+  for (int k = 0; k < kHostWords; ++k)
+    m_host_words[k] = 0;
 }
 
 Engine::~Engine() {
   if (m_check_ev)
     cudaEventDestroy(m_check_ev);
-  if (m_flag_host)
-    cudaFreeHost(m_flag_host);
+  if (m_host_words)
+    cudaFreeHost(const_cast<int *>(m_host_words));
   if (m_stream)
     cudaStreamDestroy(m_stream);
 }
@@ -149,6 +159,11 @@ Engine::~Engine() {
 void Engine::set_pair_table(int ntypes, std::vector<PairIA> const &tab) {
   if (ntypes < 1 || static_cast<int>(tab.size()) != ntypes * ntypes)
     throw Error(1, "pair table must hold ntypes^2 entries");
+  // the table of the current lists and block tables: nothing to do (scripts
+  // set it before every force calculation)
+  if (ntypes == m_ntypes && m_ia_d.p != nullptr && !m_conf.empty() &&
+      std::memcmp(tab.data(), m_ia.data(), tab.size() * sizeof(PairIA)) == 0)
+    return;
   m_ntypes = ntypes;
   m_ia = tab;
   upload_vec(m_ia_d, m_ia, m_stream);
@@ -515,6 +530,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   // sort-brick counts, then one word per replica: the bits of its largest
   // |q| (FP32, rounded up), which the assignment's fixed-point scale needs
   m_cnt.ensure((m_nkeys + 1 + R) * sizeof(int));
+  m_cnt_dirty = true;
   m_start.ensure((m_nkeys + 1) * sizeof(int));
   m_scan_tiles.ensure((ceil_div(std::max(m_nkeys, m_oct_mult * m_cells) + 1, kScanTile) + 1) * sizeof(int));
   m_dist.ensure(3 * n * rsz);
@@ -548,14 +564,6 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_overflow.ensure(static_cast<size_t>(std::max(R, 1)) * sizeof(int));
   m_rflag.ensure(static_cast<size_t>(std::max(R, 1)) * sizeof(int));
   m_flag.ensure(sizeof(int));
-  // the list check's two alternating flag words, both zero
-  m_chk.ensure(2 * sizeof(int));
-  P3MX_CUDA(cudaMemsetAsync(m_chk.p, 0, 2 * sizeof(int), st));
-  m_chk_slot = 0;
-  if (m_kerr.p == nullptr) {
-    m_kerr.ensure(4 * sizeof(int));
-    P3MX_CUDA(cudaMemsetAsync(m_kerr.p, 0, 4 * sizeof(int), st));
-  }
   m_pos_ref.ensure(3 * n * sizeof(double));
   m_type_ref.ensure(n * sizeof(int));
   m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes() * 20 * sizeof(double));
@@ -567,11 +575,45 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   P3MX_CUDA(cudaStreamSynchronize(st));
 }
 
+// Positions, charges and types (nullptr: zero) from the caller's device
+// arrays into the engine's, one launch in place of three copies.
+__global__ void __launch_bounds__(256)
+k_stage(long long n, const double *__restrict__ pos, const double *__restrict__ q,
+        const int *__restrict__ type, double *__restrict__ dpos, double *__restrict__ dq,
+        int *__restrict__ dtype) {
+  long long const i0 = static_cast<long long>(blockIdx.x) * 1024 + threadIdx.x;
+  // a block takes 1024 particles: their 3072 coordinates, then charges, types
+  double c[12];
+  long long const p0 = static_cast<long long>(blockIdx.x) * 3072 + threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < 12; ++u)
+    if (p0 + 256 * u < 3 * n)
+      c[u] = pos[p0 + 256 * u];
+#pragma unroll
+  for (int u = 0; u < 12; ++u)
+    if (p0 + 256 * u < 3 * n)
+      dpos[p0 + 256 * u] = c[u];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    long long const i = i0 + 256 * u;
+    if (i < n) {
+      dq[i] = q[i];
+      dtype[i] = type ? type[i] : 0;
+    }
+  }
+}
+
 void Engine::upload(const double *pos, const double *q, const int *type, bool device_ptrs,
                     cudaStream_t st) {
-  cudaMemcpyKind const k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  cudaMemcpyKind const k = cudaMemcpyHostToDevice;
   if (m_n == 0)
     return;
+  if (device_ptrs) {
+    k_stage<<<ceil_div(m_n, 1024), 256, 0, st>>>(m_n, pos, q, type, d_pos(), d_q(), d_type());
+    ++m_launches;
+    P3MX_CUDA(cudaGetLastError());
+    return;
+  }
   P3MX_CUDA(cudaMemcpyAsync(m_pos.p, pos, 3 * m_n * sizeof(double), k, st));
   P3MX_CUDA(cudaMemcpyAsync(m_q.p, q, m_n * sizeof(double), k, st));
   if (type)
@@ -611,14 +653,35 @@ void Engine::census(cudaStream_t st) {
 
 void Engine::sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, long long nkeys,
                        cudaStream_t st, const int *cond, bool index_order) {
-  m_launches += exclusive_scan(cnt, start, m_scan_tiles.as<int>(), nkeys, st, cond);
-  k_place<<<ceil_div(m_n, 256), 256, 0, st>>>(key, slot, start, perm, m_n, cond); ++m_launches;
+  m_launches += exclusive_scan(cnt, start, m_scan_tiles.as<int>(), nkeys, st, cond, !index_order);
+  pdl_launch(k_place, ceil_div(m_n, 256), 256, 0, st, !index_order, key, slot, start, perm, m_n,
+             cond, index_order ? nullptr : cnt, index_order ? 0 : nkeys + 1);
+  ++m_launches;
   if (!index_order)
     return;
   k_fix_buckets<<<ceil_div(nkeys * 32, 256), 256, 0, st>>>(start, perm, nkeys, cond); ++m_launches;
   k_fix_big_buckets<<<static_cast<int>(std::min<long long>(ceil_div(nkeys, 256), 296)), 256, 0,
                       st>>>(
       start, perm, nkeys, cond); ++m_launches;
+}
+
+// Corner binning and the brick sort of the particles (qmax_bits: the words the
+// weight kernel raises, cleared here).  The brick counts are zero on entry
+// (cleared by the sort before; by a memset after a failed one).
+template <typename Real> void Engine::bin_and_sort(unsigned *qmax_bits, int nq, cudaStream_t st) {
+  if (m_cnt_dirty)
+    P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
+  m_cnt_dirty = true;
+  pdl_launch(k_p3m_bin<Real>, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(),
+             m_rep_of.as<int>(), d_pos(), m_n, m_key.as<int>(), m_bkey.as<int>(), m_slot.as<int>(),
+             m_cnt.as<int>(), m_dist.as<Real>(), qmax_bits, nq);
+  ++m_launches;
+  // the order inside a brick is left as the atomic slots made it: the
+  // fixed-point assignment sums integers and the interpolation treats
+  // every particle on its own, so the results do not depend on it
+  sort_keys(m_bkey.as<int>(), m_slot.as<int>(), m_cnt.as<int>(), m_start.as<int>(),
+            m_perm.as<int>(), m_nkeys, st, nullptr, false);
+  m_cnt_dirty = false;
 }
 
 namespace {
@@ -680,9 +743,9 @@ void launch_assign(int edge, int cnt, cudaStream_t st, RepGeom const *geom, int2
                    Real *tiles, int *err, int ncomp = 1, long long comp_w = 0,
                    long long comp_tile = 0, int comp_q = 0) {
   auto go = [&](auto kern, size_t smem) {
-    kern<<<dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp)), 32 * kSbWarps, smem,
-           st>>>(geom, tab, cnt, start, W, s_key, qmax_bits, tiles, err, comp_w, comp_tile,
-                 comp_q);
+    pdl_launch(kern, dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp)), 32 * kSbWarps,
+               smem, st, true, geom, tab, cnt, start, W, s_key, qmax_bits, tiles, err, comp_w,
+               comp_tile, comp_q);
   };
   if (edge == kSbEdgeSmall)
     go(ncomp > 1 ? k_p3m_assign_sb<Real, P, kSbEdgeSmall, true>
@@ -736,27 +799,20 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     m_ginf_valid = true;
   }
   mark("start", st);
-  // 1. corner binning + deterministic counting sort
-  P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1 + R) * sizeof(int), st));
+  // 1. corner binning, brick sort, weight records.  From here on every kernel
+  // is a programmatic dependent of the one before
   unsigned *qmax_bits = reinterpret_cast<unsigned *>(m_cnt.as<int>() + m_nkeys + 1);
-  int const nb = ceil_div(m_n, 256);
   if (m_n > 0) {
-    k_p3m_bin<Real><<<nb, 256, 0, st>>>(geom, m_rep_of.as<int>(), d_pos(), m_n, m_key.as<int>(),
-                                        m_bkey.as<int>(),
-                                        m_slot.as<int>(), m_cnt.as<int>(), m_dist.as<Real>()); ++m_launches;
-    // the order inside a brick is left as the atomic slots made it: the
-    // fixed-point assignment sums integers and the interpolation treats
-    // every particle on its own, so the results do not depend on it
-    sort_keys(m_bkey.as<int>(), m_slot.as<int>(), m_cnt.as<int>(), m_start.as<int>(),
-              m_perm.as<int>(), m_nkeys, st, nullptr, false);
+    bin_and_sort<Real>(qmax_bits, R, st);
     mark("p3m_sort", st);
-    k_p3m_weights<Real><<<nb, 256, 0, st>>>(geom, m_perm.as<int>(), m_key.as<int>(),
-                                            m_dist.as<Real>(), d_q(), m_rep_of.as<int>(), m_n,
-                                            m_W.as<Real>(), m_skey.as<int>(), qmax_bits);
+    pdl_launch(k_p3m_weights<Real>, ceil_div(m_n, 256), 256, 0, st, true, geom, m_perm.as<int>(),
+               m_key.as<int>(), m_dist.as<Real>(), d_q(), m_rep_of.as<int>(), m_n, m_W.as<Real>(),
+               m_skey.as<int>(), qmax_bits);
     ++m_launches;
     mark("p3m_weights", st);
   } else {
     P3MX_CUDA(cudaMemsetAsync(m_start.p, 0, (m_nkeys + 1) * sizeof(int), st));
+    P3MX_CUDA(cudaMemsetAsync(qmax_bits, 0, R * sizeof(int), st));
   }
   // 2. charge assignment: one block per super-brick, its tile stored whole
   for (int c = 1; c <= 7; ++c) {
@@ -766,7 +822,7 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
     P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, geom, tab, m_start.as<int>(),
                                                    m_W.as<Real>(), m_skey.as<int>(), qmax_bits,
-                                                   m_tiles.as<Real>(), m_kerr.as<int>())));
+                                                   m_tiles.as<Real>(), kerr())));
     ++m_launches;
   }
   mark("p3m_assign", st);
@@ -780,9 +836,9 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   {
     auto const kern = want_ev ? (m_two[0] ? k_fft_x_kspace<Real, true, true> : k_fft_x_kspace<Real, true, false>)
                               : (m_two[0] ? k_fft_x_kspace<Real, false, true> : k_fft_x_kspace<Real, false, false>);
-    kern<<<m_n_blk_x, 256, m_smem_x, st>>>(geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(),
-                                           m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0,
-                                           m_part_x.as<double>(), m_tw.as<C>());
+    pdl_launch(kern, m_n_blk_x, 256, m_smem_x, st, true, geom, m_blk_x.as<Blk>(), m_ck.as<C>(),
+               m_ginf.as<Real>(), m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0,
+               m_part_x.as<double>(), m_tw.as<C>());
   }
   ++m_launches;
   if (want_ev) {
@@ -804,12 +860,11 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     if (nbr == 0)
       continue;
     int2 const *tab = m_blk_brick.as<int2>() + m_brick_off[c];
-    P3MX_CAO_DISPATCH_R(c, (k_p3m_interp<Real, P><<<interp_grid<Real, P>(nbr),
-                               32 * (1 + kInterpWarps), interp_smem<Real, P>(), st>>>(
+    P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>, interp_grid<Real, P>(nbr),
+                               32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true,
                                geom, tab, nbr, m_start.as<int>(), m_perm.as<int>(),
-                               m_skey.as<int>(), m_W.as<Real>(),
-                               m_tmap.as<CUtensorMap>(), 0, d_q(), m_dipole.as<double>(), f, 0,
-                               overwrite ? 1 : 0, m_kerr.as<int>())));
+                               m_skey.as<int>(), m_W.as<Real>(), m_tmap.as<CUtensorMap>(), 0,
+                               d_q(), m_dipole.as<double>(), f, 0, overwrite ? 1 : 0, kerr())));
     ++m_launches;
   }
   mark("p3m_interp", st);
@@ -902,8 +957,8 @@ void Engine::build_lists(cudaStream_t st) {
       throw Error(2, "Verlet list overflow");
     layout_lists(st);
   }
-  P3MX_CUDA(cudaMemcpyAsync(m_pos_ref.p, d_pos(), 3 * m_n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  P3MX_CUDA(cudaMemcpyAsync(m_type_ref.p, d_type(), m_n * sizeof(int), cudaMemcpyDeviceToDevice, st));
+  k_copy_pos_ref<<<nb, 256, 0, st>>>(m_pos_ref.as<double>(), d_pos(), m_type_ref.as<int>(), d_type(),
+                                     d_q(), m_rep_of.as<int>(), nullptr, m_n, nullptr); ++m_launches;
   m_lists_valid = true;
 }
 
@@ -925,43 +980,44 @@ __global__ void k_refresh_spq(const RepGeom *__restrict__ reps, const int *__res
                        qi);
 }
 
-// Displacement check fused with the sorted-position refresh: sets *flag
-// when a particle moved more than skin/2 or changed type since the last
-// build (k_displacement_check's test) and writes the pair kernel's sorted
+// Displacement check fused with the sorted-position refresh: sets *flag (in
+// mapped host memory: one store per block that found a change) when a
+// particle moved more than skin/2 or changed its kind since the last build
+// (k_displacement_check's test) and writes the pair kernel's sorted
 // records as k_refresh_spq does (a rebuild that follows rewrites them).
 // One thread per particle in index order (coalesced reads of positions,
 // reference positions, types and build-time cells), each writing its
 // records to its sorted slot inv[i].
-__global__ void k_check_refresh(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
-                                const int *__restrict__ inv, const double *__restrict__ pos,
-                                const double *__restrict__ q, const int *__restrict__ ckey,
-                                const double *__restrict__ pos_ref, const int *__restrict__ type,
-                                const int *__restrict__ type_ref, long long n,
-                                double4 *__restrict__ spq, float4 *__restrict__ spf,
-                                int *__restrict__ flag, int *__restrict__ flag_next) {
-  // the flag word of the next check starts at zero (no memset between checks)
-  if (blockIdx.x == 0 && threadIdx.x == 0)
-    *flag_next = 0;
+__global__ void __launch_bounds__(256)
+k_check_refresh(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
+                const int *__restrict__ inv, const double *__restrict__ pos,
+                const double *__restrict__ q, const int *__restrict__ ckey,
+                const double *__restrict__ pos_ref, const int *__restrict__ type,
+                const int *__restrict__ type_ref, long long n, double4 *__restrict__ spq,
+                float4 *__restrict__ spf, volatile int *flag) {
+  pdl_enter();
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  int const s = inv[i];
-  RepGeom const &G = reps[rep_of[i]];
-  double d2 = 0.0;
+  bool moved = false;
+  if (i < n) {
+    int const s = inv[i];
+    RepGeom const &G = reps[rep_of[i]];
+    double d2 = 0.0;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double const dx = pos[3 * i + d] - pos_ref[3 * i + d];
-    d2 += dx * dx;
+    for (int d = 0; d < 3; ++d) {
+      double const dx = pos[3 * i + d] - pos_ref[3 * i + d];
+      d2 += dx * dx;
+    }
+    double const lim = 0.5 * G.skin;
+    double const qi = q[i];
+    moved = d2 > lim * lim || list_kind(type[i], qi) != type_ref[i];
+    if (spq)
+      spq[s] = make_double4(fold_coord(pos[3 * i], G.box[0]), fold_coord(pos[3 * i + 1], G.box[1]),
+                            fold_coord(pos[3 * i + 2], G.box[2]), qi);
+    spf[s] = cell_offset(G, ckey[i] - static_cast<int>(G.cell_off), pos_ref + 3 * i, pos + 3 * i,
+                         qi);
   }
-  double const lim = 0.5 * G.skin;
-  if (d2 > lim * lim || type[i] != type_ref[i])
-    atomicOr(flag, 1);
-  double const qi = q[i];
-  if (spq)
-    spq[s] = make_double4(fold_coord(pos[3 * i], G.box[0]), fold_coord(pos[3 * i + 1], G.box[1]),
-                          fold_coord(pos[3 * i + 2], G.box[2]), qi);
-  spf[s] = cell_offset(G, ckey[i] - static_cast<int>(G.cell_off), pos_ref + 3 * i, pos + 3 * i,
-                       qi);
+  if (__syncthreads_or(moved) && threadIdx.x == 0)
+    *flag = 1;
 }
 
 void Engine::refresh_sorted_positions(cudaStream_t st, bool want_spq) {
@@ -979,23 +1035,17 @@ void Engine::check_lists(cudaStream_t st, bool need_spq) {
   m_check_rebuild = !m_lists_valid;
   if (m_check_rebuild)
     return;
-  if (!m_flag_host) {
-    P3MX_CUDA(cudaMallocHost(&m_flag_host, sizeof(int)));
+  if (!m_check_ev)
     P3MX_CUDA(cudaEventCreateWithFlags(&m_check_ev, cudaEventDisableTiming));
-  }
   // check and refresh in one pass; the records it writes stand unless a
-  // rebuild follows
-  RepGeom const *geom = m_geom_d.as<RepGeom>();
-  int const nb = ceil_div(m_n, 256);
-  int *const flag = m_chk.as<int>() + m_chk_slot;
-  m_chk_slot ^= 1;
-  k_check_refresh<<<nb, 256, 0, st>>>(geom, m_rep_of.as<int>(), m_cinv.as<int>(), d_pos(), d_q(),
-                                      m_ckey.as<int>(), m_pos_ref.as<double>(), d_type(),
-                                      m_type_ref.as<int>(), m_n,
-                                      need_spq ? m_spq.as<double4>() : nullptr,
-                                      m_spf.as<float4>(), flag, m_chk.as<int>() + m_chk_slot);
+  // rebuild follows.  The host consumed the flag of the check before.
+  m_host_words[kFlagWord] = 0;
+  pdl_launch(k_check_refresh, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(),
+             m_rep_of.as<int>(), m_cinv.as<int>(), d_pos(), d_q(), m_ckey.as<int>(),
+             m_pos_ref.as<double>(), d_type(), m_type_ref.as<int>(), m_n,
+             need_spq ? m_spq.as<double4>() : nullptr, m_spf.as<float4>(),
+             m_host_words + kFlagWord);
   ++m_launches;
-  P3MX_CUDA(cudaMemcpyAsync(m_flag_host, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   P3MX_CUDA(cudaEventRecord(m_check_ev, st));
 }
 
@@ -1006,7 +1056,7 @@ void Engine::prepare_short_range(cudaStream_t st, bool need_spq) {
   bool rebuild = m_check_rebuild;
   if (!rebuild) {
     P3MX_CUDA(cudaEventSynchronize(m_check_ev));
-    rebuild = (*m_flag_host != 0);
+    rebuild = (m_host_words[kFlagWord] != 0);
   }
   mark("sr_check", st);
   if (rebuild) {
@@ -1023,8 +1073,9 @@ template <typename Real>
 void Engine::launch_fft_z_fwd(const Real *tiles, void *spectra, int sets, cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
   auto const kern = m_two[2] ? k_fft_z_fwd<Real, true> : k_fft_z_fwd<Real, false>;
-  kern<<<dim3(m_n_blk_zf, sets), 256, m_smem_zf, st>>>(
-      m_geom_d.as<RepGeom>(), m_blk_zf.as<Blk>(), tiles, m_tiles_n, m_cov.as<int>(), m_sb_edge,
+  pdl_launch(
+      kern, dim3(m_n_blk_zf, sets), 256, m_smem_zf, st, true, m_geom_d.as<RepGeom>(),
+      m_blk_zf.as<Blk>(), tiles, m_tiles_n, m_cov.as<int>(), m_sb_edge,
       static_cast<C *>(spectra), m_cplx, m_tw.as<C>());
   ++m_launches;
 }
@@ -1034,8 +1085,8 @@ void Engine::launch_fft_y(void *c0, long long field_stride, YPass const &job, bo
   using C = typename CplxOf<Real>::type;
   auto const kern = inv ? (m_two[1] ? k_fft_y<Real, true, true> : k_fft_y<Real, true, false>)
                         : (m_two[1] ? k_fft_y<Real, false, true> : k_fft_y<Real, false, false>);
-  kern<<<m_n_blk_y * job.n, 256, m_smem_y, st>>>(
-      m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(), static_cast<C *>(c0), field_stride, job, kscale,
+  pdl_launch(
+      kern, m_n_blk_y * job.n, 256, m_smem_y, st, true, m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(), static_cast<C *>(c0), field_stride, job, kscale,
       m_tile_y, m_tw.as<C>());
   ++m_launches;
 }
@@ -1044,8 +1095,8 @@ void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp,
                               int kscale, void *fields, cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
   auto const kern = m_two[2] ? k_fft_z_inv3<Real, true> : k_fft_z_inv3<Real, false>;
-  kern<<<dim3(m_n_blk_zi, sets), 256, m_smem_zi, st>>>(
-      m_geom_d.as<RepGeom>(), m_blk_zi.as<Blk>(), static_cast<C *>(c0), field_stride, zp, kscale,
+  pdl_launch(
+      kern, dim3(m_n_blk_zi, sets), 256, m_smem_zi, st, true, m_geom_d.as<RepGeom>(), m_blk_zi.as<Blk>(), static_cast<C *>(c0), field_stride, zp, kscale,
       static_cast<Real *>(fields), m_ebins, m_tw.as<C>());
   ++m_launches;
 }
@@ -1064,10 +1115,12 @@ void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t s
   RepGeom const *geom = m_geom_d.as<RepGeom>();
   int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes();
   auto go = [&](auto kern, auto const *pos, size_t smem) {
-    kern<<<m_n_blk_pair * lanes, 256, smem, st>>>(
-        geom, m_blk_pair.as<int2>(), pos, m_stype.as<int>(), m_cperm.as<int>(),
-        m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(), m_nb_cnt.as<int>(), f, overwrite ? 1 : 0,
-        m_part_pair.as<double>());
+    // not chained where the launch fills the GPU: its blocks would start in
+    // the interpolation's shared-memory configuration, with too little L1
+    // left for the position gathers (1.58 -> 1.80 ms per pass at 2^20 ions)
+    pdl_launch(kern, m_n_blk_pair * lanes, 256, smem, st, lanes > 1, geom, m_blk_pair.as<int2>(), pos,
+               m_stype.as<int>(), m_cperm.as<int>(), m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(),
+               m_nb_cnt.as<int>(), f, overwrite ? 1 : 0, m_part_pair.as<double>());
     ++m_launches;
   };
   size_t const nt2 = static_cast<size_t>(m_ntypes) * m_ntypes;
@@ -1209,7 +1262,7 @@ void Engine::short_range_graph(double *f, bool overwrite, cudaStream_t st) {
   k_fill_int<<<1, 32, 0, st>>>(flag, 0, 1, nullptr); ++m_launches;
   k_fill_int<<<ceil_div(R, 256), 256, 0, st>>>(rflag, 0, R, nullptr); ++m_launches;
   k_displacement_check<<<nb, 256, 0, st>>>(geom, m_rep_of.as<int>(), d_pos(), m_pos_ref.as<double>(),
-                                           d_type(), m_type_ref.as<int>(), m_n, flag, rflag);
+                                           d_type(), d_q(), m_type_ref.as<int>(), m_n, flag, rflag);
   ++m_launches;
   k_fill_int<<<ceil_div(m_oct_mult * m_cells + 1, 256), 256, 0, st>>>(m_ccnt.as<int>(), 0, m_oct_mult * m_cells + 1, flag); ++m_launches;
   k_cell_bin<<<nb, 256, 0, st>>>(geom, m_rep_of.as<int>(), d_pos(), d_q(), m_n, m_ckey.as<int>(),
@@ -1225,7 +1278,7 @@ void Engine::short_range_graph(double *f, bool overwrite, cudaStream_t st) {
                                      m_ntypes, m_n, m_nb.as<int>(), m_nb_cnt.as<int>(),
                                      m_overflow.as<int>(), flag, rflag); ++m_launches;
   k_copy_pos_ref<<<nb, 256, 0, st>>>(m_pos_ref.as<double>(), d_pos(), m_type_ref.as<int>(),
-                                     d_type(), m_rep_of.as<int>(), rflag, m_n,
+                                     d_type(), d_q(), m_rep_of.as<int>(), rflag, m_n,
                                      flag); ++m_launches;
   refresh_sorted_positions(st, !m_fp32);
   if (m_fp32)
@@ -1379,13 +1432,13 @@ double Engine::ks_error(const int *mesh, int cao, int n_c_part, double sum_q2, d
 }
 
 void Engine::check_kernel_error(cudaStream_t st) {
-  if (m_kerr.p == nullptr)
-    return;
-  int w[4] = {0, 0, 0, 0};
-  P3MX_CUDA(cudaMemcpyAsync(w, m_kerr.p, sizeof(w), cudaMemcpyDeviceToHost, st));
   P3MX_CUDA(cudaStreamSynchronize(st));
+  int w[4];
+  for (int k = 0; k < 4; ++k)
+    w[k] = m_host_words[k];
   if (w[0] || w[1]) {
-    P3MX_CUDA(cudaMemsetAsync(m_kerr.p, 0, sizeof(w), st));
+    for (int k = 0; k < 4; ++k)
+      m_host_words[k] = 0;
     if (w[0])
       throw Error(3, "a bulk copy into shared memory did not complete within the wait limit");
     // bond_error.cpp:28-35 and the zero-distance messages of fene.hpp /
@@ -1566,7 +1619,7 @@ void Engine::bond_forces(double *f, cudaStream_t st) {
     throw Error(2, "bonds were set for a different particle count");
   k_bond_forces<<<ceil_div(m_n, 256), 256, 0, st>>>(
       m_geom_d.as<RepGeom>(), m_rep_of.as<int>(), d_pos(), m_bstart.as<int>(), m_bent.as<int2>(),
-      m_bparam.as<BondParam>(), m_n, f, m_kerr.as<int>());
+      m_bparam.as<BondParam>(), m_n, f, kerr());
   ++m_launches;
 }
 
@@ -1580,7 +1633,7 @@ std::vector<double> Engine::bond_energies(cudaStream_t st) {
   e_pp.ensure(static_cast<size_t>(m_n) * sizeof(double));
   k_bond_energy_pp<<<ceil_div(m_n, 256), 256, 0, st>>>(
       m_geom_d.as<RepGeom>(), m_rep_of.as<int>(), d_pos(), m_bstart.as<int>(), m_bent.as<int2>(),
-      m_bparam.as<BondParam>(), m_n, e_pp.as<double>(), m_kerr.as<int>());
+      m_bparam.as<BondParam>(), m_n, e_pp.as<double>(), kerr());
   ++m_launches;
   std::vector<double> h(static_cast<size_t>(m_n));
   P3MX_CUDA(cudaMemcpyAsync(h.data(), e_pp.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1604,7 +1657,7 @@ void Engine::bond_observables(cudaStream_t st, double *energy, double *virial9) 
   k_bond_observables<<<nblk, 256, 0, st>>>(m_geom_d.as<RepGeom>(), m_rep_of.as<int>(), d_pos(),
                                            m_bstart.as<int>(), m_bent.as<int2>(),
                                            m_bparam.as<BondParam>(), m_n, m_bpart.as<double>(),
-                                           m_kerr.as<int>());
+                                           kerr());
   ++m_launches;
   std::vector<double> part(static_cast<size_t>(nblk) * 10);
   P3MX_CUDA(cudaMemcpyAsync(part.data(), m_bpart.p, part.size() * sizeof(double),

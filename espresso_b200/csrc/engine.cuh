@@ -165,7 +165,7 @@ private:
                                             cudaStream_t st);
   void prepare_short_range(cudaStream_t st, bool need_spq);
   // the list check of prepare_short_range issued early: its flag lands in
-  // pinned host memory behind m_check_ev, so the host can wait for it while
+  // mapped host memory ahead of m_check_ev, so the host can wait for it while
   // later work keeps the GPU busy; prepare_short_range consumes it
   void check_lists(cudaStream_t st, bool need_spq);
   void build_lists(cudaStream_t st);
@@ -177,6 +177,8 @@ private:
   // Counting sort by key (perm: sorted position -> particle); index_order
   // orders each bucket by particle index (deterministic), else the order
   // inside a bucket is that of the atomic slots.
+  template <typename Real> void bin_and_sort(unsigned *qmax_bits, int nq, cudaStream_t st);
+  bool m_cnt_dirty = true; // the brick counts are not known to be zero
   void sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, long long nkeys,
                  cudaStream_t st, const int *cond = nullptr, bool index_order = true);
 
@@ -239,20 +241,22 @@ private:
   DevBuf m_elc_epart;
   DevBuf m_nb, m_nb_cnt, m_overflow, m_pos_ref, m_flag, m_rflag, m_part_pair, m_sums_pair;
   DevBuf m_type_ref; // types at the last list build (a change triggers a rebuild)
-  // kernel error word: [0] a bounded wait ran out; [1] bond status (1 broken,
-  // 2 zero length), [2], [3] the two particles of the first failing bond
-  DevBuf m_kerr;
+  // Words in mapped host memory that kernels write and the host reads after
+  // an event or a synchronisation (no copy on the stream): the kernel error
+  // words [0] a bounded wait ran out, [1] bond status (1 broken, 2 zero
+  // length), [2], [3] the two particles of the first failing bond; and the
+  // list check's flag.
+  static constexpr int kFlagWord = 4, kHostWords = 8;
+  volatile int *m_host_words = nullptr;
+  int *kerr() const { return const_cast<int *>(m_host_words); }
   long long m_nbonds = 0, m_bond_n = 0; // bonds, particle count they were set for
   DevBuf m_bstart, m_bent, m_bparam, m_bpart;
   std::vector<int> m_cap; // neighbour capacity per replica
   bool m_lists_valid = false;
-  // pending early list check (check_lists): rebuild regardless, or read the
-  // flag copied to m_flag_host once m_check_ev has completed
+  // pending early list check (check_lists): rebuild regardless, or read its
+  // flag word once m_check_ev has completed
   bool m_check_pending = false, m_check_rebuild = false;
-  int *m_flag_host = nullptr;
   cudaEvent_t m_check_ev = nullptr;
-  DevBuf m_chk;       // the check's two flag words (slot m_chk_slot is next)
-  int m_chk_slot = 0;
   // misc host staging
   DevBuf m_ks_part;
 };

@@ -440,6 +440,7 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
             int E, typename CplxOf<Real>::type *__restrict__ cmesh, long long c_stride,
             const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ long long s_bx[kZfLines][3];
   __shared__ int s_by[kZfLines][3];
@@ -554,6 +555,7 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
         typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, YPass const job,
         int kscale, int tile, const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int const blk = blockIdx.x / job.n, jb = blockIdx.x - blk * job.n;
   Blk const bk = blks[blk];
@@ -627,6 +629,7 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
                double *__restrict__ partials,
                const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
@@ -766,6 +769,7 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              ZPass const zp, int kscale, Real *__restrict__ efield, long long e_stride,
              const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];

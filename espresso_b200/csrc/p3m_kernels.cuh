@@ -58,8 +58,12 @@ template <typename Real>
 __global__ void k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
                           const double *__restrict__ pos, long long n,
                           int *__restrict__ key, int *__restrict__ bkey, int *__restrict__ slot,
-                          int *__restrict__ cnt, Real *__restrict__ dist) {
+                          int *__restrict__ cnt, Real *__restrict__ dist,
+                          unsigned *__restrict__ zero, int nzero) {
+  pdl_enter();
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
+    zero[k] = 0u; // the |q| maxima that the weight kernel raises next
   if (i >= n)
     return;
   RepGeom const &G = reps[rep_of[i]];
@@ -151,6 +155,7 @@ k_p3m_weights(const RepGeom *__restrict__ reps, const int *__restrict__ perm,
   // addresses; a thread's own record would be 7 stores 112 bytes apart
   constexpr bool kStage = sizeof(Real) == 4;
   __shared__ __align__(16) Real s_rec[kStage ? 256 * kRecStride : 1];
+  pdl_enter();
   long long const s = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   int const lane = threadIdx.x & 31;
   if (s < n) {
@@ -373,6 +378,7 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_r0[kSbMaxRuns], s_r1[kSbMaxRuns];
   __shared__ int s_count;
+  pdl_enter();
   if (static_cast<int>(blockIdx.x) >= nsb)
     return; // whole block
   Word *tile = reinterpret_cast<Word *>(smem_raw);
@@ -702,6 +708,7 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long full[S], empty[S];
   __shared__ InterpInfo s_info[S];
+  pdl_enter();
   int const tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
 #pragma unroll

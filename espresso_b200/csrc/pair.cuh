@@ -693,6 +693,7 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
                   const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
                   const int *__restrict__ nb, const int *__restrict__ nb_cnt,
                   double *__restrict__ f, int overwrite, double *__restrict__) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PairF *ia = reinterpret_cast<PairF *>(smem_raw);
   for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
@@ -930,6 +931,7 @@ k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ 
                      const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
                      const int *__restrict__ nb, const int *__restrict__ nb_cnt,
                      double *__restrict__ f, int overwrite, double *__restrict__ partials) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PairIA *ia = reinterpret_cast<PairIA *>(smem_raw);
   for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
@@ -1017,6 +1019,7 @@ k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
               const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
               const int *__restrict__ nb, const int *__restrict__ nb_cnt, double *__restrict__ f,
               int overwrite, double *__restrict__ partials) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PairIA *ia = reinterpret_cast<PairIA *>(smem_raw);
   for (int k = threadIdx.x; k < ntypes * ntypes; k += blockDim.x)
@@ -1128,12 +1131,14 @@ k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
 // Largest squared displacement since the last list build, as a flag:
 // set when any particle moved more than skin/2 (check_resort_required,
 // CellStructure.hpp:393-401).
-// A particle whose type differs from its type at the last build also
-// triggers the rebuild: the lists hold per-type-pair cutoffs and the sorted
-// types (as the reference resorts on a particle type change).
+// A particle whose type differs from its type at the last build, or that
+// became charged or neutral, also triggers the rebuild: the lists hold
+// per-type-pair cutoffs, the sorted types and the Coulomb pairs of charged
+// particles (as the reference resorts on a particle change).
+__device__ inline int list_kind(int type, double q) { return 2 * type + (q != 0.0 ? 1 : 0); }
 __global__ void k_displacement_check(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
                                      const double *__restrict__ pos, const double *__restrict__ pos_ref,
-                                     const int *__restrict__ type,
+                                     const int *__restrict__ type, const double *__restrict__ q,
                                      const int *__restrict__ type_ref, long long n,
                                      int *__restrict__ flag, int *__restrict__ rflag) {
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1148,18 +1153,18 @@ __global__ void k_displacement_check(const RepGeom *__restrict__ reps, const int
     d2 += dx * dx;
   }
   double const lim = 0.5 * G.skin;
-  if (d2 > lim * lim || type[i] != type_ref[i]) {
+  if (d2 > lim * lim || list_kind(type[i], q[i]) != type_ref[i]) {
     atomicOr(flag, 1);
     if (rflag) // per-replica decision: only this replica rebuilds
       atomicOr(&rflag[r], 1);
   }
 }
 
-// Reference positions and types of the replicas that rebuilt (all when
-// rflag is null).
+// Reference positions and kinds (list_kind) of the replicas that rebuilt
+// (all when rflag is null).
 __global__ void k_copy_pos_ref(double *__restrict__ pos_ref, const double *__restrict__ pos,
                                int *__restrict__ type_ref, const int *__restrict__ type,
-                               const int *__restrict__ rep_of, const int *__restrict__ rflag,
+                               const double *__restrict__ q, const int *__restrict__ rep_of, const int *__restrict__ rflag,
                                long long n, const int *__restrict__ cond) {
   if (cond && !*cond)
     return;
@@ -1169,7 +1174,7 @@ __global__ void k_copy_pos_ref(double *__restrict__ pos_ref, const double *__res
 #pragma unroll
   for (int d = 0; d < 3; ++d)
     pos_ref[3 * i + d] = pos[3 * i + d];
-  type_ref[i] = type[i];
+  type_ref[i] = list_kind(type[i], q[i]);
 }
 
 } // namespace p3mx

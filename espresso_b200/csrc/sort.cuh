@@ -52,6 +52,7 @@ __device__ inline int block_excl_scan(int v, int &total) {
 __global__ void k_scan_tiles(const int *__restrict__ in, int *__restrict__ out,
                              int *__restrict__ tile_sums, long long n,
                              const int *__restrict__ cond) {
+  pdl_enter();
   if (cond && !*cond)
     return;
   long long const base = static_cast<long long>(blockIdx.x) * kScanTile +
@@ -80,6 +81,7 @@ __global__ void k_scan_tiles(const int *__restrict__ in, int *__restrict__ out,
 __global__ void k_scan_tile_sums(int *__restrict__ tile_sums, int ntiles,
                                  int *__restrict__ out, long long n,
                                  const int *__restrict__ cond) {
+  pdl_enter();
   if (cond && !*cond)
     return;
   int const per = (ntiles + blockDim.x - 1) / blockDim.x;
@@ -104,6 +106,7 @@ __global__ void k_scan_tile_sums(int *__restrict__ tile_sums, int ntiles,
 // Pass 3: add tile offsets.
 __global__ void k_scan_add(int *__restrict__ out, const int *__restrict__ tile_sums,
                            long long n, const int *__restrict__ cond) {
+  pdl_enter();
   if (cond && !*cond)
     return;
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -111,15 +114,21 @@ __global__ void k_scan_add(int *__restrict__ out, const int *__restrict__ tile_s
     out[i] += tile_sums[i / kScanTile];
 }
 
-// Place every item at start[key] + slot (slot from the counting atomics).
+// Place every item at start[key] + slot (slot from the counting atomics);
+// the nzero words at `zero` (the counts, already scanned) are cleared for the
+// next sort.
 __global__ void k_place(const int *__restrict__ key, const int *__restrict__ slot,
                         const int *__restrict__ start, int *__restrict__ perm,
-                        long long n, const int *__restrict__ cond) {
+                        long long n, const int *__restrict__ cond, int *__restrict__ zero,
+                        long long nzero) {
+  pdl_enter();
   if (cond && !*cond)
     return;
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n)
     perm[start[key[i]] + slot[i]] = static_cast<int>(i);
+  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
+    zero[k] = 0;
 }
 
 // Restore particle-index order inside every bucket (the atomic slots of the
@@ -244,6 +253,7 @@ constexpr long long kScanOneMax = 32LL * 32 * kScanOneRounds;
 __global__ void __launch_bounds__(1024) k_scan_one(const int *__restrict__ in,
                                                    int *__restrict__ out, long long n,
                                                    const int *__restrict__ cond) {
+  pdl_enter();
   if (cond && !*cond)
     return;
   int const lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -281,16 +291,18 @@ __global__ void __launch_bounds__(1024) k_scan_one(const int *__restrict__ in,
 // to kScanOneMax items, else three passes; returns the kernels launched.
 // `cond` (device int, may be NULL) skips the whole scan when zero, so the
 // scan can sit inside a captured CUDA graph behind a device-side decision.
+// chained: programmatic dependent launches (the kernel before is part of the
+// chain).
 inline int exclusive_scan(const int *in, int *out, int *tile_buf, long long n,
-                          cudaStream_t st, const int *cond = nullptr) {
+                          cudaStream_t st, const int *cond = nullptr, bool chained = false) {
   if (n <= kScanOneMax) {
-    k_scan_one<<<1, 1024, 0, st>>>(in, out, n, cond);
+    pdl_launch(k_scan_one, 1, 1024, 0, st, chained, in, out, n, cond);
     return 1;
   }
   int const ntiles = ceil_div(n, kScanTile);
-  k_scan_tiles<<<ntiles, kScanThreads, 0, st>>>(in, out, tile_buf, n, cond);
-  k_scan_tile_sums<<<1, 1024, 0, st>>>(tile_buf, ntiles, out, n, cond);
-  k_scan_add<<<ceil_div(n, 256), 256, 0, st>>>(out, tile_buf, n, cond);
+  pdl_launch(k_scan_tiles, ntiles, kScanThreads, 0, st, chained, in, out, tile_buf, n, cond);
+  pdl_launch(k_scan_tile_sums, 1, 1024, 0, st, chained, tile_buf, ntiles, out, n, cond);
+  pdl_launch(k_scan_add, ceil_div(n, 256), 256, 0, st, chained, out, tile_buf, n, cond);
   return 3;
 }
 

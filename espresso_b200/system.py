@@ -501,7 +501,8 @@ class System:
             h = solver._handle
             self._sync_pairs(h, t)
             self._sync_bonds(solver)
-            rc = lib.p3mx_forces(h, n, _lib.dptr(pos), _lib.dptr(q), _lib.dptr(t), _lib.dptr(f),
+            rc = lib.p3mx_forces(h, n, _lib.dptr(pos), _lib.dptr(q), _lib.dptr(t),
+                                 _lib.dptr(f) if forces else None,
                                  e3.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
                                  v27.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), flags, None)
             _lib.check(rc, h)
