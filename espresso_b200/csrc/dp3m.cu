@@ -3,10 +3,10 @@
 // (DipolarTuningAlgorithm, dp3m.cpp:535-660) and the device pipeline.
 //
 // Pipeline of one force/torque/energy evaluation (one cubic system):
-//  1. k_dp3m_prepare: moment components, list selector, census partials;
-//  2. brick binning and sort of the particles (once), weight records with
-//     q = mu_d for each component d = x, y, z, one super-brick assignment
-//     launch, one r2c z pass and one y pass over the three;
+//  1. k_dp3m_prepare: list selector, census partials;
+//  2. brick binning and sort of the particles into records with the three
+//     moment components as charges, one super-brick assignment launch, one
+//     r2c z pass and one y pass over the three;
 //  3. k_fft_x_dp3m (energy sum, five spectra), the backward y and z passes to
 //     the three torque fields and the six entries of the force-field tensor,
 //     and the back-interpolation of the nine with unit-charge weights;
@@ -67,13 +67,11 @@ public:
     size_t const csz = 2 * rsz;
     long long const nn = std::max<long long>(1, n);
     m_mu.ensure(3 * nn * sizeof(double));
-    m_comp.ensure(3 * nn * sizeof(double));
     m_out.ensure(9 * nn * sizeof(double));
     m_smu.ensure(nn * sizeof(double4));
     m_ck3.ensure(3 * E.m_cplx * csz);
     m_ge.ensure(E.m_cplx * rsz);
-    // three weight-record sets and tile sets for the one-launch assignment
-    m_W3.ensure(3 * static_cast<size_t>(kRecStride) * nn * rsz);
+    // three tile sets for the one-launch assignment
     m_tiles3.ensure(3 * static_cast<size_t>(E.m_tiles_n) * rsz);
     m_qmax3.ensure(4 * sizeof(unsigned));
     m_gf.ensure(E.m_cplx * rsz);
@@ -142,7 +140,7 @@ public:
     P3MX_CUDA(cudaMemcpyAsync(m_mu.p, dip, 3 * n * sizeof(double), k, st));
     P3MX_CUDA(cudaMemsetAsync(m_flag.p, 0, sizeof(int), st));
     int const nb = static_cast<int>(ceil_div(n, 256));
-    k_dp3m_prepare<<<nb, 256, 0, st>>>(n, m_mu.as<double>(), m_comp.as<double>(), E.d_q(),
+    k_dp3m_prepare<<<nb, 256, 0, st>>>(n, m_mu.as<double>(), E.d_q(),
                                        m_flag.as<int>(), m_part.as<double>());
     ++E.m_launches;
     k_dp3m_sum_rows<<<1, 32 * 5, 0, st>>>(m_part.as<double>(), nb, 5, m_sums.as<double>());
@@ -170,47 +168,28 @@ public:
       m_g_valid = true;
     }
     // 1. brick binning and sort (shared by the three components)
-    unsigned *qmax_bits = reinterpret_cast<unsigned *>(E.m_cnt.as<int>() + E.m_nkeys + 1);
-    int const nb = static_cast<int>(ceil_div(n, 256));
-    E.bin_and_sort<Real>(qmax_bits, 1, st);
-    E.mark("dp_sort", st);
-    // 2. the three component meshes: weight records per component, then one
-    // assignment and one z pass over all three (blockIdx.y = component)
-    C *ck3 = m_ck3.as<C>();
-    long long const wst = static_cast<long long>(kRecStride) * n;
+    // records with the three moment components as charges
     unsigned *qmax3 = m_qmax3.as<unsigned>();
-    P3MX_CUDA(cudaMemsetAsync(qmax3, 0, 3 * sizeof(unsigned), st));
-    for (int d = 0; d < 3; ++d) {
-      k_p3m_weights<Real><<<nb, 256, 0, st>>>(geom, E.m_perm.as<int>(), E.m_key.as<int>(),
-                                              E.m_dist.as<Real>(), m_comp.as<double>() + d * n,
-                                              E.m_rep_of.as<int>(), n, m_W3.as<Real>() + d * wst,
-                                              E.m_skey.as<int>(), qmax3 + d);
-      ++E.m_launches;
-    }
+    E.bin_and_sort<Real>(m_mu.as<double>(), 3, qmax3, st);
+    E.mark("dp_sort", st);
+    // 2. the three component meshes: one assignment and one z pass over all
+    // three (blockIdx.y = component)
+    C *ck3 = m_ck3.as<C>();
     for (int c = 1; c <= 7; ++c) {
       int const cnt = E.m_sb_off[c + 1] - E.m_sb_off[c];
       if (cnt == 0)
         continue;
       int2 const *tab = E.m_blk_mesh.as<int2>() + E.m_sb_off[c];
       P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(E.m_sb_edge, cnt, st, geom, tab,
-                                                     E.m_start.as<int>(), m_W3.as<Real>(),
-                                                     E.m_skey.as<int>(), qmax3,
-                                                     m_tiles3.as<Real>(), E.kerr(), 3,
-                                                     wst, E.m_tiles_n, 1)));
+                                                     E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(),
+                                                     qmax3, m_tiles3.as<Real>(), E.kerr(), 3,
+                                                     E.m_tiles_n, 1)));
       ++E.m_launches;
     }
     E.launch_fft_z_fwd<Real>(m_tiles3.as<Real>(), ck3, 3, st);
     E.mark("dp_assign_fft_z", st);
     E.launch_fft_y<Real>(ck3, E.m_cplx, y_plain(3), false, 0, st);
-    // unit-charge weights of the magnetic particles (selector) for the
-    // back-interpolation
-    if (want_ft) {
-      k_p3m_weights<Real><<<nb, 256, 0, st>>>(geom, E.m_perm.as<int>(), E.m_key.as<int>(),
-                                              E.m_dist.as<Real>(), E.d_q(), E.m_rep_of.as<int>(), n,
-                                              E.m_W.as<Real>(), E.m_skey.as<int>(), qmax_bits);
-      ++E.m_launches;
-    }
-    E.mark("dp_fft_y_weights", st);
+    E.mark("dp_fft_y", st);
     // 3. one x pass, backward y and z passes over the nine fields, one
     // interpolation of the three field sets
     if (!want_ft && !want_e)
@@ -249,12 +228,12 @@ public:
       if (nbr == 0)
         continue;
       int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
-      P3MX_CAO_DISPATCH_R(c, (k_p3m_interp<Real, P><<<dim3(ceil_div(interp_grid<Real, P>(3 * nbr), 3), 3),
-                                 32 * (1 + kInterpWarps), interp_smem<Real, P>(), st>>>(
-                                 gi, tab, nbr, E.m_start.as<int>(), E.m_perm.as<int>(),
-                                 E.m_skey.as<int>(), E.m_W.as<Real>(), E.m_tmap.as<CUtensorMap>(),
-                                 1, E.d_q(), E.m_dipole.as<double>(), out, 3 * n, 1,
-                                 E.kerr())));
+      P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>,
+                                 dim3(ceil_div(interp_grid<Real, P>(3 * nbr), 3), 3),
+                                 32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true, gi, tab,
+                                 nbr, E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(), 1,
+                                 E.m_tmap.as<CUtensorMap>(), 1, E.d_q(), E.m_dipole.as<double>(),
+                                 out, 3 * n, 1, E.kerr())));
       ++E.m_launches;
     }
     E.mark("dp_interp", st);
@@ -432,8 +411,8 @@ public:
 
 private:
   Engine m_eng;
-  DevBuf m_mu, m_comp, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
-  DevBuf m_W3, m_tiles3, m_qmax3;
+  DevBuf m_mu, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
+  DevBuf m_tiles3, m_qmax3;
   bool m_g_valid = false, m_phi_valid = false, m_table_set = false;
   double m_phi = 0.0;
   int m_M = 0, m_cao = 0;

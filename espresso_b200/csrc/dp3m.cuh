@@ -167,21 +167,17 @@ __global__ void k_dp3m_ks_error(int M, int cao, double alpha_L, double *__restri
   }
 }
 
-// Dipole moments (AoS, 3 per particle) -> the three components as separate
-// arrays (the charge slot of the assignment weights), the list selector
+// Dipole moments (AoS, 3 per particle) -> the list selector
 // sel = 1 for a particle with a non-zero moment (0 otherwise: it has no
 // real-space partners), a flag set when a selector changed since the last
 // call, and per-block partials {n_dipoles, sum mu^2, M_x, M_y, M_z}.
 __global__ void k_dp3m_prepare(long long n, const double *__restrict__ mu,
-                               double *__restrict__ comp, double *__restrict__ sel,
+                               double *__restrict__ sel,
                                int *__restrict__ sel_changed, double *__restrict__ partials) {
   double acc[5] = {0, 0, 0, 0, 0};
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) {
     double const m0 = mu[3 * i], m1 = mu[3 * i + 1], m2 = mu[3 * i + 2];
-    comp[i] = m0;
-    comp[n + i] = m1;
-    comp[2 * n + i] = m2;
     double const m2s = m0 * m0 + m1 * m1 + m2 * m2;
     double const s = (m2s != 0.0) ? 1.0 : 0.0;
     if (sel[i] != s) {

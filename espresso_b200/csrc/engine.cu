@@ -523,10 +523,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_type.ensure(n * sizeof(int));
   m_force.ensure(3 * n * sizeof(double));
   m_key.ensure(n * sizeof(int));
-  m_bkey.ensure(n * sizeof(int));
   m_slot.ensure(n * sizeof(int));
-  // + 8: the back-interpolation copies 16-byte aligned windows of these
-  m_perm.ensure((n + 8) * sizeof(int));
   // sort-brick counts, then one word per replica: the bits of its largest
   // |q| (FP32, rounded up), which the assignment's fixed-point scale needs
   m_cnt.ensure((m_nkeys + 1 + R) * sizeof(int));
@@ -534,8 +531,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_start.ensure((m_nkeys + 1) * sizeof(int));
   m_scan_tiles.ensure((ceil_div(std::max(m_nkeys, m_oct_mult * m_cells) + 1, kScanTile) + 1) * sizeof(int));
   m_dist.ensure(3 * n * rsz);
-  m_W.ensure(static_cast<size_t>(wstride<7, 4>()) * n * rsz);
-  m_skey.ensure((n + 8) * sizeof(int));
+  m_rec.ensure(n * (m_fp32 ? sizeof(PRec<float>) : sizeof(PRec<double>)));
   m_tiles.ensure(static_cast<size_t>(m_tiles_n) * rsz);
   m_E.ensure(4 * m_ebins * rsz);
   encode_field_maps(st);
@@ -652,35 +648,39 @@ void Engine::census(cudaStream_t st) {
 }
 
 void Engine::sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, long long nkeys,
-                       cudaStream_t st, const int *cond, bool index_order) {
-  m_launches += exclusive_scan(cnt, start, m_scan_tiles.as<int>(), nkeys, st, cond, !index_order);
-  pdl_launch(k_place, ceil_div(m_n, 256), 256, 0, st, !index_order, key, slot, start, perm, m_n,
-             cond, index_order ? nullptr : cnt, index_order ? 0 : nkeys + 1);
-  ++m_launches;
-  if (!index_order)
-    return;
+                       cudaStream_t st, const int *cond) {
+  m_launches += exclusive_scan(cnt, start, m_scan_tiles.as<int>(), nkeys, st, cond);
+  k_place<<<ceil_div(m_n, 256), 256, 0, st>>>(key, slot, start, perm, m_n, cond); ++m_launches;
   k_fix_buckets<<<ceil_div(nkeys * 32, 256), 256, 0, st>>>(start, perm, nkeys, cond); ++m_launches;
   k_fix_big_buckets<<<static_cast<int>(std::min<long long>(ceil_div(nkeys, 256), 296)), 256, 0,
                       st>>>(
       start, perm, nkeys, cond); ++m_launches;
 }
 
-// Corner binning and the brick sort of the particles (qmax_bits: the words the
-// weight kernel raises, cleared here).  The brick counts are zero on entry
-// (cleared by the sort before; by a memset after a failed one).
-template <typename Real> void Engine::bin_and_sort(unsigned *qmax_bits, int nq, cudaStream_t st) {
+// Corner binning and brick sort of the particles into records; q holds nc (1
+// or 3) charges per particle, qmax receives nc words per replica.  The brick
+// counts are zero on entry (cleared by the sort before; by a memset after a
+// failed one).  The order inside a brick is left as the atomic slots made
+// it: the fixed-point assignment sums integers and the interpolation treats
+// every particle on its own, so the results do not depend on it.
+template <typename Real>
+void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t st) {
+  int const R = n_rep();
+  const int *rep_of = R > 1 ? m_rep_of.as<int>() : nullptr;
   if (m_cnt_dirty)
     P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
   m_cnt_dirty = true;
-  pdl_launch(k_p3m_bin<Real>, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(),
-             m_rep_of.as<int>(), d_pos(), m_n, m_key.as<int>(), m_bkey.as<int>(), m_slot.as<int>(),
-             m_cnt.as<int>(), m_dist.as<Real>(), qmax_bits, nq);
+  pdl_launch(k_p3m_bin<Real>, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(), rep_of,
+             d_pos(), m_n, m_key.as<int>(), m_slot.as<int>(), m_cnt.as<int>(), m_dist.as<Real>(),
+             qmax, nc * R);
   ++m_launches;
-  // the order inside a brick is left as the atomic slots made it: the
-  // fixed-point assignment sums integers and the interpolation treats
-  // every particle on its own, so the results do not depend on it
-  sort_keys(m_bkey.as<int>(), m_slot.as<int>(), m_cnt.as<int>(), m_start.as<int>(),
-            m_perm.as<int>(), m_nkeys, st, nullptr, false);
+  m_launches += exclusive_scan(m_cnt.as<int>(), m_start.as<int>(), m_scan_tiles.as<int>(), m_nkeys,
+                               st, nullptr, true);
+  pdl_launch(nc == 1 ? k_p3m_place<Real, 1> : k_p3m_place<Real, 3>, ceil_div(m_n, 256), 256, 0, st,
+             true, m_geom_d.as<RepGeom>(), rep_of, R, m_key.as<int>(), m_slot.as<int>(),
+             m_start.as<int>(), m_dist.as<Real>(), q, m_n, m_rec.as<PRec<Real>>(), qmax,
+             m_cnt.as<int>(), m_nkeys + 1);
+  ++m_launches;
   m_cnt_dirty = false;
 }
 
@@ -736,16 +736,16 @@ void Engine::encode_field_maps(cudaStream_t st, int sets) {
 
 namespace {
 // The charge assignment of cnt super-bricks of edge E (16 or 8); ncomp charge
-// sets (records, tiles and |q| maxima comp_w / comp_tile / comp_q apart).
+// sets (tiles and |q| maxima comp_tile / comp_q apart).
 template <typename Real, int P>
 void launch_assign(int edge, int cnt, cudaStream_t st, RepGeom const *geom, int2 const *tab,
-                   int const *start, Real const *W, int const *s_key, unsigned const *qmax_bits,
-                   Real *tiles, int *err, int ncomp = 1, long long comp_w = 0,
-                   long long comp_tile = 0, int comp_q = 0) {
+                   int const *start, PRec<Real> const *recs, unsigned const *qmax_bits,
+                   Real *tiles, int *err, int ncomp = 1, long long comp_tile = 0,
+                   int comp_q = 0) {
   auto go = [&](auto kern, size_t smem) {
     pdl_launch(kern, dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp)), 32 * kSbWarps,
-               smem, st, true, geom, tab, cnt, start, W, s_key, qmax_bits, tiles, err, comp_w,
-               comp_tile, comp_q);
+               smem, st, true, geom, tab, cnt, start, recs, qmax_bits, tiles, err, comp_tile,
+               comp_q);
   };
   if (edge == kSbEdgeSmall)
     go(ncomp > 1 ? k_p3m_assign_sb<Real, P, kSbEdgeSmall, true>
@@ -799,17 +799,12 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     m_ginf_valid = true;
   }
   mark("start", st);
-  // 1. corner binning, brick sort, weight records.  From here on every kernel
-  // is a programmatic dependent of the one before
+  // 1. corner binning and brick sort.  From here on every kernel is a
+  // programmatic dependent of the one before
   unsigned *qmax_bits = reinterpret_cast<unsigned *>(m_cnt.as<int>() + m_nkeys + 1);
   if (m_n > 0) {
-    bin_and_sort<Real>(qmax_bits, R, st);
+    bin_and_sort<Real>(d_q(), 1, qmax_bits, st);
     mark("p3m_sort", st);
-    pdl_launch(k_p3m_weights<Real>, ceil_div(m_n, 256), 256, 0, st, true, geom, m_perm.as<int>(),
-               m_key.as<int>(), m_dist.as<Real>(), d_q(), m_rep_of.as<int>(), m_n, m_W.as<Real>(),
-               m_skey.as<int>(), qmax_bits);
-    ++m_launches;
-    mark("p3m_weights", st);
   } else {
     P3MX_CUDA(cudaMemsetAsync(m_start.p, 0, (m_nkeys + 1) * sizeof(int), st));
     P3MX_CUDA(cudaMemsetAsync(qmax_bits, 0, R * sizeof(int), st));
@@ -821,7 +816,7 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
       continue;
     int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
     P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, geom, tab, m_start.as<int>(),
-                                                   m_W.as<Real>(), m_skey.as<int>(), qmax_bits,
+                                                   m_rec.as<PRec<Real>>(), qmax_bits,
                                                    m_tiles.as<Real>(), kerr())));
     ++m_launches;
   }
@@ -862,9 +857,8 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     int2 const *tab = m_blk_brick.as<int2>() + m_brick_off[c];
     P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>, interp_grid<Real, P>(nbr),
                                32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true,
-                               geom, tab, nbr, m_start.as<int>(), m_perm.as<int>(),
-                               m_skey.as<int>(), m_W.as<Real>(), m_tmap.as<CUtensorMap>(), 0,
-                               d_q(), m_dipole.as<double>(), f, 0, overwrite ? 1 : 0, kerr())));
+                               geom, tab, nbr, m_start.as<int>(), m_rec.as<PRec<Real>>(), 0,
+                               m_tmap.as<CUtensorMap>(), 0, d_q(), m_dipole.as<double>(), f, 0, overwrite ? 1 : 0, kerr())));
     ++m_launches;
   }
   mark("p3m_interp", st);

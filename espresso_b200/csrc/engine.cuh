@@ -174,13 +174,13 @@ private:
   void encode_field_maps(cudaStream_t st, int sets = 1);
   // want_spq: also the FP64 double4 positions (FP64 pair kernel)
   void refresh_sorted_positions(cudaStream_t st, bool want_spq = true);
-  // Counting sort by key (perm: sorted position -> particle); index_order
-  // orders each bucket by particle index (deterministic), else the order
-  // inside a bucket is that of the atomic slots.
-  template <typename Real> void bin_and_sort(unsigned *qmax_bits, int nq, cudaStream_t st);
+  // Counting sort by key (perm: sorted position -> particle), each bucket
+  // ordered by particle index (deterministic).
+  template <typename Real>
+  void bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t st);
   bool m_cnt_dirty = true; // the brick counts are not known to be zero
   void sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, long long nkeys,
-                 cudaStream_t st, const int *cond = nullptr, bool index_order = true);
+                 cudaStream_t st, const int *cond = nullptr);
 
   void mark(const char *name, cudaStream_t st);
 
@@ -225,8 +225,8 @@ private:
   // particles
   DevBuf m_pos, m_q, m_type, m_force;
   // p3m
-  DevBuf m_key, m_bkey, m_slot, m_cnt, m_start, m_perm, m_scan_tiles;
-  DevBuf m_dist, m_W, m_skey;
+  DevBuf m_key, m_slot, m_cnt, m_start, m_scan_tiles;
+  DevBuf m_dist, m_rec; // distances to the mesh points; brick-sorted records
   DevBuf m_rho; // charge mesh of one replica (mesh_copy only)
   DevBuf m_tiles, m_ck, m_field, m_E, m_ginf;
   DevBuf m_tmap; // per replica: tensor map of its field mesh (interpolation tiles)

@@ -24,49 +24,92 @@ __device__ inline double fold_coord(double x, double L) {
 }
 
 // Cardinal B-spline weights of order P at the P points around a particle
-// (x = distance to the nearest mesh point, [-0.5, 0.5]) by the Cox-de Boor
-// recursion; w[i] = M_P(x + 1/2 + P-1-i), the values tabulated in
-// utils/math/bspline.hpp:30-177.
-template <int P, typename Real>
-__device__ inline void bspline_weights(Real x, Real *w) {
-  Real c[P];
-  Real const u = x + Real(0.5);
-  c[0] = Real(1);
-#pragma unroll
-  for (int n = 1; n < P; ++n) {
-    Real const inv_n = Real(1) / Real(n);
-    c[n] = Real(0);
-#pragma unroll
-    for (int k = n; k >= 0; --k) {
-      Real const left = (k > 0) ? c[k - 1] : Real(0);
-      c[k] = ((u + Real(k)) * c[k] + (Real(n + 1) - u - Real(k)) * left) * inv_n;
+// (x = distance to the nearest mesh point, [-0.5, 0.5]): w[i] = M_P(x + 1/2 +
+// P-1-i), the values tabulated in utils/math/bspline.hpp:30-177.  Weight i is
+// one polynomial in x; its coefficients follow from
+//   M_P(t) = sum_l (-1)^l binom(P, l) max(t - l, 0)^(P-1) / (P-1)!
+// (every term a dyadic fraction, exact in FP64 before the division).
+struct SplineTable {
+  double c[8][8][8]; // [order][weight][power of x]
+};
+constexpr SplineTable spline_table() {
+  SplineTable t{};
+  for (int P = 1; P <= 7; ++P) {
+    double binom_p[8] = {1}, binom_n[8] = {1}, fact = 1.0;
+    for (int k = 1; k <= P; ++k)
+      binom_p[k] = binom_p[k - 1] * (P - k + 1) / k;
+    for (int k = 1; k < P; ++k) {
+      binom_n[k] = binom_n[k - 1] * (P - k) / k;
+      fact *= k;
     }
+    for (int i = 0; i < P; ++i)
+      for (int m = 0; m < P; ++m) {
+        int const j = P - 1 - i;
+        double sum = 0.0;
+        for (int l = 0; l <= j; ++l) {
+          double pw = 1.0;
+          for (int e = 0; e < P - 1 - m; ++e)
+            pw *= 0.5 + j - l;
+          sum += ((l & 1) ? -1.0 : 1.0) * binom_p[l] * pw;
+        }
+        t.c[P][i][m] = binom_n[m] * sum / fact;
+      }
   }
-#pragma unroll
-  for (int i = 0; i < P; ++i)
-    w[i] = c[P - 1 - i];
+  return t;
 }
+__constant__ SplineTable kSpline = spline_table();
+// Weight i of order P at x, coefficients c[0 .. P-1].
+template <int P, typename Real> __device__ inline Real spline_eval(const Real *c, Real x) {
+  Real w = c[P - 1];
+#pragma unroll
+  for (int m = P - 2; m >= 0; --m)
+    w = w * x + c[m];
+  return w;
+}
+template <int P, typename Real> __device__ inline void spline_coef(int i, Real *c) {
+#pragma unroll
+  for (int m = 0; m < P; ++m)
+    c[m] = static_cast<Real>(kSpline.c[P][i][m]);
+}
+
+// Record of a particle in brick-sorted order: the distances to its nearest
+// mesh point, up to three charges (a charge, or the moment components), the
+// corner key inside the replica and the particle index -- one 32-byte sector
+// in FP32.  The assignment and the interpolation compute the 3 P stencil
+// weights from it in shared memory (8 lanes per particle, one weight of each
+// axis per lane): the weight records they replace were 112 bytes, written by
+// a gathering kernel and read twice.
+template <typename Real> struct PRec;
+template <> struct __align__(32) PRec<float> {
+  float d[3], q[3];
+  int key, idx;
+};
+template <> struct __align__(64) PRec<double> {
+  double d[3], q[3];
+  int key, idx;
+  double pad;
+};
 
 // Per particle: nearest-mesh-point corner and the distance to it, following
 // p3m_calculate_interpolation_weights (p3m/interpolation.hpp:138-178) with
 // the single-rank CA-mesh origin of P3MLocalMesh (p3m/common.cpp:34-106).
-// key = corner, brick-major: bin_off + brick*B^3 + (lx*B + ly)*B + lz with
+// key = corner, brick-major: brick*B^3 + (lx*B + ly)*B + lz with
 // brick = (bx*nby + by)*nbz + bz and (lx, ly, lz) the corner inside it; the
-// sort key bkey = brk_off + brick, so the particles of one brick form one
-// contiguous range of the sorted order (particle index order inside it).
+// sort key is brk_off + brick, so the particles of one brick form one
+// contiguous range of the sorted order.  rep_of: nullptr for one replica.
 template <typename Real>
 __global__ void k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
                           const double *__restrict__ pos, long long n,
-                          int *__restrict__ key, int *__restrict__ bkey, int *__restrict__ slot,
+                          int *__restrict__ key, int *__restrict__ slot,
                           int *__restrict__ cnt, Real *__restrict__ dist,
                           unsigned *__restrict__ zero, int nzero) {
   pdl_enter();
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
-    zero[k] = 0u; // the |q| maxima that the weight kernel raises next
+    zero[k] = 0u; // the |q| maxima that the placing kernel raises next
   if (i >= n)
     return;
-  RepGeom const &G = reps[rep_of[i]];
+  RepGeom const &G = reps[rep_of ? rep_of[i] : 0];
   int g[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -82,119 +125,59 @@ __global__ void k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restric
   }
   int const B = G.brick;
   int const brick = ((g[0] / B) * G.nby + g[1] / B) * G.nbz + g[2] / B;
-  int const k = static_cast<int>(G.bin_off) + brick * B * B * B +
-                ((g[0] % B) * B + g[1] % B) * B + g[2] % B;
-  key[i] = k;
-  int const b = static_cast<int>(G.brk_off) + brick;
-  bkey[i] = b;
-  slot[i] = atomicAdd(&cnt[b], 1);
+  key[i] = brick * B * B * B + ((g[0] % B) * B + g[1] % B) * B + g[2] % B;
+  slot[i] = atomicAdd(&cnt[static_cast<int>(G.brk_off) + brick], 1);
 }
 
-// Per-particle weight record for order P (R = 4):
-// {q*wx[0..P), wy[0..P), 0[R-1], wz[0..P), 0[R-1]}, zero-padded; the stride
-// is a multiple of 4 elements (16 bytes in FP32, 32 in FP64) so that records
-// are stored as vectors and runs of records are legal 16-byte asynchronous
-// copies.
-template <int P, int R> __host__ __device__ constexpr int wstride() {
-  return (3 * P + 2 * (R - 1) + 3) / 4 * 4;
-}
-template <int P, int R> __host__ __device__ constexpr int wz_off() { return 2 * P + (R - 1); }
-// Record stride of every order (that of order 7), so that replicas of one
-// batch may use different orders: a sorted particle's record starts at
-// s * kRecStride whatever its replica's order.
-constexpr int kRecStride = wstride<7, 4>();
-
-// Weight record of one sorted particle for order P (R = 4):
-// {q*wx[0..P), wy[0..P), 0[R-1], wz[0..P), 0[R-1]}, zero-padded to the
-// common stride kRecStride, stored as 16- or 32-byte vectors.
-template <typename Real, int P>
-__device__ inline void weights_record(const Real *dist3, double q, Real *__restrict__ out) {
-  constexpr int R = 4;
-  Real w[3][P];
-  bspline_weights<P>(dist3[0], w[0]);
-  bspline_weights<P>(dist3[1], w[1]);
-  bspline_weights<P>(dist3[2], w[2]);
-  Real const qi = static_cast<Real>(q);
-  constexpr int WS = kRecStride;
-  Real rec[WS];
-#pragma unroll
-  for (int k = 0; k < WS; ++k)
-    rec[k] = Real(0);
-#pragma unroll
-  for (int k = 0; k < P; ++k) {
-    rec[k] = qi * w[0][k];
-    rec[P + k] = w[1][k];
-    rec[wz_off<P, R>() + k] = w[2][k];
-  }
-  using R4 = typename Real4Of<Real>::type;
-  R4 *o = reinterpret_cast<R4 *>(out);
-#pragma unroll
-  for (int k = 0; k < WS / 4; ++k) {
-    R4 v;
-    v.x = rec[4 * k];
-    v.y = rec[4 * k + 1];
-    v.z = rec[4 * k + 2];
-    v.w = rec[4 * k + 3];
-    o[k] = v;
-  }
-}
-
-// Weights in brick-sorted order (each replica's order), the corner key
-// (relative to the replica's corner range) of every sorted particle, and
-// each replica's largest |q| (FP32 bits rounded up, atomic maximum:
-// order-independent) for the fixed-point scale of the charge assignment.
-template <typename Real>
+// Every particle's record to its sorted place (start of its brick plus the
+// slot from the counting atomics), and each replica's largest |q| per charge
+// (FP32 bits rounded up, atomic maximum: order-independent; set c at
+// qmax_bits + c * n_rep) for the fixed-point scale of the charge assignment.
+// NC charges per particle, q[NC i + c].  The nzero words at `zero` (the brick
+// counts, already scanned) are cleared for the next sort.  A particle is one
+// full 32-byte sector (FP32) written at random: the gathering weight kernel
+// it replaces read five random sectors and wrote 112 bytes.
+template <typename Real, int NC>
 __global__ void __launch_bounds__(256)
-k_p3m_weights(const RepGeom *__restrict__ reps, const int *__restrict__ perm,
-              const int *__restrict__ key, const Real *__restrict__ dist,
-              const double *__restrict__ q, const int *__restrict__ rep_of,
-              long long n, Real *__restrict__ W, int *__restrict__ s_key,
-              unsigned *__restrict__ qmax_bits) {
-  // FP32 records are built in shared memory and each warp's 32 records
-  // (contiguous in W) leave with 16-byte lane stores of consecutive
-  // addresses; a thread's own record would be 7 stores 112 bytes apart
-  constexpr bool kStage = sizeof(Real) == 4;
-  __shared__ __align__(16) Real s_rec[kStage ? 256 * kRecStride : 1];
+k_p3m_place(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, int n_rep,
+            const int *__restrict__ key, const int *__restrict__ slot,
+            const int *__restrict__ start, const Real *__restrict__ dist,
+            const double *__restrict__ q, long long n, PRec<Real> *__restrict__ rec,
+            unsigned *__restrict__ qmax_bits, int *__restrict__ zero, long long nzero) {
   pdl_enter();
-  long long const s = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  int const lane = threadIdx.x & 31;
-  if (s < n) {
-    int const i = perm[s];
-    int const rep = rep_of[i];
-    RepGeom const &G = reps[rep];
-    {
-      // one atomic per group of lanes of the same replica
-      unsigned const qb = __float_as_uint(__double2float_ru(fabs(q[i])));
-      unsigned const act = __activemask();
-      unsigned const grp = __match_any_sync(act, rep);
-      unsigned const mx = __reduce_max_sync(grp, qb);
-      if (lane == __ffs(grp) - 1)
-        atomicMax(&qmax_bits[rep], mx);
-    }
-    Real *out = kStage ? s_rec + threadIdx.x * kRecStride : W + s * kRecStride;
-    const Real *d3 = dist + 3 * i;
-    switch (G.cao) {
-    case 1: weights_record<Real, 1>(d3, q[i], out); break;
-    case 2: weights_record<Real, 2>(d3, q[i], out); break;
-    case 3: weights_record<Real, 3>(d3, q[i], out); break;
-    case 4: weights_record<Real, 4>(d3, q[i], out); break;
-    case 5: weights_record<Real, 5>(d3, q[i], out); break;
-    case 6: weights_record<Real, 6>(d3, q[i], out); break;
-    default: weights_record<Real, 7>(d3, q[i], out); break;
-    }
-    s_key[s] = key[i] - static_cast<int>(G.bin_off);
+  long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
+    zero[k] = 0;
+  if (i >= n)
+    return;
+  int const rep = rep_of ? rep_of[i] : 0;
+  RepGeom const &G = reps[rep];
+  PRec<Real> r;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    r.d[d] = dist[3 * i + d];
+    r.q[d] = Real(0);
   }
-  if constexpr (kStage) {
-    __syncwarp();
-    long long const s0 = s - lane;
-    if (s0 >= n)
-      return;
-    int const nv = static_cast<int>(min(32LL, n - s0));
-    const float4 *src = reinterpret_cast<const float4 *>(s_rec + (threadIdx.x - lane) * kRecStride);
-    float4 *dst = reinterpret_cast<float4 *>(W + s0 * kRecStride);
-    for (int k = lane; k < nv * (kRecStride / 4); k += 32)
-      dst[k] = src[k];
+  r.key = key[i];
+  r.idx = static_cast<int>(i);
+  unsigned const act = __activemask();
+  unsigned const grp = __match_any_sync(act, rep);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    double const qi = q[NC * i + c];
+    r.q[c] = static_cast<Real>(qi);
+    // one atomic per group of lanes of the same replica, and only where the
+    // maximum seen so far is smaller
+    unsigned const mx =
+        __reduce_max_sync(grp, __float_as_uint(__double2float_ru(fabs(qi))));
+    unsigned *const w = qmax_bits + c * n_rep + rep;
+    if (static_cast<int>(threadIdx.x & 31) == __ffs(grp) - 1 &&
+        mx > *reinterpret_cast<volatile unsigned *>(w))
+      atomicMax(w, mx);
   }
+  int const lb = G.brick == 4 ? 6 : 9; // log2 of the corners per brick
+  int const s = start[static_cast<int>(G.brk_off) + (r.key >> lb)] + slot[i];
+  rec[s] = r;
 }
 
 // Edge (mesh points) of the sort bricks that bin the particles by stencil
@@ -322,13 +305,14 @@ template <int P, int WB, int E> __host__ __device__ constexpr TileStrides sb_str
 template <typename Real, int P, int E> __host__ __device__ constexpr size_t sb_tile_bytes() {
   using W = typename SbWord<Real>::type;
   return (sizeof(W) * sb_tile_edge<P, E>() * static_cast<size_t>(sb_strides<P, sizeof(W), E>().sx) +
-          15) / 16 * 16;
+          63) / 64 * 64;
 }
-// shared memory: tile, staged weight records, per staged particle its z
-// weights times S in FP64 (8 slots) and its tile offset
+// shared memory: tile, staged records, per staged particle its z weights
+// times S in FP64, its x weights times the charge and its y weights (8 slots
+// each), and its tile offset
 template <typename Real, int P, int E> __host__ __device__ constexpr size_t sb_smem() {
-  return sb_tile_bytes<Real, P, E>() + sizeof(Real) * kSbChunk * kRecStride +
-         sizeof(double) * 8 * kSbChunk + sizeof(int) * kSbChunk;
+  return sb_tile_bytes<Real, P, E>() + (sizeof(PRec<Real>) + 8 * sizeof(double) +
+                                        16 * sizeof(Real) + sizeof(int)) * kSbChunk;
 }
 // The stored tiles of a replica, TE = E + P - 1 points per edge, z rows
 // padded to TZ values (a multiple of 4): value (lx, ly, lz) of super-brick
@@ -343,25 +327,19 @@ constexpr int kSbMaxRuns = (kSbEdge / 4) * (kSbEdge / 4);
 template <typename Real, int P, int E, bool MC>
 __global__ void __launch_bounds__(32 * kSbWarps, sizeof(Real) == 4 ? 4 : 1)
 k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, int nsb,
-                const int *__restrict__ start, const Real *__restrict__ W,
-                const int *__restrict__ s_key, const unsigned *__restrict__ qmax_bits,
-                Real *__restrict__ tiles, int *__restrict__ err, long long comp_w,
-                long long comp_tile, int comp_q) {
+                const int *__restrict__ start, const PRec<Real> *__restrict__ recs,
+                const unsigned *__restrict__ qmax_bits, Real *__restrict__ tiles,
+                int *__restrict__ err, long long comp_tile, int comp_q) {
   // MC: blockIdx.y picks one of several charge sets assigned by one launch
-  // (the dipole components): its weight records, tiles and |q| maxima lie
-  // comp_w / comp_tile / comp_q elements after the previous set's. The
-  // single-set instance leaves the three pointers as kernel parameters: the
-  // offset copies cost six registers at the FP32 instances' 64-register
-  // bound.
+  // (the dipole components): its tiles and |q| maxima lie comp_tile / comp_q
+  // elements after the previous set's. The single-set instance leaves the
+  // pointers as kernel parameters: the offset copies cost registers at the
+  // FP32 instances' 64-register bound.
   if constexpr (MC) {
-    W += blockIdx.y * comp_w;
     tiles += blockIdx.y * comp_tile;
     qmax_bits += blockIdx.y * comp_q;
   }
   using Word = typename SbWord<Real>::type;
-  constexpr int R = 4;
-  constexpr int WS = kRecStride;
-  constexpr int WZ = wz_off<P, R>();
   constexpr int P2 = P * P;
   constexpr int NQ = (P2 + 31) / 32;
   constexpr int NT = 32 * kSbWarps;
@@ -382,9 +360,10 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   if (static_cast<int>(blockIdx.x) >= nsb)
     return; // whole block
   Word *tile = reinterpret_cast<Word *>(smem_raw);
-  Real *rec = reinterpret_cast<Real *>(smem_raw + sb_tile_bytes<Real, P, E>());
-  double *wzd = reinterpret_cast<double *>(rec + CH * WS);
-  int *toff = reinterpret_cast<int *>(wzd + 8 * CH);
+  PRec<Real> *rec = reinterpret_cast<PRec<Real> *>(smem_raw + sb_tile_bytes<Real, P, E>());
+  double *wzd = reinterpret_cast<double *>(rec + CH);
+  Real *wxs = reinterpret_cast<Real *>(wzd + 8 * CH), *wys = wxs + 8 * CH;
+  int *toff = reinterpret_cast<int *>(wys + 8 * CH);
   int const tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   int2 const sb = sbs[blockIdx.x];
@@ -468,19 +447,10 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
       int const cn = min(CH, s1 - c0);
       __syncthreads(); // the previous chunk is consumed
       if (tid == 0) {
-        unsigned const nbytes = static_cast<unsigned>(cn * WS * sizeof(Real));
+        unsigned const nbytes = static_cast<unsigned>(cn * sizeof(PRec<Real>));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive_expect_tx(&bar, nbytes);
-        bulk_g2s(rec, W + static_cast<long long>(c0) * WS, nbytes, &bar);
-      }
-      for (int j = tid; j < cn; j += NT) {
-        // corner offset inside the super-brick, [0, E)^3
-        int const sk = s_key[c0 + j];
-        int const bz = bz0 + ((sk >> (3 * LB)) - b0);
-        int const l = sk & (B3 - 1);
-        int const dx = bx * B + (l >> (2 * LB)) - o0, dy = by * B + ((l >> LB) & (B - 1)) - o1,
-                  dz = bz * B + (l & (B - 1)) - o2;
-        toff[j] = dx * SX + dy * SY + dz;
+        bulk_g2s(rec, recs + c0, nbytes, &bar);
       }
       bool const got = mbar_wait(&bar, parity);
       parity ^= 1u;
@@ -491,23 +461,43 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
         }
         return;
       }
-      // z weights of the staged records in FP64, times S
-      for (int t = tid; t < cn * P; t += NT) {
-        int const j = t / P, k = t - j * P;
-        wzd[8 * j + k] = static_cast<double>(rec[j * WS + WZ + k]) * S;
+      // weights of the staged particles: lane k of a particle's 8 the weight k
+      // of each axis (z in FP64, times S), lane 7 the tile offset
+      {
+        int const k = tid & 7;
+        Real cf[P];
+        spline_coef<P>(min(k, P - 1), cf);
+        for (int j = tid >> 3; j < cn; j += NT / 8) {
+          PRec<Real> const &r = rec[j];
+          if (k < P) {
+            wxs[8 * j + k] = r.q[MC ? blockIdx.y : 0] * spline_eval<P>(cf, r.d[0]);
+            wys[8 * j + k] = spline_eval<P>(cf, r.d[1]);
+            wzd[8 * j + k] = static_cast<double>(spline_eval<P>(cf, r.d[2])) * S;
+          } else if (k == 7) {
+            // corner offset inside the super-brick, [0, E)^3
+            int const sk = r.key;
+            int const bz = bz0 + ((sk >> (3 * LB)) - b0);
+            int const l = sk & (B3 - 1);
+            int const dx = bx * B + (l >> (2 * LB)) - o0, dy = by * B + ((l >> LB) & (B - 1)) - o1,
+                      dz = bz * B + (l & (B - 1)) - o2;
+            toff[j] = dx * SX + dy * SY + dz;
+          }
+        }
       }
       __syncthreads();
       for (int j = warp; j < cn; j += kSbWarps) {
         int const base = toff[j];
-        const Real *w = rec + j * WS;
-        double wz[P];
+        double wz[8];
 #pragma unroll
-        for (int k = 0; k < P; ++k)
-          wz[k] = wzd[8 * j + k];
+        for (int k = 0; k < P; k += 2) {
+          double2 const w = reinterpret_cast<const double2 *>(wzd)[4 * j + k / 2];
+          wz[k] = w.x;
+          wz[k + 1] = w.y;
+        }
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
           if (lane + 32 * q < P2) {
-            double const wxy = static_cast<double>(w[qx[q]] * w[P + qy[q]]);
+            double const wxy = static_cast<double>(wxs[8 * j + qx[q]] * wys[8 * j + qy[q]]);
             Word *pt = tile + base + qoff[q];
 #pragma unroll
             for (int k = 0; k < P; ++k)
@@ -665,16 +655,15 @@ template <typename Real, int P> struct InterpStage {
   using R4 = typename Real4Of<Real>::type;
   static constexpr int Ed = brick_edge<P>() + P - 1;
   static constexpr size_t tile = sizeof(R4) * Ed * Ed * Ed;
-  static constexpr size_t rec = sizeof(Real) * kInterpCap * kRecStride;
-  // key / index window: the 16-byte aligned superset of the staged range
-  static constexpr size_t ids = sizeof(int) * (kInterpCap + 8);
+  static constexpr size_t rec_at = (tile + 63) / 64 * 64;
+  static constexpr size_t rec = sizeof(PRec<Real>) * kInterpCap;
   // stages start on 128-byte boundaries (tensor copy destinations)
-  static constexpr size_t bytes = (tile + rec + 2 * ids + 127) / 128 * 128;
-  static_assert(tile % 16 == 0 && rec % 16 == 0 && ids % 16 == 0, "bulk copy alignment");
+  static constexpr size_t bytes = (rec_at + rec + 127) / 128 * 128;
 };
-// (+ 128: the kernel rounds the dynamic shared-memory base up to 128 bytes)
+// (stages, then per consumer warp the x and y weights of its four particles;
+// + 128: the kernel rounds the dynamic shared-memory base up to 128 bytes)
 template <typename Real, int P> __host__ __device__ constexpr size_t interp_smem() {
-  return kInterpStages * InterpStage<Real, P>::bytes + 128;
+  return kInterpStages * InterpStage<Real, P>::bytes + kInterpWarps * 4 * 16 * sizeof(Real) + 128;
 }
 
 struct InterpInfo {
@@ -689,18 +678,15 @@ __device__ inline void mbar_arrive(unsigned long long *bar) {
 template <typename Real, int P>
 __global__ void __launch_bounds__(32 * (1 + kInterpWarps), sizeof(Real) == 4 ? 2 : 1)
 k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, int nbricks,
-             const int *__restrict__ start, const int *__restrict__ perm,
-             const int *__restrict__ s_key, const Real *__restrict__ W,
+             const int *__restrict__ start, const PRec<Real> *__restrict__ recs, int unit,
              const CUtensorMap *__restrict__ tmaps, int map_stride,
              const double *__restrict__ q, const double *__restrict__ dipole,
              double *__restrict__ f, long long f_stride, int overwrite, int *__restrict__ err) {
-  // blockIdx.y: field set (tensor maps and outputs map_stride / f_stride apart)
+  // blockIdx.y: field set (tensor maps and outputs map_stride / f_stride
+  // apart); unit: charges of one instead of the records'
   tmaps += blockIdx.y * map_stride;
   f += blockIdx.y * f_stride;
   static_assert(P <= 8, "one lane per stencil z offset");
-  constexpr int R = 4;
-  constexpr int WS = kRecStride;
-  constexpr int WZ = wz_off<P, R>();
   constexpr int S = kInterpStages, CW = kInterpWarps, CAP = kInterpCap;
   using L = InterpStage<Real, P>;
   using R4 = typename L::R4;
@@ -749,11 +735,8 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
         }
         unsigned char *sp = stage_ptr(k);
         R4 *tile = reinterpret_cast<R4 *>(sp);
-        Real *rec = reinterpret_cast<Real *>(sp + L::tile);
-        int *keys = reinterpret_cast<int *>(sp + L::tile + L::rec);
-        int *pm = reinterpret_cast<int *>(sp + L::tile + L::rec + L::ids);
+        PRec<Real> *rec = reinterpret_cast<PRec<Real> *>(sp + L::rec_at);
         int const cn = min(s1 - s0, CAP);
-        int const a0 = s0 & ~3, a1 = (s0 + cn + 3) & ~3;
         if (lane == 0) {
           InterpInfo inf;
           inf.rep = bk.x;
@@ -770,14 +753,12 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
         // order them before the asynchronous-proxy writes that refill it
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         int const bz = bk.y % G.nbz, by = (bk.y / G.nbz) % G.nby, bx = bk.y / (G.nbz * G.nby);
-        // lane 0: the tile; lanes 1..3: one particle array each
+        // lane 0: the tile; lane 1: the particle records
         unsigned bytes = 0;
         if (lane == 0)
           bytes = static_cast<unsigned>(E2 * Ed * sizeof(R4));
         else if (lane == 1)
-          bytes = static_cast<unsigned>(cn * WS * sizeof(Real));
-        else if (lane == 2 || lane == 3)
-          bytes = static_cast<unsigned>((a1 - a0) * sizeof(int));
+          bytes = static_cast<unsigned>(cn * sizeof(PRec<Real>));
         mbar_arrive_expect_tx(&full[k], bytes);
         if (lane == 0) {
           if (bk.x != last_rep) {
@@ -786,12 +767,7 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
           }
           tma_load_3d(tile, &tmaps[bk.x], 4 * bz * B, by * B, bx * B, &full[k]);
         } else if (lane == 1) {
-          bulk_g2s(rec, W + static_cast<long long>(s0) * WS,
-                   static_cast<unsigned>(cn * WS * sizeof(Real)), &full[k]);
-        } else if (lane == 2) {
-          bulk_g2s(keys, s_key + a0, static_cast<unsigned>((a1 - a0) * sizeof(int)), &full[k]);
-        } else if (lane == 3) {
-          bulk_g2s(pm, perm + a0, static_cast<unsigned>((a1 - a0) * sizeof(int)), &full[k]);
+          bulk_g2s(rec, recs + s0, bytes, &full[k]);
         }
         ++it;
       }
@@ -829,6 +805,11 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
 
   // ---------------- consumers ----------------
   int const cw = warp - 1, g = lane >> 3, kz = lane & 7;
+  // weight kz of an axis is this lane's polynomial; x and y weights meet in
+  // the warp's slots
+  Real cf[P];
+  spline_coef<P>(min(kz, P - 1), cf);
+  Real *const wsl = reinterpret_cast<Real *>(smem_base + S * L::bytes) + (4 * cw + g) * 16;
   for (int it = 0;; ++it) {
     int const k = it % S;
     bool const got = mbar_wait(&full[k], (it / S) & 1);
@@ -842,28 +823,38 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
       return;
     unsigned char *sp = stage_ptr(k);
     const R4 *tile = reinterpret_cast<const R4 *>(sp);
-    const Real *rec = reinterpret_cast<const Real *>(sp + L::tile);
-    const int *keys = reinterpret_cast<const int *>(sp + L::tile + L::rec);
-    const int *pm = reinterpret_cast<const int *>(sp + L::tile + L::rec + L::ids);
-    int const s0 = inf.s0, s1 = inf.s1, a0 = s0 & ~3;
+    const PRec<Real> *rec = reinterpret_cast<const PRec<Real> *>(sp + L::rec_at);
+    int const s0 = inf.s0, s1 = inf.s1;
     // four particles per warp (one per 8-lane group), warps interleaved
     for (int sb = s0 + 4 * cw; sb < s1; sb += 4 * CW) {
       int const s = sb + g, j = s - s0;
       bool const live = s < s1;
-      Real ax = Real(0), ay = Real(0), az = Real(0);
+      Real ax = Real(0), ay = Real(0), az = Real(0), wzk = Real(0);
+      int l = 0, idx = 0;
+      if (live) {
+        PRec<Real> r;
+        if (j < CAP)
+          r = rec[j];
+        else
+          r = recs[s];
+        l = r.key - inf.brick * B3;
+        idx = r.idx;
+        wsl[kz] = (unit ? Real(1) : r.q[0]) * spline_eval<P>(cf, r.d[0]);
+        wsl[8 + kz] = spline_eval<P>(cf, r.d[1]);
+        wzk = spline_eval<P>(cf, r.d[2]);
+      }
+      __syncwarp();
       if (live && kz < P) {
-        bool const staged = j < CAP;
-        int const l = (staged ? keys[s - a0] : s_key[s]) - inf.brick * B3;
         int const lb = __ffs(B) - 1; // B is a power of two
         int const lx = l >> (2 * lb), ly = (l >> lb) & (B - 1), lz = l & (B - 1);
-        const Real *w = staged ? rec + j * WS : W + static_cast<long long>(s) * WS;
-        Real wx[P], wy[P];
+        Real wx[8], wy[8];
 #pragma unroll
-        for (int kk = 0; kk < P; ++kk) {
-          wx[kk] = w[kk];
-          wy[kk] = w[P + kk];
+        for (int h = 0; h < P; h += 4) {
+          R4 const u = reinterpret_cast<const R4 *>(wsl)[h / 4];
+          R4 const v = reinterpret_cast<const R4 *>(wsl)[2 + h / 4];
+          wx[h] = u.x, wx[h + 1] = u.y, wx[h + 2] = u.z, wx[h + 3] = u.w;
+          wy[h] = v.x, wy[h + 1] = v.y, wy[h + 2] = v.z, wy[h + 3] = v.w;
         }
-        Real const wzk = w[WZ + kz];
         const R4 *tp = tile + (lx * Ed + ly) * Ed + lz + kz;
 #pragma unroll
         for (int kx = 0; kx < P; ++kx) {
@@ -878,6 +869,7 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
           }
         }
       }
+      __syncwarp(); // the slots are refilled for the next four particles
       double fx = static_cast<double>(ax), fy = static_cast<double>(ay),
              fz = static_cast<double>(az);
 #pragma unroll
@@ -887,7 +879,7 @@ k_p3m_interp(const RepGeom *__restrict__ reps, const int2 *__restrict__ bricks, 
         fz += __shfl_xor_sync(0xffffffffu, fz, o);
       }
       if (live && kz == 0) {
-        int const i = (j < CAP) ? pm[s - a0] : perm[s];
+        int const i = idx;
         double ox = -inf.pref * fx, oy = -inf.pref * fy, oz = -inf.pref * fz;
         if (inf.cdip != 0.0) {
           double const qi = q[i];

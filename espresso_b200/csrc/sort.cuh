@@ -114,21 +114,15 @@ __global__ void k_scan_add(int *__restrict__ out, const int *__restrict__ tile_s
     out[i] += tile_sums[i / kScanTile];
 }
 
-// Place every item at start[key] + slot (slot from the counting atomics);
-// the nzero words at `zero` (the counts, already scanned) are cleared for the
-// next sort.
+// Place every item at start[key] + slot (slot from the counting atomics).
 __global__ void k_place(const int *__restrict__ key, const int *__restrict__ slot,
                         const int *__restrict__ start, int *__restrict__ perm,
-                        long long n, const int *__restrict__ cond, int *__restrict__ zero,
-                        long long nzero) {
-  pdl_enter();
+                        long long n, const int *__restrict__ cond) {
   if (cond && !*cond)
     return;
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n)
     perm[start[key[i]] + slot[i]] = static_cast<int>(i);
-  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
-    zero[k] = 0;
 }
 
 // Restore particle-index order inside every bucket (the atomic slots of the
