@@ -354,10 +354,12 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       a[tq * ld + pix(x)] = tor ? C{c * m.y, c * m.x} : C{-c * m.x, c * m.y};
     }
   __syncthreads();
-  C const *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw);
-  if (col)
-    for (int x = xq; x < M0; x += 16)
-      field0[fstride * o + base + x * stride_x] = cswap(res[tq * ld + pix(x)]);
+  C const *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
+  int const rows = col ? (M0 - xq + 15) >> 4 : 0;
+  C *q = field0 + fstride * o + base + xq * stride_x;
+#pragma unroll 4
+  for (int u = 0; u < rows; ++u)
+    q[u * 16 * stride_x] = cswap(res[17 * u]);
 }
 
 // Backward y pass over the x pass's five arrays: nine fields (E_x, E_y, E_z in
@@ -452,18 +454,25 @@ __global__ void k_dp3m_sort_mu(long long n, const int *__restrict__ perm,
 // of 8 entries each, as k_pair_forces_rel): 16 384 dipoles fill the GPU only
 // with 8 lanes each.
 
-// Sums of the LPP lanes of a particle, its outputs (times pref; f may be
-// nullptr) and the block's energy partial.
+// The particle's own moment leaves the sums:
+//   F = sum (cd d + q mu_j) + mu_i sum s,  T = mu_i x sum (s d - B mu_j)
+// with cd = (mu_i.mu_j) C - (mu_i.d)(mu_j.d) D, s = (mu_j.d) C, q = (mu_i.d) C:
+// seven sums, nine operations per pair fewer than six sums of whole terms.
+// Sums w of the LPP lanes of a particle (force part, torque part, sum s), its
+// outputs (times pref; f may be nullptr) and the block's energy partial.
 template <bool EV, int LPP>
-__device__ inline void dp_pairs_finish(double (&v)[6], double energy, double pref, bool active,
+__device__ inline void dp_pairs_finish(double (&w)[7], double mx, double my, double mz,
+                                       double energy, double pref, bool active,
                                        long long a, const int *__restrict__ perm,
                                        double *__restrict__ f, double *__restrict__ tq,
                                        int overwrite, double *__restrict__ partials) {
 #pragma unroll
   for (int o = 1; o < LPP; o <<= 1)
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-      v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    for (int k = 0; k < 7; ++k)
+      w[k] += __shfl_xor_sync(0xffffffffu, w[k], o);
+  double const v[6] = {w[0] + mx * w[6], w[1] + my * w[6], w[2] + mz * w[6],
+                       my * w[5] - mz * w[4], mz * w[3] - mx * w[5], mx * w[4] - my * w[3]};
   if (f && active && threadIdx.x % LPP == 0) {
     int const i = perm[a];
 #pragma unroll
@@ -499,10 +508,10 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
   bool const active = la < G.np;
   long long const a = G.p0 + la;
   double energy = 0.0;
-  double s6[6] = {0, 0, 0, 0, 0, 0};
+  double s7[7] = {0, 0, 0, 0, 0, 0, 0};
+  double4 const ma = active ? smu[a] : make_double4(0.0, 0.0, 0.0, 0.0);
   if (active) {
     double4 const pa = spq[a];
-    double4 const ma = smu[a];
     double const alpha = G.alpha, rc = G.r_cut;
     double const coeff = 2.0 * alpha / sqrt(kPi);
     double const a2 = alpha * alpha;
@@ -560,19 +569,19 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
           energy += mimj * B - mir * mjr * Cc;
         double const cd = mimj * Cc - mir * mjr * Dd;
         double const s = mjr * Cc, q = mir * Cc;
-        s6[0] += cd * d0 + s * ma.x + q * mb.x;
-        s6[1] += cd * d1 + s * ma.y + q * mb.y;
-        s6[2] += cd * d2 + s * ma.z + q * mb.z;
-        // -mu_i x (B mu_j - s d)
-        double const w0 = s * d0 - B * mb.x, w1 = s * d1 - B * mb.y, w2 = s * d2 - B * mb.z;
-        s6[3] += ma.y * w2 - ma.z * w1;
-        s6[4] += ma.z * w0 - ma.x * w2;
-        s6[5] += ma.x * w1 - ma.y * w0;
+        s7[0] += cd * d0 + q * mb.x;
+        s7[1] += cd * d1 + q * mb.y;
+        s7[2] += cd * d2 + q * mb.z;
+        s7[3] += s * d0 - B * mb.x;
+        s7[4] += s * d1 - B * mb.y;
+        s7[5] += s * d2 - B * mb.z;
+        s7[6] += s;
       }
       gp = gn;
     }
   }
-  dp_pairs_finish<EV, LPP>(s6, energy, pref, active, a, perm, f, tq, overwrite, partials);
+  dp_pairs_finish<EV, LPP>(s7, ma.x, ma.y, ma.z, energy, pref, active, a, perm, f, tq, overwrite,
+                           partials);
 }
 
 // Sum of FP32 terms in an unevaluated pair hi + lo (two-sum, Knuth: the
@@ -616,10 +625,10 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
   bool const active = la < G.np;
   long long const a = G.p0 + la;
   double energy = 0.0;
-  double s6[6] = {0, 0, 0, 0, 0, 0};
+  double s7[7] = {0, 0, 0, 0, 0, 0, 0};
+  float4 const ma = active ? smu[a] : make_float4(0.f, 0.f, 0.f, 0.f);
   if (active) {
     float4 const pa = spf[a];
-    float4 const ma = smu[a];
     float const alpha = static_cast<float>(G.alpha);
     float const rc2 = static_cast<float>(G.r_cut * G.r_cut);
     float const coeff = static_cast<float>(2.0 * G.alpha / sqrt(kPi));
@@ -630,6 +639,7 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
     float const ncs_y = -0.25f * static_cast<float>(G.box[1] / G.cg[1]);
     float const ncs_z = -0.0625f * static_cast<float>(G.box[2] / G.cg[2]);
     Sum2 s01{0, 0}, s23{0, 0}, s45{0, 0};
+    double ss = 0.0;
     int const cw = nb_cnt[a];
     int const ga = (nb_count_a(cw) + 7) >> 3, gt = ga + ((nb_count_b(cw) + 7) >> 3);
     const int *nbp = nb + nb_base(G.nb_off, G.max_nb, la);
@@ -685,18 +695,20 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
             energy += static_cast<double>(mimj * B - mir * mjr * Cc);
           float const cd = mimj * Cc - mir * mjr * Dd;
           float const s = mjr * Cc, q = mir * Cc;
-          float const w0 = s * d0 - B * mb.x, w1 = s * d1 - B * mb.y, w2 = s * d2 - B * mb.z;
-          s01.add(pk2(cd * d0 + s * ma.x + q * mb.x, cd * d1 + s * ma.y + q * mb.y));
-          s23.add(pk2(cd * d2 + s * ma.z + q * mb.z, ma.y * w2 - ma.z * w1));
-          s45.add(pk2(ma.z * w0 - ma.x * w2, ma.x * w1 - ma.y * w0));
+          s01.add(pk2(cd * d0 + q * mb.x, cd * d1 + q * mb.y));
+          s23.add(pk2(cd * d2 + q * mb.z, s * d0 - B * mb.x));
+          s45.add(pk2(s * d1 - B * mb.y, s * d2 - B * mb.z));
+          ss += static_cast<double>(s);
         }
       }
     }
-    s01.get(s6[0], s6[1]);
-    s23.get(s6[2], s6[3]);
-    s45.get(s6[4], s6[5]);
+    s01.get(s7[0], s7[1]);
+    s23.get(s7[2], s7[3]);
+    s45.get(s7[4], s7[5]);
+    s7[6] = ss;
   }
-  dp_pairs_finish<EV, LPP>(s6, energy, pref, active, a, perm, f, tq, overwrite, partials);
+  dp_pairs_finish<EV, LPP>(s7, ma.x, ma.y, ma.z, energy, pref, active, a, perm, f, tq, overwrite,
+                           partials);
 }
 
 } // namespace p3mx

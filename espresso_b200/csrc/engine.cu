@@ -442,7 +442,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
         return ((two ? 1 : 2) * static_cast<size_t>(nl + (nl + 1) / 2) * ldz + M2) * csz;
       };
       int lzi = 2;
-      while (3 * (lzi + 2) / 2 <= want && zi_smem(lzi + 2) <= z_budget)
+      while (3 * (lzi + 2) / 2 <= want && lzi + 2 <= kZiLines && zi_smem(lzi + 2) <= z_budget)
         lzi += 2;
       lzi = std::min(lzi, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2));
       for (int l = 0; l < lines; l += lzi)

@@ -340,6 +340,49 @@ __device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
     }
   }
 }
+// The two steps for compile-time factors (powers of two): the padded indices
+// fold to a base and immediate offsets (128^3: 150 -> about 90 instructions per
+// point and pass against the runtime factors).  Blocks of 256 threads.
+template <typename C, int N1, int N2>
+__device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__restrict__ tw) {
+  unsigned const tid = threadIdx.x;
+  for (unsigned it = tid; it < static_cast<unsigned>(nlines * N2); it += 256) {
+    int const l = it / N2, t = it % N2;
+    C *s = a + l * ld + t;
+    C v[N1];
+#pragma unroll
+    for (int m = 0; m < N1; ++m)
+      v[m] = s[pix(N2 * m)]; // t < 16 never crosses a pad
+    dft<C, N1>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1)
+      v[k1] = cmul(v[k1], tw[t * k1]);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1)
+      s[pix(N2 * k1)] = v[k1];
+  }
+  __syncthreads();
+  constexpr int per = 256 / N1;
+  int const lq = tid / N1, k1 = tid % N1;
+  for (int l0 = 0; l0 < nlines; l0 += per) {
+    bool const act = l0 + lq < nlines;
+    C *s = a + (l0 + lq) * ld;
+    C v[N2];
+    if (act) {
+      C const *r = s + pix(N2 * k1);
+#pragma unroll
+      for (int t = 0; t < N2; ++t)
+        v[t] = r[t];
+      dft<C, N2>(v);
+    }
+    __syncthreads();
+    if (act) {
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        s[k1 + pix(N1 * k2)] = v[k2];
+    }
+  }
+}
 #define P3MX_FACTOR_DISPATCH(N, CALL)                                          \
   switch (N) {                                                                 \
   case 2: { constexpr int R = 2; CALL; } break;                                \
@@ -361,18 +404,16 @@ __device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
 template <typename C>
 __device__ __forceinline__ void fft_lines_2(C *a, int nlines, int ld, AxisPlan const &pl,
                                             const C *__restrict__ tw) {
-  if (pl.n == 256) {
-    fft_step1<C, 16>(a, nlines, ld, 16, tw);
-    __syncthreads();
-    fft_step2<C, 16>(a, nlines, ld, 16);
-  } else if (pl.n == 128) {
-    fft_step1<C, 16>(a, nlines, ld, 8, tw);
-    __syncthreads();
-    fft_step2<C, 8>(a, nlines, ld, 16);
-  } else {
+  switch (pl.n) {
+  case 32: fft_pow2<C, 8, 4>(a, nlines, ld, tw); break;
+  case 64: fft_pow2<C, 8, 8>(a, nlines, ld, tw); break;
+  case 128: fft_pow2<C, 16, 8>(a, nlines, ld, tw); break;
+  case 256: fft_pow2<C, 16, 16>(a, nlines, ld, tw); break;
+  default:
     P3MX_FACTOR_DISPATCH(pl.n1, (fft_step1<C, R>(a, nlines, ld, pl.n2, tw)))
     __syncthreads();
     P3MX_FACTOR_DISPATCH(pl.n2, (fft_step2<C, R>(a, nlines, ld, pl.n1)))
+    break;
   }
   __syncthreads();
 }
@@ -579,36 +620,37 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const pw = INV ? job.pw[jb] : 0;
   Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[1]) : Real(1);
   // all of a thread's rows in flight at once (up to 16: M1 <= 256 in one
-  // round)
-  for (int y0 = yq; y0 < M1; y0 += 256) {
+  // round); row y = yq + 16 u of column tq lies at tq ld + yq + 17 u
+  C *const sl = a + tq * ld + yq;
+  int const rows = col ? (M1 - yq + 15) >> 4 : 0;
+  long long const step = 16 * hp;
+  for (int u0 = 0; u0 < rows; u0 += 16) {
     C v[16];
+    const C *p = src + (yq + 16 * u0) * hp;
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      int const y = y0 + 16 * u;
-      if (col && y < M1)
-        v[u] = src[y * hp];
-    }
+    for (int u = 0; u < 16; ++u, p += step)
+      if (u0 + u < rows)
+        v[u] = *p;
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      int const y = y0 + 16 * u;
-      if (col && y < M1) {
+    for (int u = 0; u < 16; ++u)
+      if (u0 + u < rows) {
         C w = INV ? cswap(v[u]) : v[u];
         if (INV && pw > 0) {
-          Real const k = static_cast<Real>(freq_dop(y, M1)) * ks;
+          Real const k = static_cast<Real>(freq_dop(yq + 16 * (u0 + u), M1)) * ks;
           Real const f = pw == 2 ? k * k : k;
           w = C{f * w.x, f * w.y};
         }
-        a[tq * ld + pix(y)] = w;
+        sl[17 * (u0 + u)] = w;
       }
-    }
   }
   __syncthreads();
-  const C *res = fft_lines<TWO>(a, b, T, ld, G.plan[1], tw);
-  if (col)
-    for (int y = yq; y < M1; y += 16) {
-      C const v = res[tq * ld + pix(y)];
-      dst[y * hp] = INV ? cswap(v) : v;
-    }
+  const C *res = fft_lines<TWO>(a, b, T, ld, G.plan[1], tw) + tq * ld + yq;
+  C *q = dst + yq * hp;
+#pragma unroll 4
+  for (int u = 0; u < rows; ++u, q += step) {
+    C const v = res[17 * u];
+    *q = INV ? cswap(v) : v;
+  }
 }
 
 // ---- pass x fused with the k-space operator -----------------------------
@@ -732,16 +774,19 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   __syncthreads();
   // without TWO the scratch of the second transform is the first's buffer
   // once that is stored
-  const C *f0 = fft_lines<TWO>(fb, c, T, ld, G.plan[0], tw);
-  if (col)
-    for (int x = xq; x < M0; x += 16)
-      field0[base + x * stride_x + tq] = cswap(f0[tq * ld + pix(x)]);
+  const C *f0 = fft_lines<TWO>(fb, c, T, ld, G.plan[0], tw) + tq * ld + xq;
+  int const rows = col ? (M0 - xq + 15) >> 4 : 0;
+  C *q = field0 + base + xq * stride_x + tq;
+#pragma unroll 4
+  for (int u = 0; u < rows; ++u)
+    q[u * 16 * stride_x] = cswap(f0[17 * u]);
   if constexpr (!TWO)
     __syncthreads();
-  const C *f1 = fft_lines<TWO>(res, fb, T, ld, G.plan[0], tw);
-  if (col)
-    for (int x = xq; x < M0; x += 16)
-      field0[field_stride + base + x * stride_x + tq] = cswap(f1[tq * ld + pix(x)]);
+  const C *f1 = fft_lines<TWO>(res, fb, T, ld, G.plan[0], tw) + tq * ld + xq;
+  q += field_stride;
+#pragma unroll 4
+  for (int u = 0; u < rows; ++u)
+    q[u * 16 * stride_x] = cswap(f1[17 * u]);
 }
 
 // ---- pass z, backward for 3 field components -> real fields -------------
@@ -762,6 +807,7 @@ inline ZPass z_charge() { return ZPass{{0, 2, 3}, {0, 0, 1}}; }
 // TWO), twiddles (n).  FP32: four blocks per SM -- the block's load, transform
 // and store phases do not overlap, so the fourth resident block pays for the
 // 64-register bound.
+constexpr int kZiLines = 128; // most lines per block
 template <typename Real, bool TWO>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
 k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
@@ -791,29 +837,36 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[2]) : Real(1);
   int const px = zp.pw[set], py = zp.pw[set + 1], pz = zp.pw[set + 2];
   float const rH = 1.0f / static_cast<float>(H);
-#pragma unroll 4
-  for (int t = threadIdx.x; t < nc * H; t += blockDim.x) {
-    int const j = qdiv(t, H, rH), k = t - j * H;
-    bool const xy = j < nl;
-    int const l0 = xy ? j : 2 * (j - nl), l1 = xy ? j : l0 + 1;
-    const C *r0 = (xy ? fx : fz) + static_cast<long long>(l0) * G.hp + k;
-    const C *r1 = (xy ? fy : fz) + static_cast<long long>(l1) * G.hp + k;
-    C X = *r0;
-    C Y = (l1 < nl) ? *r1 : C{Real(0), Real(0)};
-    int const p0 = xy ? px : pz, p1 = xy ? py : pz;
-    Real const kz = static_cast<Real>(freq_dop(k, n)) * ks;
-    Real const f0 = p0 == 0 ? Real(1) : (p0 == 2 ? kz * kz : kz);
-    Real const f1 = p1 == 0 ? Real(1) : (p1 == 2 ? kz * kz : kz);
-    X = C{f0 * X.x, f0 * X.y};
-    Y = C{f1 * Y.x, f1 * Y.y};
+  long long const hp = G.hp;
+  // entry k of the half rows X and Y (times k_z^p0, k_z^p1) into slot j
+  auto put = [&](int j, int k, C X, C Y, int p0, int p1) {
+    if (p0 | p1) {
+      Real const kz = static_cast<Real>(freq_dop(k, n)) * ks;
+      Real const f0 = p0 == 0 ? Real(1) : (p0 == 2 ? kz * kz : kz);
+      Real const f1 = p1 == 0 ? Real(1) : (p1 == 2 ? kz * kz : kz);
+      X = C{f0 * X.x, f0 * X.y};
+      Y = C{f1 * Y.x, f1 * Y.y};
+    }
+    C *s = a + j * ld;
     if (k == 0 || 2 * k == n) {
       // swapped (X.x + i Y.x)
-      a[j * ld + pix(k)] = C{Y.x, X.x};
+      s[pix(k)] = C{Y.x, X.x};
     } else {
       // X + i Y at k, conj(X) + i conj(Y) at n - k, swapped
-      a[j * ld + pix(k)] = C{X.y + Y.x, X.x - Y.y};
-      a[j * ld + pix(n - k)] = C{Y.x - X.y, X.x + Y.y};
+      s[pix(k)] = C{X.y + Y.x, X.x - Y.y};
+      s[pix(n - k)] = C{Y.x - X.y, X.x + Y.y};
     }
+  };
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nl * H; t += 256) {
+    int const j = qdiv(t, H, rH), k = t - j * H;
+    put(j, k, fx[j * hp + k], fy[j * hp + k], px, py);
+  }
+#pragma unroll 2
+  for (int t = threadIdx.x; t < nz * H; t += 256) {
+    int const j = qdiv(t, H, rH), k = t - j * H;
+    const C *r = fz + 2 * j * hp + k;
+    put(nl + j, k, r[0], (2 * j + 1 < nl) ? r[hp] : C{Real(0), Real(0)}, pz, pz);
   }
   __syncthreads();
   const C *res = fft_lines<TWO>(a, b, nc, ld, G.plan[2], tw);
@@ -825,7 +878,15 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   R4 *out = reinterpret_cast<R4 *>(efield) + blockIdx.y * e_stride + G.re_off;
   int const M1 = G.mesh[1], M0 = G.mesh[0];
   int const P0 = G.epad[0], P1 = G.epad[1], P2 = G.epad[2];
-  int const x0 = static_cast<int>(line0 / M1), y0 = static_cast<int>(line0 - static_cast<long long>(x0) * M1);
+  // per line: its row of the field mesh, and whether it has ghost images along
+  // x or y
+  __shared__ long long s_row[kZiLines];
+  for (int l = threadIdx.x; l < nl; l += 256) {
+    int const x = static_cast<int>((line0 + l) / M1), y = static_cast<int>((line0 + l) % M1);
+    long long const row = (static_cast<long long>(x) * P1 + y) * P2;
+    s_row[l] = (x + M0 < P0 || y + M1 < P1) ? ~row : row;
+  }
+  __syncthreads();
   for_lines(nl, n, [&](int l, int k) {
     C const xy = res[l * ld + pix(k)];
     C const zz = res[(nl + (l >> 1)) * ld + pix(k)];
@@ -834,16 +895,19 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     v.y = xy.x;
     v.z = (l & 1) ? zz.x : zz.y;
     v.w = Real(0);
-    int x = x0, y = y0 + l;
-    while (y >= M1) {
-      y -= M1;
-      ++x;
+    long long const row = s_row[l];
+    if (row >= 0) {
+      out[row + k] = v;
+      for (int zg = k + n; zg < P2; zg += n)
+        out[row + zg] = v;
+      return;
     }
+    int const x = static_cast<int>((line0 + l) / M1), y = static_cast<int>((line0 + l) % M1);
     for (int xg = x; xg < P0; xg += M0)
       for (int yg = y; yg < P1; yg += M1) {
-        R4 *row = out + (static_cast<long long>(xg) * P1 + yg) * P2;
+        R4 *r = out + (static_cast<long long>(xg) * P1 + yg) * P2;
         for (int zg = k; zg < P2; zg += n)
-          row[zg] = v;
+          r[zg] = v;
       }
   });
 }

@@ -686,8 +686,11 @@ constexpr int kPairFill = 768;
 // Bound by instruction issue (about 45 scalar instructions per entry and
 // three MUFU operations): the range-independent arithmetic runs on two
 // entries at a time in packed FP32, with the scalar code's roundings.
+#ifndef P3MX_PAIR_MINB
+#define P3MX_PAIR_MINB 3
+#endif
 template <int MODE, int LPP>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, P3MX_PAIR_MINB)
 k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                   const float4 *__restrict__ spf, const int *__restrict__ stype,
                   const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
@@ -816,11 +819,14 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
       sz += ft * dz[u];
     }
   };
-  auto group = [&](auto lj, int v) {
-    // the lane's group v: class A group v, or class B group v - ga
+  // the lane's group v: class A group v, or class B group v - ga
+  auto entries = [&](int v, int4 &g0, int4 &g1) {
     int const grp = v < ga ? v : ngroups - 1 - (v - ga);
     const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
-    int4 const g0 = gp[0], g1 = gp[1];
+    g0 = gp[0];
+    g1 = gp[1];
+  };
+  auto group = [&](auto lj, int4 const &g0, int4 const &g1) {
     unsigned const ent[8] = {static_cast<unsigned>(g0.x), static_cast<unsigned>(g0.y),
                              static_cast<unsigned>(g0.z), static_cast<unsigned>(g0.w),
                              static_cast<unsigned>(g1.x), static_cast<unsigned>(g1.y),
@@ -840,14 +846,21 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
     fy += static_cast<double>(sy);
     fz += static_cast<double>(sz);
   };
+  // the next group's entries are loaded before the current group's pairs
+  int4 n0 = make_int4(0, 0, 0, 0), n1 = n0;
+  if (sub < gt)
+    entries(sub, n0, n1);
   for (int v0 = 0; v0 < gmax; v0 += LPP) {
     int const v = v0 + sub;
+    int4 const g0 = n0, g1 = n1;
+    if (v + LPP < gt)
+      entries(v + LPP, n0, n1);
     bool const any_a = __any_sync(0xffffffffu, v < ga);
     if (v < gt) {
       if (any_a)
-        group(std::true_type{}, v);
+        group(std::true_type{}, g0, g1);
       else
-        group(std::false_type{}, v);
+        group(std::false_type{}, g0, g1);
     }
   }
 #pragma unroll
@@ -1064,44 +1077,53 @@ k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           pv[u] = pos[idx[u]];
+        // two pairs at a time, selected instead of branched around: their
+        // dependent chains (rsqrt, exp, polynomial) overlap
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          double4 const pb = pv[u];
-          double const d0 = mi_d(pa.x - pb.x, L0, Li0);
-          double const d1 = mi_d(pa.y - pb.y, L1, Li1);
-          double const d2 = mi_d(pa.z - pb.z, L2, Li2);
-          double const dist2 = d0 * d0 + d1 * d1 + d2 * d2;
-          if (!(dist2 > 0.0))
-            continue;
-          double const inv_d = rsqrt(dist2);
-          double const dist = dist2 * inv_d;
-          double fc = 0.0, ec = 0.0;
-          if (pb.w != 0.0 && pref_qa != 0.0 && dist < r_cut) {
-            double const adist = alpha * dist;
+        for (int w = 0; w < 4; w += 2) {
+          double d0[2], d1[2], d2[2], dist2[2], inv[2], dist[2], fc[2], ec[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            double4 const pb = pv[w + u];
+            d0[u] = mi_d(pa.x - pb.x, L0, Li0);
+            d1[u] = mi_d(pa.y - pb.y, L1, Li1);
+            d2[u] = mi_d(pa.z - pb.z, L2, Li2);
+            dist2[u] = d0[u] * d0[u] + d1[u] * d1[u] + d2[u] * d2[u];
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            // zero distance (the list's filling): no term
+            inv[u] = rsqrt(dist2[u] > 0.0 ? dist2[u] : 1.0);
+            dist[u] = dist2[u] > 0.0 ? dist2[u] * inv[u] : 2.0 * r_cut;
+            double const adist = alpha * dist[u];
             double const ex = exp(-adist * adist);
             double const t = rcp_newton(fma(0.3275911, adist, 1.0));
             double const asp =
                 t * (0.254829592 +
                      t * (-0.284496736 +
                           t * (1.421413741 + t * (-1.453152027 + t * 1.061405429))));
-            double const er = asp * inv_d;
-            double const pq = pref_qa * pb.w;
-            fc = pq * (ex * (er + two_a) * (inv_d * inv_d));
+            double const er = asp * inv[u];
+            double const pq = pref_qa * pv[w + u].w;
+            bool const in = dist[u] < r_cut;
+            fc[u] = in ? pq * (ex * (er + two_a) * (inv[u] * inv[u])) : 0.0;
             if constexpr (EV)
-              ec = pq * er * ex;
+              ec[u] = in ? pq * er * ex : 0.0;
           }
-          double fn = 0.0, en = 0.0;
-          if (cls_a) {
-            PairR<double> const p(ia[ta + typ[idx[u]]]);
-            if (p.active)
-              lj_wca(p, dist, inv_d, fn, en);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            double fn = 0.0, en = 0.0;
+            if (cls_a && dist2[u] > 0.0) {
+              PairR<double> const p(ia[ta + typ[idx[w + u]]]);
+              if (p.active)
+                lj_wca(p, dist[u], inv[u], fn, en);
+            }
+            double const ft = fc[u] + fn;
+            fx += ft * d0[u];
+            fy += ft * d1[u];
+            fz += ft * d2[u];
+            if constexpr (EV)
+              ev_add(ev, ec[u], en, fc[u], fn, d0[u], d1[u], d2[u]);
           }
-          double const ft = fc + fn;
-          fx += ft * d0;
-          fy += ft * d1;
-          fz += ft * d2;
-          if constexpr (EV)
-            ev_add(ev, ec, en, fc, fn, d0, d1, d2);
         }
       }
     }

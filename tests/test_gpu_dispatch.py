@@ -1,0 +1,208 @@
+"""GPU tests of the size rules: every path that a rule on sizes, types or
+alignment chooses, against the FP64 oracle (or against the same system
+computed through another path).
+
+Tolerances: FP64 1e-9 of the largest component (the oracle's own sums); FP32
+2e-5, the FP32-mixed mesh and pair arithmetic as in test_gpu_p3m.py.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+import espresso_b200 as eb
+from espresso_b200 import _lib
+from espresso_b200.electrostatics import P3M, P3MGPU
+from espresso_b200.magnetostatics import DipolarP3M
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DP = ctypes.POINTER(ctypes.c_double)
+RTOL = {P3M: 1e-9, P3MGPU: 2e-5}
+
+
+def _ions(n, box, seed=0):
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    cell = np.asarray(box) / side
+    sites = rng.choice(side ** 3, n, replace=False)
+    idx = np.stack(np.unravel_index(sites, (side,) * 3), 1)
+    pos = (idx + 0.5 + rng.uniform(-0.1, 0.1, (n, 3))) * cell
+    return pos, np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+
+
+def _actor(cls, box, pos, q, mesh, cao, alpha=1.0, r_cut=2.0):
+    act = cls(prefactor=1.0, accuracy=1e-4, mesh=list(mesh), cao=cao, alpha=alpha, r_cut=r_cut,
+              tune=False, check_neutrality=False)
+    act._set_system(box, 0.4, (True, True, True))
+    act._activate(pos, q)
+    return act
+
+
+def _long_range(act, pos, q, mesh):
+    lib = _lib.load()
+    f = np.zeros((len(q), 3))
+    e, v = np.zeros(1), np.zeros(9)
+    flags = _lib.P3MX_FORCES | _lib.P3MX_ENERGY | _lib.P3MX_VIRIAL | _lib.P3MX_OVERWRITE
+    _lib.check(lib.p3mx_long_range(act._handle, len(q), _lib.dptr(pos), _lib.dptr(q), _lib.dptr(f),
+                                   e.ctypes.data_as(DP), v.ctypes.data_as(DP), flags, None),
+               act._handle)
+    rho = np.zeros(mesh)
+    _lib.check(lib.p3mx_copy_mesh(act._handle, rho.ctypes.data_as(DP), rho.size), act._handle)
+    return f, e[0], v.reshape(3, 3), rho
+
+
+# meshes: last super-bricks shorter than the stencil (three covers of the first
+# points), one super-brick per axis, 16-point super-bricks (many of them) with
+# whole and ragged ends; axis lengths with every transform factor (2..10, 12,
+# 14, 15, 16), powers of two, no two factors (22, 34, 200), odd factor pairs
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+@pytest.mark.parametrize("mesh,cao", [
+    ((10, 18, 26), 7), ((8, 8, 8), 7), ((12, 20, 28), 3), ((18, 34, 22), 5), ((30, 42, 54), 6),
+    ((64, 32, 48), 4), ((90, 70, 84), 1), ((100, 126, 140), 7), ((130, 98, 120), 7),
+    ((144, 150, 210), 2), ((224, 96, 16), 6), ((128, 16, 256), 5), ((200, 50, 36), 7)])
+def test_long_range_meshes(cls, mesh, cao):
+    box = np.array([9.0, 10.0, 11.0]) if max(mesh) < 100 else np.array([21.0, 20.0, 23.0])
+    pos, q = _ions(700, box, seed=cao)
+    # particles on the box faces and corners: stencils that wrap every axis
+    pos[:8] = np.stack(np.meshgrid([0, 1], [0, 1], [0, 1]), -1).reshape(-1, 3) * box * (1 - 1e-9)
+    alpha = 0.5 * min(mesh) / max(box)
+    act = _actor(cls, box, pos, q, mesh, cao, alpha=alpha, r_cut=1.0)
+    f, e, v, rho = _long_range(act, pos, q, mesh)
+    prm = O.make_params(box, mesh, cao, alpha, 1.0, 1.0)
+    fo, eo, vo, rho_o = O.p3m_kspace(prm, pos, q, want_mesh=True)
+    tol = RTOL[cls]
+    np.testing.assert_allclose(rho, rho_o, rtol=0, atol=tol * np.abs(rho_o).max())
+    np.testing.assert_allclose(f, fo, rtol=0, atol=tol * np.abs(fo).max())
+    # energies and virials of both actors are FP64 sums (self terms cancel)
+    assert abs(e - eo) <= 1e-9 * (abs(eo) + (q * q).sum() * alpha)
+    np.testing.assert_allclose(v, vo, rtol=0, atol=1e-9 * np.abs(vo).max())
+
+
+# one particle number for 8, 4, 2 and 1 lanes per particle of the pair kernels
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+@pytest.mark.parametrize("n", [3001, 30000, 60000, 116001])
+@pytest.mark.parametrize("form", ["wca", "types", "offset"])
+def test_pair_lanes_and_types(cls, n, form):
+    box = np.full(3, (n / 0.4) ** (1.0 / 3.0))
+    pos, q = _ions(n, box, seed=1)
+    if n % 2:
+        q[-1] = 0.0
+    types = (np.arange(n) % 3 == 0).astype(np.int32) if form != "wca" else np.zeros(n, np.int32)
+    s = eb.System(box_l=box)
+    s.time_step = 0.01
+    s.part.add(pos=pos, q=q, type=types)
+    if form == "wca":
+        pairs = {(0, 0): dict(wca_eps=1.0, wca_sig=1.0)}
+        s.non_bonded_inter[0, 0].wca.set_params(epsilon=1.0, sigma=1.0)
+    else:
+        off = 0.2 if form == "offset" else 0.0
+        lj = dict(lj_eps=1.3, lj_sig=0.9, lj_cut=2.0, lj_shift=0.1, lj_offset=off)
+        pairs = {(0, 0): dict(wca_eps=1.0, wca_sig=1.0), (0, 1): lj}  # (1, 1): none
+        s.non_bonded_inter[0, 0].wca.set_params(epsilon=1.0, sigma=1.0)
+        s.non_bonded_inter[0, 1].lennard_jones.set_params(epsilon=1.3, sigma=0.9, cutoff=2.0,
+                                                          shift=0.1, offset=off)
+    s.electrostatics.solver = cls(prefactor=1.5, accuracy=1e-3, mesh=32, cao=3, r_cut=2.4,
+                                  alpha=1.1, tune=False)
+    act = s.electrostatics.solver
+    s._sync_pairs(act._handle, types)
+    lib = _lib.load()
+    f = np.zeros((n, 3))
+    e, v = np.zeros(2), np.zeros(18)
+    flags = _lib.P3MX_FORCES | _lib.P3MX_ENERGY | _lib.P3MX_VIRIAL | _lib.P3MX_OVERWRITE
+    _lib.check(lib.p3mx_short_range(act._handle, n, _lib.dptr(pos), _lib.dptr(q), _lib.dptr(types),
+                                    _lib.dptr(f), e.ctypes.data_as(DP), v.ctypes.data_as(DP),
+                                    flags, None), act._handle)
+    prm = O.make_params(box, [32] * 3, 3, 1.1, 2.4, 1.5)
+    nt = 1 + int(types.max())
+    fo, eo, vc, vn = O.short_range(prm, pos, q, types, nt, O.pair_table(nt, pairs))
+    scale = np.abs(fo).max()
+    # a pair within FP32 rounding of the LJ cutoff changes two particles by the
+    # force there (0.06 at 2.0): counted apart
+    bad = np.abs(f - fo).max(1) > RTOL[cls] * scale
+    assert bad.sum() <= (0 if cls is P3M or form == "wca" else 2 * (1 + n // 20000))
+    assert np.abs(f - fo).max() <= max(RTOL[cls] * scale, 0.1 if bad.any() else 0.0)
+    np.testing.assert_allclose(e, eo, rtol=1e-9, atol=1e-9 * n)
+    np.testing.assert_allclose(v.reshape(2, 3, 3), [vc, vn], rtol=0,
+                               atol=1e-9 * max(np.abs(vc).max(), np.abs(vn).max()))
+
+
+# dipolar pair lanes: a 2x2x2 supercell (twice the mesh) gives every copy of a
+# dipole the forces and torques of the single cell
+@pytest.mark.parametrize("single,tol", [(False, 1e-9), (True, 2e-5)])
+@pytest.mark.parametrize("n,mesh", [(500, 10), (3750, 22), (7500, 28), (15000, 36)])
+def test_dipole_supercell(single, tol, n, mesh):
+    rng = np.random.default_rng(n)
+    edge = (n / 0.5) ** (1.0 / 3.0)
+    pos, _ = _ions(n, [edge] * 3, seed=n)
+    mu = rng.normal(size=(n, 3))
+    mu[::7] = 0.0  # non-magnetic particles
+
+    def compute(x, m, length, points):
+        act = DipolarP3M(prefactor=1.1, accuracy=1e-4, mesh=points, cao=5, r_cut=3.2, alpha=0.9,
+                         tune=False, single_precision=single)
+        act._set_system([length] * 3, 0.4, (True, True, True))
+        act._activate(x, m)
+        return act._compute(x, m, forces=True, energy=True)
+    f1, t1, e1 = compute(pos, mu, edge, mesh)
+    shifts = np.stack(np.meshgrid(*[[0, edge]] * 3, indexing="ij"), -1).reshape(-1, 3)
+    big = np.concatenate([pos + s for s in shifts])
+    f8, t8, e8 = compute(big, np.tile(mu, (8, 1)), 2 * edge, 2 * mesh)
+    np.testing.assert_allclose(f8.reshape(8, n, 3), np.broadcast_to(f1, (8, n, 3)), rtol=0,
+                               atol=tol * np.abs(f1).max())
+    np.testing.assert_allclose(t8.reshape(8, n, 3), np.broadcast_to(t1, (8, n, 3)), rtol=0,
+                               atol=tol * np.abs(t1).max())
+
+
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+def test_charge_change_and_table_change(cls):
+    """Setting the same pair table keeps the lists; another table, and a
+    particle that becomes charged, rebuild them."""
+    box = np.full(3, 14.0)
+    pos, q = _ions(1000, box, seed=4)
+    q[:100] = 0.0
+    s = eb.System(box_l=box)
+    s.time_step = 0.01
+    s.part.add(pos=pos, q=q)
+    s.non_bonded_inter[0, 0].wca.set_params(epsilon=1.0, sigma=1.0)
+    s.electrostatics.solver = cls(prefactor=1.0, accuracy=1e-3, mesh=24, cao=5, r_cut=2.5,
+                                  alpha=1.1, tune=False)
+    prm = O.make_params(box, [24] * 3, 5, 1.1, 2.5, 1.0)
+
+    def check(tab):
+        s.integrator.run(0)
+        fo = O.p3m_kspace(prm, pos, s.part.all().q)[0] + \
+            O.short_range(prm, pos, s.part.all().q, None, 1, O.pair_table(1, {(0, 0): tab}))[0]
+        np.testing.assert_allclose(s.part.all().f, fo, rtol=0, atol=RTOL[cls] * np.abs(fo).max())
+    count = ctypes.c_longlong()
+    check(dict(wca_eps=1.0, wca_sig=1.0))
+    _lib.load().p3mx_launch_count(s.electrostatics.solver._handle, ctypes.byref(count))
+    before = count.value
+    check(dict(wca_eps=1.0, wca_sig=1.0))
+    _lib.load().p3mx_launch_count(s.electrostatics.solver._handle, ctypes.byref(count))
+    assert count.value - before <= 15  # no rebuild: no cell sort, no list build
+    q[:100] = np.where(np.arange(100) % 2 == 0, 0.5, -0.5)
+    s.part.all().q = q
+    check(dict(wca_eps=1.0, wca_sig=1.0))
+    s.non_bonded_inter[0, 0].wca.set_params(epsilon=2.0, sigma=1.1)
+    check(dict(wca_eps=2.0, wca_sig=1.1))
+
+
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+def test_observables_without_forces(cls):
+    """p3mx_forces without a force array returns the energies and virials that
+    it returns with one."""
+    box = np.full(3, 15.0)
+    pos, q = _ions(1500, box, seed=5)
+    act = _actor(cls, box, pos, q, [32] * 3, 5, alpha=1.2, r_cut=2.5)
+    lib = _lib.load()
+    out = []
+    for force in (np.zeros((1500, 3)), None):
+        e, v = np.zeros(3), np.zeros(27)
+        _lib.check(lib.p3mx_forces(act._handle, 1500, _lib.dptr(pos), _lib.dptr(q), None,
+                                   _lib.dptr(force), e.ctypes.data_as(DP), v.ctypes.data_as(DP),
+                                   _lib.P3MX_ENERGY | _lib.P3MX_VIRIAL | _lib.P3MX_OVERWRITE, None),
+                   act._handle)
+        out.append(np.concatenate([e, v]))
+    np.testing.assert_array_equal(out[0], out[1])
