@@ -251,9 +251,8 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
   int const M0 = G.mesh[0], M1 = G.mesh[1], M2 = G.mesh[2];
-  int const H = M2 / 2 + 1;
   int const y = bk.a, kz0 = bk.b;
-  int const T = min(tile, H - kz0);
+  int const T = bk.w;
   int const ld = line_ld(M0);
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);
@@ -331,7 +330,7 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Blk const bk = blks[blk];
   RepGeom const &G = reps[bk.rep];
   int const M0 = G.mesh[0], M1 = G.mesh[1];
-  int const T = min(tile, G.mesh[2] / 2 + 1 - bk.b);
+  int const T = bk.w;
   int const ld = line_ld(M0);
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = TWO ? nullptr : a + tile * ld;

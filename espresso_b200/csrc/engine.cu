@@ -418,22 +418,29 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       int const H = M2 / 2 + 1;
       int const lines = M0 * M1;
       int const ldz = line_ld(M2);
-      // z passes: as many complex lines as give every thread of a block one
-      // transform of the smaller factor, within a quarter (FP64: half) of the
-      // SM's shared memory, and fewer where the launch would have less than
-      // two blocks per SM (meshes up to 64)
+      // z passes: at most as many complex lines as give every thread of a block
+      // one transform of the smaller factor, within a quarter (FP64: half) of
+      // the SM's shared memory; then as few as fill the same number of whole
+      // waves of resident blocks (a last wave that is nearly empty costs a
+      // whole one)
       AxisPlan const &pz = G.plan[2];
       bool const two = m_two[2];
       size_t const z_budget = m_fp32 ? 54 * 1024 : 100 * 1024;
       int const want = two ? 256 / std::min(pz.n1, pz.n2) : 256;
+      long long const slots = static_cast<long long>(m_fp32 ? 4 : 2) * sms;
+      auto const fill = [&](int most) {
+        long long const waves = (all_lines + most * slots - 1) / (most * slots);
+        int const l = ceil_div(all_lines, waves * slots);
+        return std::min(most, std::max(2, (l + 1) / 2 * 2));
+      };
       auto const zf_smem = [&](int pairs) {
-        return ((two ? 1 : 2) * static_cast<size_t>(pairs) * ldz + M2) * csz + 3 * M2 * sizeof(int);
+        return ((two ? 1 : 2) * static_cast<size_t>(pairs) * ldz + M2) * csz;
       };
       // forward: two real lines per complex transform
       int lz = 2;
       while (lz / 2 < want && lz + 2 <= kZfLines && zf_smem(lz / 2 + 1) <= z_budget)
         lz += 2;
-      lz = std::min(lz, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2));
+      lz = fill(lz);
       for (int l = 0; l < lines; l += lz)
         zf.push_back(Blk{r, l, std::min(lz, lines - l), 0});
       smem_zf = std::max(smem_zf, zf_smem((std::min(lz, lines) + 1) / 2));
@@ -444,16 +451,18 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       int lzi = 2;
       while (3 * (lzi + 2) / 2 <= want && lzi + 2 <= kZiLines && zi_smem(lzi + 2) <= z_budget)
         lzi += 2;
-      lzi = std::min(lzi, std::max(2, ceil_div(all_lines, 2 * sms) / 2 * 2));
+      lzi = fill(lzi);
       for (int l = 0; l < lines; l += lzi)
         zi.push_back(Blk{r, l, std::min(lzi, lines - l), 0});
       smem_zi = std::max(smem_zi, zi_smem(std::min(lzi, lines)));
+      // column tiles of equal width (no last tile of one column)
+      int const ty = ceil_div(H, ceil_div(H, m_tile_y)), tx = ceil_div(H, ceil_div(H, m_tile_x));
       for (int xx = 0; xx < M0; ++xx)
-        for (int k0 = 0; k0 < H; k0 += m_tile_y)
-          y.push_back(Blk{r, xx, k0, 0});
+        for (int k0 = 0; k0 < H; k0 += ty)
+          y.push_back(Blk{r, xx, k0, std::min(ty, H - k0)});
       for (int yy = 0; yy < M1; ++yy)
-        for (int k0 = 0; k0 < H; k0 += m_tile_x)
-          x.push_back(Blk{r, yy, k0, 0});
+        for (int k0 = 0; k0 < H; k0 += tx)
+          x.push_back(Blk{r, yy, k0, std::min(tx, H - k0)});
       m_blk_x_start.push_back(static_cast<int>(x.size()));
     }
     m_smem_zf = smem_zf;

@@ -33,8 +33,8 @@ namespace p3mx {
 struct Blk {
   int rep;
   int a;   // first line / x / y index
-  int b;   // second index (kz tile start) or unused
-  int pad;
+  int b;   // line count, or second index (kz tile start)
+  int w;   // columns of the kz tile (y and x passes)
 };
 
 // Shared-memory position of element i of a staged line: one pad slot per 16
@@ -466,13 +466,14 @@ template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 // X0[k] = (Z[k] + conj Z[n-k]) / 2 and X1[k] = -i (Z[k] - conj Z[n-k]) / 2.
 // bk.b real lines per block (an odd last line is paired with zeros).
 // The charge mesh exists only as the assignment's tiles: the block sums, for
-// every (x, y) line, the 1 to 4 tile rows that cover it (contiguous along z),
-// first each point's own super-brick (four points per load), then the points
-// in a halo of the previous one along z.
+// every (x, y) line, the 1 to 4 (in wrap corners 9) tile rows that cover it,
+// contiguous along z: first the points of each super-brick, four per load,
+// then its halo, added to the points of the next one.  Bound by instructions
+// (integer ones run at half rate), so the rows of a line are listed once in
+// shared memory and a warp works on one line at a time.
 // blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
 // Shared memory: bk.b/2 staged lines of line_ld(n) (twice that unless TWO),
-// twiddles (n), the halo points' z and offsets (3 n ints).  Meshes are even,
-// so is bk.b.
+// twiddles (n).  Meshes are even, so is bk.b.
 constexpr int kZfLines = 64; // most real lines per block
 template <typename Real, bool TWO>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
@@ -483,8 +484,8 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   using C = typename CplxOf<Real>::type;
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ long long s_bx[kZfLines][3];
-  __shared__ int s_by[kZfLines][3];
+  __shared__ long long s_row[kZfLines][9];
+  __shared__ int s_nrow[kZfLines];
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
   int const n = G.mesh[2];
@@ -494,75 +495,128 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = TWO ? nullptr : a + np * ld;
   C *tw = a + (TWO ? 1 : 2) * np * ld;
-  int *zc = reinterpret_cast<int *>(tw + n);
   tiles += blockIdx.y * tile_stride + G.tl_off;
   cmesh += blockIdx.y * c_stride;
   load_twiddles(tw, twtab, G.plan[2]);
   long long const line0 = bk.a;
-  int const nh = cov[G.cov_off[2] + 3 * n];
-  {
-    TileMap const tm(G, E);
+  TileMap const tm(G, E);
+  if (static_cast<int>(threadIdx.x) < nl) {
     int const M0 = G.mesh[0], M1 = G.mesh[1];
-    const int *cz = cov + G.cov_off[2];
-    for (int t = threadIdx.x; t < nh; t += blockDim.x) {
-      int const z = cz[3 * n + 1 + t];
-      zc[t] = z;
-      zc[n + t] = tm.z(cz[n + z]);
-      zc[2 * n + t] = tm.z(cz[2 * n + z]);
-    }
-    for (int t = threadIdx.x; t < 3 * nl; t += blockDim.x) {
-      int const l = t / 3, j = t - 3 * l;
-      int const x = static_cast<int>((line0 + l) / M1), y = static_cast<int>((line0 + l) % M1);
-      s_bx[l][j] = tm.x(cov[G.cov_off[0] + j * M0 + x]);
-      s_by[l][j] = tm.y(cov[G.cov_off[1] + j * M1 + y]);
-    }
+    int const x = static_cast<int>((line0 + threadIdx.x) / M1),
+              y = static_cast<int>((line0 + threadIdx.x) % M1);
+    int c = 0;
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) {
+        long long const bx = tm.x(cov[G.cov_off[0] + i * M0 + x]);
+        int const by = tm.y(cov[G.cov_off[1] + j * M1 + y]);
+        if (bx >= 0 && by >= 0)
+          s_row[threadIdx.x][c++] = bx + by;
+      }
+    s_nrow[threadIdx.x] = c;
   }
   __syncthreads();
   // real line l, element k -> real or imaginary part of slot l/2
   Real *ar = reinterpret_cast<Real *>(a);
   using R4 = typename Real4Of<Real>::type;
-  int const tz = sb_tile_z(E + G.cao - 1);
-  int const g4 = (n + 3) >> 2, total = nl * g4;
-  float const rg4 = 1.0f / static_cast<float>(g4);
+  auto row_sum = [&](int l, int z) {
+    int const c = s_nrow[l];
+    const long long *r = s_row[l];
+    const Real *t = tiles + z;
+    R4 s = *reinterpret_cast<const R4 *>(t + r[0]);
+    if (c == 2) {
+      s = tile_add(s, *reinterpret_cast<const R4 *>(t + r[1]));
+    } else if (c > 2) {
+      // three rows (wrap corners) or four and more
+      R4 const u = *reinterpret_cast<const R4 *>(t + r[1]),
+               v = *reinterpret_cast<const R4 *>(t + r[2]);
+      s = tile_add(s, u);
+      if (c == 3) {
+        s = tile_add(s, v);
+      } else {
+        s = tile_add(s, tile_add(v, *reinterpret_cast<const R4 *>(t + r[3])));
+        for (int k = 4; k < c; ++k)
+          s = tile_add(s, *reinterpret_cast<const R4 *>(t + r[k]));
+      }
+    }
+    return s;
+  };
+  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int const g4 = (n + 3) >> 2;
+  int const le = 31 - __clz(E), tz = tm.tz;
+  for (int l = warp; l < nl; l += 8) {
+    Real *o = ar + 2 * ((l >> 1) * ld) + (l & 1);
 #pragma unroll 2
-  for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    int const l = qdiv(t, g4, rg4), k = 4 * (t - l * g4);
-    // E is a multiple of 4: the four points lie in one super-brick (rows are
-    // padded, so the last group may reach past the mesh)
-    R4 const v = tile_rows<R4>(tiles, s_bx[l], s_by[l], (k / E) * tz + k % E);
-    Real *o = ar + 2 * ((l >> 1) * ld + pix(k)) + (l & 1);
-    o[0] = v.x;
-    o[2] = v.y;
-    if (k + 2 < n) {
-      o[4] = v.z;
-      o[6] = v.w;
+    for (int g = lane; g < g4; g += 32) {
+      // E is a multiple of 4: the four points lie in one super-brick (rows are
+      // padded, so the last group may reach past the mesh)
+      int const k = 4 * g;
+      R4 const v = row_sum(l, (k >> le) * tz + (k & (E - 1)));
+      Real *p = o + 2 * pix(k);
+      p[0] = v.x;
+      p[2] = v.y;
+      if (k + 2 < n) {
+        p[4] = v.z;
+        p[6] = v.w;
+      }
     }
   }
-  __syncthreads();
-  float const rnh = 1.0f / static_cast<float>(max(nh, 1));
-#pragma unroll 2
-  for (int t = threadIdx.x; t < nl * nh; t += blockDim.x) {
-    int const l = qdiv(t, nh, rnh), h = t - l * nh;
-    Real v = tile_rows<Real>(tiles, s_bx[l], s_by[l], zc[n + h]);
-    if (zc[2 * n + h] >= 0)
-      v += tile_rows<Real>(tiles, s_bx[l], s_by[l], zc[2 * n + h]);
-    ar[2 * ((l >> 1) * ld + pix(zc[h])) + (l & 1)] += v;
+  // halos: group h of super-brick b's, points (b E + len_b + 4 h ...) mod n.
+  // The last super-brick's length need not be a multiple of 4: its row
+  // segment is then read point by point
+  int const halo = G.cao - 1, nb = G.sbn[2], hg = (halo + 3) >> 2;
+  int const last = n - (nb - 1) * E; // length of the last super-brick
+  float const rhg = 1.0f / static_cast<float>(max(hg, 1));
+  // the halo of the one before the last may reach around the axis to the same
+  // points as the last one's: added after it
+  bool const around = nb > 1 && last < halo;
+  for (int pass = 0; pass < (around ? 2 : 1); ++pass) {
+    __syncthreads();
+    for (int l = warp; l < nl; l += 8) {
+      Real *o = ar + 2 * ((l >> 1) * ld) + (l & 1);
+      for (int t = lane; t < nb * hg; t += 32) {
+        int const bz = qdiv(t, hg, rhg), h = 4 * (t - bz * hg);
+        if (around && (bz == nb - 2) != (pass == 1))
+          continue;
+        int const len = bz == nb - 1 ? last : E;
+        Real v[4];
+        if ((len & 3) == 0) {
+          R4 const q = row_sum(l, bz * tz + len + h);
+          v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
+          for (int e = 0; e < 4; ++e) {
+            v[e] = Real(0);
+            if (h + e < halo)
+              for (int c = 0; c < s_nrow[l]; ++c)
+                v[e] += tiles[s_row[l][c] + bz * tz + len + h + e];
+          }
+        }
+        int z = bz * E + len + h;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          int const zz = z + e >= n ? (z + e) % n : z + e;
+          if (h + e < halo)
+            o[2 * pix(zz)] += v[e];
+        }
+      }
+    }
   }
   __syncthreads();
   C *res = fft_lines<TWO>(a, b, np, ld, G.plan[2], tw);
   int const H = n / 2 + 1;
   int const hp = G.hp;
-  for_lines(nl, hp, [&](int l, int k) {
-    C v{Real(0), Real(0)};
+  // both lines of a slot from one pair of entries
+  C *const out = cmesh + G.km_off + line0 * hp;
+  for_lines(np, hp, [&](int p, int k) {
+    C v0{Real(0), Real(0)}, v1 = v0;
     if (k < H) {
-      C const z = res[(l >> 1) * ld + pix(k)];
-      C const zc = res[(l >> 1) * ld + pix(k == 0 ? 0 : n - k)];
-      if ((l & 1) == 0)
-        v = C{Real(0.5) * (z.x + zc.x), Real(0.5) * (z.y - zc.y)};
-      else
-        v = C{Real(0.5) * (z.y + zc.y), Real(0.5) * (zc.x - z.x)};
+      C const z = res[p * ld + pix(k)];
+      C const zc = res[p * ld + pix(k == 0 ? 0 : n - k)];
+      v0 = C{Real(0.5) * (z.x + zc.x), Real(0.5) * (z.y - zc.y)};
+      v1 = C{Real(0.5) * (z.y + zc.y), Real(0.5) * (zc.x - z.x)};
     }
-    cmesh[G.km_off + (line0 + l) * hp + k] = v;
+    C *q = out + 2 * p * hp + k;
+    q[0] = v0;
+    q[hp] = v1;
   });
 }
 
@@ -602,9 +656,8 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Blk const bk = blks[blk];
   RepGeom const &G = reps[bk.rep];
   int const M1 = G.mesh[1];
-  int const H = G.mesh[2] / 2 + 1;
   int const x = bk.a, kz0 = bk.b;
-  int const T = min(tile, H - kz0);
+  int const T = bk.w;
   int const ld = line_ld(M1);
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = TWO ? nullptr : a + tile * ld;
@@ -676,9 +729,8 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
   int const M0 = G.mesh[0], M1 = G.mesh[1], M2 = G.mesh[2];
-  int const H = M2 / 2 + 1;
   int const y = bk.a, kz0 = bk.b;
-  int const T = min(tile, H - kz0);
+  int const T = bk.w;
   int const ld = line_ld(M0);
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);

@@ -354,8 +354,8 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   static_assert(NBS * NBS <= kSbMaxRuns, "run table too small");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bar;
-  __shared__ int s_r0[kSbMaxRuns], s_r1[kSbMaxRuns];
-  __shared__ int s_count;
+  __shared__ int s_r0[kSbMaxRuns], s_pre[kSbMaxRuns + 1];
+  __shared__ Real s_cf[8 * 8];
   pdl_enter();
   if (static_cast<int>(blockIdx.x) >= nsb)
     return; // whole block
@@ -376,28 +376,37 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   int const bx0 = o0 / B, by0 = o1 / B, bz0 = o2 / B;
   int const nbx = min(NBS, G.nbx - bx0), nby = min(NBS, G.nby - by0), nbz = min(NBS, G.nbz - bz0);
   int const ncol = nbx * nby;
-  if (tid < ncol) {
-    const int *st = start + G.brk_off;
-    int const col = ((bx0 + tid / nby) * G.nby + (by0 + tid % nby)) * G.nbz + bz0;
-    s_r0[tid] = st[col];
-    s_r1[tid] = st[col + nbz];
+  if (warp == 0) {
+    // the runs' first particles and the prefix of their counts
+    int r0 = 0, c = 0;
+    if (lane < ncol) {
+      const int *st = start + G.brk_off;
+      int const col = ((bx0 + lane / nby) * G.nby + (by0 + lane % nby)) * G.nbz + bz0;
+      r0 = st[col];
+      c = st[col + nbz] - r0;
+    }
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < kSbMaxRuns; o <<= 1) {
+      int const t = __shfl_up_sync(0xffffffffu, incl, o);
+      incl += lane >= o ? t : 0;
+    }
+    if (lane < ncol) {
+      s_r0[lane] = r0;
+      s_pre[lane + 1] = incl;
+    }
+    if (lane == 0)
+      s_pre[0] = 0;
   }
+  if (tid < 64 && (tid & 7) < P && (tid >> 3) < P)
+    s_cf[tid] = static_cast<Real>(kSpline.c[P][tid >> 3][tid & 7]);
   // zero the tile; initialise the staging barrier
   for (int t = tid; t < TW; t += NT)
     tile[t] = Word(0);
   if (tid == 0)
     mbar_init(&bar, 1);
   __syncthreads();
-  if (warp == 0) {
-    int c = (lane < ncol) ? s_r1[lane] - s_r0[lane] : 0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-      c += __shfl_xor_sync(0xffffffffu, c, off);
-    if (lane == 0)
-      s_count = c;
-  }
-  __syncthreads();
-  int const count = s_count;
+  int const count = s_pre[ncol];
   float const qmax = __uint_as_float(qmax_bits[sb.x]);
   // store the tile, value(x, y, z) (lanes along z: conflict-free shared
   // reads, row segments stored whole; the row padding is zero)
@@ -439,18 +448,24 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
     qoff[q] = qx[q] * SX + qy[q] * SY;
   }
   unsigned parity = 0;
-  for (int run = 0; run < ncol; ++run) {
-    int const s0 = s_r0[run], s1 = s_r1[run];
-    int const bx = bx0 + run / nby, by = by0 + run % nby;
-    int const b0 = (bx * G.nby + by) * G.nbz + bz0;
-    for (int c0 = s0; c0 < s1; c0 += CH) {
-      int const cn = min(CH, s1 - c0);
+  // chunks of particles across the runs (a chunk per run would end in a short
+  // one for every other run)
+  for (int c0 = 0; c0 < count; c0 += CH) {
+    {
+      int const cn = min(CH, count - c0);
       __syncthreads(); // the previous chunk is consumed
-      if (tid == 0) {
-        unsigned const nbytes = static_cast<unsigned>(cn * sizeof(PRec<Real>));
+      if (warp == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive_expect_tx(&bar, nbytes);
-        bulk_g2s(rec, recs + c0, nbytes, &bar);
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&bar, static_cast<unsigned>(cn * sizeof(PRec<Real>)));
+        }
+        __syncwarp();
+        if (lane < ncol) {
+          int const lo = max(c0, s_pre[lane]), hi = min(c0 + cn, s_pre[lane + 1]);
+          if (lo < hi)
+            bulk_g2s(rec + (lo - c0), recs + (s_r0[lane] + lo - s_pre[lane]),
+                     static_cast<unsigned>((hi - lo) * sizeof(PRec<Real>)), &bar);
+        }
       }
       bool const got = mbar_wait(&bar, parity);
       parity ^= 1u;
@@ -466,7 +481,9 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
       {
         int const k = tid & 7;
         Real cf[P];
-        spline_coef<P>(min(k, P - 1), cf);
+#pragma unroll
+        for (int m = 0; m < P; ++m)
+          cf[m] = s_cf[8 * min(k, P - 1) + m];
         for (int j = tid >> 3; j < cn; j += NT / 8) {
           PRec<Real> const &r = rec[j];
           if (k < P) {
@@ -476,7 +493,11 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
           } else if (k == 7) {
             // corner offset inside the super-brick, [0, E)^3
             int const sk = r.key;
-            int const bz = bz0 + ((sk >> (3 * LB)) - b0);
+            int run = 0;
+            while (c0 + j >= s_pre[run + 1])
+              ++run;
+            int const bx = bx0 + run / nby, by = by0 + run % nby;
+            int const bz = (sk >> (3 * LB)) - (bx * G.nby + by) * G.nbz;
             int const l = sk & (B3 - 1);
             int const dx = bx * B + (l >> (2 * LB)) - o0, dy = by * B + ((l >> LB) & (B - 1)) - o1,
                       dz = bz * B + (l & (B - 1)) - o2;
@@ -518,8 +539,7 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
 // point's own super-brick comes first.  A point lies in its own super-brick's
 // tile and maybe in the halo of the one before; the first P - 1 points of an
 // axis whose last super-brick is shorter than P - 1 also in that of the one
-// before the last.  Entry j of point i is at cov[cov_off + j M + i]; behind
-// the 3 M entries the number of points with a second cover and their list.
+// before the last.  Entry j of point i is at cov[cov_off + j M + i].
 inline void cover_table(int M, int E, int P, std::vector<int> &cov) {
   size_t const at = cov.size();
   cov.resize(at + 3 * static_cast<size_t>(M), -1);
@@ -534,13 +554,6 @@ inline void cover_table(int M, int E, int P, std::vector<int> &cov) {
           throw Error(3, "assignment tiles: more than three covers of a mesh point");
         cov[at + static_cast<size_t>(n[i]++) * M + i] = (b << 8) | l;
       }
-    }
-  cov.push_back(0);
-  size_t const cnt = cov.size() - 1;
-  for (int i = 0; i < M; ++i)
-    if (n[i] > 1) {
-      ++cov[cnt];
-      cov.push_back(i);
     }
 }
 

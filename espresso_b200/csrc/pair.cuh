@@ -686,11 +686,8 @@ constexpr int kPairFill = 768;
 // Bound by instruction issue (about 45 scalar instructions per entry and
 // three MUFU operations): the range-independent arithmetic runs on two
 // entries at a time in packed FP32, with the scalar code's roundings.
-#ifndef P3MX_PAIR_MINB
-#define P3MX_PAIR_MINB 3
-#endif
 template <int MODE, int LPP>
-__global__ void __launch_bounds__(256, P3MX_PAIR_MINB)
+__global__ void __launch_bounds__(256, 4)
 k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                   const float4 *__restrict__ spf, const int *__restrict__ stype,
                   const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
@@ -819,14 +816,11 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
       sz += ft * dz[u];
     }
   };
-  // the lane's group v: class A group v, or class B group v - ga
-  auto entries = [&](int v, int4 &g0, int4 &g1) {
+  auto group = [&](auto lj, int v) {
+    // the lane's group v: class A group v, or class B group v - ga
     int const grp = v < ga ? v : ngroups - 1 - (v - ga);
     const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
-    g0 = gp[0];
-    g1 = gp[1];
-  };
-  auto group = [&](auto lj, int4 const &g0, int4 const &g1) {
+    int4 const g0 = gp[0], g1 = gp[1];
     unsigned const ent[8] = {static_cast<unsigned>(g0.x), static_cast<unsigned>(g0.y),
                              static_cast<unsigned>(g0.z), static_cast<unsigned>(g0.w),
                              static_cast<unsigned>(g1.x), static_cast<unsigned>(g1.y),
@@ -846,21 +840,14 @@ k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
     fy += static_cast<double>(sy);
     fz += static_cast<double>(sz);
   };
-  // the next group's entries are loaded before the current group's pairs
-  int4 n0 = make_int4(0, 0, 0, 0), n1 = n0;
-  if (sub < gt)
-    entries(sub, n0, n1);
   for (int v0 = 0; v0 < gmax; v0 += LPP) {
     int const v = v0 + sub;
-    int4 const g0 = n0, g1 = n1;
-    if (v + LPP < gt)
-      entries(v + LPP, n0, n1);
     bool const any_a = __any_sync(0xffffffffu, v < ga);
     if (v < gt) {
       if (any_a)
-        group(std::true_type{}, g0, g1);
+        group(std::true_type{}, v);
       else
-        group(std::false_type{}, g0, g1);
+        group(std::false_type{}, v);
     }
   }
 #pragma unroll
