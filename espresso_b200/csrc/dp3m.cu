@@ -99,20 +99,19 @@ public:
       P3MX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(limit)));
     };
-    auto attrs = [&](auto zero, auto two) {
+    auto attrs = [&](auto zero) {
       using Real = decltype(zero);
-      constexpr bool TWO = decltype(two)::value;
-      attr(k_fft_x_dp3m<Real, true, TWO>);
-      attr(k_fft_x_dp3m<Real, false, TWO>);
-      attr(k_fft_x_dp3m_inv<Real, TWO>);
+      fft_pick(E.m_kind[0], [&](auto kind) {
+        constexpr int K = decltype(kind)::value;
+        attr(k_fft_x_dp3m<Real, true, K>);
+        attr(k_fft_x_dp3m<Real, false, K>);
+        attr(k_fft_x_dp3m_inv<Real, K>);
+      });
     };
-    if (E.fp32()) {
-      attrs(0.0f, std::true_type{});
-      attrs(0.0f, std::false_type{});
-    } else {
-      attrs(0.0, std::true_type{});
-      attrs(0.0, std::false_type{});
-    }
+    if (E.fp32())
+      attrs(0.0f);
+    else
+      attrs(0.0);
     // the field spectra and three field meshes
     E.m_field.ensure(kDipoleSpectra * E.m_cplx * csz);
     E.m_E.ensure(3 * 4 * E.m_ebins * rsz);
@@ -195,25 +194,24 @@ public:
     if (!want_ft && !want_e)
       return;
     {
-      auto const kern =
-          want_e ? (E.m_two[0] ? k_fft_x_dp3m<Real, true, true> : k_fft_x_dp3m<Real, true, false>)
-                 : (E.m_two[0] ? k_fft_x_dp3m<Real, false, true> : k_fft_x_dp3m<Real, false, false>);
-      kern<<<E.m_n_blk_x, 256, E.m_smem_x, st>>>(geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx,
-                                                 m_ge.as<Real>(), E.m_tile_x, m_part.as<double>(),
-                                                 E.m_tw.as<C>());
-      ++E.m_launches;
+      fft_pick(E.m_kind[0], [&](auto kind) {
+        constexpr int K = decltype(kind)::value;
+        pdl_launch(want_e ? k_fft_x_dp3m<Real, true, K> : k_fft_x_dp3m<Real, false, K>, E.m_n_blk_x,
+                   256, E.m_smem_x, st, true, geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx,
+                   m_ge.as<Real>(), E.m_tile_x, m_part.as<double>(), E.m_tw.as<C>());
+        ++E.m_launches;
+        if (want_ft) {
+          pdl_launch(k_fft_x_dp3m_inv<Real, K>, 5 * E.m_n_blk_x, 256, E.m_smem_x, st, true, geom,
+                     E.m_blk_x.as<Blk>(), ck3, E.m_cplx, m_ge.as<Real>(), m_gf.as<Real>(),
+                     E.m_field.as<C>(), E.m_tile_x, E.m_tw.as<C>());
+          ++E.m_launches;
+        }
+      });
       if (want_e) {
         k_dp3m_sum_rows<<<1, 32 * 1, 0, st>>>(m_part.as<double>(), E.m_n_blk_x, 1,
                                               m_sums.as<double>() + 5);
         ++E.m_launches;
       }
-    }
-    if (want_ft) {
-      auto const kern = E.m_two[0] ? k_fft_x_dp3m_inv<Real, true> : k_fft_x_dp3m_inv<Real, false>;
-      kern<<<5 * E.m_n_blk_x, 256, E.m_smem_x, st>>>(geom, E.m_blk_x.as<Blk>(), ck3, E.m_cplx,
-                                                     m_ge.as<Real>(), m_gf.as<Real>(),
-                                                     E.m_field.as<C>(), E.m_tile_x, E.m_tw.as<C>());
-      ++E.m_launches;
     }
     E.mark("dp_x_pass", st);
     if (!want_ft)

@@ -238,15 +238,16 @@ __global__ void k_dp3m_sum_rows(const double *__restrict__ partials, int nblk, i
 // the lines it read).
 // EV: per-block partial of the k-space energy sum G_energy |mk|^2 with the
 // Hermitian weights of the half mesh (1 at kz = 0 and M/2, else 2).
-// Shared memory: 2 x tile staged lines of line_ld(M) (3 x unless TWO: a
+// Shared memory: 2 x tile staged lines of line_ld(M) (3 x for KIND 0: a
 // scratch buffer), twiddles (M): the charge x pass's layout.
-template <typename Real, bool EV, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 && TWO ? 3 : 2)
+template <typename Real, bool EV, int KIND>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && KIND ? 3 : 2)
 k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              typename CplxOf<Real>::type *__restrict__ comp_hat, long long fstride,
              const Real *__restrict__ g_e, int tile, double *__restrict__ partials,
              const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Blk const bk = blks[blockIdx.x];
   RepGeom const &G = reps[bk.rep];
@@ -257,8 +258,8 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = a + L;
-  C *c = TWO ? nullptr : b + L;
-  C *tw = a + (TWO ? 2 : 3) * L;
+  C *c = KIND ? nullptr : b + L;
+  C *tw = a + (KIND ? 2 : 3) * L;
   load_twiddles(tw, twtab, G.plan[0]);
   long long const stride_x = static_cast<long long>(M1) * G.hp;
   int const tq = threadIdx.x & 15, xq = threadIdx.x >> 4;
@@ -275,9 +276,9 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       b[tq * ld + pix(x)] = C{dop_y * vy.x + dop_z * vz.x, dop_y * vy.y + dop_z * vz.y};
     }
   __syncthreads();
-  C *ra = fft_lines<TWO>(a, c, T, ld, G.plan[0], tw);
-  // without TWO: the buffer that the first transform left free
-  C *rb = fft_lines<TWO>(b, ra == a ? c : a, T, ld, G.plan[0], tw);
+  C *ra = fft_lines<KIND>(a, c, T, ld, G.plan[0], tw);
+  // with KIND 0: the buffer that the first transform left free
+  C *rb = fft_lines<KIND>(b, ra == a ? c : a, T, ld, G.plan[0], tw);
   double acc = 0.0;
   double const wgt = (kz == 0 || kz == M2 / 2) ? 1.0 : 2.0;
   for (int x = xq; col && x < M0; x += 16) {
@@ -317,14 +318,15 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
 // its powers (dp_y_pass, dp_z_pass), so 5 backward x transforms serve the
 // three torque fields and the six entries of the symmetric force-field tensor.
 // Shared memory: the forward pass's.
-template <typename Real, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 && TWO ? 3 : 2)
+template <typename Real, int KIND>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && KIND ? 3 : 2)
 k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
                  const typename CplxOf<Real>::type *__restrict__ mk_hat, long long fstride,
                  const Real *__restrict__ g_e, const Real *__restrict__ g_f,
                  typename CplxOf<Real>::type *__restrict__ field0, int tile,
                  const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int const blk = blockIdx.x / 5, o = blockIdx.x - 5 * blk;
   Blk const bk = blks[blk];
@@ -333,8 +335,8 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const T = bk.w;
   int const ld = line_ld(M0);
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = TWO ? nullptr : a + tile * ld;
-  C *tw = a + (TWO ? 2 : 3) * tile * ld;
+  C *b = KIND ? nullptr : a + tile * ld;
+  C *tw = a + (KIND ? 2 : 3) * tile * ld;
   load_twiddles(tw, twtab, G.plan[0]);
   long long const stride_x = static_cast<long long>(M1) * G.hp;
   int const tq = threadIdx.x & 15, xq = threadIdx.x >> 4;
@@ -353,7 +355,7 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       a[tq * ld + pix(x)] = tor ? C{c * m.y, c * m.x} : C{-c * m.x, c * m.y};
     }
   __syncthreads();
-  C const *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
+  C const *res = fft_lines<KIND>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
   int const rows = col ? (M0 - xq + 15) >> 4 : 0;
   C *q = field0 + fstride * o + base + xq * stride_x;
 #pragma unroll 4

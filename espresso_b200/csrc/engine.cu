@@ -398,15 +398,18 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     // twiddle table (n complex) in shared memory.  Axes whose lines all have
     // two-factor plans transform in place (one buffer fewer per pass)
     for (int d = 0; d < 3; ++d) {
-      m_two[d] = true;
-      for (auto const &G : m_geom)
-        m_two[d] = m_two[d] && G.plan[d].n1 > 0;
+      m_kind[d] = kFftPow2;
+      for (auto const &G : m_geom) {
+        int const n = G.mesh[d];
+        bool const pow2 = n >= 32 && n <= 256 && (n & (n - 1)) == 0;
+        m_kind[d] = std::min(m_kind[d], pow2 ? kFftPow2 : (G.plan[d].n1 > 0 ? kFftTwo : kFftAny));
+      }
     }
     size_t const ldy = line_ld(maxM1), ldx = line_ld(maxM0);
     // y and x passes: tiles of up to 16 kz columns; 72 KB keep three FP32
     // blocks of the x pass per SM at 256
-    size_t const y_budget = 72 * 1024, x_budget = m_two[0] ? 72 * 1024 : 96 * 1024;
-    size_t const y_bufs = m_two[1] ? 1 : 2, x_bufs = m_two[0] ? 2 : 3;
+    size_t const y_budget = 72 * 1024, x_budget = m_kind[0] ? 72 * 1024 : 96 * 1024;
+    size_t const y_bufs = m_kind[1] ? 1 : 2, x_bufs = m_kind[0] ? 2 : 3;
     m_tile_y = static_cast<int>(
         std::max<size_t>(1, std::min<size_t>(16, y_budget / (y_bufs * ldy * csz))));
     m_tile_x = static_cast<int>(
@@ -424,10 +427,10 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       // waves of resident blocks (a last wave that is nearly empty costs a
       // whole one)
       AxisPlan const &pz = G.plan[2];
-      bool const two = m_two[2];
+      bool const two = m_kind[2] != kFftAny;
       size_t const z_budget = m_fp32 ? 54 * 1024 : 100 * 1024;
       int const want = two ? 256 / std::min(pz.n1, pz.n2) : 256;
-      long long const slots = static_cast<long long>(m_fp32 ? 4 : 2) * sms;
+      long long const slots = static_cast<long long>(m_fp32 ? (m_kind[2] == kFftTwo ? 3 : 4) : 2) * sms;
       auto const fill = [&](int most) {
         long long const waves = (all_lines + most * slots - 1) / (most * slots);
         int const l = ceil_div(all_lines, waves * slots);
@@ -506,22 +509,23 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
         aset(k_p3m_interp<double, 7>);
       }
     }
-    auto fft_attrs = [&](auto zero, auto two) {
+    auto fft_attrs = [&](auto zero, int two) {
       using Real = decltype(zero);
-      constexpr bool TWO = decltype(two)::value;
-      attr(k_fft_z_fwd<Real, TWO>, m_smem_zf);
-      attr(k_fft_y<Real, false, TWO>, m_smem_y);
-      attr(k_fft_y<Real, true, TWO>, m_smem_y);
-      attr(k_fft_x_kspace<Real, true, TWO>, m_smem_x);
-      attr(k_fft_x_kspace<Real, false, TWO>, m_smem_x);
-      attr(k_fft_z_inv3<Real, TWO>, m_smem_zi);
+      fft_pick(two, [&](auto kind) {
+        constexpr int K = decltype(kind)::value;
+        attr(k_fft_z_fwd<Real, K>, m_smem_zf);
+        attr(k_fft_y<Real, false, K>, m_smem_y);
+        attr(k_fft_y<Real, true, K>, m_smem_y);
+        attr(k_fft_x_kspace<Real, true, K>, m_smem_x);
+        attr(k_fft_x_kspace<Real, false, K>, m_smem_x);
+        attr(k_fft_z_inv3<Real, K>, m_smem_zi);
+      });
     };
-    if (m_fp32) {
-      fft_attrs(0.0f, std::true_type{});
-      fft_attrs(0.0f, std::false_type{});
-    } else {
-      fft_attrs(0.0, std::true_type{});
-      fft_attrs(0.0, std::false_type{});
+    for (int k : {m_kind[0], m_kind[1], m_kind[2]}) {
+      if (m_fp32)
+        fft_attrs(0.0f, k);
+      else
+        fft_attrs(0.0, k);
     }
   }
   // buffers
@@ -837,13 +841,13 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   // 4. x pass fused with the k-space operator (+ energy/virial partials)
   bool const want_f = (f != nullptr);
   bool const want_ev = want_e || want_v;
-  {
-    auto const kern = want_ev ? (m_two[0] ? k_fft_x_kspace<Real, true, true> : k_fft_x_kspace<Real, true, false>)
-                              : (m_two[0] ? k_fft_x_kspace<Real, false, true> : k_fft_x_kspace<Real, false, false>);
-    pdl_launch(kern, m_n_blk_x, 256, m_smem_x, st, true, geom, m_blk_x.as<Blk>(), m_ck.as<C>(),
-               m_ginf.as<Real>(), m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0,
-               m_part_x.as<double>(), m_tw.as<C>());
-  }
+  fft_pick(m_kind[0], [&](auto kind) {
+    constexpr int K = decltype(kind)::value;
+    pdl_launch(want_ev ? k_fft_x_kspace<Real, true, K> : k_fft_x_kspace<Real, false, K>, m_n_blk_x,
+               256, m_smem_x, st, true, geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(),
+               m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0, m_part_x.as<double>(),
+               m_tw.as<C>());
+  });
   ++m_launches;
   if (want_ev) {
     k_reduce_partials<<<dim3(R, 8), 256, 0, st>>>(m_part_x.as<double>(), 8,
@@ -1075,32 +1079,34 @@ void Engine::prepare_short_range(cudaStream_t st, bool need_spq) {
 template <typename Real>
 void Engine::launch_fft_z_fwd(const Real *tiles, void *spectra, int sets, cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
-  auto const kern = m_two[2] ? k_fft_z_fwd<Real, true> : k_fft_z_fwd<Real, false>;
-  pdl_launch(
-      kern, dim3(m_n_blk_zf, sets), 256, m_smem_zf, st, true, m_geom_d.as<RepGeom>(),
-      m_blk_zf.as<Blk>(), tiles, m_tiles_n, m_cov.as<int>(), m_sb_edge,
-      static_cast<C *>(spectra), m_cplx, m_tw.as<C>());
+  fft_pick(m_kind[2], [&](auto kind) {
+    pdl_launch(k_fft_z_fwd<Real, decltype(kind)::value>, dim3(m_n_blk_zf, sets), 256, m_smem_zf, st,
+               true, m_geom_d.as<RepGeom>(), m_blk_zf.as<Blk>(), tiles, m_tiles_n, m_cov.as<int>(),
+               m_sb_edge, static_cast<C *>(spectra), m_cplx, m_tw.as<C>());
+  });
   ++m_launches;
 }
 template <typename Real>
 void Engine::launch_fft_y(void *c0, long long field_stride, YPass const &job, bool inv, int kscale,
                           cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
-  auto const kern = inv ? (m_two[1] ? k_fft_y<Real, true, true> : k_fft_y<Real, true, false>)
-                        : (m_two[1] ? k_fft_y<Real, false, true> : k_fft_y<Real, false, false>);
-  pdl_launch(
-      kern, m_n_blk_y * job.n, 256, m_smem_y, st, true, m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(), static_cast<C *>(c0), field_stride, job, kscale,
-      m_tile_y, m_tw.as<C>());
+  fft_pick(m_kind[1], [&](auto kind) {
+    constexpr int K = decltype(kind)::value;
+    pdl_launch(inv ? k_fft_y<Real, true, K> : k_fft_y<Real, false, K>, m_n_blk_y * job.n, 256,
+               m_smem_y, st, true, m_geom_d.as<RepGeom>(), m_blk_y.as<Blk>(), static_cast<C *>(c0),
+               field_stride, job, kscale, m_tile_y, m_tw.as<C>());
+  });
   ++m_launches;
 }
 template <typename Real>
 void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp, int sets,
                               int kscale, void *fields, cudaStream_t st) {
   using C = typename CplxOf<Real>::type;
-  auto const kern = m_two[2] ? k_fft_z_inv3<Real, true> : k_fft_z_inv3<Real, false>;
-  pdl_launch(
-      kern, dim3(m_n_blk_zi, sets), 256, m_smem_zi, st, true, m_geom_d.as<RepGeom>(), m_blk_zi.as<Blk>(), static_cast<C *>(c0), field_stride, zp, kscale,
-      static_cast<Real *>(fields), m_ebins, m_tw.as<C>());
+  fft_pick(m_kind[2], [&](auto kind) {
+    pdl_launch(k_fft_z_inv3<Real, decltype(kind)::value>, dim3(m_n_blk_zi, sets), 256, m_smem_zi, st,
+               true, m_geom_d.as<RepGeom>(), m_blk_zi.as<Blk>(), static_cast<C *>(c0), field_stride,
+               zp, kscale, static_cast<Real *>(fields), m_ebins, m_tw.as<C>());
+  });
   ++m_launches;
 }
 

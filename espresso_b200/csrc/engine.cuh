@@ -219,7 +219,7 @@ private:
   int m_n_blk_mesh = 0, m_n_blk_cplx = 0, m_n_blk_census = 0, m_n_blk_pair = 0;
   int m_n_blk_zf = 0, m_n_blk_y = 0, m_n_blk_x = 0, m_n_blk_zi = 0;
   int m_tile_y = 16, m_tile_x = 16;
-  bool m_two[3] = {true, true, true}; // every replica's lines of the axis have two-factor plans
+  int m_kind[3] = {0, 0, 0}; // per axis the transform kind that serves every replica (kFft...)
   size_t m_smem_zf = 0, m_smem_y = 0, m_smem_x = 0, m_smem_zi = 0;
 
   // particles

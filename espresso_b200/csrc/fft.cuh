@@ -399,35 +399,32 @@ __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__re
   case 15: { constexpr int R = 15; CALL; } break;                              \
   default: { constexpr int R = 16; CALL; } break;                              \
   }
-// In-place transform of nlines lines (plan with n1, n2); the caller's block
-// of at least 16 threads synchronises before, the result is visible after.
-template <typename C>
-__device__ __forceinline__ void fft_lines_2(C *a, int nlines, int ld, AxisPlan const &pl,
-                                            const C *__restrict__ tw) {
-  switch (pl.n) {
-  case 32: fft_pow2<C, 8, 4>(a, nlines, ld, tw); break;
-  case 64: fft_pow2<C, 8, 8>(a, nlines, ld, tw); break;
-  case 128: fft_pow2<C, 16, 8>(a, nlines, ld, tw); break;
-  case 256: fft_pow2<C, 16, 16>(a, nlines, ld, tw); break;
-  default:
+// Forward transform of nlines lines in `a` (element i of line l at
+// l*ld + pix(i)); tw = the axis twiddle table (shared memory).  KIND, for all
+// lines of a launch: kFftPow2 -- powers of two 32 to 256, in place,
+// compile-time factors (without the other factors' code a pass needs no
+// spills at four blocks per SM); kFftTwo -- two-factor plans, in place;
+// kFftAny -- Stockham stages with `b`, a second buffer of the same size.
+// Returns the buffer holding the result.  All threads of the block call it
+// behind a barrier; the result is visible when it returns.
+constexpr int kFftAny = 0, kFftTwo = 1, kFftPow2 = 2;
+template <int KIND, typename C>
+__device__ __forceinline__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
+                                        const C *__restrict__ tw) {
+  if constexpr (KIND == kFftPow2) {
+    switch (pl.n) {
+    case 32: fft_pow2<C, 8, 4>(a, nlines, ld, tw); break;
+    case 64: fft_pow2<C, 8, 8>(a, nlines, ld, tw); break;
+    case 128: fft_pow2<C, 16, 8>(a, nlines, ld, tw); break;
+    default: fft_pow2<C, 16, 16>(a, nlines, ld, tw); break;
+    }
+    __syncthreads();
+    return a;
+  } else if constexpr (KIND == kFftTwo) {
     P3MX_FACTOR_DISPATCH(pl.n1, (fft_step1<C, R>(a, nlines, ld, pl.n2, tw)))
     __syncthreads();
     P3MX_FACTOR_DISPATCH(pl.n2, (fft_step2<C, R>(a, nlines, ld, pl.n1)))
-    break;
-  }
-  __syncthreads();
-}
-
-// Forward transform of nlines lines in `a` (element i of line l at
-// l*ld + pix(i)); tw = the axis twiddle table (shared memory).  TWO: the
-// launch's lines all have two-factor plans and transform in place (b
-// unused); otherwise `b` is a second buffer of the same size.  Returns the
-// buffer holding the result.  All threads of the block must call it.
-template <bool TWO, typename C>
-__device__ __forceinline__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
-                                        const C *__restrict__ tw) {
-  if constexpr (TWO) {
-    fft_lines_2(a, nlines, ld, pl, tw);
+    __syncthreads();
     return a;
   } else {
     int const n = pl.n;
@@ -455,6 +452,21 @@ __device__ __forceinline__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan
   }
 }
 
+// f(integral_constant<int, kind>) for a runtime kind.
+template <typename Fn> inline void fft_pick(int kind, Fn &&f) {
+  if (kind == kFftPow2)
+    f(std::integral_constant<int, kFftPow2>{});
+  else if (kind == kFftTwo)
+    f(std::integral_constant<int, kFftTwo>{});
+  else
+    f(std::integral_constant<int, kFftAny>{});
+}
+
+// Blocks per SM of the z and y passes (their registers are sized for it).
+template <typename Real, int KIND> __host__ __device__ constexpr int fft_blocks() {
+  return sizeof(Real) == 4 ? (KIND == kFftTwo ? 3 : 4) : 2;
+}
+
 // Signed frequency of index i in an axis of m points, the Nyquist index as
 // zero (calc_meshift with the differential operator's convention,
 // p3m/common.hpp:248-264).
@@ -472,11 +484,11 @@ template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 // (integer ones run at half rate), so the rows of a line are listed once in
 // shared memory and a warp works on one line at a time.
 // blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
-// Shared memory: bk.b/2 staged lines of line_ld(n) (twice that unless TWO),
+// Shared memory: bk.b/2 staged lines of line_ld(n) (twice that for KIND 0),
 // twiddles (n).  Meshes are even, so is bk.b.
 constexpr int kZfLines = 64; // most real lines per block
-template <typename Real, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
+template <typename Real, int KIND>
+__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
 k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
             const Real *__restrict__ tiles, long long tile_stride, const int *__restrict__ cov,
             int E, typename CplxOf<Real>::type *__restrict__ cmesh, long long c_stride,
@@ -493,8 +505,8 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const nl = bk.b;          // real lines in this block
   int const np = (nl + 1) >> 1; // complex lines
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = TWO ? nullptr : a + np * ld;
-  C *tw = a + (TWO ? 1 : 2) * np * ld;
+  C *b = KIND ? nullptr : a + np * ld;
+  C *tw = a + (KIND ? 1 : 2) * np * ld;
   tiles += blockIdx.y * tile_stride + G.tl_off;
   cmesh += blockIdx.y * c_stride;
   load_twiddles(tw, twtab, G.plan[2]);
@@ -601,7 +613,7 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
   }
   __syncthreads();
-  C *res = fft_lines<TWO>(a, b, np, ld, G.plan[2], tw);
+  C *res = fft_lines<KIND>(a, b, np, ld, G.plan[2], tw);
   int const H = n / 2 + 1;
   int const hp = G.hp;
   // both lines of a slot from one pair of entries
@@ -641,11 +653,11 @@ inline YPass y_plain(int nf) {
 // and phi (arrays 2 and 3) from phi (array 1)
 inline YPass y_charge() { return YPass{3, {1, 1, 0}, {2, 3, 0}, {1, 0, 0}}; }
 constexpr int kChargeSpectra = 4; // arrays of the charge fields' spectra
-// TWO: every replica's y lines transform in place (the host checks).  kscale:
+// KIND: every replica's y lines transform in place (the host checks).  kscale:
 // k_y in units of 2 pi / box (1) or as an integer (0).  Shared memory: tile
-// staged lines of line_ld(M1) (two sets unless TWO), twiddles (M1).
-template <typename Real, bool INV, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
+// staged lines of line_ld(M1) (two sets for KIND 0), twiddles (M1).
+template <typename Real, bool INV, int KIND>
+__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
 k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
         typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, YPass const job,
         int kscale, int tile, const typename CplxOf<Real>::type *__restrict__ twtab) {
@@ -660,8 +672,8 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const T = bk.w;
   int const ld = line_ld(M1);
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = TWO ? nullptr : a + tile * ld;
-  C *tw = a + (TWO ? 1 : 2) * tile * ld;
+  C *b = KIND ? nullptr : a + tile * ld;
+  C *tw = a + (KIND ? 1 : 2) * tile * ld;
   load_twiddles(tw, twtab, G.plan[1]);
   long long const hp = G.hp;
   // 16 x 16 thread mapping (tile <= 16 columns): column tq, rows yq + 16 i
@@ -697,7 +709,7 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       }
   }
   __syncthreads();
-  const C *res = fft_lines<TWO>(a, b, T, ld, G.plan[1], tw) + tq * ld + yq;
+  const C *res = fft_lines<KIND>(a, b, T, ld, G.plan[1], tw) + tq * ld + yq;
   C *q = dst + yq * hp;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u, q += step) {
@@ -712,11 +724,11 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
 // Emits two backward-x-transformed spectra: array 0 i k_x phi, array 1 i phi
 // (the y and z passes apply k_y and k_z).
 // Shared memory: 2 x tile staged lines of line_ld(M0) (phi, k_x phi; 3 x
-// unless TWO: a scratch buffer), twiddles (M0).
+// for KIND 0: a scratch buffer), twiddles (M0).
 // EV: energy / virial partials (a template parameter, so that the
 // forces-only instance carries none of their registers).
-template <typename Real, bool EV, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 && !EV && TWO ? 3 : 2)
+template <typename Real, bool EV, int KIND>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 && !EV && KIND ? 3 : 2)
 k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
                const typename CplxOf<Real>::type *__restrict__ rho_hat,
                const Real *__restrict__ ginf, typename CplxOf<Real>::type *__restrict__ field0,
@@ -735,8 +747,8 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const L = tile * ld;
   C *a = reinterpret_cast<C *>(smem_raw);
   C *b = a + L;
-  C *c = TWO ? nullptr : b + L;
-  C *tw = a + (TWO ? 2 : 3) * L;
+  C *c = KIND ? nullptr : b + L;
+  C *tw = a + (KIND ? 2 : 3) * L;
   load_twiddles(tw, twtab, G.plan[0]);
   long long const stride_x = static_cast<long long>(M1) * G.hp;
   long long const base = G.km_off + static_cast<long long>(y) * G.hp + kz0;
@@ -759,7 +771,7 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
   }
   __syncthreads();
-  C *res = fft_lines<TWO>(a, b, T, ld, G.plan[0], tw);
+  C *res = fft_lines<KIND>(a, b, T, ld, G.plan[0], tw);
   C *fb = (res == a) ? b : a; // k_x phi goes to the free buffer
   // k-space operator
   double const wv[3] = {2.0 * kPi * G.box_i[0], 2.0 * kPi * G.box_i[1],
@@ -824,17 +836,17 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   if (!want_fields)
     return;
   __syncthreads();
-  // without TWO the scratch of the second transform is the first's buffer
+  // with KIND 0 the scratch of the second transform is the first's buffer
   // once that is stored
-  const C *f0 = fft_lines<TWO>(fb, c, T, ld, G.plan[0], tw) + tq * ld + xq;
+  const C *f0 = fft_lines<KIND>(fb, c, T, ld, G.plan[0], tw) + tq * ld + xq;
   int const rows = col ? (M0 - xq + 15) >> 4 : 0;
   C *q = field0 + base + xq * stride_x + tq;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u)
     q[u * 16 * stride_x] = cswap(f0[17 * u]);
-  if constexpr (!TWO)
+  if constexpr (!KIND)
     __syncthreads();
-  const C *f1 = fft_lines<TWO>(res, fb, T, ld, G.plan[0], tw) + tq * ld + xq;
+  const C *f1 = fft_lines<KIND>(res, fb, T, ld, G.plan[0], tw) + tq * ld + xq;
   q += field_stride;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u)
@@ -855,13 +867,13 @@ inline ZPass z_charge() { return ZPass{{0, 2, 3}, {0, 0, 1}}; }
 // a thread reads entry k of the slot's two half rows and writes entries k and
 // n - k (real and imaginary parts swapped: a backward transform).
 // Set blockIdx.y writes the field mesh e_stride records further on.
-// Shared memory: nl + ceil(nl/2) staged lines of line_ld(n) (twice unless
-// TWO), twiddles (n).  FP32: four blocks per SM -- the block's load, transform
+// Shared memory: nl + ceil(nl/2) staged lines of line_ld(n) (twice for
+// KIND 0), twiddles (n).  FP32: four blocks per SM -- the block's load, transform
 // and store phases do not overlap, so the fourth resident block pays for the
 // 64-register bound.
 constexpr int kZiLines = 128; // most lines per block
-template <typename Real, bool TWO>
-__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
+template <typename Real, int KIND>
+__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
 k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              const typename CplxOf<Real>::type *__restrict__ field0, long long field_stride,
              ZPass const zp, int kscale, Real *__restrict__ efield, long long e_stride,
@@ -879,8 +891,8 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const nc = nl + nz;
   long long const line0 = bk.a;
   C *a = reinterpret_cast<C *>(smem_raw);
-  C *b = TWO ? nullptr : a + nc * ld;
-  C *tw = a + (TWO ? 1 : 2) * nc * ld;
+  C *b = KIND ? nullptr : a + nc * ld;
+  C *tw = a + (KIND ? 1 : 2) * nc * ld;
   load_twiddles(tw, twtab, G.plan[2]);
   const C *fsrc = field0 + G.km_off + line0 * G.hp;
   int const set = 3 * blockIdx.y;
@@ -921,7 +933,7 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     put(nl + j, k, r[0], (2 * j + 1 < nl) ? r[hp] : C{Real(0), Real(0)}, pz, pz);
   }
   __syncthreads();
-  const C *res = fft_lines<TWO>(a, b, nc, ld, G.plan[2], tw);
+  const C *res = fft_lines<KIND>(a, b, nc, ld, G.plan[2], tw);
   // packed field mesh: one (Ex, Ey, Ez, 0) record per mesh point, so the
   // interpolation gathers one 16-byte (FP32) record per stencil point
   // (ghost-padded: every record also goes to its periodic images in the
