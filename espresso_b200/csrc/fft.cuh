@@ -129,7 +129,8 @@ template <int K, int N, typename C> __device__ __forceinline__ C mul_root(C v) {
 
 // In-register forward DFT of length R, natural order in and out: 2 and 4
 // directly, odd primes from the sums and differences of mirrored inputs,
-// composites R = A B as B transforms of length A, twiddles, A of length B.
+// 8 and 16 from halves, other composites R = A B as B transforms of length A,
+// twiddles, A of length B.
 template <typename C, int R> __device__ __forceinline__ void dft(C *v) {
   using Real = decltype(v[0].x);
   if constexpr (R == 2) {
@@ -171,6 +172,22 @@ template <typename C, int R> __device__ __forceinline__ void dft(C *v) {
       // X_K = a - i b, X_{R-K} = a + i b
       v[K] = C{a.x + b.y, a.y - b.x};
       v[R - K] = C{a.x - b.y, a.y + b.x};
+    });
+  } else if constexpr (R == 8 || R == 16) {
+    // halves of even and odd inputs (the fewest live registers)
+    constexpr int H = R / 2;
+    C e[H], o[H];
+    static_for<0, H>([&](auto i) {
+      e[decltype(i)::value] = v[2 * decltype(i)::value];
+      o[decltype(i)::value] = v[2 * decltype(i)::value + 1];
+    });
+    dft<C, H>(e);
+    dft<C, H>(o);
+    static_for<0, H>([&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      C const t = mul_root<K, R>(o[K]);
+      v[K] = cadd(e[K], t);
+      v[K + H] = csub(e[K], t);
     });
   } else {
     constexpr int A = R % 4 == 0 ? 4 : (R % 2 == 0 ? 2 : 3), B = R / A;
@@ -482,7 +499,7 @@ template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 // contiguous along z: first the points of each super-brick, four per load,
 // then its halo, added to the points of the next one.  Bound by instructions
 // (integer ones run at half rate), so the rows of a line are listed once in
-// shared memory and a warp works on one line at a time.
+// shared memory.
 // blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
 // Shared memory: bk.b/2 staged lines of line_ld(n) (twice that for KIND 0),
 // twiddles (n).  Meshes are even, so is bk.b.
@@ -552,24 +569,21 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
     return s;
   };
-  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int const g4 = (n + 3) >> 2;
   int const le = 31 - __clz(E), tz = tm.tz;
-  for (int l = warp; l < nl; l += 8) {
-    Real *o = ar + 2 * ((l >> 1) * ld) + (l & 1);
+  float const rg4 = 1.0f / static_cast<float>(g4);
 #pragma unroll 2
-    for (int g = lane; g < g4; g += 32) {
-      // E is a multiple of 4: the four points lie in one super-brick (rows are
-      // padded, so the last group may reach past the mesh)
-      int const k = 4 * g;
-      R4 const v = row_sum(l, (k >> le) * tz + (k & (E - 1)));
-      Real *p = o + 2 * pix(k);
-      p[0] = v.x;
-      p[2] = v.y;
-      if (k + 2 < n) {
-        p[4] = v.z;
-        p[6] = v.w;
-      }
+  for (int t = threadIdx.x; t < nl * g4; t += 256) {
+    // E is a multiple of 4: the four points lie in one super-brick (rows are
+    // padded, so the last group may reach past the mesh)
+    int const l = qdiv(t, g4, rg4), k = 4 * (t - l * g4);
+    R4 const v = row_sum(l, (k >> le) * tz + (k & (E - 1)));
+    Real *p = ar + 2 * ((l >> 1) * ld + pix(k)) + (l & 1);
+    p[0] = v.x;
+    p[2] = v.y;
+    if (k + 2 < n) {
+      p[4] = v.z;
+      p[6] = v.w;
     }
   }
   // halos: group h of super-brick b's, points (b E + len_b + 4 h ...) mod n.
@@ -577,38 +591,39 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   // segment is then read point by point
   int const halo = G.cao - 1, nb = G.sbn[2], hg = (halo + 3) >> 2;
   int const last = n - (nb - 1) * E; // length of the last super-brick
+  int const per = nb * hg;           // halo groups of a line
+  float const rper = 1.0f / static_cast<float>(max(per, 1));
   float const rhg = 1.0f / static_cast<float>(max(hg, 1));
   // the halo of the one before the last may reach around the axis to the same
   // points as the last one's: added after it
   bool const around = nb > 1 && last < halo;
   for (int pass = 0; pass < (around ? 2 : 1); ++pass) {
     __syncthreads();
-    for (int l = warp; l < nl; l += 8) {
-      Real *o = ar + 2 * ((l >> 1) * ld) + (l & 1);
-      for (int t = lane; t < nb * hg; t += 32) {
-        int const bz = qdiv(t, hg, rhg), h = 4 * (t - bz * hg);
-        if (around && (bz == nb - 2) != (pass == 1))
-          continue;
-        int const len = bz == nb - 1 ? last : E;
-        Real v[4];
-        if ((len & 3) == 0) {
-          R4 const q = row_sum(l, bz * tz + len + h);
-          v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-        } else {
-          for (int e = 0; e < 4; ++e) {
-            v[e] = Real(0);
-            if (h + e < halo)
-              for (int c = 0; c < s_nrow[l]; ++c)
-                v[e] += tiles[s_row[l][c] + bz * tz + len + h + e];
-          }
-        }
-        int z = bz * E + len + h;
-#pragma unroll
+    for (int t = threadIdx.x; t < nl * per; t += 256) {
+      int const l = qdiv(t, per, rper), u = t - l * per;
+      int const bz = qdiv(u, hg, rhg), h = 4 * (u - bz * hg);
+      if (around && (bz == nb - 2) != (pass == 1))
+        continue;
+      int const len = bz == nb - 1 ? last : E;
+      Real v[4];
+      if ((len & 3) == 0) {
+        R4 const q = row_sum(l, bz * tz + len + h);
+        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+      } else {
         for (int e = 0; e < 4; ++e) {
-          int const zz = z + e >= n ? (z + e) % n : z + e;
+          v[e] = Real(0);
           if (h + e < halo)
-            o[2 * pix(zz)] += v[e];
+            for (int c = 0; c < s_nrow[l]; ++c)
+              v[e] += tiles[s_row[l][c] + bz * tz + len + h + e];
         }
+      }
+      Real *o = ar + 2 * ((l >> 1) * ld) + (l & 1);
+      int const z = bz * E + len + h;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        int const zz = z + e >= n ? (z + e) % n : z + e;
+        if (h + e < halo)
+          o[2 * pix(zz)] += v[e];
       }
     }
   }
