@@ -142,6 +142,8 @@ struct p3mx_batch {
   std::vector<std::vector<BatchChoice>> by_cao;
   std::vector<int> caos; // the cao of every replica
   DevBuf vel, step;
+  Pinned h_out; // staging of p3mx_batch_get
+  ChunkEvents out_events;
   bool forces_valid = false;
   cudaGraphExec_t graph = nullptr;
   double g_dt = 0, g_kT = -1, g_gamma = -1;
@@ -770,12 +772,42 @@ int p3mx_batch_get(p3mx_batch *b, double *pos, double *f, double *vel) {
     Engine &e = *b->eng;
     cudaStream_t st = e.stream();
     size_t const bytes = 3 * static_cast<size_t>(e.n_part()) * sizeof(double);
-    if (pos)
-      P3MX_CUDA(cudaMemcpyAsync(pos, e.d_pos(), bytes, cudaMemcpyDeviceToHost, st));
-    if (f)
-      P3MX_CUDA(cudaMemcpyAsync(f, e.d_force(), bytes, cudaMemcpyDeviceToHost, st));
-    if (vel)
-      P3MX_CUDA(cudaMemcpyAsync(vel, b->vel.p, bytes, cudaMemcpyDeviceToHost, st));
+    // through a ring of pinned chunks, each copied to the caller's array by the
+    // host pool while the next ones are in flight (a copy to pageable memory
+    // runs at a sixth of the link's rate)
+    constexpr size_t kChunk = size_t(1) << 20, kSlots = 4;
+    struct Chunk {
+      char *dst;
+      const char *src;
+      size_t n;
+    };
+    std::vector<Chunk> chunks;
+    auto add = [&](double *dst, const void *src) {
+      for (size_t off = 0; dst && off < bytes; off += kChunk)
+        chunks.push_back(Chunk{reinterpret_cast<char *>(dst) + off,
+                               static_cast<const char *>(src) + off,
+                               std::min(kChunk, bytes - off)});
+    };
+    add(pos, e.d_pos());
+    add(f, e.d_force());
+    add(vel, b->vel.p);
+    b->h_out.ensure(kSlots * kChunk);
+    char *const buf = b->h_out.as<char>();
+    auto issue = [&](size_t k) {
+      P3MX_CUDA(cudaMemcpyAsync(buf + (k % kSlots) * kChunk, chunks[k].src, chunks[k].n,
+                                cudaMemcpyDeviceToHost, st));
+      P3MX_CUDA(cudaEventRecord(b->out_events.get(k % kSlots), st));
+    };
+    std::unique_lock<std::mutex> lk;
+    HostPool &pool = host_pool(lk);
+    for (size_t k = 0; k < std::min(kSlots, chunks.size()); ++k)
+      issue(k);
+    for (size_t k = 0; k < chunks.size(); ++k) {
+      P3MX_CUDA(cudaEventSynchronize(b->out_events.get(k % kSlots)));
+      pool.copy(chunks[k].dst, buf + (k % kSlots) * kChunk, chunks[k].n);
+      if (k + kSlots < chunks.size())
+        issue(k + kSlots);
+    }
     P3MX_CUDA(cudaStreamSynchronize(st));
   });
 }
