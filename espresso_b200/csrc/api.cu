@@ -1187,7 +1187,14 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
     // charges and types).
     bool const spec = !dev && f && !want_e && !want_v && n > 0 && h->h_in.p &&
                       h->staged_n == n && h->staged_q && (type != nullptr) == h->staged_type;
-    stage_in(h, n, pos, q, type, dev, st, true, !spec);
+    // device arrays and forces only: staged by the evaluation's first kernel
+    ParticleArrays direct;
+    if (dev && n > 0 && !want_e && !want_v && h->prm.epsilon == 0.) {
+      direct = ParticleArrays{pos, q, type};
+      h->staged_q = h->staged_type = false;
+    } else {
+      stage_in(h, n, pos, q, type, dev, st, true, !spec);
+    }
     if (spec) {
       auto forces = [&] {
         if (h->prm.epsilon != 0.)
@@ -1211,8 +1218,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
     std::vector<double> enk, virk, ens, virs;
     bool const obs64 = h->prm.single_precision && !(flags & P3MX_MIXED_OBSERVABLES);
     if (!want_e && !want_v) {
-      // forces only: real-space pairs concurrent with the k-space chain
-      e.forces_all(fd, dev ? ow : true, st);
+      e.forces_all(fd, dev ? ow : true, st, direct);
     } else if (f) {
       e.long_range(fd, dev ? ow : true, want_e && !obs64, want_v && !obs64, st, &enk, &virk);
       e.short_range(fd, false, (want_e || want_v) && !obs64, st, &ens, &virs);

@@ -680,13 +680,16 @@ template <typename Real>
 void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t st) {
   int const R = n_rep();
   const int *rep_of = R > 1 ? m_rep_of.as<int>() : nullptr;
-  if (m_cnt_dirty)
-    P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
-  m_cnt_dirty = true;
-  pdl_launch(k_p3m_bin<Real>, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(), rep_of,
-             d_pos(), m_n, m_key.as<int>(), m_slot.as<int>(), m_cnt.as<int>(), m_dist.as<Real>(),
-             qmax, nc * R);
-  ++m_launches;
+  if (!m_binned) {
+    if (m_cnt_dirty)
+      P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
+    m_cnt_dirty = true;
+    pdl_launch(k_p3m_bin<Real>, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(),
+               rep_of, d_pos(), m_n, m_key.as<int>(), m_slot.as<int>(), m_cnt.as<int>(),
+               m_dist.as<Real>(), qmax, nc * R);
+    ++m_launches;
+  }
+  m_binned = false;
   m_launches += exclusive_scan(m_cnt.as<int>(), m_start.as<int>(), m_scan_tiles.as<int>(), m_nkeys,
                                st, nullptr, true);
   pdl_launch(nc == 1 ? k_p3m_place<Real, 1> : k_p3m_place<Real, 3>, ceil_div(m_n, 256), 256, 0, st,
@@ -987,44 +990,88 @@ __global__ void k_refresh_spq(const RepGeom *__restrict__ reps, const int *__res
                        qi);
 }
 
-// Displacement check fused with the sorted-position refresh: sets *flag (in
-// mapped host memory: one store per block that found a change) when a
-// particle moved more than skin/2 or changed its kind since the last build
-// (k_displacement_check's test) and writes the pair kernel's sorted
-// records as k_refresh_spq does (a rebuild that follows rewrites them).
+// Displacement check and sorted-position refresh of particle i: true when it
+// moved more than skin/2 or changed its kind since the last build
+// (k_displacement_check's test); writes the pair kernel's records to its
+// sorted slot as k_refresh_spq does (a rebuild that follows rewrites them).
+struct CheckArrays {
+  const int *inv, *ckey, *type_ref;
+  const double *pos_ref;
+  double4 *spq; // or nullptr: FP32 records only
+  float4 *spf;
+  volatile int *flag; // mapped host memory: one store per block that found a change
+};
+__device__ inline bool check_particle(RepGeom const &G, long long i, double const (&x)[3],
+                                      double qi, int type, CheckArrays const &c) {
+  int const s = c.inv[i];
+  double d2 = 0.0;
+  double ref[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    ref[d] = c.pos_ref[3 * i + d];
+    double const dx = x[d] - ref[d];
+    d2 += dx * dx;
+  }
+  double const lim = 0.5 * G.skin;
+  if (c.spq)
+    c.spq[s] = make_double4(fold_coord(x[0], G.box[0]), fold_coord(x[1], G.box[1]),
+                            fold_coord(x[2], G.box[2]), qi);
+  c.spf[s] = cell_offset(G, c.ckey[i] - static_cast<int>(G.cell_off), ref, x, qi);
+  return d2 > lim * lim || list_kind(type, qi) != c.type_ref[i];
+}
 // One thread per particle in index order (coalesced reads of positions,
-// reference positions, types and build-time cells), each writing its
-// records to its sorted slot inv[i].
+// reference positions, types and build-time cells).
 __global__ void __launch_bounds__(256)
 k_check_refresh(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
-                const int *__restrict__ inv, const double *__restrict__ pos,
-                const double *__restrict__ q, const int *__restrict__ ckey,
-                const double *__restrict__ pos_ref, const int *__restrict__ type,
-                const int *__restrict__ type_ref, long long n, double4 *__restrict__ spq,
-                float4 *__restrict__ spf, volatile int *flag) {
+                const double *__restrict__ pos, const double *__restrict__ q,
+                const int *__restrict__ type, long long n, CheckArrays const chk) {
   pdl_enter();
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   bool moved = false;
   if (i < n) {
-    int const s = inv[i];
-    RepGeom const &G = reps[rep_of[i]];
-    double d2 = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double const dx = pos[3 * i + d] - pos_ref[3 * i + d];
-      d2 += dx * dx;
-    }
-    double const lim = 0.5 * G.skin;
-    double const qi = q[i];
-    moved = d2 > lim * lim || list_kind(type[i], qi) != type_ref[i];
-    if (spq)
-      spq[s] = make_double4(fold_coord(pos[3 * i], G.box[0]), fold_coord(pos[3 * i + 1], G.box[1]),
-                            fold_coord(pos[3 * i + 2], G.box[2]), qi);
-    spf[s] = cell_offset(G, ckey[i] - static_cast<int>(G.cell_off), pos_ref + 3 * i, pos + 3 * i,
-                         qi);
+    double const x[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+    moved = check_particle(reps[rep_of[i]], i, x, q[i], type[i], chk);
   }
   if (__syncthreads_or(moved) && threadIdx.x == 0)
-    *flag = 1;
+    *chk.flag = 1;
+}
+
+// The particle passes at the front of a force evaluation in one: the caller's
+// device arrays staged into the engine's (in.pos != nullptr; in.type nullptr:
+// types zero), the list check with its record refresh (chk.inv != nullptr)
+// and the mesh binning.  The three read the same positions in index order;
+// apart they are three launches (of 13) and two more reads of the positions.
+template <typename Real>
+__global__ void __launch_bounds__(256)
+k_front(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, long long n,
+        ParticleArrays const in, double *__restrict__ pos, double *__restrict__ q,
+        int *__restrict__ type, CheckArrays const chk, int *__restrict__ key,
+        int *__restrict__ slot, int *__restrict__ cnt, Real *__restrict__ dist,
+        unsigned *__restrict__ zero, int nzero) {
+  long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
+    zero[k] = 0u;
+  bool moved = false;
+  if (i < n) {
+    bool const stage = in.pos != nullptr;
+    const double *xs = stage ? in.pos : pos;
+    double const x[3] = {xs[3 * i], xs[3 * i + 1], xs[3 * i + 2]};
+    double const qi = stage ? in.q[i] : q[i];
+    int const ti = stage ? (in.type ? in.type[i] : 0) : type[i];
+    if (stage) {
+      pos[3 * i] = x[0];
+      pos[3 * i + 1] = x[1];
+      pos[3 * i + 2] = x[2];
+      q[i] = qi;
+      type[i] = ti;
+    }
+    RepGeom const &G = reps[rep_of ? rep_of[i] : 0];
+    if (chk.inv)
+      moved = check_particle(G, i, x, qi, ti, chk);
+    bin_particle(G, i, x, key, slot, cnt, dist);
+  }
+  if (chk.inv && __syncthreads_or(moved) && threadIdx.x == 0)
+    *chk.flag = 1;
 }
 
 void Engine::refresh_sorted_positions(cudaStream_t st, bool want_spq) {
@@ -1048,12 +1095,42 @@ void Engine::check_lists(cudaStream_t st, bool need_spq) {
   // rebuild follows.  The host consumed the flag of the check before.
   m_host_words[kFlagWord] = 0;
   pdl_launch(k_check_refresh, ceil_div(m_n, 256), 256, 0, st, false, m_geom_d.as<RepGeom>(),
-             m_rep_of.as<int>(), m_cinv.as<int>(), d_pos(), d_q(), m_ckey.as<int>(),
-             m_pos_ref.as<double>(), d_type(), m_type_ref.as<int>(), m_n,
-             need_spq ? m_spq.as<double4>() : nullptr, m_spf.as<float4>(),
-             m_host_words + kFlagWord);
+             m_rep_of.as<int>(), d_pos(), d_q(), d_type(), m_n, check_arrays(need_spq));
   ++m_launches;
   P3MX_CUDA(cudaEventRecord(m_check_ev, st));
+}
+
+// The arrays of the list check (empty while there are no valid lists).
+CheckArrays Engine::check_arrays(bool need_spq) const {
+  if (!m_lists_valid)
+    return CheckArrays{};
+  return CheckArrays{m_cinv.as<int>(),       m_ckey.as<int>(),
+                     m_type_ref.as<int>(),   m_pos_ref.as<double>(),
+                     need_spq ? m_spq.as<double4>() : nullptr,
+                     m_spf.as<float4>(),     m_host_words + kFlagWord};
+}
+
+// Staging (in.pos != nullptr), list check and mesh binning in one launch; the
+// check is then pending as after check_lists, the binning done (m_binned).
+template <typename Real> void Engine::front(ParticleArrays const &in, cudaStream_t st) {
+  bool const spq = sizeof(Real) == 8;
+  m_check_pending = true;
+  m_check_rebuild = !m_lists_valid;
+  if (!m_check_ev)
+    P3MX_CUDA(cudaEventCreateWithFlags(&m_check_ev, cudaEventDisableTiming));
+  m_host_words[kFlagWord] = 0;
+  if (m_cnt_dirty)
+    P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
+  m_cnt_dirty = true;
+  int const R = n_rep();
+  k_front<Real><<<ceil_div(m_n, 256), 256, 0, st>>>(
+      m_geom_d.as<RepGeom>(), R > 1 ? m_rep_of.as<int>() : nullptr, m_n, in, d_pos(), d_q(),
+      d_type(), check_arrays(spq), m_key.as<int>(), m_slot.as<int>(), m_cnt.as<int>(),
+      m_dist.as<Real>(), reinterpret_cast<unsigned *>(m_cnt.as<int>() + m_nkeys + 1), R);
+  ++m_launches;
+  P3MX_CUDA(cudaGetLastError());
+  P3MX_CUDA(cudaEventRecord(m_check_ev, st));
+  m_binned = true;
 }
 
 void Engine::prepare_short_range(cudaStream_t st, bool need_spq) {
@@ -1188,29 +1265,35 @@ void Engine::short_range_t(double *f, bool overwrite, bool want_ev, cudaStream_t
   mark("pair_forces", st);
 }
 
-// Forces only (no energies or virials): the pair kernel runs on a side
-// stream, concurrently with the k-space chain (sort, assignment, FFTs); the
-// interpolation waits for it and adds the k-space forces on top.
-void Engine::forces_all(double *f, bool overwrite, cudaStream_t st) {
+// Forces only (no energies or virials); in: the caller's device arrays to stage
+// first, or none.
+void Engine::forces_all(double *f, bool overwrite, cudaStream_t st, ParticleArrays const &in) {
   if (m_n == 0 || m_profiling) {
+    if (in.pos)
+      upload(in.pos, in.q, in.type, true, st);
     long_range(f, overwrite, false, false, st, nullptr, nullptr);
     short_range(f, false, false, st, nullptr, nullptr);
     bond_forces(f, st);
     return;
   }
-  // one stream: the list check, the k-space chain, then the pair kernel.
+  // one stream: staging, list check and binning, the k-space chain, then the
+  // pair kernel.
   // The host waits for the check's flag (an event behind it) while the GPU
   // runs the k-space chain, so the pair kernel (or the list rebuild) is
   // queued before the GPU gets to it.  The stage kernels each fill the GPU;
   // this measured faster than the pair kernel on a second stream beside the
   // k-space chain (1.58 vs 1.62 ms at 2^20 ions)
-  check_lists(st, !m_fp32);
   try {
+    if (m_fp32)
+      front<float>(in, st);
+    else
+      front<double>(in, st);
     long_range(f, overwrite, false, false, st, nullptr, nullptr);
   } catch (...) {
-    m_check_pending = false;
+    m_check_pending = m_binned = false;
     throw;
   }
+  m_binned = false; // also where long_range returned without sorting
   prepare_short_range(st, !m_fp32);
   if (m_fp32)
     launch_pair<float>(f, false, false, st);

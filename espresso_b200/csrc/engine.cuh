@@ -61,6 +61,13 @@ struct Timing {
   float ms_long = 0.f, ms_short = 0.f;
 };
 
+// A caller's device arrays (pos == nullptr: none; type == nullptr: all zero).
+struct ParticleArrays {
+  const double *pos = nullptr, *q = nullptr;
+  const int *type = nullptr;
+};
+struct CheckArrays; // arrays of the list check (engine.cu)
+
 class Dp3mEngine;
 
 class Engine {
@@ -106,7 +113,7 @@ public:
                    bool fp64_math = false);
   // Forces of the whole path (k-space + real-space + LJ/WCA), no energies:
   // the k-space chain, the list check, then the pair kernel, on one stream.
-  void forces_all(double *f, bool overwrite, cudaStream_t st);
+  void forces_all(double *f, bool overwrite, cudaStream_t st, ParticleArrays const &in = {});
   // Graph-capturable short-range evaluation (device-side rebuild decision).
   void short_range_graph(double *f, bool overwrite, cudaStream_t st);
   // Build lists now if invalid (capacity margin factor for graph use).
@@ -168,6 +175,9 @@ private:
   // mapped host memory ahead of m_check_ev, so the host can wait for it while
   // later work keeps the GPU busy; prepare_short_range consumes it
   void check_lists(cudaStream_t st, bool need_spq);
+  CheckArrays check_arrays(bool need_spq) const;
+  template <typename Real> void front(ParticleArrays const &in, cudaStream_t st);
+  bool m_binned = false; // the mesh binning of the coming sort is done (front)
   void build_lists(cudaStream_t st);
   void set_list_capacity(double margin);
   void layout_lists(cudaStream_t st);

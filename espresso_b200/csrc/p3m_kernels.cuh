@@ -98,22 +98,13 @@ template <> struct __align__(64) PRec<double> {
 // sort key is brk_off + brick, so the particles of one brick form one
 // contiguous range of the sorted order.  rep_of: nullptr for one replica.
 template <typename Real>
-__global__ void k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
-                          const double *__restrict__ pos, long long n,
-                          int *__restrict__ key, int *__restrict__ slot,
-                          int *__restrict__ cnt, Real *__restrict__ dist,
-                          unsigned *__restrict__ zero, int nzero) {
-  pdl_enter();
-  long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
-    zero[k] = 0u; // the |q| maxima that the placing kernel raises next
-  if (i >= n)
-    return;
-  RepGeom const &G = reps[rep_of ? rep_of[i] : 0];
+__device__ inline void bin_particle(RepGeom const &G, long long i, double const (&x)[3],
+                                    int *__restrict__ key, int *__restrict__ slot,
+                                    int *__restrict__ cnt, Real *__restrict__ dist) {
   int g[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    double const xf = fold_coord(pos[3 * i + d], G.box[d]);
+    double const xf = fold_coord(x[d], G.box[d]);
     double const p = ((xf - G.ld_pos[d]) * G.ai[d]) - G.pos_shift;
     int const nmp = static_cast<int>(p);
     double const ds = (p - nmp) - 0.5;
@@ -127,6 +118,22 @@ __global__ void k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restric
   int const brick = ((g[0] / B) * G.nby + g[1] / B) * G.nbz + g[2] / B;
   key[i] = brick * B * B * B + ((g[0] % B) * B + g[1] % B) * B + g[2] % B;
   slot[i] = atomicAdd(&cnt[static_cast<int>(G.brk_off) + brick], 1);
+}
+// zero: nzero words cleared (the |q| maxima that the placing kernel raises next).
+template <typename Real>
+__global__ void __launch_bounds__(256)
+k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
+          const double *__restrict__ pos, long long n, int *__restrict__ key,
+          int *__restrict__ slot, int *__restrict__ cnt, Real *__restrict__ dist,
+          unsigned *__restrict__ zero, int nzero) {
+  pdl_enter();
+  long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
+    zero[k] = 0u;
+  if (i >= n)
+    return;
+  double const x[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+  bin_particle(reps[rep_of ? rep_of[i] : 0], i, x, key, slot, cnt, dist);
 }
 
 // Every particle's record to its sorted place (start of its brick plus the
