@@ -276,9 +276,9 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       b[tq * ld + pix(x)] = C{dop_y * vy.x + dop_z * vz.x, dop_y * vy.y + dop_z * vz.y};
     }
   __syncthreads();
-  C *ra = fft_lines<KIND>(a, c, T, ld, G.plan[0], tw);
+  C *ra = fft_lines<KIND, true>(a, c, T, ld, G.plan[0], tw);
   // with KIND 0: the buffer that the first transform left free
-  C *rb = fft_lines<KIND>(b, ra == a ? c : a, T, ld, G.plan[0], tw);
+  C *rb = fft_lines<KIND, true>(b, ra == a ? c : a, T, ld, G.plan[0], tw);
   double acc = 0.0;
   double const wgt = (kz == 0 || kz == M2 / 2) ? 1.0 : 2.0;
   for (int x = xq; col && x < M0; x += 16) {
@@ -355,7 +355,7 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       a[tq * ld + pix(x)] = tor ? C{c * m.y, c * m.x} : C{-c * m.x, c * m.y};
     }
   __syncthreads();
-  C const *res = fft_lines<KIND>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
+  C const *res = fft_lines<KIND, true>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
   int const rows = col ? (M0 - xq + 15) >> 4 : 0;
   C *q = field0 + fstride * o + base + xq * stride_x;
 #pragma unroll 4

@@ -430,7 +430,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       bool const two = m_kind[2] != kFftAny;
       size_t const z_budget = m_fp32 ? 54 * 1024 : 100 * 1024;
       int const want = two ? 256 / std::min(pz.n1, pz.n2) : 256;
-      long long const slots = static_cast<long long>(m_fp32 ? (m_kind[2] == kFftTwo ? 3 : 4) : 2) * sms;
+      long long const slots = static_cast<long long>(m_fp32 ? kFftBlocks<float> : kFftBlocks<double>) * sms;
       auto const fill = [&](int most) {
         long long const waves = (all_lines + most * slots - 1) / (most * slots);
         int const l = ceil_div(all_lines, waves * slots);
@@ -458,8 +458,13 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       for (int l = 0; l < lines; l += lzi)
         zi.push_back(Blk{r, l, std::min(lzi, lines - l), 0});
       smem_zi = std::max(smem_zi, zi_smem(std::min(lzi, lines)));
-      // column tiles of equal width (no last tile of one column)
-      int const ty = ceil_div(H, ceil_div(H, m_tile_y)), tx = ceil_div(H, ceil_div(H, m_tile_x));
+      // column tiles of about equal width, rounded up to 4 columns (whole
+      // 32-byte sectors)
+      auto const cols = [H](int most) {
+        int const w = ceil_div(H, ceil_div(H, most));
+        return std::min(most, (w + 3) / 4 * 4);
+      };
+      int const ty = cols(m_tile_y), tx = cols(m_tile_x);
       for (int xx = 0; xx < M0; ++xx)
         for (int k0 = 0; k0 < H; k0 += ty)
           y.push_back(Blk{r, xx, k0, std::min(ty, H - k0)});

@@ -310,30 +310,31 @@ __device__ __forceinline__ int opaque(int x) {
   asm volatile("" : "+r"(x));
   return x;
 }
+// A block takes at most 256 / n2 lines, n2 the smaller factor: step 1 is one
+// item per thread.
 template <typename C, int N1>
 __device__ __forceinline__ void fft_step1(C *a, int nlines, int ld, int n2,
                                           const C *__restrict__ tw) {
-  float const rn2 = 1.0f / static_cast<float>(n2);
-#pragma unroll 1
-  for (int it = opaque(threadIdx.x); it < nlines * n2; it += blockDim.x) {
-    int const l = qdiv(it, n2, rn2);
-    int t = it - l * n2;
-    C *s = a + l * ld;
-    C v[N1];
+  int const it = opaque(threadIdx.x);
+  if (it >= nlines * n2)
+    return;
+  int const l = qdiv(it, n2, 1.0f / static_cast<float>(n2));
+  int t = it - l * n2;
+  C *s = a + l * ld;
+  C v[N1];
 #pragma unroll
-    for (int m = 0; m < N1; ++m)
-      v[m] = s[pix(t + n2 * m)];
-    dft<C, N1>(v);
+  for (int m = 0; m < N1; ++m)
+    v[m] = s[pix(t + n2 * m)];
+  dft<C, N1>(v);
 #pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1)
-      v[k1] = cmul(v[k1], tw[t * k1]);
-    t = opaque(t);
+  for (int k1 = 1; k1 < N1; ++k1)
+    v[k1] = cmul(v[k1], tw[t * k1]);
+  t = opaque(t);
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1)
-      s[pix(t + n2 * k1)] = v[k1];
-  }
+  for (int k1 = 0; k1 < N1; ++k1)
+    s[pix(t + n2 * k1)] = v[k1];
 }
-template <typename C, int N2>
+template <typename C, int N2, bool ONE>
 __device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
   int const per = blockDim.x / n1; // lines per round
   int const tid = opaque(threadIdx.x);
@@ -355,16 +356,18 @@ __device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
       for (int k2 = 0; k2 < N2; ++k2)
         s[pix(k1 + n1 * k2)] = v[k2];
     }
+    if (ONE)
+      break;
   }
 }
 // The two steps for compile-time factors (powers of two): the padded indices
 // fold to a base and immediate offsets (128^3: 150 -> about 90 instructions per
 // point and pass against the runtime factors).  Blocks of 256 threads.
-template <typename C, int N1, int N2>
+template <typename C, int N1, int N2, bool ONE>
 __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__restrict__ tw) {
   unsigned const tid = threadIdx.x;
-  for (unsigned it = tid; it < static_cast<unsigned>(nlines * N2); it += 256) {
-    int const l = it / N2, t = it % N2;
+  if (tid < static_cast<unsigned>(nlines * N2)) {
+    int const l = tid / N2, t = tid % N2;
     C *s = a + l * ld + t;
     C v[N1];
 #pragma unroll
@@ -381,6 +384,7 @@ __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__re
   __syncthreads();
   constexpr int per = 256 / N1;
   int const lq = tid / N1, k1 = tid % N1;
+#pragma unroll 1
   for (int l0 = 0; l0 < nlines; l0 += per) {
     bool const act = l0 + lq < nlines;
     C *s = a + (l0 + lq) * ld;
@@ -398,6 +402,8 @@ __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__re
       for (int k2 = 0; k2 < N2; ++k2)
         s[k1 + pix(N1 * k2)] = v[k2];
     }
+    if (ONE)
+      break;
   }
 }
 #define P3MX_FACTOR_DISPATCH(N, CALL)                                          \
@@ -422,25 +428,26 @@ __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__re
 // compile-time factors (without the other factors' code a pass needs no
 // spills at four blocks per SM); kFftTwo -- two-factor plans, in place;
 // kFftAny -- Stockham stages with `b`, a second buffer of the same size.
-// Returns the buffer holding the result.  All threads of the block call it
+// ONE: at most 16 lines, so that a thread has one item per step (no loops, and
+// nothing hoisted out of them).  Returns the buffer holding the result.  All threads of the block call it
 // behind a barrier; the result is visible when it returns.
 constexpr int kFftAny = 0, kFftTwo = 1, kFftPow2 = 2;
-template <int KIND, typename C>
+template <int KIND, bool ONE, typename C>
 __device__ __forceinline__ C *fft_lines(C *a, C *b, int nlines, int ld, AxisPlan const &pl,
                                         const C *__restrict__ tw) {
   if constexpr (KIND == kFftPow2) {
     switch (pl.n) {
-    case 32: fft_pow2<C, 8, 4>(a, nlines, ld, tw); break;
-    case 64: fft_pow2<C, 8, 8>(a, nlines, ld, tw); break;
-    case 128: fft_pow2<C, 16, 8>(a, nlines, ld, tw); break;
-    default: fft_pow2<C, 16, 16>(a, nlines, ld, tw); break;
+    case 32: fft_pow2<C, 8, 4, ONE>(a, nlines, ld, tw); break;
+    case 64: fft_pow2<C, 8, 8, ONE>(a, nlines, ld, tw); break;
+    case 128: fft_pow2<C, 16, 8, ONE>(a, nlines, ld, tw); break;
+    default: fft_pow2<C, 16, 16, ONE>(a, nlines, ld, tw); break;
     }
     __syncthreads();
     return a;
   } else if constexpr (KIND == kFftTwo) {
     P3MX_FACTOR_DISPATCH(pl.n1, (fft_step1<C, R>(a, nlines, ld, pl.n2, tw)))
     __syncthreads();
-    P3MX_FACTOR_DISPATCH(pl.n2, (fft_step2<C, R>(a, nlines, ld, pl.n1)))
+    P3MX_FACTOR_DISPATCH(pl.n2, (fft_step2<C, R, ONE>(a, nlines, ld, pl.n1)))
     __syncthreads();
     return a;
   } else {
@@ -479,10 +486,10 @@ template <typename Fn> inline void fft_pick(int kind, Fn &&f) {
     f(std::integral_constant<int, kFftAny>{});
 }
 
-// Blocks per SM of the z and y passes (their registers are sized for it).
-template <typename Real, int KIND> __host__ __device__ constexpr int fft_blocks() {
-  return sizeof(Real) == 4 ? (KIND == kFftTwo ? 3 : 4) : 2;
-}
+// Blocks per SM of the z and y passes (their registers are sized for it).  Four
+// also for two-factor lines, with some spills: three without measured 888 ->
+// 916 us (131 072 dipoles), 335 -> 345 us (98 304 ions on 112 x 112 x 144).
+template <typename Real> constexpr int kFftBlocks = sizeof(Real) == 4 ? 4 : 2;
 
 // Signed frequency of index i in an axis of m points, the Nyquist index as
 // zero (calc_meshift with the differential operator's convention,
@@ -505,7 +512,7 @@ template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 // twiddles (n).  Meshes are even, so is bk.b.
 constexpr int kZfLines = 64; // most real lines per block
 template <typename Real, int KIND>
-__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
+__global__ void __launch_bounds__(256, kFftBlocks<Real>)
 k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
             const Real *__restrict__ tiles, long long tile_stride, const int *__restrict__ cov,
             int E, typename CplxOf<Real>::type *__restrict__ cmesh, long long c_stride,
@@ -628,7 +635,7 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
   }
   __syncthreads();
-  C *res = fft_lines<KIND>(a, b, np, ld, G.plan[2], tw);
+  C *res = fft_lines<KIND, false>(a, b, np, ld, G.plan[2], tw);
   int const H = n / 2 + 1;
   int const hp = G.hp;
   // both lines of a slot from one pair of entries
@@ -672,9 +679,9 @@ constexpr int kChargeSpectra = 4; // arrays of the charge fields' spectra
 // k_y in units of 2 pi / box (1) or as an integer (0).  Shared memory: tile
 // staged lines of line_ld(M1) (two sets for KIND 0), twiddles (M1).
 template <typename Real, bool INV, int KIND>
-__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
+__global__ void __launch_bounds__(256, kFftBlocks<Real>)
 k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
-        typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, YPass const job,
+        typename CplxOf<Real>::type *__restrict__ c0, long long field_stride, const __grid_constant__ YPass job,
         int kscale, int tile, const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   pdl_enter();
@@ -694,23 +701,26 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   // 16 x 16 thread mapping (tile <= 16 columns): column tq, rows yq + 16 i
   int const tq = threadIdx.x & 15, yq = threadIdx.x >> 4;
   bool const col = tq < T;
-  long long const base = G.km_off + static_cast<long long>(x) * M1 * hp + kz0 + tq;
-  const C *src = c0 + field_stride * job.src[jb] + base;
-  C *dst = c0 + field_stride * job.dst[jb] + base;
+  long long const base = G.km_off + static_cast<long long>(x) * M1 * hp + kz0;
+  const C *src = c0 + field_stride * job.src[jb] + base + min(tq, T - 1);
+  C *dst = c0 + field_stride * job.dst[jb] + base + tq;
   int const pw = INV ? job.pw[jb] : 0;
   Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[1]) : Real(1);
   // all of a thread's rows in flight at once (up to 16: M1 <= 256 in one
-  // round); row y = yq + 16 u of column tq lies at tq ld + yq + 17 u
+  // round), rows and columns past the tile read a valid one in their place, so
+  // that the loads are unconditional (guarded, the compiler waits for each
+  // before the next: 12 -> 19 us at 128^3); row y = yq + 16 u of column tq lies
+  // at tq ld + yq + 17 u
   C *const sl = a + tq * ld + yq;
   int const rows = col ? (M1 - yq + 15) >> 4 : 0;
   long long const step = 16 * hp;
   for (int u0 = 0; u0 < rows; u0 += 16) {
     C v[16];
-    const C *p = src + (yq + 16 * u0) * hp;
+    int const last = M1 - 1 - 16 * u0;
+    const C *p = src + 16 * u0 * hp;
 #pragma unroll
-    for (int u = 0; u < 16; ++u, p += step)
-      if (u0 + u < rows)
-        v[u] = *p;
+    for (int u = 0; u < 16; ++u)
+      v[u] = p[min(yq + 16 * u, last) * hp];
 #pragma unroll
     for (int u = 0; u < 16; ++u)
       if (u0 + u < rows) {
@@ -724,7 +734,7 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       }
   }
   __syncthreads();
-  const C *res = fft_lines<KIND>(a, b, T, ld, G.plan[1], tw) + tq * ld + yq;
+  const C *res = fft_lines<KIND, true>(a, b, T, ld, G.plan[1], tw) + tq * ld + yq;
   C *q = dst + yq * hp;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u, q += step) {
@@ -786,7 +796,7 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     }
   }
   __syncthreads();
-  C *res = fft_lines<KIND>(a, b, T, ld, G.plan[0], tw);
+  C *res = fft_lines<KIND, true>(a, b, T, ld, G.plan[0], tw);
   C *fb = (res == a) ? b : a; // k_x phi goes to the free buffer
   // k-space operator
   double const wv[3] = {2.0 * kPi * G.box_i[0], 2.0 * kPi * G.box_i[1],
@@ -853,7 +863,7 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   __syncthreads();
   // with KIND 0 the scratch of the second transform is the first's buffer
   // once that is stored
-  const C *f0 = fft_lines<KIND>(fb, c, T, ld, G.plan[0], tw) + tq * ld + xq;
+  const C *f0 = fft_lines<KIND, true>(fb, c, T, ld, G.plan[0], tw) + tq * ld + xq;
   int const rows = col ? (M0 - xq + 15) >> 4 : 0;
   C *q = field0 + base + xq * stride_x + tq;
 #pragma unroll 4
@@ -861,7 +871,7 @@ k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     q[u * 16 * stride_x] = cswap(f0[17 * u]);
   if constexpr (!KIND)
     __syncthreads();
-  const C *f1 = fft_lines<KIND>(res, fb, T, ld, G.plan[0], tw) + tq * ld + xq;
+  const C *f1 = fft_lines<KIND, true>(res, fb, T, ld, G.plan[0], tw) + tq * ld + xq;
   q += field_stride;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u)
@@ -888,10 +898,10 @@ inline ZPass z_charge() { return ZPass{{0, 2, 3}, {0, 0, 1}}; }
 // 64-register bound.
 constexpr int kZiLines = 128; // most lines per block
 template <typename Real, int KIND>
-__global__ void __launch_bounds__(256, fft_blocks<Real, KIND>())
+__global__ void __launch_bounds__(256, kFftBlocks<Real>)
 k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
              const typename CplxOf<Real>::type *__restrict__ field0, long long field_stride,
-             ZPass const zp, int kscale, Real *__restrict__ efield, long long e_stride,
+             const __grid_constant__ ZPass zp, int kscale, Real *__restrict__ efield, long long e_stride,
              const typename CplxOf<Real>::type *__restrict__ twtab) {
   using C = typename CplxOf<Real>::type;
   pdl_enter();
@@ -948,7 +958,7 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     put(nl + j, k, r[0], (2 * j + 1 < nl) ? r[hp] : C{Real(0), Real(0)}, pz, pz);
   }
   __syncthreads();
-  const C *res = fft_lines<KIND>(a, b, nc, ld, G.plan[2], tw);
+  const C *res = fft_lines<KIND, false>(a, b, nc, ld, G.plan[2], tw);
   // packed field mesh: one (Ex, Ey, Ez, 0) record per mesh point, so the
   // interpolation gathers one 16-byte (FP32) record per stencil point
   // (ghost-padded: every record also goes to its periodic images in the
