@@ -84,7 +84,6 @@ struct RepGeom {
   int cov_off[3];    // per axis: its cover table (see cover_entry)
   long long re_off;  // field mesh offset (records of 4 values)
   int epad[3];       // field mesh extent: mesh plus high-side ghost layers
-  long long bin_off; // corner key offset: bricks of brick^3 corners
   long long brk_off; // brick (sort key) offset
   int brick;         // brick edge (corner units) of the charge assignment
   int nbx, nby, nbz; // bricks per dimension

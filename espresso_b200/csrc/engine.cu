@@ -228,7 +228,6 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     G.nbx = (c.mesh[0] + G.brick - 1) / G.brick;
     G.nby = (c.mesh[1] + G.brick - 1) / G.brick;
     G.nbz = (c.mesh[2] + G.brick - 1) / G.brick;
-    G.bin_off = m_ncorner;
     m_ncorner += static_cast<long long>(G.nbx) * G.nby * G.nbz * G.brick * G.brick * G.brick;
     G.brk_off = m_nkeys;
     m_nkeys += static_cast<long long>(G.nbx) * G.nby * G.nbz;
@@ -695,12 +694,19 @@ void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t 
     ++m_launches;
   }
   m_binned = false;
-  m_launches += exclusive_scan(m_cnt.as<int>(), m_start.as<int>(), m_scan_tiles.as<int>(), m_nkeys,
-                               st, nullptr, true);
-  pdl_launch(nc == 1 ? k_p3m_place<Real, 1> : k_p3m_place<Real, 3>, ceil_div(m_n, 256), 256, 0, st,
-             true, m_geom_d.as<RepGeom>(), rep_of, R, m_key.as<int>(), m_slot.as<int>(),
-             m_start.as<int>(), m_dist.as<Real>(), q, m_n, m_rec.as<PRec<Real>>(), qmax,
-             m_cnt.as<int>(), m_nkeys + 1);
+  // few bricks and at most a block per SM: the placing kernel scans the counts
+  // itself (2000 ions 70.4 -> 67.0 us a pass, 23 457 ions 106.2 -> 102.7); with
+  // more blocks their scans cost more than the launch (sort of 131 072 ions 25.6
+  // -> 31.1 us, of 98 304 ions 22.7 -> 25.7)
+  bool const scan = m_nkeys <= kPlaceScan && ceil_div(m_n, 256) <= m_sms;
+  if (!scan)
+    m_launches += exclusive_scan(m_cnt.as<int>(), m_start.as<int>(), m_scan_tiles.as<int>(),
+                                 m_nkeys, st, nullptr, true);
+  pdl_launch(scan ? (nc == 1 ? k_p3m_place<Real, 1, true> : k_p3m_place<Real, 3, true>)
+                  : (nc == 1 ? k_p3m_place<Real, 1, false> : k_p3m_place<Real, 3, false>),
+             ceil_div(m_n, 256), 256, 0, st, true, m_geom_d.as<RepGeom>(), rep_of, R,
+             m_key.as<int>(), m_slot.as<int>(), m_start.as<int>(), m_dist.as<Real>(), q, m_n,
+             m_rec.as<PRec<Real>>(), qmax, m_cnt.as<int>(), static_cast<int>(m_nkeys));
   ++m_launches;
   m_cnt_dirty = false;
 }

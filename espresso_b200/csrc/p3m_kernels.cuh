@@ -1,9 +1,11 @@
-// P3M particle <-> mesh kernels (sm_100a): corner binning, B-spline weights,
-// gather-based deterministic charge assignment, force back-interpolation,
-// influence function, charge census and the k-space error sum.
+// P3M particle <-> mesh kernels (sm_100a): corner binning and brick-sorted
+// particle records, B-spline weights, deterministic charge assignment by
+// super-bricks, force back-interpolation, influence function, charge census and
+// the k-space error sum.
 #pragma once
 
 #include "common.cuh"
+#include "sort.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -140,21 +142,58 @@ k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
 // slot from the counting atomics), and each replica's largest |q| per charge
 // (FP32 bits rounded up, atomic maximum: order-independent; set c at
 // qmax_bits + c * n_rep) for the fixed-point scale of the charge assignment.
-// NC charges per particle, q[NC i + c].  The nzero words at `zero` (the brick
-// counts, already scanned) are cleared for the next sort.  A particle is one
-// full 32-byte sector (FP32) written at random: the gathering weight kernel
-// it replaces read five random sectors and wrote 112 bytes.
-template <typename Real, int NC>
+// NC charges per particle, q[NC i + c].  The brick counts `cnt` are cleared for
+// the next sort.  A particle is one full 32-byte sector (FP32) written at
+// random: the gathering weight kernel it replaces read five random sectors and
+// wrote 112 bytes.
+// SCAN (small systems, up to kPlaceScan bricks): `start` is not given but made, every block
+// scanning all counts for itself (16 KB from L2 at most) and block 0 storing the
+// result; the last block to have read the counts clears them (ticket cnt[nkeys]).
+// A small system's pass is bound by the number of dependent launches, and this
+// is one less.
+constexpr int kPlaceScan = 4096;
+template <typename Real, int NC, bool SCAN>
 __global__ void __launch_bounds__(256)
 k_p3m_place(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, int n_rep,
             const int *__restrict__ key, const int *__restrict__ slot,
-            const int *__restrict__ start, const Real *__restrict__ dist,
+            int *__restrict__ start, const Real *__restrict__ dist,
             const double *__restrict__ q, long long n, PRec<Real> *__restrict__ rec,
-            unsigned *__restrict__ qmax_bits, int *__restrict__ zero, long long nzero) {
+            unsigned *__restrict__ qmax_bits, int *__restrict__ cnt, int nkeys) {
+  __shared__ int s_start[SCAN ? kPlaceScan : 1];
   pdl_enter();
   long long const i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (long long k = i; k < nzero; k += static_cast<long long>(gridDim.x) * blockDim.x)
-    zero[k] = 0;
+  if constexpr (SCAN) {
+    constexpr int PER = kPlaceScan / 256;
+    int v[PER], sum = 0, total;
+    int const k0 = threadIdx.x * PER;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      v[k] = k0 + k < nkeys ? cnt[k0 + k] : 0;
+      sum += v[k];
+    }
+    int run = block_excl_scan(sum, total);
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (k0 + k < nkeys) {
+        s_start[k0 + k] = run;
+        if (blockIdx.x == 0)
+          start[k0 + k] = run;
+        run += v[k];
+      }
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) {
+      if (blockIdx.x == 0)
+        start[nkeys] = total;
+      s_last = atomicAdd(cnt + nkeys, 1) == static_cast<int>(gridDim.x) - 1;
+    }
+    __syncthreads();
+    if (s_last) // every block has read the counts
+      for (int k = threadIdx.x; k <= nkeys; k += 256)
+        cnt[k] = 0;
+  } else {
+    for (long long k = i; k <= nkeys; k += static_cast<long long>(gridDim.x) * blockDim.x)
+      cnt[k] = 0;
+  }
   if (i >= n)
     return;
   int const rep = rep_of ? rep_of[i] : 0;
@@ -183,8 +222,8 @@ k_p3m_place(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, in
       atomicMax(w, mx);
   }
   int const lb = G.brick == 4 ? 6 : 9; // log2 of the corners per brick
-  int const s = start[static_cast<int>(G.brk_off) + (r.key >> lb)] + slot[i];
-  rec[s] = r;
+  int const b = static_cast<int>(G.brk_off) + (r.key >> lb);
+  rec[(SCAN ? s_start[b] : start[b]) + slot[i]] = r;
 }
 
 // Edge (mesh points) of the sort bricks that bin the particles by stencil
@@ -205,7 +244,7 @@ struct TileStrides {
 // particle is visited once.  For each particle one warp covers its P^2
 // (x, y) stencil rows (one row per lane, the P z points of a row unrolled)
 // and adds q wx wy wz into a shared-memory tile of (E + P - 1)^3
-// points, in fixed point; the tile is then added to the mesh.  E = 16, or 8
+// points, in fixed point.  E = 16, or 8
 // when the 16^3 super-bricks would not give every SM two blocks (small
 // meshes: more, smaller tiles with a larger halo share).  Tiles of
 // neighbouring super-bricks overlap by P - 1 points.  Every block stores its
@@ -215,7 +254,10 @@ struct TileStrides {
 // is read back and rewritten, and the sum over the (up to 8, in wrap corners
 // 27) tiles has a fixed order, so the mesh is bitwise reproducible.  The
 // tiles hold ((16 + P - 1) / 16)^3 = 2.6 mesh sizes at P = 7.  The kernel is
-// bound by the shared-memory atomics and loads of the stencil terms.
+// bound by the shared-memory atomics and loads of the stencil terms: 2^20 ions on
+// 256^3 at order 7 257 us against 241 us in eight coloured launches that added
+// to the mesh, which also needed 79 us of weight records; 131 072 ions on 128^3
+// 47 against 64 + 17 us, 23 457 ions 10 against 55 + 9 us.
 //
 // Fixed point: a term v = q wx wy wz becomes t = rint(v S) by one FP64 FMA
 // with the magic constant 1.5 * 2^52 (the bits of the sum are those of the
@@ -230,7 +272,7 @@ struct TileStrides {
 // cancels).  Integer sums do not depend on the order of the atomics; the
 // quantum 1/S is about 2^-25 of a charge at 2^20 ions on a 256^3 mesh
 // (FP32-mixed) and 2^-56 in FP64, and each tile point is rounded once to
-// the working precision before it is added to the mesh.
+// the working precision before it is stored.
 constexpr int kSbEdge = 16;   // corner positions per dimension of a super-brick (multiple of 4 and 8)
 constexpr int kSbEdgeSmall = 8; // the edge for meshes with too few 16^3 super-bricks to fill the GPU
 constexpr int kSbWarps = 8;   // warps per super-brick block
