@@ -1,8 +1,8 @@
 // Dipolar P3M kernels (magnetostatics/dp3m.cpp, p3m/influence_function_dipolar.hpp).
 //
 // The three dipole-moment components are assigned to three meshes with the
-// charge-assignment kernels (a component of mu in the charge slot of the
-// weight record) and transformed forward with the z and y passes of the
+// charge-assignment kernels (three charges in one particle record) and
+// transformed forward with the z and y passes of the
 // charge path.  This file adds what is specific to point dipoles:
 //  * the dipolar influence functions G_energy (S = 2) and G_force (S = 3)
 //    on the r2c half mesh, and the aliasing sum of the energy correction;
@@ -267,14 +267,26 @@ k_fft_x_dp3m(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const kz = kz0 + tq;
   long long const base = G.km_off + static_cast<long long>(y) * G.hp + kz;
   Real const dop_y = static_cast<Real>(dp_dop(y, M1)), dop_z = static_cast<Real>(dp_dop(kz, M2));
-#pragma unroll 4
-  for (int x = xq; x < M0; x += 16)
-    if (col) {
-      long long const at = base + x * stride_x;
-      C const vx = comp_hat[at], vy = comp_hat[at + fstride], vz = comp_hat[at + 2 * fstride];
-      a[tq * ld + pix(x)] = vx;
-      b[tq * ld + pix(x)] = C{dop_y * vy.x + dop_z * vz.x, dop_y * vy.y + dop_z * vz.y};
+  // 4 rows of the three components in flight, unconditional as in the y pass
+  int const rows = col ? (M0 - xq + 15) >> 4 : 0;
+  const C *src = comp_hat + base - tq + min(tq, T - 1);
+  for (int u0 = 0; u0 < rows; u0 += 4) {
+    C v[3][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const C *p = src + min(xq + 16 * (u0 + u), M0 - 1) * stride_x;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        v[d][u] = p[d * fstride];
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u0 + u < rows) {
+        int const at = tq * ld + xq + 17 * (u0 + u);
+        a[at] = v[0][u];
+        b[at] = C{dop_y * v[1][u].x + dop_z * v[2][u].x, dop_y * v[1][u].y + dop_z * v[2][u].y};
+      }
+  }
   __syncthreads();
   C *ra = fft_lines<KIND, true>(a, c, T, ld, G.plan[0], tw);
   // with KIND 0: the buffer that the first transform left free
@@ -345,18 +357,29 @@ k_fft_x_dp3m_inv(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   bool const tor = o < 2;
   int const p = tor ? 1 - o : 4 - o; // power of d_op_x
   const Real *g = tor ? g_e : g_f;
-#pragma unroll 4
-  for (int x = xq; x < M0; x += 16)
-    if (col) {
-      C const m = mk_hat[base + x * stride_x];
-      int const dx = dp_dop(x, M0);
-      Real const c = static_cast<Real>(p == 0 ? 1 : (p == 1 ? dx : dx * dx)) * g[base + x * stride_x];
-      // c mk, or -i c mk; real and imaginary parts swapped (backward)
-      a[tq * ld + pix(x)] = tor ? C{c * m.y, c * m.x} : C{-c * m.x, c * m.y};
+  // 8 rows in flight, unconditional as in the y pass
+  int const rows = col ? (M0 - xq + 15) >> 4 : 0;
+  long long const first = base - tq + min(tq, T - 1);
+  for (int u0 = 0; u0 < rows; u0 += 8) {
+    C v[8];
+    Real gv[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      long long const at = first + min(xq + 16 * (u0 + u), M0 - 1) * stride_x;
+      v[u] = mk_hat[at];
+      gv[u] = g[at];
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (u0 + u < rows) {
+        int const dx = dp_dop(xq + 16 * (u0 + u), M0);
+        Real const c = static_cast<Real>(p == 0 ? 1 : (p == 1 ? dx : dx * dx)) * gv[u];
+        // c mk, or -i c mk; real and imaginary parts swapped (backward)
+        a[tq * ld + xq + 17 * (u0 + u)] = tor ? C{c * v[u].y, c * v[u].x} : C{-c * v[u].x, c * v[u].y};
+      }
+  }
   __syncthreads();
   C const *res = fft_lines<KIND, true>(a, b, T, ld, G.plan[0], tw) + tq * ld + xq;
-  int const rows = col ? (M0 - xq + 15) >> 4 : 0;
   C *q = field0 + fstride * o + base + xq * stride_x;
 #pragma unroll 4
   for (int u = 0; u < rows; ++u)

@@ -45,22 +45,6 @@ __host__ __device__ inline int pix(int i) { return i + (i >> 4); }
 // that consecutive lines start in different banks.
 __host__ __device__ inline int line_ld(int n) { return (n + ((n - 1) >> 4)) | 1; }
 
-// body(l, k) for l < nl, k < n over the block: lines shorter than the block
-// run several at a time (one division per thread, not per element).
-template <typename F> __device__ inline void for_lines(int nl, int n, F const &body) {
-  int const per = blockDim.x / n;
-  if (per > 0) {
-    int const lq = threadIdx.x / n, k = threadIdx.x - lq * n;
-    if (lq < per)
-      for (int l = lq; l < nl; l += per)
-        body(l, k);
-  } else {
-    for (int l = 0; l < nl; ++l)
-      for (int k = threadIdx.x; k < n; k += blockDim.x)
-        body(l, k);
-  }
-}
-
 // Copy the twiddle table exp(-2 pi i k / n), k < n, of one axis to shared
 // memory (caller synchronises).
 template <typename C>
@@ -361,8 +345,9 @@ __device__ __forceinline__ void fft_step2(C *a, int nlines, int ld, int n1) {
   }
 }
 // The two steps for compile-time factors (powers of two): the padded indices
-// fold to a base and immediate offsets (128^3: 150 -> about 90 instructions per
-// point and pass against the runtime factors).  Blocks of 256 threads.
+// fold to a base and immediate offsets.  Blocks of 256 threads, one item per
+// thread in the first step; a loop around either step made the compiler keep
+// addresses live across it (64-84 bytes of spills at 64 registers, now none).
 template <typename C, int N1, int N2, bool ONE>
 __device__ __forceinline__ void fft_pow2(C *a, int nlines, int ld, const C *__restrict__ tw) {
   unsigned const tid = threadIdx.x;
@@ -506,7 +491,9 @@ template <typename C> __device__ inline C cswap(C v) { return C{v.y, v.x}; }
 // contiguous along z: first the points of each super-brick, four per load,
 // then its halo, added to the points of the next one.  Bound by instructions
 // (integer ones run at half rate), so the rows of a line are listed once in
-// shared memory.
+// shared memory, and lines, groups and half rows are flat index ranges (a warp
+// per line left lanes idle on short lines: 48 small meshes 45 -> 109 us).  At
+// 256^3 84 us; from a mesh 54 us, but the mesh cost the assignment its flushes.
 // blockIdx.y: charge set (tiles and spectra tile_stride / c_stride apart).
 // Shared memory: bk.b/2 staged lines of line_ld(n) (twice that for KIND 0),
 // twiddles (n).  Meshes are even, so is bk.b.
@@ -640,7 +627,10 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   int const hp = G.hp;
   // both lines of a slot from one pair of entries
   C *const out = cmesh + G.km_off + line0 * hp;
-  for_lines(np, hp, [&](int p, int k) {
+  float const rhp = 1.0f / static_cast<float>(hp);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < np * hp; t += 256) {
+    int const p = qdiv(t, hp, rhp), k = t - p * hp;
     C v0{Real(0), Real(0)}, v1 = v0;
     if (k < H) {
       C const z = res[p * ld + pix(k)];
@@ -651,10 +641,12 @@ k_fft_z_fwd(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     C *q = out + 2 * p * hp + k;
     q[0] = v0;
     q[hp] = v1;
-  });
+  }
 }
 
 // ---- pass y ---------------------------------------------------------------
+// Bound by the latency of its row loads, then by instructions; at 256^3 36 us
+// forward and 100 us for the three backward spectra (two of them inputs).
 // Jobs of a y pass: job k transforms array src[k], times k_y^pw[k], into array
 // dst[k].  Array src[k] is read by other jobs unless dst[k] = src[k].  The
 // jobs of one tile are neighbouring blocks, so a shared source is read from
@@ -708,9 +700,9 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
   Real const ks = kscale ? static_cast<Real>(2.0 * kPi * G.box_i[1]) : Real(1);
   // all of a thread's rows in flight at once (up to 16: M1 <= 256 in one
   // round), rows and columns past the tile read a valid one in their place, so
-  // that the loads are unconditional (guarded, the compiler waits for each
-  // before the next: 12 -> 19 us at 128^3); row y = yq + 16 u of column tq lies
-  // at tq ld + yq + 17 u
+  // that the loads are unconditional (guarded they were not all in flight
+  // together: with the spills, the two y passes of 256^3 took 64 + 125 us
+  // against 36 + 100); row y = yq + 16 u of column tq lies at tq ld + yq + 17 u
   C *const sl = a + tq * ld + yq;
   int const rows = col ? (M1 - yq + 15) >> 4 : 0;
   long long const step = 16 * hp;
@@ -895,7 +887,9 @@ inline ZPass z_charge() { return ZPass{{0, 2, 3}, {0, 0, 1}}; }
 // Shared memory: nl + ceil(nl/2) staged lines of line_ld(n) (twice for
 // KIND 0), twiddles (n).  FP32: four blocks per SM -- the block's load, transform
 // and store phases do not overlap, so the fourth resident block pays for the
-// 64-register bound.
+// 64-register bound.  The half rows are read straight into the slots: staging
+// them first cost a pass over shared memory and half the lines per block (128^3
+// 32 -> 26 us; at 256^3, where the spectra come from HBM, 156 -> 162 us).
 constexpr int kZiLines = 128; // most lines per block
 template <typename Real, int KIND>
 __global__ void __launch_bounds__(256, kFftBlocks<Real>)
@@ -976,7 +970,10 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
     s_row[l] = (x + M0 < P0 || y + M1 < P1) ? ~row : row;
   }
   __syncthreads();
-  for_lines(nl, n, [&](int l, int k) {
+  float const rn = 1.0f / static_cast<float>(n);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < nl * n; t += 256) {
+    int const l = KIND == kFftPow2 ? t >> (__ffs(n) - 1) : qdiv(t, n, rn), k = t - l * n;
     C const xy = res[l * ld + pix(k)];
     C const zz = res[(nl + (l >> 1)) * ld + pix(k)];
     R4 v;
@@ -989,7 +986,7 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
       out[row + k] = v;
       for (int zg = k + n; zg < P2; zg += n)
         out[row + zg] = v;
-      return;
+      continue;
     }
     int const x = static_cast<int>((line0 + l) / M1), y = static_cast<int>((line0 + l) % M1);
     for (int xg = x; xg < P0; xg += M0)
@@ -998,7 +995,7 @@ k_fft_z_inv3(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
         for (int zg = k; zg < P2; zg += n)
           r[zg] = v;
       }
-  });
+  }
 }
 
 } // namespace p3mx
