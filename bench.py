@@ -1289,11 +1289,10 @@ def main():
         "p3m_assign": 28 * N + 4 * M3,
         "p3m_interp": 28 * N + 12 * M3 + 24 * N,
         "fft_fwd_zy": 4 * M3 + 8 * K + 8 * K + 8 * K,
-        "fft_x_kspace": 8 * K + 4 * K + 3 * 8 * K,
-        "fft_inv_yz": 3 * (8 * K + 8 * K) + 3 * (8 * K + 4 * M3),
+        "fft_x_kspace": 8 * K + 4 * K + 2 * 8 * K,
+        "fft_inv_yz": (2 + 3) * 8 * K + 3 * 8 * K + 3 * 4 * M3,
         "pair_forces": N * nb_full * 4 + 32 * N + 24 * N,
         "p3m_sort": 2 * (24 + 4 + 4) * N + 8 * M3,
-        "p3m_weights": 24 * N + 8 * N + 3 * 4 * c * N,
     }
     dom = max(stages, key=stages.get)
     dom_ms = stages[dom]

@@ -50,9 +50,6 @@ template <typename C> __host__ __device__ inline C cadd(C a, C b) {
 template <typename C> __host__ __device__ inline C csub(C a, C b) {
   return C{a.x - b.x, a.y - b.y};
 }
-template <typename C> __host__ __device__ inline C cconj(C a) {
-  return C{a.x, -a.y};
-}
 
 // Maximum number of radix stages of one FFT length.
 constexpr int kMaxStages = 12;
@@ -101,27 +98,6 @@ struct RepGeom {
   long long nb_off;
   int max_nb;
 };
-
-// Batched global -> shared copy: each thread issues U loads before its
-// stores, so U loads are in flight per thread.
-template <int U, typename L, typename S>
-__device__ inline void staged_copy(int total, L const &load, S const &store) {
-  for (int e0 = threadIdx.x; e0 < total; e0 += U * blockDim.x) {
-    decltype(load(0)) v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      int const e = e0 + u * blockDim.x;
-      if (e < total)
-        v[u] = load(e);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      int const e = e0 + u * blockDim.x;
-      if (e < total)
-        store(e, v[u]);
-    }
-  }
-}
 
 // ---- bulk-copy engine (TMA) helpers: cp.async.bulk global -> shared with
 // completion on an mbarrier (transaction bytes); waits are bounded.

@@ -77,7 +77,8 @@ public:
     m_gf.ensure(E.m_cplx * rsz);
     long long const nprep = ceil_div(nn, 256);
     size_t const np = std::max<size_t>({static_cast<size_t>(E.m_n_blk_x), 5 * static_cast<size_t>(nprep),
-                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(), size_t(kSumBlocks)});
+                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(kDpPairBlocks64),
+                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(kDpPairBlocks32), size_t(kSumBlocks)});
     m_part.ensure(np * sizeof(double));
     m_sums.ensure(8 * sizeof(double));
     m_flag.ensure(sizeof(int));
@@ -293,7 +294,7 @@ public:
       int const exact = accuracy > 5e-6 ? 0 : 1;
       RepGeom const *geom = E.m_geom_d.as<RepGeom>();
       // FP32-mesh mode: the pair terms in FP32 on the cell-relative offsets
-      int const lanes = E.pair_lanes();
+      int const lanes = E.pair_lanes(rel ? kDpPairBlocks32 : kDpPairBlocks64);
       auto pairs = [&](auto ev, double *fo, double *part) {
         constexpr bool EV = decltype(ev)::value;
         auto go = [&](auto lpp) {

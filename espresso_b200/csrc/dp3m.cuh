@@ -20,6 +20,9 @@
 
 namespace p3mx {
 
+// Resident blocks per SM of the pair kernels (Engine::pair_lanes), FP32 and FP64.
+constexpr int kDpPairBlocks32 = 3, kDpPairBlocks64 = 2;
+
 // calc_meshift (p3m/common.hpp:248-264): index shift of the influence
 // function (M/2 -> -M/2) and of the differential operator (M/2 -> 0).
 __host__ __device__ inline int dp_shift(int i, int m) { return (i < m / 2) ? i : i - m; }
@@ -517,7 +520,7 @@ __device__ inline void dp_pairs_finish(double (&w)[7], double mx, double my, dou
 }
 
 template <bool EV, int LPP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kDpPairBlocks64)
 k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
              const double4 *__restrict__ spq, const double4 *__restrict__ smu,
              const int *__restrict__ perm, const int *__restrict__ nb,
@@ -634,7 +637,7 @@ struct Sum2 {
 // square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; each pair's force and
 // torque terms summed in FP32 pairs (Sum2), its energy in FP64.
 template <bool EV, int LPP>
-__global__ void __launch_bounds__(256, EV ? 1 : 3)
+__global__ void __launch_bounds__(256, EV ? 1 : kDpPairBlocks32)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                  const float4 *__restrict__ spf, const float4 *__restrict__ smu,
                  const int *__restrict__ perm, const int *__restrict__ nb,

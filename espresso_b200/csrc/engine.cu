@@ -579,7 +579,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_flag.ensure(sizeof(int));
   m_pos_ref.ensure(3 * n * sizeof(double));
   m_type_ref.ensure(n * sizeof(int));
-  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes() * 20 * sizeof(double));
+  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes(kPairBlocks64) * 20 * sizeof(double));
   m_sums_pair.ensure(static_cast<size_t>(R) * 20 * sizeof(double));
   if (m_ia_d.p == nullptr)
     upload_vec(m_ia_d, m_ia, st);
@@ -1198,24 +1198,35 @@ void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp,
   ++m_launches;
 }
 
-// Lanes per particle of the pair kernels: lists are split over 1, 2, 4 or 8
-// lanes until the launch fills the GPU (kPairFill threads per SM).
-int Engine::pair_lanes() const {
+// Lanes per particle of the pair kernels (1, 2, 4 or 8, whole groups of 8 list
+// entries each), for `per_sm` resident blocks per SM: the most with which all
+// blocks are resident at once; two where the blocks are more than one but less
+// than 1.7 waves (the second wave would cost as much as a full one).  Kernel
+// times in us at 1 / 2 / 4 / 8 lanes, those chosen in brackets: FP32 23 457 ions
+// 33 / 25 / [22] / 26, 98 304 ions [37] / 39 / 41 / 53, 131 072 ions [52] / 53 / 62
+// / 79, 250 000 ions in a dense melt 142 / [126] / 139 / 180, 2^20 ions [240] / 265
+// / 335 / 456; FP64 131 072 ions [187] / 196 / 203 / 243; dipoles 16 384 FP64 197
+// / 108 / [71] / 80, 131 072 FP32 352 / [288] / 281 / 310.
+int Engine::pair_lanes(int per_sm) const {
+  long long const room = static_cast<long long>(m_sms) * per_sm, blocks = m_n_blk_pair;
   int l = 1;
-  while (l < 8 && m_n * l < static_cast<long long>(m_sms) * kPairFill)
+  while (l < 8 && 2 * l * blocks <= room)
     l *= 2;
-  return l;
+  return blocks > room && 10 * blocks < 17 * room ? 2 : l;
 }
 
 template <typename Real>
 void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t st) {
   RepGeom const *geom = m_geom_d.as<RepGeom>();
-  int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes();
+  constexpr int per_sm = sizeof(Real) == 4 ? kPairBlocks32 : kPairBlocks64;
+  int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes(per_sm);
+  bool const chained = lanes > 1 && m_n_blk_pair * lanes <= m_sms * per_sm;
   auto go = [&](auto kern, auto const *pos, size_t smem) {
     // not chained where the launch fills the GPU: its blocks would start in
     // the interpolation's shared-memory configuration, with too little L1
-    // left for the position gathers (1.58 -> 1.80 ms per pass at 2^20 ions)
-    pdl_launch(kern, m_n_blk_pair * lanes, 256, smem, st, lanes > 1, geom, m_blk_pair.as<int2>(), pos,
+    // left for the position gathers (1.58 -> 1.80 ms per pass at 2^20 ions, 0.274
+    // -> 0.296 ms at 131 072)
+    pdl_launch(kern, m_n_blk_pair * lanes, 256, smem, st, chained, geom, m_blk_pair.as<int2>(), pos,
                m_stype.as<int>(), m_cperm.as<int>(), m_ia_d.as<PairIA>(), m_ntypes, m_nb.as<int>(),
                m_nb_cnt.as<int>(), f, overwrite ? 1 : 0, m_part_pair.as<double>());
     ++m_launches;
@@ -1326,7 +1337,7 @@ void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t s
     bool const one = m_fp32 && !fp64_math;
     k_reduce_partials<<<dim3(R, 20), 256, 0, st>>>(m_part_pair.as<double>(), 20,
                                                    m_blk_pair_start_d.as<int>(),
-                                                   one ? 1 : pair_lanes(),
+                                                   one ? 1 : pair_lanes(kPairBlocks64),
                                                    m_sums_pair.as<double>()); ++m_launches;
     std::vector<double> sums(static_cast<size_t>(R) * 20);
     P3MX_CUDA(cudaMemcpyAsync(sums.data(), m_sums_pair.p, sums.size() * sizeof(double),

@@ -195,7 +195,7 @@ private:
   void mark(const char *name, cudaStream_t st);
 
   // lanes per particle of the pair kernels for the current particle number
-  int pair_lanes() const;
+  int pair_lanes(int per_sm) const;
 
   bool m_fp32;
   int m_sms = 148;

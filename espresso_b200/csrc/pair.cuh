@@ -665,11 +665,8 @@ __device__ inline PairF pair_f(PairIA const &p) {
 // (parameters in registers, the LJ powers from the Coulomb term's 1/r^2),
 // several types without offsets, LJ offsets.
 constexpr int kPairOneType = 0, kPairTypes = 1, kPairOffset = 2;
-// Threads per SM at which a pair launch counts as filling the GPU.  Below,
-// each particle's list is split over up to 8 lanes, whole groups of 8
-// entries each: 12 000 ions 25 -> 10 us, 131 072 ions are the faster the
-// fewer lanes.
-constexpr int kPairFill = 768;
+// Resident blocks per SM of the force kernels (Engine::pair_lanes), FP32 and FP64.
+constexpr int kPairBlocks32 = 4, kPairBlocks64 = 2;
 
 // Force kernel of the FP32-mixed path over the Verlet list: real-space Coulomb
 // (CoulombP3M::pair_force, p3m.hpp:146-180) plus LJ and WCA (lj.hpp:41-60,
@@ -685,9 +682,10 @@ constexpr int kPairFill = 768;
 // a group and FP64 across groups.
 // Bound by instruction issue (about 45 scalar instructions per entry and
 // three MUFU operations): the range-independent arithmetic runs on two
-// entries at a time in packed FP32, with the scalar code's roundings.
+// entries at a time in packed FP32, with the scalar code's roundings: 2^20 ions
+// 311 -> 241 us, 131 072 ions 57 -> 52 us.
 template <int MODE, int LPP>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, kPairBlocks32)
 k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                   const float4 *__restrict__ spf, const int *__restrict__ stype,
                   const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
@@ -1010,10 +1008,12 @@ k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ 
 // k_pair_forces_rel (LJ / WCA for class A groups only).  EV adds energies and
 // virials: per-block FP64 partials {E_coul, E_nb, Vc[9], Vn[9]} (width 20).
 // Blocks map to replicas through the block table so partials never straddle
-// replicas.  Bound by the FP64 pipe: the inverse distance is one rsqrt, the
-// A&S reciprocal one FP32 seed with a third-order step.
+// replicas.  Bound by latency and the FP64 pipe: the inverse distance is one rsqrt, the
+// A&S reciprocal one FP32 seed with a third-order step; two pairs at a time, since
+// a pair's chain (rsqrt, exp, polynomial) is long and two blocks per SM do not
+// hide it (131 072 ions 234 -> 187 us).
 template <bool EV, int LPP>
-__global__ void __launch_bounds__(256, EV ? 1 : 2)
+__global__ void __launch_bounds__(256, EV ? 1 : kPairBlocks64)
 k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
               const double4 *__restrict__ spq, const int *__restrict__ stype,
               const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
