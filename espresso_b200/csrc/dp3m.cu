@@ -227,8 +227,11 @@ public:
       if (nbr == 0)
         continue;
       int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
+      // a third of the resident blocks per field set, rounded down: rounded up,
+      // one or two blocks had to wait for a second wave as long as the first
+      // (131 072 dipoles FP32 166 -> 113 us, 16 384 FP64 78 -> 58 us)
       P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>,
-                                 dim3(ceil_div(interp_grid<Real, P>(3 * nbr), 3), 3),
+                                 dim3(std::max(1, interp_grid<Real, P>(3 * nbr) / 3), 3),
                                  32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true, gi, tab,
                                  nbr, E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(), 1,
                                  E.m_tmap.as<CUtensorMap>(), 1, E.d_q(), E.m_dipole.as<double>(),
