@@ -635,7 +635,8 @@ struct Sum2 {
 // offsets (as k_pair_forces_rel: d = (off_a - off_b) - dc cs with dc from
 // the entry's offset code, no minimum-image arithmetic): hardware reciprocal
 // square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; each pair's force and
-// torque terms summed in FP32 pairs (Sum2), its energy in FP64.
+// torque terms summed in FP32 pairs (Sum2), its energy in FP64.  Bound by
+// instruction issue (about 130 per entry): 131 072 dipoles 347 -> 288 us.
 template <bool EV, int LPP>
 __global__ void __launch_bounds__(256, EV ? 1 : kDpPairBlocks32)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,

@@ -743,7 +743,8 @@ k_fft_y(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
 // Shared memory: 2 x tile staged lines of line_ld(M0) (phi, k_x phi; 3 x
 // for KIND 0: a scratch buffer), twiddles (M0).
 // EV: energy / virial partials (a template parameter, so that the
-// forces-only instance carries none of their registers).
+// forces-only instance carries none of their registers).  Bound by instructions:
+// 101 us at 256^3 (three backward transforms per mode: 181 us).
 template <typename Real, bool EV, int KIND>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 && !EV && KIND ? 3 : 2)
 k_fft_x_kspace(const RepGeom *__restrict__ reps, const Blk *__restrict__ blks,
