@@ -231,7 +231,7 @@ void configure_engine(p3mx_handle *h) {
   c.skin = h->sys.skin;
   c.p0 = 0;
   c.np = static_cast<long long>(h->n);
-  h->eng->set_pair_table(h->ntypes, h->table);
+  h->eng->store_pair_table(h->ntypes, h->table);
   h->eng->configure({c}, static_cast<long long>(h->n));
   h->eng64.reset();
   if (h->elc)
@@ -239,10 +239,10 @@ void configure_engine(p3mx_handle *h) {
 }
 
 Engine &observables_engine(p3mx_handle *h) {
-  if (!h->eng64) {
+  if (!h->eng64 || !h->eng64->configured()) {
     h->eng64 = std::make_unique<Engine>(false);
     ReplicaConf c = h->eng->conf(0);
-    h->eng64->set_pair_table(h->ntypes, h->table);
+    h->eng64->store_pair_table(h->ntypes, h->table);
     h->eng64->configure({c}, static_cast<long long>(h->n));
   }
   return *h->eng64;
@@ -628,10 +628,10 @@ void host_census(p3mx_handle *h, size_t n, const double *q, bool dev) {
 void ensure_ready(p3mx_handle *h, size_t n) {
   if (!h->activated)
     throw Error(P3MX_ERUNTIME, "actor not activated: call p3mx_activate first");
-  if (n != h->n || !h->eng) {
+  if (n != h->n || !h->eng || !h->eng->configured()) {
     h->n = n;
-    configure_engine(h);
     h->bonds_dirty = !h->bonds.empty();
+    configure_engine(h);
   }
   if (h->bonds_dirty) {
     h->eng->set_bonds(h->bond_types, h->bonds, h->eng->stream());
@@ -994,11 +994,11 @@ static void elc_contrast_forces(p3mx_handle *h, double *fd, double *energy3, dou
                     energy3 ? &e_img_pairs : nullptr, st);
   long long const n = static_cast<long long>(h->n);
   long long const n3 = 3 * n;
-  if (!s.img) {
+  if (!s.img || !s.img->configured()) {
     s.img = std::make_unique<Engine>(false);
     ReplicaConf c = e.conf(0);
     c.np = n3;
-    s.img->set_pair_table(h->ntypes, h->table);
+    s.img->store_pair_table(h->ntypes, h->table);
     s.img->configure({c}, n3);
   }
   Engine &im = *s.img;

@@ -38,9 +38,13 @@ public:
   Engine &engine() { return m_eng; }
   long long n() const { return m_eng.n_part(); }
 
+  // False until the first configuration and after one that threw.
+  bool configured() const { return m_configured && m_eng.configured(); }
+
   // One cubic replica of edge L with mesh M^3.
   void configure(double L, int M, int cao, double alpha, double r_cut, double skin,
                  const double *mesh_off, long long n) {
+    m_configured = false;
     ReplicaConf c;
     for (int d = 0; d < 3; ++d) {
       c.box[d] = L;
@@ -124,6 +128,7 @@ public:
     m_alpha = alpha;
     m_cao = cao;
     P3MX_CUDA(cudaStreamSynchronize(st));
+    m_configured = true;
   }
 
   // Stages positions and moments; returns {n_dipoles, sum mu^2, Mx, My, Mz}
@@ -415,6 +420,7 @@ private:
   Engine m_eng;
   DevBuf m_mu, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
   DevBuf m_tiles3, m_qmax3;
+  bool m_configured = false;
   bool m_g_valid = false, m_phi_valid = false, m_table_set = false;
   double m_phi = 0.0;
   int m_M = 0, m_cao = 0;
@@ -997,7 +1003,7 @@ int p3mx_dp3m_compute(p3mx_dp3m *h, size_t n, const double *pos, const double *d
       throw Error(P3MX_EDOMAIN, "forces requested with a NULL force or torque array");
     if (n && (!pos || !dip))
       throw Error(P3MX_EDOMAIN, "NULL position or dipole array");
-    if (n != h->n || !h->de) {
+    if (n != h->n || !h->de || !h->de->configured()) {
       h->n = n;
       dp_configure(h);
     }
@@ -1041,7 +1047,7 @@ int p3mx_dp3m_profile(p3mx_dp3m *h, size_t n, const double *pos, const double *d
   return dp_guarded(h, [&] {
     if (!h->activated)
       throw Error(P3MX_ERUNTIME, "DipolarP3M: actor not activated");
-    if (n != h->n || !h->de) {
+    if (n != h->n || !h->de || !h->de->configured()) {
       h->n = n;
       dp_configure(h);
     }

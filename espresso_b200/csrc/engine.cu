@@ -156,23 +156,35 @@ Engine::~Engine() {
     cudaStreamDestroy(m_stream);
 }
 
-void Engine::set_pair_table(int ntypes, std::vector<PairIA> const &tab) {
+void Engine::store_pair_table(int ntypes, std::vector<PairIA> const &tab) {
   if (ntypes < 1 || static_cast<int>(tab.size()) != ntypes * ntypes)
     throw Error(1, "pair table must hold ntypes^2 entries");
-  // the table of the current lists and block tables: nothing to do (scripts
-  // set it before every force calculation)
-  if (ntypes == m_ntypes && m_ia_d.p != nullptr && !m_conf.empty() &&
-      std::memcmp(tab.data(), m_ia.data(), tab.size() * sizeof(PairIA)) == 0)
-    return;
+  m_configured = false; // the cell grid and the lists belong to the table
+  m_lists_valid = false;
   m_ntypes = ntypes;
   m_ia = tab;
   upload_vec(m_ia_d, m_ia, m_stream);
-  m_lists_valid = false;
+}
+
+void Engine::set_pair_table(int ntypes, std::vector<PairIA> const &tab) {
+  // the table of the current lists and block tables: nothing to do (scripts
+  // set it before every force calculation).  After a configuration that threw,
+  // the same table is tried again and throws again
+  if (m_configured && ntypes == m_ntypes && tab.size() == m_ia.size() &&
+      std::memcmp(tab.data(), m_ia.data(), tab.size() * sizeof(PairIA)) == 0)
+    return;
+  store_pair_table(ntypes, tab);
   if (!m_conf.empty())
     configure(std::vector<ReplicaConf>(m_conf), m_n);
 }
 
+void Engine::require_configured() const {
+  if (!m_configured)
+    throw Error(2, "the engine is not configured: its last configuration failed");
+}
+
 void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) {
+  m_configured = false; // until the end: a throw leaves members of both states
   m_conf = conf;
   m_n = n_total;
   int const R = static_cast<int>(conf.size());
@@ -586,6 +598,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_ginf_valid = false;
   m_lists_valid = false;
   P3MX_CUDA(cudaStreamSynchronize(st));
+  m_configured = true;
 }
 
 // Positions, charges and types (nullptr: zero) from the caller's device
@@ -618,6 +631,7 @@ k_stage(long long n, const double *__restrict__ pos, const double *__restrict__ 
 
 void Engine::upload(const double *pos, const double *q, const int *type, bool device_ptrs,
                     cudaStream_t st) {
+  require_configured();
   cudaMemcpyKind const k = cudaMemcpyHostToDevice;
   if (m_n == 0)
     return;
@@ -636,6 +650,7 @@ void Engine::upload(const double *pos, const double *q, const int *type, bool de
 }
 
 void Engine::upload_positions(const double *pos, bool device_ptrs, cudaStream_t st) {
+  require_configured();
   if (m_n == 0)
     return;
   P3MX_CUDA(cudaMemcpyAsync(m_pos.p, pos, 3 * m_n * sizeof(double),
@@ -643,6 +658,7 @@ void Engine::upload_positions(const double *pos, bool device_ptrs, cudaStream_t 
 }
 
 void Engine::census(cudaStream_t st) {
+  require_configured();
   int const R = n_rep();
   k_census<<<m_n_blk_census, 256, 0, st>>>(m_blk_census.as<int2>(), m_geom_d.as<RepGeom>(),
                                            d_pos(), d_q(), m_part_census.as<double>()); ++m_launches;
@@ -894,6 +910,7 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
 void Engine::long_range(double *f, bool overwrite, bool want_energy, bool want_virial,
                         cudaStream_t st, std::vector<double> *energies,
                         std::vector<double> *virials) {
+  require_configured();
   if (m_fp32)
     long_range_t<float>(f, overwrite, want_energy, want_virial, st);
   else
@@ -1290,6 +1307,7 @@ void Engine::short_range_t(double *f, bool overwrite, bool want_ev, cudaStream_t
 // Forces only (no energies or virials); in: the caller's device arrays to stage
 // first, or none.
 void Engine::forces_all(double *f, bool overwrite, cudaStream_t st, ParticleArrays const &in) {
+  require_configured();
   if (m_n == 0 || m_profiling) {
     if (in.pos)
       upload(in.pos, in.q, in.type, true, st);
@@ -1327,6 +1345,7 @@ void Engine::forces_all(double *f, bool overwrite, cudaStream_t st, ParticleArra
 void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t st,
                          std::vector<double> *energies, std::vector<double> *virials,
                          bool fp64_math) {
+  require_configured();
   if (m_fp32 && !fp64_math)
     short_range_t<float>(f, overwrite, want_ev, st);
   else
@@ -1366,6 +1385,7 @@ void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t s
 // particles moved more than skin/2 rebuild: the others keep their cell keys,
 // hence their sorted order, lists and reference positions.
 void Engine::short_range_graph(double *f, bool overwrite, cudaStream_t st) {
+  require_configured();
   if (m_n == 0)
     return;
   RepGeom const *geom = m_geom_d.as<RepGeom>();
@@ -1443,6 +1463,7 @@ void Engine::layout_lists(cudaStream_t st) {
 }
 
 void Engine::ensure_lists(cudaStream_t st, double nb_margin) {
+  require_configured();
   std::vector<int> before = m_cap;
   if (m_cap.size() != m_geom.size() || nb_margin > 1.0)
     set_list_capacity(std::max(nb_margin, 1.5));
@@ -1453,6 +1474,7 @@ void Engine::ensure_lists(cudaStream_t st, double nb_margin) {
 }
 
 std::vector<int> Engine::cell_index_ghost(cudaStream_t st) {
+  require_configured();
   std::vector<int> out(m_n);
   if (m_n == 0)
     return out;
@@ -1471,6 +1493,7 @@ std::vector<int> Engine::cell_index_ghost(cudaStream_t st) {
 }
 
 std::vector<int> Engine::verlet_pairs(cudaStream_t st) {
+  require_configured();
   build_lists(st);
   std::vector<int> cnt(m_n), perm(m_n);
   long long total = 0;
@@ -1498,6 +1521,7 @@ std::vector<int> Engine::verlet_pairs(cudaStream_t st) {
 }
 
 std::vector<double> Engine::mesh_copy(int r, cudaStream_t st) {
+  require_configured();
   auto const &G = m_geom[r];
   long long const ms = static_cast<long long>(G.mesh[0]) * G.mesh[1] * G.mesh[2];
   std::vector<double> out(ms);
@@ -1523,6 +1547,7 @@ std::vector<double> Engine::mesh_copy(int r, cudaStream_t st) {
 }
 
 void Engine::cell_grid(int r, int *cg, double *cs) const {
+  require_configured();
   for (int d = 0; d < 3; ++d) {
     cg[d] = m_geom[r].cg[d];
     cs[d] = 1.0 / m_geom[r].inv_cs[d];
@@ -1568,6 +1593,7 @@ void Engine::check_kernel_error(cudaStream_t st) {
 
 void Engine::set_bonds(std::vector<BondParam> const &types, std::vector<int> const &bonds,
                        cudaStream_t st) {
+  require_configured();
   long long const nb = static_cast<long long>(bonds.size() / 3);
   m_nbonds = 0;
   if (nb == 0)
@@ -1700,6 +1726,7 @@ k_elc_image_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk
 
 void Engine::elc_image_pairs(double sl, double h, double db, double dt, double *f,
                              double *energy, cudaStream_t st) {
+  require_configured();
   if (energy)
     *energy = 0.0;
   if (m_n == 0)
@@ -1727,6 +1754,7 @@ void Engine::elc_image_pairs(double sl, double h, double db, double dt, double *
 }
 
 void Engine::bond_forces(double *f, cudaStream_t st) {
+  require_configured();
   if (m_nbonds == 0)
     return;
   if (m_bond_n != m_n)
@@ -1738,6 +1766,7 @@ void Engine::bond_forces(double *f, cudaStream_t st) {
 }
 
 std::vector<double> Engine::bond_energies(cudaStream_t st) {
+  require_configured();
   std::vector<double> out(m_geom.size(), 0.0);
   if (m_nbonds == 0)
     return out;
@@ -1760,6 +1789,7 @@ std::vector<double> Engine::bond_energies(cudaStream_t st) {
 }
 
 void Engine::bond_observables(cudaStream_t st, double *energy, double *virial9) {
+  require_configured();
   for (int k = 0; k < 9; ++k)
     virial9[k] = 0.0;
   *energy = 0.0;

@@ -84,7 +84,13 @@ public:
 
   // (Re)builds geometry, plans, block tables; allocates the buffers.
   void configure(std::vector<ReplicaConf> const &conf, long long n_total);
-  // LJ/WCA table (ntypes^2 entries, symmetric).
+  // False until the first configuration and after one that threw: every other
+  // call that works on the configuration then throws.
+  bool configured() const { return m_configured; }
+  void require_configured() const;
+  // LJ/WCA table (ntypes^2 entries, symmetric): for the configure() that
+  // follows, or with the current configuration made again where it differs.
+  void store_pair_table(int ntypes, std::vector<PairIA> const &tab);
   void set_pair_table(int ntypes, std::vector<PairIA> const &tab);
 
   // Device-resident particle arrays in user order (AoS positions/forces).
@@ -198,6 +204,7 @@ private:
   int pair_lanes(int per_sm) const;
 
   bool m_fp32;
+  bool m_configured = false;
   int m_sms = 148;
   cudaStream_t m_stream = nullptr;
   long long m_launches = 0;
