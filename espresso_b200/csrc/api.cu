@@ -1189,7 +1189,8 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
                       h->staged_n == n && h->staged_q && (type != nullptr) == h->staged_type;
     // device arrays and forces only: staged by the evaluation's first kernel
     ParticleArrays direct;
-    if (dev && n > 0 && !want_e && !want_v && h->prm.epsilon == 0.) {
+    if (dev && n > 0 && !want_e && !want_v && h->prm.epsilon == 0. &&
+        e.kernel_readable(pos, q, type)) {
       direct = ParticleArrays{pos, q, type};
       h->staged_q = h->staged_type = false;
     } else {

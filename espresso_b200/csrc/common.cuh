@@ -23,10 +23,12 @@ struct Error : std::runtime_error {
 #define P3MX_CUDA(call)                                                       \
   do {                                                                        \
     cudaError_t err_ = (call);                                                \
-    if (err_ != cudaSuccess)                                                  \
+    if (err_ != cudaSuccess) {                                                \
+      cudaGetLastError(); /* reported here, not by the next check as well */  \
       throw ::p3mx::Error(3, std::string("CUDA error: ") +                    \
                                  cudaGetErrorString(err_) + " at " +          \
                                  __FILE__ + ":" + std::to_string(__LINE__));  \
+    }                                                                         \
   } while (0)
 
 template <typename Real> struct CplxOf;

@@ -133,9 +133,8 @@ template <typename T> void upload_vec(DevBuf &b, std::vector<T> const &v, cudaSt
 Engine::Engine(bool fp32) : m_fp32(fp32) {
   P3MX_CUDA(cudaStreamCreateWithFlags(&m_stream, cudaStreamNonBlocking));
   m_ia.assign(1, PairIA{0, 0, 0, 0, 0, 0, 0, 0, 0, -1.0});
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess)
-    cudaDeviceGetAttribute(&m_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaGetDevice(&m_device) == cudaSuccess)
+    cudaDeviceGetAttribute(&m_sms, cudaDevAttrMultiProcessorCount, m_device);
   void *w = nullptr;
   if (cudaHostAlloc(&w, kHostWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) !=
       cudaSuccess) {
@@ -601,6 +600,23 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_configured = true;
 }
 
+// Whether kernels of this device may read the caller's arrays in place of
+// copies: aligned memory of the device.  Anything else (NULL, host or managed
+// memory, another device's, a misaligned address) is left to the copies, which
+// take it or return an error; a kernel would fault.
+bool Engine::kernel_readable(const double *pos, const double *q, const int *type) const {
+  auto ok = [&](const void *p, size_t align) {
+    cudaPointerAttributes a;
+    if (reinterpret_cast<uintptr_t>(p) % align != 0 ||
+        cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == m_device;
+  };
+  return ok(pos, sizeof(double)) && ok(q, sizeof(double)) && (!type || ok(type, sizeof(int)));
+}
+
 // Positions, charges and types (nullptr: zero) from the caller's device
 // arrays into the engine's, one launch in place of three copies.
 __global__ void __launch_bounds__(256)
@@ -632,10 +648,12 @@ k_stage(long long n, const double *__restrict__ pos, const double *__restrict__ 
 void Engine::upload(const double *pos, const double *q, const int *type, bool device_ptrs,
                     cudaStream_t st) {
   require_configured();
-  cudaMemcpyKind const k = cudaMemcpyHostToDevice;
+  cudaMemcpyKind const k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   if (m_n == 0)
     return;
-  if (device_ptrs) {
+  if (!pos || !q)
+    throw Error(3, "NULL position or charge array");
+  if (device_ptrs && kernel_readable(pos, q, type)) {
     k_stage<<<ceil_div(m_n, 1024), 256, 0, st>>>(m_n, pos, q, type, d_pos(), d_q(), d_type());
     ++m_launches;
     P3MX_CUDA(cudaGetLastError());

@@ -100,6 +100,7 @@ public:
   double *d_force() const { return m_force.as<double>(); }
   void upload(const double *pos, const double *q, const int *type, bool device_ptrs,
               cudaStream_t st);
+  bool kernel_readable(const double *pos, const double *q, const int *type) const;
   void upload_positions(const double *pos, bool device_ptrs, cudaStream_t st);
 
   // Charge census (n_charged, sum q, sum q^2, dipole) per replica -> host.
@@ -205,7 +206,7 @@ private:
 
   bool m_fp32;
   bool m_configured = false;
-  int m_sms = 148;
+  int m_device = 0, m_sms = 148;
   cudaStream_t m_stream = nullptr;
   long long m_launches = 0;
   bool m_profiling = false;

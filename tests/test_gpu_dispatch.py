@@ -9,6 +9,7 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 from scipy.spatial import cKDTree
 
 import espresso_b200 as eb
@@ -221,3 +222,48 @@ def test_observables_without_forces(cls):
                    act._handle)
         out.append(np.concatenate([e, v]))
     np.testing.assert_array_equal(out[0], out[1])
+
+
+def _device_call(lib, act, fn, n, pos, q, types, f):
+    flags = _lib.P3MX_DEVICE_PTRS | _lib.P3MX_FORCES | _lib.P3MX_OVERWRITE
+    if fn == "forces":
+        return lib.p3mx_forces(act._handle, n, pos, q, types, f, None, None, flags, None)
+    if fn == "short":
+        return lib.p3mx_short_range(act._handle, n, pos, q, types, f, None, None, flags, None)
+    return lib.p3mx_long_range(act._handle, n, pos, q, f, None, None, flags, None)
+
+
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+@pytest.mark.parametrize("fn", ["forces", "short", "long"])
+def test_device_arrays_that_kernels_cannot_read(cls, fn):
+    """Device arrays are read by kernels where these can: a NULL array is an
+    error and not a fault, and arrays off their alignment are copied."""
+    n, box = 1000, np.full(3, 13.0)
+    pos, q = _ions(n, box, seed=6)
+    types = (np.arange(n) % 2).astype(np.int32)
+    act = _actor(cls, box, pos, q, [24] * 3, 5, alpha=1.1, r_cut=2.5)
+    lib = _lib.load()
+    tab = (_lib.PairParams * 4)()
+    tab[1].wca_eps = tab[2].wca_eps = tab[1].wca_sig = tab[2].wca_sig = 1.0
+    _lib.check(lib.p3mx_set_pair_params(act._handle, 2, tab), act._handle)
+    d = [torch.from_numpy(a).cuda() for a in (pos, q, types)]
+    f = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ptr = [_lib.dptr(a) for a in d]
+    assert _device_call(lib, act, fn, n, *ptr, _lib.dptr(f)) == 0
+    want = f.clone()
+    for k in range(2):
+        bad = list(ptr)
+        bad[k] = None
+        assert _device_call(lib, act, fn, n, *bad, _lib.dptr(f)) != 0
+    off = []  # the same arrays, 4 and 2 bytes off their alignment
+    for a in d:
+        raw = a.contiguous().view(torch.uint8).reshape(-1)
+        buf = torch.empty(len(raw) + 16, dtype=torch.uint8, device="cuda")
+        shift = a.element_size() // 2
+        buf[shift:shift + len(raw)] = raw
+        off.append((buf, ctypes.c_void_p(buf.data_ptr() + shift)))
+    f.zero_()
+    torch.cuda.synchronize()
+    assert _device_call(lib, act, fn, n, *[p for _, p in off], _lib.dptr(f)) == 0
+    assert torch.equal(f, want)
