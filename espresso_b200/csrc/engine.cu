@@ -424,6 +424,9 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
         std::max<size_t>(1, std::min<size_t>(16, y_budget / (y_bufs * ldy * csz))));
     m_tile_x = static_cast<int>(
         std::max<size_t>(1, std::min<size_t>(16, x_budget / (x_bufs * ldx * csz))));
+    // dynamic shared memory of a block: the 227 KB limit less the kernels' static
+    // arrays
+    size_t const limit = 220 * 1024;
     size_t smem_zf = 0, smem_zi = 0;
     for (int r = 0; r < R; ++r) {
       auto const &G = m_geom[r];
@@ -461,10 +464,14 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       auto const zi_smem = [&](int nl) {
         return ((two ? 1 : 2) * static_cast<size_t>(nl + (nl + 1) / 2) * ldz + M2) * csz;
       };
-      int lzi = 2;
-      while (3 * (lzi + 2) / 2 <= want && lzi + 2 <= kZiLines && zi_smem(lzi + 2) <= z_budget)
-        lzi += 2;
-      lzi = fill(lzi);
+      // (one line where two exceed a block's shared memory: 2048 points in FP64)
+      int lzi = 1;
+      if (zi_smem(2) <= limit) {
+        lzi = 2;
+        while (3 * (lzi + 2) / 2 <= want && lzi + 2 <= kZiLines && zi_smem(lzi + 2) <= z_budget)
+          lzi += 2;
+        lzi = fill(lzi);
+      }
       for (int l = 0; l < lines; l += lzi)
         zi.push_back(Blk{r, l, std::min(lzi, lines - l), 0});
       smem_zi = std::max(smem_zi, zi_smem(std::min(lzi, lines)));
@@ -496,9 +503,6 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     upload_vec(m_blk_x, x, st);
     upload_vec(m_blk_zi, zi, st);
     upload_vec(m_blk_x_start_d, m_blk_x_start, st);
-    // opt-in dynamic shared memory; static arrays of the kernels (<= 2 KB)
-    // stay inside the 227 KB per-block limit
-    size_t const limit = 220 * 1024;
     if (std::max({m_smem_zf, m_smem_zi, m_smem_y, m_smem_x}) > limit)
       throw Error(1, "mesh too large for the shared-memory FFT tiles");
     // one process-wide opt-in value, so engines of different sizes coexist

@@ -267,3 +267,22 @@ def test_device_arrays_that_kernels_cannot_read(cls, fn):
     torch.cuda.synchronize()
     assert _device_call(lib, act, fn, n, *[p for _, p in off], _lib.dptr(f)) == 0
     assert torch.equal(f, want)
+
+
+# axis lengths whose backward z pass takes one line per block: 2048 points in
+# FP64 (two lines would need 241 568 bytes of shared memory), 3840 in FP32
+@pytest.mark.parametrize("cls,mz,energy", [(P3M, 2048, True), (P3MGPU, 2048, True),
+                                           (P3MGPU, 3840, False)])
+def test_long_z_axis(cls, mz, energy):
+    mesh, box = (8, 6, mz), np.array([6.0, 5.0, 0.4 * mz])
+    pos, q = _ions(700, box, seed=9)
+    act = _actor(cls, box, pos, q, mesh, 3, alpha=0.9, r_cut=1.0)
+    lib = _lib.load()
+    f, e = np.zeros((len(q), 3)), np.zeros(1)
+    flags = _lib.P3MX_FORCES | _lib.P3MX_OVERWRITE | (_lib.P3MX_ENERGY if energy else 0)
+    _lib.check(lib.p3mx_long_range(act._handle, len(q), _lib.dptr(pos), _lib.dptr(q), _lib.dptr(f),
+                                   e.ctypes.data_as(DP), None, flags, None), act._handle)
+    fo, eo, _ = O.p3m_kspace(O.make_params(box, mesh, 3, 0.9, 1.0, 1.0), pos, q)
+    np.testing.assert_allclose(f, fo, rtol=0, atol=RTOL[cls] * np.abs(fo).max())
+    if energy:
+        assert abs(e[0] - eo) <= 1e-9 * (abs(eo) + (q * q).sum() * 0.9)
