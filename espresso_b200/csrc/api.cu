@@ -127,6 +127,9 @@ struct p3mx_handle {
   // pressures are evaluated in FP64, as the reference GPU actor evaluates
   // them with its double-precision CPU kernels (p3m.impl.hpp:328-343)
   std::unique_ptr<Engine> eng64;
+  // the last evaluation ran the mesh of eng64 alone (observables without
+  // forces): p3mx_copy_mesh reads it there
+  bool mesh_in_eng64 = false;
   size_t n = 0;
   int ntypes = 1;
   std::vector<PairIA> table{PairIA{0, 0, 0, 0, 0, 0, 0, 0, 0, -1.0}};
@@ -234,6 +237,7 @@ void configure_engine(p3mx_handle *h) {
   h->eng->store_pair_table(h->ntypes, h->table);
   h->eng->configure({c}, static_cast<long long>(h->n));
   h->eng64.reset();
+  h->mesh_in_eng64 = false;
   if (h->elc)
     h->elc->img.reset();
 }
@@ -1102,6 +1106,7 @@ int p3mx_long_range(p3mx_handle *h, size_t n, const double *pos, const double *q
     bool const want_v = virial9 && (flags & P3MX_VIRIAL);
     bool const obs64 = h->prm.single_precision && !(flags & P3MX_MIXED_OBSERVABLES);
     e.long_range(fd, dev ? ow : true, want_e && !obs64, want_v && !obs64, st, &en, &vir);
+    h->mesh_in_eng64 = false;
     if (obs64 && (want_e || want_v))
       fp64_kspace_observables(h, st, want_e, want_v, en, vir);
     double e_elc = 0.0;
@@ -1201,6 +1206,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
         if (h->prm.epsilon != 0.)
           e.census(st);
         e.forces_all(fd, true, st);
+        h->mesh_in_eng64 = false;
         if (h->elc)
           elc_add(h, fd, nullptr, st);
       };
@@ -1218,6 +1224,7 @@ int p3mx_forces(p3mx_handle *h, size_t n, const double *pos, const double *q, co
       e.census(st);
     std::vector<double> enk, virk, ens, virs;
     bool const obs64 = h->prm.single_precision && !(flags & P3MX_MIXED_OBSERVABLES);
+    h->mesh_in_eng64 = !f && obs64 && (want_e || want_v);
     if (!want_e && !want_v) {
       e.forces_all(fd, dev ? ow : true, st, direct);
     } else if (f) {
@@ -1299,7 +1306,8 @@ int p3mx_copy_mesh(p3mx_handle *h, double *out, size_t cap) {
   return guarded(h, [&] {
     if (!h->eng)
       throw Error(P3MX_ERUNTIME, "actor not activated");
-    auto v = h->eng->mesh_copy(0, h->eng->stream());
+    Engine &e = h->mesh_in_eng64 && h->eng64 ? *h->eng64 : *h->eng;
+    auto v = e.mesh_copy(0, e.stream());
     if (cap < v.size())
       throw Error(P3MX_EDOMAIN, "output buffer too small for the mesh");
     std::memcpy(out, v.data(), v.size() * sizeof(double));
@@ -1313,6 +1321,7 @@ int p3mx_profile(p3mx_handle *h, int reps, double *ms, const char **names, int c
       throw Error(P3MX_ERUNTIME, "actor not activated");
     static std::vector<std::string> keep;
     auto prof = h->eng->profile(std::max(1, reps), h->eng->stream());
+    h->mesh_in_eng64 = false;
     if (h->elc) {
       Engine &e = *h->eng;
       auto pe = elc_profile(*h->elc, h->sys.box, h->prm.prefactor, h->r_cut,

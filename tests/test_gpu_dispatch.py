@@ -222,6 +222,18 @@ def test_observables_without_forces(cls):
                    act._handle)
         out.append(np.concatenate([e, v]))
     np.testing.assert_array_equal(out[0], out[1])
+    # ... and leaves the mesh of its own positions to p3mx_copy_mesh, as does
+    # a call with forces after it
+    prm = O.make_params(box, [32] * 3, 5, 1.2, 2.5, 1.0)
+    for k, force in enumerate((None, np.zeros((1500, 3)), None)):
+        x = np.mod(pos + 0.37 * (k + 1), box)
+        _lib.check(lib.p3mx_forces(act._handle, 1500, _lib.dptr(x), _lib.dptr(q), None,
+                                   _lib.dptr(force), e.ctypes.data_as(DP), v.ctypes.data_as(DP),
+                                   _lib.P3MX_ENERGY | _lib.P3MX_OVERWRITE, None), act._handle)
+        rho = np.zeros((32, 32, 32))
+        _lib.check(lib.p3mx_copy_mesh(act._handle, rho.ctypes.data_as(DP), rho.size), act._handle)
+        rho_o = O.p3m_kspace(prm, x, q, want_mesh=True)[3]
+        np.testing.assert_allclose(rho, rho_o, rtol=0, atol=RTOL[cls] * np.abs(rho_o).max())
 
 
 def _device_call(lib, act, fn, n, pos, q, types, f):
