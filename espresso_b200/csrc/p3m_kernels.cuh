@@ -184,7 +184,11 @@ k_p3m_place(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, in
     if (threadIdx.x == 0) {
       if (blockIdx.x == 0)
         start[nkeys] = total;
+      // the block's reads of the counts (behind the scan's barrier) come before
+      // its ticket, the last ticket before the clearing
+      __threadfence();
       s_last = atomicAdd(cnt + nkeys, 1) == static_cast<int>(gridDim.x) - 1;
+      __threadfence();
     }
     __syncthreads();
     if (s_last) // every block has read the counts
