@@ -993,7 +993,7 @@ void Engine::build_lists(cudaStream_t st) {
   k_cell_gather<<<nb, 256, 0, st>>>(geom, m_rep_of.as<int>(), m_cperm.as<int>(), m_pq.as<double4>(), d_type(), m_ckey.as<int>(),
                                     m_n, m_spq.as<double4>(), m_spf.as<float4>(), m_stype.as<int>(), m_scell.as<int>(), m_cinv.as<int>(), nullptr); ++m_launches;
   if (m_cap.size() != m_geom.size())
-    set_list_capacity(1.5);
+    set_list_capacity(1.5, st);
   int const R = n_rep();
   for (int attempt = 0; attempt < 4; ++attempt) {
     P3MX_CUDA(cudaMemsetAsync(m_overflow.p, 0, R * sizeof(int), st));
@@ -1452,7 +1452,9 @@ int Engine::list_overflow(cudaStream_t st) {
 
 // Per-replica neighbour capacity from the densest local estimate
 // margin * 4/3 pi (max_cut + skin)^3 rho + 48, never shrinking an existing one.
-void Engine::set_list_capacity(double margin) {
+// The replica records are written on st, behind the kernels that still read
+// them and ahead of the list build.
+void Engine::set_list_capacity(double margin, cudaStream_t st) {
   int const R = n_rep();
   bool changed = (static_cast<int>(m_cap.size()) != R) || m_nb.p == nullptr;
   m_cap.resize(R, 0);
@@ -1468,7 +1470,7 @@ void Engine::set_list_capacity(double margin) {
   }
   // a new layout invalidates the lists; an unchanged one keeps them
   if (changed)
-    layout_lists(m_stream);
+    layout_lists(st);
 }
 
 void Engine::layout_lists(cudaStream_t st) {
@@ -1488,7 +1490,7 @@ void Engine::ensure_lists(cudaStream_t st, double nb_margin) {
   require_configured();
   std::vector<int> before = m_cap;
   if (m_cap.size() != m_geom.size() || nb_margin > 1.0)
-    set_list_capacity(std::max(nb_margin, 1.5));
+    set_list_capacity(std::max(nb_margin, 1.5), st);
   if (m_cap != before)
     m_lists_valid = false;
   if (!m_lists_valid)

@@ -186,7 +186,7 @@ private:
   template <typename Real> void front(ParticleArrays const &in, cudaStream_t st);
   bool m_binned = false; // the mesh binning of the coming sort is done (front)
   void build_lists(cudaStream_t st);
-  void set_list_capacity(double margin);
+  void set_list_capacity(double margin, cudaStream_t st);
   void layout_lists(cudaStream_t st);
   void encode_field_maps(cudaStream_t st, int sets = 1);
   // want_spq: also the FP64 double4 positions (FP64 pair kernel)
