@@ -611,32 +611,14 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                            partials);
 }
 
-// Sum of FP32 terms in an unevaluated pair hi + lo (two-sum, Knuth: the
-// rounding error of every addition is exact and goes to lo), two sums at a
-// time: the precision of FP64 sums without six conversions and additions in
-// FP64 per pair.
-struct Sum2 {
-  f32x2 hi, lo;
-  __device__ void add(f32x2 v) {
-    f32x2 const s = add2(hi, v);
-    f32x2 const bb = sub2(s, hi);
-    f32x2 const e = add2(sub2(hi, sub2(s, bb)), sub2(v, bb));
-    hi = s;
-    lo = add2(lo, e);
-  }
-  __device__ void get(double &a, double &b) const {
-    float2 const h = up2(hi), l = up2(lo);
-    a = static_cast<double>(h.x) + static_cast<double>(l.x);
-    b = static_cast<double>(h.y) + static_cast<double>(l.y);
-  }
-};
-
 // The same pair terms for the FP32-mesh mode, in FP32 from the cell-relative
 // offsets (as k_pair_forces_rel: d = (off_a - off_b) - dc cs with dc from
 // the entry's offset code, no minimum-image arithmetic): hardware reciprocal
-// square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; each pair's force and
-// torque terms summed in FP32 pairs (Sum2), its energy in FP64.  Bound by
-// instruction issue (about 130 per entry): 131 072 dipoles 347 -> 288 us.
+// square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; the pairs' force and
+// torque terms and energies summed in FP64.  Bound by instruction issue: at
+// 131 072 dipoles 207 us (215 us with the six sums in pairs of FP32 values,
+// whose two-sums take more issue slots than the conversions and FP64 additions
+// and hold 48 bits), at 30 000 64 (69).
 template <bool EV, int LPP>
 __global__ void __launch_bounds__(256, EV ? 1 : kDpPairBlocks32)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
@@ -666,8 +648,6 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
     float const ncs_x = -static_cast<float>(G.box[0] / G.cg[0]);
     float const ncs_y = -0.25f * static_cast<float>(G.box[1] / G.cg[1]);
     float const ncs_z = -0.0625f * static_cast<float>(G.box[2] / G.cg[2]);
-    Sum2 s01{0, 0}, s23{0, 0}, s45{0, 0};
-    double ss = 0.0;
     int const cw = nb_cnt[a];
     int const ga = (nb_count_a(cw) + 7) >> 3, gt = ga + ((nb_count_b(cw) + 7) >> 3);
     const int *nbp = nb + nb_base(G.nb_off, G.max_nb, la);
@@ -723,17 +703,16 @@ k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
             energy += static_cast<double>(mimj * B - mir * mjr * Cc);
           float const cd = mimj * Cc - mir * mjr * Dd;
           float const s = mjr * Cc, q = mir * Cc;
-          s01.add(pk2(cd * d0 + q * mb.x, cd * d1 + q * mb.y));
-          s23.add(pk2(cd * d2 + q * mb.z, s * d0 - B * mb.x));
-          s45.add(pk2(s * d1 - B * mb.y, s * d2 - B * mb.z));
-          ss += static_cast<double>(s);
+          s7[0] += static_cast<double>(cd * d0 + q * mb.x);
+          s7[1] += static_cast<double>(cd * d1 + q * mb.y);
+          s7[2] += static_cast<double>(cd * d2 + q * mb.z);
+          s7[3] += static_cast<double>(s * d0 - B * mb.x);
+          s7[4] += static_cast<double>(s * d1 - B * mb.y);
+          s7[5] += static_cast<double>(s * d2 - B * mb.z);
+          s7[6] += static_cast<double>(s);
         }
       }
     }
-    s01.get(s7[0], s7[1]);
-    s23.get(s7[2], s7[3]);
-    s45.get(s7[4], s7[5]);
-    s7[6] = ss;
   }
   dp_pairs_finish<EV, LPP>(s7, ma.x, ma.y, ma.z, energy, pref, active, a, perm, f, tq, overwrite,
                            partials);
