@@ -247,6 +247,9 @@ int p3mx_launch_count(const p3mx_handle *h, long long *count);
  * to the device array out (3n floats) exp_fast(x), the single hardware
  * ex2 of x log2(e) the force-only kernel uses, and CUDA's expf(x). */
 int p3mx_exp_check(size_t n, const float *x, float *out, void *stream);
+/* The same for the FP64 pair kernels: for n device values x, the reciprocal
+ * of the erfc approximation's argument and CUDA's rsqrt(x) (2n doubles). */
+int p3mx_rcp_check(size_t n, const double *x, double *out, void *stream);
 
 /* Tuning error estimates (p3m.cpp:187-243; GPU k-space sum of
  * p3m_gpu_error_cuda.cu:87-143). */

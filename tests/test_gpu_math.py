@@ -11,6 +11,11 @@ force the kernel sums):
   2^-24 |x log2 e| ln 2 = 2^-24 |x|), so <= 2^-21 + |x| 2^-23 (1e-5 at
   x = -87, 1.2e-6 at the real-space cutoff's x ~ -10);
   CUDA's expf: <= 2 ulp (2^-22).
+
+FP64 (p3mx_rcp_check), over the arguments 1 + 0.3275911 alpha r of the erfc
+approximation and beyond: the third-order step on the hardware's FP32 reciprocal
+(PTX ISA: 1 ulp) leaves |x y - 1| <= 2^-53 (1 + 2^-8); rsqrt(x): <= 1 ulp (CUDA's
+table), and no larger than 1 / sqrt(x) rounded twice.
 """
 import numpy as np
 import pytest
@@ -54,3 +59,25 @@ def test_exponentials_at_the_ends():
     np.testing.assert_allclose(fast[:4], ref[:4], rtol=2.0 ** -20, atol=0)
     # subnormal results flush to zero, never to anything larger
     assert np.all(fast[4:] <= 1.2e-38) and np.all(fast[4:] >= 0.0)
+
+
+def test_fp64_reciprocals_over_the_pair_range():
+    rng = np.random.default_rng(7)
+    x = np.concatenate([np.linspace(1.0, 8.0, 1 << 19), np.exp(rng.uniform(0, 13.8, 1 << 18)),
+                        1.0 + np.arange(4096) * 2.0 ** -52])
+    dev = torch.device("cuda", 0)
+    xd = torch.from_numpy(x).to(dev)
+    out = torch.empty(2 * len(x), dtype=torch.float64, device=dev)
+    assert _lib.load().p3mx_rcp_check(len(x), _lib.dptr(xd), _lib.dptr(out), None) == 0
+    torch.cuda.synchronize(dev)
+    rcp, rsq = out.cpu().numpy().reshape(2, -1)
+    assert np.finfo(np.longdouble).nmant >= 63  # residuals good to 2^-63
+    xl = x.astype(np.longdouble)
+    err = np.abs(rcp.astype(np.longdouble) * xl - 1)
+    assert err.max() <= 2.0 ** -53 * (1 + 2.0 ** -8)
+    quot = 1.0 / x  # correctly rounded: the same but for near ties
+    assert np.abs(rcp - quot).max() <= np.spacing(1.0) and np.mean(rcp != quot) < 2.0 ** -7
+    ref = 1 / np.sqrt(xl)
+    ulp = lambda y: np.abs((y.astype(np.longdouble) - ref) / np.spacing(y))
+    assert ulp(rsq).max() <= 1.0
+    assert ulp(rsq).max() <= ulp(1.0 / np.sqrt(x)).max()
