@@ -936,7 +936,9 @@ __device__ inline void ev_add(double *ev, double ec, double en, double fc, doubl
 }
 
 // The FP32-mixed pair kernel with energies and virials in FP32 arithmetic
-// (P3MX_MIXED_OBSERVABLES): one thread per particle, pairs one at a time.
+// (P3MX_MIXED_OBSERVABLES, the energies of the batch): one thread per particle,
+// whole groups of entries with four gathers in flight, LJ / WCA for class A
+// groups, sums in FP64.
 __global__ void __launch_bounds__(256)
 k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                      const float4 *__restrict__ spf, const int *__restrict__ stype,
@@ -961,9 +963,9 @@ k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ 
     ev[k] = 0.0;
   if (a < G.p0 + G.np) {
     int const c = nb_cnt[a];
-    int const na = nb_count_a(c), cnt = nb_count(c);
+    int const ga = (nb_count_a(c) + 7) >> 3, gt = ga + ((nb_count_b(c) + 7) >> 3);
     float4 const pa = spf[a];
-    int const ta = stype[a];
+    int const ta = stype[a] * ntypes;
     float const rc2 = static_cast<float>(G.r_cut * G.r_cut);
     float const two_a = static_cast<float>(2.0 * G.alpha / sqrt(kPi));
     float const pref_qa = static_cast<float>(G.prefactor) * pa.w;
@@ -971,37 +973,54 @@ k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ 
     float const p_alpha = static_cast<float>(0.3275911 * G.alpha);
     double fx = 0.0, fy = 0.0, fz = 0.0;
     const int *nbp = nb + nb_base(G.nb_off, G.max_nb, a - G.p0);
-    for (int k = 0; k < cnt; ++k) {
-      unsigned const e = static_cast<unsigned>(nbp[nb_logical(0, G.max_nb, na, k)]);
-      long long const b = G.p0 + nb_index(e);
-      float4 const pb = spf[b];
-      float const d0 = fmaf(code_axis(e, 0), -cs_x, pa.x - pb.x);
-      float const d1 = fmaf(code_axis(e, 1), -0.25f * cs_y, pa.y - pb.y);
-      float const d2 = fmaf(code_axis(e, 2), -0.0625f * cs_z, pa.z - pb.z);
-      float const r2 = d0 * d0 + d1 * d1 + d2 * d2;
-      if (!(r2 > 0.f))
-        continue;
-      float const inv_d = rsqrt_approx(r2);
-      float const dist = r2 * inv_d;
-      float const ex = ex2_approx(c_exp * r2);
-      float const t = rcp_r(fmaf(p_alpha, dist, 1.f));
-      float const asp =
-          t * (0.254829592f +
-               t * (-0.284496736f + t * (1.421413741f + t * (-1.453152027f + t * 1.061405429f))));
-      float const er = asp * inv_d;
-      float const pq = pref_qa * pb.w;
-      bool const in_c = r2 < rc2;
-      float const fc = in_c ? (pq * ex) * (er + two_a) * (inv_d * inv_d) : 0.f;
-      float const ec = in_c ? pq * er * ex : 0.f;
-      float fn = 0.f, en = 0.f;
-      PairR<float> const p(ia[ta * ntypes + stype[b]]);
-      if (p.active)
-        lj_wca_sel(p, dist, inv_d, fn, en);
-      float const ft = fc + fn;
-      fx += static_cast<double>(ft * d0);
-      fy += static_cast<double>(ft * d1);
-      fz += static_cast<double>(ft * d2);
-      ev_add(ev, ec, en, fc, fn, d0, d1, d2);
+    int const ngroups = G.max_nb >> 3;
+    const float4 *pos = spf + G.p0;
+    const int *typ = stype + G.p0;
+    for (int v = 0; v < gt; ++v) {
+      bool const cls_a = v < ga;
+      int const grp = cls_a ? v : ngroups - 1 - (v - ga);
+      const int4 *gp = reinterpret_cast<const int4 *>(nbp + (static_cast<long long>(grp) << 8));
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        int4 const g = gp[h];
+        unsigned const ent[4] = {static_cast<unsigned>(g.x), static_cast<unsigned>(g.y),
+                                 static_cast<unsigned>(g.z), static_cast<unsigned>(g.w)};
+        float4 pb[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          pb[u] = pos[nb_index(ent[u])];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float const d0 = fmaf(code_axis(ent[u], 0), -cs_x, pa.x - pb[u].x);
+          float const d1 = fmaf(code_axis(ent[u], 1), -0.25f * cs_y, pa.y - pb[u].y);
+          float const d2 = fmaf(code_axis(ent[u], 2), -0.0625f * cs_z, pa.z - pb[u].z);
+          float const r2 = d0 * d0 + d1 * d1 + d2 * d2;
+          // zero distance (the list's filling): no term
+          bool const on = r2 > 0.f, in_c = on && r2 < rc2;
+          float const inv_d = rsqrt_approx(r2);
+          float const dist = r2 * inv_d;
+          float const ex = ex2_approx(c_exp * r2);
+          float const t = rcp_r(fmaf(p_alpha, dist, 1.f));
+          float const asp =
+              t * (0.254829592f +
+                   t * (-0.284496736f + t * (1.421413741f + t * (-1.453152027f + t * 1.061405429f))));
+          float const er = asp * inv_d;
+          float const pq = pref_qa * pb[u].w;
+          float const fc = in_c ? (pq * ex) * (er + two_a) * (inv_d * inv_d) : 0.f;
+          float const ec = in_c ? pq * er * ex : 0.f;
+          float fn = 0.f, en = 0.f;
+          if (cls_a && on) {
+            PairR<float> const p(ia[ta + (ntypes == 1 ? 0 : typ[nb_index(ent[u])])]);
+            if (p.active)
+              lj_wca_sel(p, dist, inv_d, fn, en);
+          }
+          float const ft = fc + fn;
+          fx += static_cast<double>(ft * d0);
+          fy += static_cast<double>(ft * d1);
+          fz += static_cast<double>(ft * d2);
+          ev_add(ev, ec, en, fc, fn, d0, d1, d2);
+        }
+      }
     }
     int const i = perm[a];
     if (overwrite) {
