@@ -81,8 +81,7 @@ public:
     m_gf.ensure(E.m_cplx * rsz);
     long long const nprep = ceil_div(nn, 256);
     size_t const np = std::max<size_t>({static_cast<size_t>(E.m_n_blk_x), 5 * static_cast<size_t>(nprep),
-                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(kDpPairBlocks64),
-                                        static_cast<size_t>(E.m_n_blk_pair) * E.pair_lanes(kDpPairBlocks32), size_t(kSumBlocks)});
+                                        static_cast<size_t>(E.m_n_blk_pair) * pair_lanes(true), size_t(kSumBlocks)});
     m_part.ensure(np * sizeof(double));
     m_sums.ensure(8 * sizeof(double));
     m_flag.ensure(sizeof(int));
@@ -302,7 +301,7 @@ public:
       int const exact = accuracy > 5e-6 ? 0 : 1;
       RepGeom const *geom = E.m_geom_d.as<RepGeom>();
       // FP32-mesh mode: the pair terms in FP32 on the cell-relative offsets
-      int const lanes = E.pair_lanes(rel ? kDpPairBlocks32 : kDpPairBlocks64);
+      int const lanes = pair_lanes(want_e);
       auto pairs = [&](auto ev, double *fo, double *part) {
         constexpr bool EV = decltype(ev)::value;
         auto go = [&](auto lpp) {
@@ -417,6 +416,12 @@ public:
   static constexpr int kSumBlocks = 296;
 
 private:
+  // lanes per particle of the pair kernel, with or without the energy
+  int pair_lanes(bool ev) const {
+    return m_eng.pair_lanes(!m_eng.fp32() ? kDpPairBlocks64
+                            : ev          ? kDpPairBlocks32Ev
+                                          : kDpPairBlocks32);
+  }
   Engine m_eng;
   DevBuf m_mu, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
   DevBuf m_tiles3, m_qmax3;

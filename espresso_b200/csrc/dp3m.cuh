@@ -20,8 +20,9 @@
 
 namespace p3mx {
 
-// Resident blocks per SM of the pair kernels (Engine::pair_lanes), FP32 and FP64.
-constexpr int kDpPairBlocks32 = 3, kDpPairBlocks64 = 2;
+// Resident blocks per SM of the pair kernels (Engine::pair_lanes): FP32, FP32 with
+// energies, FP64.
+constexpr int kDpPairBlocks32 = 3, kDpPairBlocks32Ev = 2, kDpPairBlocks64 = 2;
 
 // calc_meshift (p3m/common.hpp:248-264): index shift of the influence
 // function (M/2 -> -M/2) and of the differential operator (M/2 -> 0).
@@ -620,7 +621,7 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
 // whose two-sums take more issue slots than the conversions and FP64 additions
 // and hold 48 bits), at 30 000 64 (69).
 template <bool EV, int LPP>
-__global__ void __launch_bounds__(256, EV ? 1 : kDpPairBlocks32)
+__global__ void __launch_bounds__(256, EV ? kDpPairBlocks32Ev : kDpPairBlocks32)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
                  const float4 *__restrict__ spf, const float4 *__restrict__ smu,
                  const int *__restrict__ perm, const int *__restrict__ nb,

@@ -594,7 +594,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_flag.ensure(sizeof(int));
   m_pos_ref.ensure(3 * n * sizeof(double));
   m_type_ref.ensure(n * sizeof(int));
-  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes(kPairBlocks64) * 20 * sizeof(double));
+  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes(kPairBlocks64Ev) * 20 * sizeof(double));
   m_sums_pair.ensure(static_cast<size_t>(R) * 20 * sizeof(double));
   if (m_ia_d.p == nullptr)
     upload_vec(m_ia_d, m_ia, st);
@@ -1257,7 +1257,7 @@ int Engine::pair_lanes(int per_sm) const {
 template <typename Real>
 void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t st) {
   RepGeom const *geom = m_geom_d.as<RepGeom>();
-  constexpr int per_sm = sizeof(Real) == 4 ? kPairBlocks32 : kPairBlocks64;
+  int const per_sm = sizeof(Real) == 4 ? kPairBlocks32 : want_ev ? kPairBlocks64Ev : kPairBlocks64;
   int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes(per_sm);
   bool const chained = lanes > 1 && m_n_blk_pair * lanes <= m_sms * per_sm;
   auto go = [&](auto kern, auto const *pos, size_t smem) {
@@ -1378,7 +1378,7 @@ void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t s
     bool const one = m_fp32 && !fp64_math;
     k_reduce_partials<<<dim3(R, 20), 256, 0, st>>>(m_part_pair.as<double>(), 20,
                                                    m_blk_pair_start_d.as<int>(),
-                                                   one ? 1 : pair_lanes(kPairBlocks64),
+                                                   one ? 1 : pair_lanes(kPairBlocks64Ev),
                                                    m_sums_pair.as<double>()); ++m_launches;
     std::vector<double> sums(static_cast<size_t>(R) * 20);
     P3MX_CUDA(cudaMemcpyAsync(sums.data(), m_sums_pair.p, sums.size() * sizeof(double),

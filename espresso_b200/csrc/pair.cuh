@@ -679,8 +679,9 @@ __device__ inline PairF pair_f(PairIA const &p) {
 // (parameters in registers, the LJ powers from the Coulomb term's 1/r^2),
 // several types without offsets, LJ offsets.
 constexpr int kPairOneType = 0, kPairTypes = 1, kPairOffset = 2;
-// Resident blocks per SM of the force kernels (Engine::pair_lanes), FP32 and FP64.
-constexpr int kPairBlocks32 = 4, kPairBlocks64 = 2;
+// Resident blocks per SM (Engine::pair_lanes) of the force kernels, FP32 and FP64,
+// and of the FP64 kernel with energies and virials (174 registers).
+constexpr int kPairBlocks32 = 4, kPairBlocks64 = 2, kPairBlocks64Ev = 1;
 
 // Force kernel of the FP32-mixed path over the Verlet list: real-space Coulomb
 // (CoulombP3M::pair_force, p3m.hpp:146-180) plus LJ and WCA (lj.hpp:41-60,
@@ -1047,7 +1048,7 @@ k_pair_forces_rel_ev(const RepGeom *__restrict__ reps, const int2 *__restrict__ 
 // a pair's chain (rsqrt, exp, polynomial) is long and two blocks per SM do not
 // hide it (131 072 ions 234 -> 187 us).
 template <bool EV, int LPP>
-__global__ void __launch_bounds__(256, EV ? 1 : kPairBlocks64)
+__global__ void __launch_bounds__(256, EV ? kPairBlocks64Ev : kPairBlocks64)
 k_pair_forces(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
               const double4 *__restrict__ spq, const int *__restrict__ stype,
               const int *__restrict__ perm, const PairIA *__restrict__ ia_g, int ntypes,
