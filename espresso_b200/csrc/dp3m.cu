@@ -420,7 +420,8 @@ private:
   int pair_lanes(bool ev) const {
     return m_eng.pair_lanes(!m_eng.fp32() ? kDpPairBlocks64
                             : ev          ? kDpPairBlocks32Ev
-                                          : kDpPairBlocks32);
+                                          : kDpPairBlocks32,
+                            kPairTailLong);
   }
   Engine m_eng;
   DevBuf m_mu, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;

@@ -594,7 +594,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_flag.ensure(sizeof(int));
   m_pos_ref.ensure(3 * n * sizeof(double));
   m_type_ref.ensure(n * sizeof(int));
-  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes(kPairBlocks64Ev) * 20 * sizeof(double));
+  m_part_pair.ensure(static_cast<size_t>(m_n_blk_pair) * pair_lanes(kPairBlocks64Ev, kPairTail) * 20 * sizeof(double));
   m_sums_pair.ensure(static_cast<size_t>(R) * 20 * sizeof(double));
   if (m_ia_d.p == nullptr)
     upload_vec(m_ia_d, m_ia, st);
@@ -1239,26 +1239,42 @@ void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp,
 
 // Lanes per particle of the pair kernels (1, 2, 4 or 8, whole groups of 8 list
 // entries each), for `per_sm` resident blocks per SM: the most with which all
-// blocks are resident at once; two where the blocks are more than one but less
-// than 1.7 waves (the second wave would cost as much as a full one).  Kernel
-// times in us at 1 / 2 / 4 / 8 lanes, those chosen in brackets: FP32 23 457 ions
-// 33 / 25 / [22] / 26, 98 304 ions [37] / 39 / 41 / 53, 131 072 ions [52] / 53 / 62
-// / 79, 250 000 ions in a dense melt 142 / [126] / 139 / 180, 2^20 ions [240] / 265
-// / 335 / 456; FP64 131 072 ions [187] / 196 / 203 / 243; dipoles 16 384 FP64 197
-// / 108 / [71] / 80, 131 072 FP32 352 / [288] / 281 / 310.
-int Engine::pair_lanes(int per_sm) const {
+// blocks are resident at once; two where the blocks are more than one wave and
+// at most tail / 10 waves.  With two lanes a wave costs half as much, so up to 1.5
+// waves three of them replace two whole ones; up to 2 waves four replace two, which
+// pays only for the kernels with the longer chains per entry (kPairTail,
+// kPairTailLong), by the shorter last wave.  Kernel times in us at 1 / 2 lanes:
+//   waves                       1.05       1.3       1.5       1.65       1.8       2.0
+//   FP32 ions, one type       62 / 57   67 / 64   72 / 72   75 / 81   84 / 85   85 / 93
+//   ... density 0.85         119 /100  127 /112  136 /124  141 /141  156 /150  160 /161
+//   FP64 ions                124 /106  124 /117  134 /123  146 /151  148 /163  151 /167
+//   ... with energies        116 / 98  118 /100  119 /102  119 /131  119 /132  121 /136
+//   FP32 ions, two types      66 / 60   74 / 67     -       88 / 84   93 / 89   96 / 97
+//   ... density 0.85         129 /102  140 /114     -      163 /143  174 /152  180 /164
+//   dipoles FP32             254 /212  263 /233  291 /261  294 /290  337 /311  340 /340
+//   dipoles FP64             394 /314  407 /344  457 /354  458 /429  459 /455  465 /470
+// Below one wave, at 1 / 2 / 4 / 8 lanes, those chosen in brackets: FP32 23 457 ions
+// 33 / 25 / [22] / 26, 98 304 ions [37] / 39 / 41 / 53; 16 384 dipoles FP64 197 / 108
+// / [71] / 80; above two waves: FP32 2^20 ions [240] / 265 / 335 / 456.
+int Engine::pair_lanes(int per_sm, int tail) const {
   long long const room = static_cast<long long>(m_sms) * per_sm, blocks = m_n_blk_pair;
   int l = 1;
   while (l < 8 && 2 * l * blocks <= room)
     l *= 2;
-  return blocks > room && 10 * blocks < 17 * room ? 2 : l;
+  return blocks > room && 10 * blocks <= tail * room ? 2 : l;
 }
 
 template <typename Real>
 void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t st) {
   RepGeom const *geom = m_geom_d.as<RepGeom>();
   int const per_sm = sizeof(Real) == 4 ? kPairBlocks32 : want_ev ? kPairBlocks64Ev : kPairBlocks64;
-  int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes(per_sm);
+  // FP32 parameter mode (kPairOneType, ...)
+  bool offset = false;
+  for (auto const &p : m_ia)
+    offset = offset || (p.ia_cut != -1.0 && p.lj_offset != 0.0);
+  int const mode_f = offset ? kPairOffset : m_ntypes == 1 ? kPairOneType : kPairTypes;
+  int const tail = sizeof(Real) == 4 && mode_f != kPairOneType ? kPairTailLong : kPairTail;
+  int const lanes = want_ev && sizeof(Real) == 4 ? 1 : pair_lanes(per_sm, tail);
   bool const chained = lanes > 1 && m_n_blk_pair * lanes <= m_sms * per_sm;
   auto go = [&](auto kern, auto const *pos, size_t smem) {
     // not chained where the launch fills the GPU: its blocks would start in
@@ -1278,9 +1294,6 @@ void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t s
       go(k_pair_forces_rel_ev, pos, nt2 * sizeof(PairIA));
       return;
     }
-    bool offset = false;
-    for (auto const &p : m_ia)
-      offset = offset || (p.ia_cut != -1.0 && p.lj_offset != 0.0);
     size_t const smem = nt2 * sizeof(PairF);
     auto mode = [&](auto m) {
       constexpr int M = decltype(m)::value;
@@ -1291,12 +1304,11 @@ void Engine::launch_pair(double *f, bool overwrite, bool want_ev, cudaStream_t s
       default: go(k_pair_forces_rel<M, 8>, pos, smem); break;
       }
     };
-    if (offset)
-      mode(std::integral_constant<int, kPairOffset>{});
-    else if (m_ntypes == 1)
-      mode(std::integral_constant<int, kPairOneType>{});
-    else
-      mode(std::integral_constant<int, kPairTypes>{});
+    switch (mode_f) {
+    case kPairOffset: mode(std::integral_constant<int, kPairOffset>{}); break;
+    case kPairOneType: mode(std::integral_constant<int, kPairOneType>{}); break;
+    default: mode(std::integral_constant<int, kPairTypes>{}); break;
+    }
   } else {
     // FP64: FP64 geometry (minimum image on absolute positions)
     const double4 *pos = m_spq.as<double4>();
@@ -1378,7 +1390,7 @@ void Engine::short_range(double *f, bool overwrite, bool want_ev, cudaStream_t s
     bool const one = m_fp32 && !fp64_math;
     k_reduce_partials<<<dim3(R, 20), 256, 0, st>>>(m_part_pair.as<double>(), 20,
                                                    m_blk_pair_start_d.as<int>(),
-                                                   one ? 1 : pair_lanes(kPairBlocks64Ev),
+                                                   one ? 1 : pair_lanes(kPairBlocks64Ev, kPairTail),
                                                    m_sums_pair.as<double>()); ++m_launches;
     std::vector<double> sums(static_cast<size_t>(R) * 20);
     P3MX_CUDA(cudaMemcpyAsync(sums.data(), m_sums_pair.p, sums.size() * sizeof(double),

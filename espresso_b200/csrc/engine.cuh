@@ -202,7 +202,7 @@ private:
   void mark(const char *name, cudaStream_t st);
 
   // lanes per particle of the pair kernels for the current particle number
-  int pair_lanes(int per_sm) const;
+  int pair_lanes(int per_sm, int tail) const;
 
   bool m_fp32;
   bool m_configured = false;

@@ -682,6 +682,9 @@ constexpr int kPairOneType = 0, kPairTypes = 1, kPairOffset = 2;
 // Resident blocks per SM (Engine::pair_lanes) of the force kernels, FP32 and FP64,
 // and of the FP64 kernel with energies and virials (174 registers).
 constexpr int kPairBlocks32 = 4, kPairBlocks64 = 2, kPairBlocks64Ev = 1;
+// Tenths of waves up to which two lanes per particle replace one
+// (Engine::pair_lanes): one particle type and FP64; several types and dipoles.
+constexpr int kPairTail = 15, kPairTailLong = 18;
 
 // Force kernel of the FP32-mixed path over the Verlet list: real-space Coulomb
 // (CoulombP3M::pair_force, p3m.hpp:146-180) plus LJ and WCA (lj.hpp:41-60,
