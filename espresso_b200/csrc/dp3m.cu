@@ -33,7 +33,7 @@ namespace p3mx {
 
 class Dp3mEngine {
 public:
-  explicit Dp3mEngine(bool fp32) : m_eng(fp32) {}
+  explicit Dp3mEngine(bool fp32) : m_eng(fp32) { m_eng.set_field_sets(3, kDipoleSpectra); }
 
   Engine &engine() { return m_eng; }
   long long n() const { return m_eng.n_part(); }
@@ -68,15 +68,11 @@ public:
     cudaStream_t const st = m_eng.stream();
     Engine &E = m_eng;
     size_t const rsz = E.fp32() ? sizeof(float) : sizeof(double);
-    size_t const csz = 2 * rsz;
     long long const nn = std::max<long long>(1, n);
     m_mu.ensure(3 * nn * sizeof(double));
     m_out.ensure(9 * nn * sizeof(double));
     m_smu.ensure(nn * sizeof(double4));
-    m_ck3.ensure(3 * E.m_cplx * csz);
     m_ge.ensure(E.m_cplx * rsz);
-    // three tile sets for the one-launch assignment
-    m_tiles3.ensure(3 * static_cast<size_t>(E.m_tiles_n) * rsz);
     m_qmax3.ensure(4 * sizeof(unsigned));
     m_gf.ensure(E.m_cplx * rsz);
     long long const nprep = ceil_div(nn, 256);
@@ -116,10 +112,6 @@ public:
       attrs(0.0f);
     else
       attrs(0.0);
-    // the field spectra and three field meshes
-    E.m_field.ensure(kDipoleSpectra * E.m_cplx * csz);
-    E.m_E.ensure(3 * 4 * E.m_ebins * rsz);
-    E.encode_field_maps(st, 3);
     m_g_valid = false;
     m_phi_valid = false;
     m_M = M;
@@ -178,7 +170,7 @@ public:
     E.mark("dp_sort", st);
     // 2. the three component meshes: one assignment and one z pass over all
     // three (blockIdx.y = component)
-    C *ck3 = m_ck3.as<C>();
+    C *ck3 = E.m_ck.as<C>();
     for (int c = 1; c <= 7; ++c) {
       int const cnt = E.m_sb_off[c + 1] - E.m_sb_off[c];
       if (cnt == 0)
@@ -186,11 +178,11 @@ public:
       int2 const *tab = E.m_blk_mesh.as<int2>() + E.m_sb_off[c];
       P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(E.m_sb_edge, cnt, st, geom, tab,
                                                      E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(),
-                                                     qmax3, m_tiles3.as<Real>(), E.kerr(), 3,
+                                                     qmax3, E.m_tiles.as<Real>(), E.kerr(), 3,
                                                      E.m_tiles_n, 1)));
       ++E.m_launches;
     }
-    E.launch_fft_z_fwd<Real>(m_tiles3.as<Real>(), ck3, 3, st);
+    E.launch_fft_z_fwd<Real>(E.m_tiles.as<Real>(), ck3, 3, st);
     E.mark("dp_assign_fft_z", st);
     E.launch_fft_y<Real>(ck3, E.m_cplx, y_plain(3), false, 0, st);
     E.mark("dp_fft_y", st);
@@ -424,8 +416,8 @@ private:
                             kPairTailLong);
   }
   Engine m_eng;
-  DevBuf m_mu, m_out, m_smu, m_ck3, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
-  DevBuf m_tiles3, m_qmax3;
+  DevBuf m_mu, m_out, m_smu, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
+  DevBuf m_qmax3;
   bool m_configured = false;
   bool m_g_valid = false, m_phi_valid = false, m_table_set = false;
   double m_phi = 0.0;

@@ -564,11 +564,11 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_scan_tiles.ensure((ceil_div(std::max(m_nkeys, m_oct_mult * m_cells) + 1, kScanTile) + 1) * sizeof(int));
   m_dist.ensure(3 * n * rsz);
   m_rec.ensure(n * (m_fp32 ? sizeof(PRec<float>) : sizeof(PRec<double>)));
-  m_tiles.ensure(static_cast<size_t>(m_tiles_n) * rsz);
-  m_E.ensure(4 * m_ebins * rsz);
+  m_tiles.ensure(m_sets * static_cast<size_t>(m_tiles_n) * rsz);
+  m_E.ensure(m_sets * 4 * m_ebins * rsz);
   encode_field_maps(st);
-  m_ck.ensure(m_cplx * csz);
-  m_field.ensure(kChargeSpectra * m_cplx * csz);
+  m_ck.ensure(m_sets * m_cplx * csz);
+  m_field.ensure(m_spectra * m_cplx * csz);
   m_ginf.ensure(m_cplx * rsz);
   m_part_x.ensure(static_cast<size_t>(m_n_blk_x) * 8 * sizeof(double));
   m_sums_x.ensure(static_cast<size_t>(R) * 8 * sizeof(double));
@@ -768,13 +768,13 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // One tensor map per replica over its packed, ghost-padded field mesh E (4
 // values per point): dims (4 E2, E1, E0) with E = epad, box (4 Ed, Ed, Ed)
-// with Ed = brick + cao - 1 (<= epad by construction); `sets` field meshes
+// with Ed = brick + cao - 1 (<= epad by construction); m_sets field meshes
 // m_ebins records apart.
-void Engine::encode_field_maps(cudaStream_t st, int sets) {
+void Engine::encode_field_maps(cudaStream_t st) {
   auto enc = tensor_map_encoder();
   size_t const es = m_fp32 ? sizeof(float) : sizeof(double);
   size_t const R = m_geom.size();
-  std::vector<CUtensorMap> maps(sets * R);
+  std::vector<CUtensorMap> maps(m_sets * R);
   for (size_t m = 0; m < maps.size(); ++m) {
     size_t const set = m / R;
     RepGeom const &G = m_geom[m - set * R];

@@ -82,6 +82,12 @@ public:
   ReplicaConf const &conf(int r) const { return m_conf[r]; }
   cudaStream_t stream() const { return m_stream; }
 
+  // Charge sets (tiles, spectra and field meshes) and field spectra that
+  // configure() allocates: one and kChargeSpectra, or a dipolar engine's.
+  void set_field_sets(int sets, int spectra) {
+    m_sets = sets;
+    m_spectra = spectra;
+  }
   // (Re)builds geometry, plans, block tables; allocates the buffers.
   void configure(std::vector<ReplicaConf> const &conf, long long n_total);
   // False until the first configuration and after one that threw: every other
@@ -188,7 +194,7 @@ private:
   void build_lists(cudaStream_t st);
   void set_list_capacity(double margin, cudaStream_t st);
   void layout_lists(cudaStream_t st);
-  void encode_field_maps(cudaStream_t st, int sets = 1);
+  void encode_field_maps(cudaStream_t st);
   // want_spq: also the FP64 double4 positions (FP64 pair kernel)
   void refresh_sorted_positions(cudaStream_t st, bool want_spq = true);
   // Counting sort by key (perm: sorted position -> particle), each bucket
@@ -206,6 +212,7 @@ private:
 
   bool m_fp32;
   bool m_configured = false;
+  int m_sets = 1, m_spectra = kChargeSpectra;
   int m_device = 0, m_sms = 148;
   cudaStream_t m_stream = nullptr;
   long long m_launches = 0;
