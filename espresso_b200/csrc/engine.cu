@@ -441,7 +441,10 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       // whole one)
       AxisPlan const &pz = G.plan[2];
       bool const two = m_kind[2] != kFftAny;
+      // (of 228 KB; beside it a block of the forward pass holds 4.9 KB of static
+      // arrays, of the backward pass 1 KB, and 1 KB is reserved per block)
       size_t const z_budget = m_fp32 ? 54 * 1024 : 100 * 1024;
+      size_t const zf_budget = m_fp32 ? 50 * 1024 : z_budget;
       int const want = two ? 256 / std::min(pz.n1, pz.n2) : 256;
       long long const slots = static_cast<long long>(m_fp32 ? kFftBlocks<float> : kFftBlocks<double>) * sms;
       auto const fill = [&](int most) {
@@ -454,7 +457,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
       };
       // forward: two real lines per complex transform
       int lz = 2;
-      while (lz / 2 < want && lz + 2 <= kZfLines && zf_smem(lz / 2 + 1) <= z_budget)
+      while (lz / 2 < want && lz + 2 <= kZfLines && zf_smem(lz / 2 + 1) <= zf_budget)
         lz += 2;
       lz = fill(lz);
       for (int l = 0; l < lines; l += lz)
