@@ -77,10 +77,9 @@ struct RepGeom {
   int hp;  // padded length of the r2c axis (>= mesh[2]/2+1, multiple of 4)
   int cao;
   long long p0, np;  // particle range
-  long long rm_off;  // real mesh offset (elements)
   long long tl_off;  // assignment tile offset (elements)
   int sbn[3];        // super-bricks of the charge assignment per dimension
-  int cov_off[3];    // per axis: its cover table (see cover_entry)
+  int cov_off[3];    // per axis: its cover table (cover_table)
   long long re_off;  // field mesh offset (records of 4 values)
   int epad[3];       // field mesh extent: mesh plus high-side ghost layers
   long long brk_off; // brick (sort key) offset

@@ -242,7 +242,6 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     m_ncorner += static_cast<long long>(G.nbx) * G.nby * G.nbz * G.brick * G.brick * G.brick;
     G.brk_off = m_nkeys;
     m_nkeys += static_cast<long long>(G.nbx) * G.nby * G.nbz;
-    G.rm_off = m_bins;
     G.km_off = m_cplx;
     // field mesh: ghost layers (periodic images) on the high side, so that
     // the interpolation tile of every brick (brick + cao - 1 points from the

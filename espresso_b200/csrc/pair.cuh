@@ -471,15 +471,6 @@ k_verlet_build(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of_
                    s_group_b + threadIdx.x * 8);
 }
 
-// A&S 7.1.26 approximation of exp(d^2) erfc(d), as the reference's real-
-// space kernel uses it (utils/math/AS_erfc_part.hpp:29-40).
-template <typename Real> __device__ inline Real as_erfc_part(Real d) {
-  Real const a1 = Real(0.254829592), a2 = Real(-0.284496736), a3 = Real(1.421413741),
-             a4 = Real(-1.453152027), a5 = Real(1.061405429), p = Real(0.3275911);
-  Real const t = Real(1) / (Real(1) + p * d);
-  return t * (a1 + t * (a2 + t * (a3 + t * (a4 + t * a5))));
-}
-
 // FP32 exp(x) for the real-space kernel (x = -(alpha r)^2 in [-88, 0]):
 // e^x = 2^y with y = x log2(e) split error-free into y_hi + y_lo (the FMA
 // residual of the product, Dekker's TwoProduct, plus the low part of the
@@ -495,16 +486,10 @@ __device__ inline float exp_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(y_hi));
   return fmaf(e, y_lo * 0.693147180559945309f, e);
 }
-template <typename Real> __device__ inline Real exp_r(Real x);
-template <> __device__ inline float exp_r<float>(float x) { return exp_fast(x); }
-template <> __device__ inline double exp_r<double>(double x) { return exp(x); }
-template <typename Real> __device__ inline Real sqrt_r(Real x);
-template <> __device__ inline float sqrt_r<float>(float x) { return sqrtf(x); }
-template <> __device__ inline double sqrt_r<double>(double x) { return sqrt(x); }
 
-// Reciprocal / reciprocal square root in the working precision: FP32 uses
-// the hardware approximations (~1 ulp; the FP32-mixed path tolerates
-// ulp-level differences); FP64 keeps IEEE division and sqrt.
+// Reciprocal in the working precision: FP32 uses the hardware approximation
+// (~1 ulp; the FP32-mixed path tolerates ulp-level differences); FP64 keeps the
+// IEEE division.
 template <typename Real> __device__ inline Real rcp_r(Real x);
 template <> __device__ inline float rcp_r<float>(float x) {
   float r;
@@ -512,9 +497,6 @@ template <> __device__ inline float rcp_r<float>(float x) {
   return r;
 }
 template <> __device__ inline double rcp_r<double>(double x) { return 1.0 / x; }
-template <typename Real> __device__ inline Real rsqrt_r(Real x);
-template <> __device__ inline float rsqrt_r<float>(float x) { return rsqrtf(x); }
-template <> __device__ inline double rsqrt_r<double>(double x) { return 1.0 / sqrt(x); }
 
 // LJ/WCA parameters of one type pair in the working precision.
 template <typename Real> struct PairR {
