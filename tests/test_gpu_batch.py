@@ -279,3 +279,35 @@ def test_batch_bonds_in_the_graph_step_match_oracle():
             assert abs(en[r] - e_ref) <= 1e-4 * (abs(e_ref) + np.abs(ek) + 1.0)
     finally:
         lib.p3mx_batch_destroy(h)
+
+
+def test_get_of_many_chunks():
+    """p3mx_batch_get copies through a ring of four 1 MB chunks: 80 000 particles'
+    three arrays (5.8 MB) wrap it, each array alone (1.9 MB) does not."""
+    lib = _lib.load()
+    rng = np.random.default_rng(11)
+    n, edge = 40000, (40000 / 0.3) ** (1 / 3)
+    side = int(np.ceil(n ** (1 / 3)))
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = np.vstack([(grid[rng.choice(len(grid), n, replace=False)] + 0.5) * (edge / side)
+                     for _ in range(2)])
+    q = np.where(np.arange(2 * n) % 2 == 0, 1.0, -1.0)
+    h = create([[edge] * 3] * 2, [1.0, 1.0], pos, q, [0, n, 2 * n], acc=0.1, cao=(5, 5))
+    try:
+        _lib.check(lib.p3mx_batch_run(h, 3, 0.01, 1.0, 1.0, 3), h, lib.p3mx_batch_last_error)
+        ptr = lambda a: None if a is None else a.ctypes.data_as(_P(ctypes.c_double))
+        one = []
+        for k in range(3):
+            a = [None] * 3
+            a[k] = np.full((2 * n, 3), np.nan)
+            _lib.check(lib.p3mx_batch_get(h, *map(ptr, a)), h, lib.p3mx_batch_last_error)
+            one.append(a[k])
+        both = [np.full((2 * n, 3), np.nan) for _ in range(3)]
+        _lib.check(lib.p3mx_batch_get(h, *map(ptr, both)), h, lib.p3mx_batch_last_error)
+        for x, y in zip(one, both):
+            np.testing.assert_array_equal(x, y)
+        # positions within a few steps of the start, velocities drawn
+        assert np.abs(both[0] - pos).max() < 0.5 and np.abs(both[2]).max() > 0
+        assert not np.isnan(both[1]).any()
+    finally:
+        lib.p3mx_batch_destroy(h)

@@ -84,10 +84,28 @@ def test_long_range_meshes(cls, mesh, cao):
     np.testing.assert_allclose(v, vo, rtol=0, atol=1e-9 * np.abs(vo).max())
 
 
+def _near(pos, box, types, cuts):
+    """Particles of pairs within FP32 rounding of a cutoff ({(type, type): r},
+    or {None: r} for every pair): such a pair may fall on either side."""
+    out = np.zeros(len(pos), bool)
+    tree = cKDTree(np.mod(pos, box), boxsize=box)
+    for kind, cut in cuts.items():
+        i, j = tree.query_pairs(cut + 1e-6, output_type="ndarray").T
+        if kind is not None:
+            sel = np.isin(types[i], kind) & np.isin(types[j], kind) & (types[i] != types[j])
+            i, j = i[sel], j[sel]
+        d = pos[i] - pos[j]
+        d -= box * np.rint(d / box)
+        sel = np.sqrt((d * d).sum(1)) > cut - 1e-6
+        out[i[sel]] = out[j[sel]] = True
+    return out
+
+
 # particle numbers for 8, 4, 2 and 1 lanes per particle of the pair kernels, in
-# either precision, and for 2 lanes above a wave of blocks
+# either precision, with and without energies, and for 2 lanes above a wave of
+# blocks
 @pytest.mark.parametrize("cls", [P3M, P3MGPU])
-@pytest.mark.parametrize("n", [3001, 15000, 30000, 60000, 116001, 160001])
+@pytest.mark.parametrize("n", [3001, 15000, 30000, 45000, 60000, 100001, 116001, 160001])
 @pytest.mark.parametrize("form", ["wca", "types", "offset"])
 def test_pair_lanes_and_types(cls, n, form):
     box = np.full(3, (n / 0.4) ** (1.0 / 3.0))
@@ -98,11 +116,11 @@ def test_pair_lanes_and_types(cls, n, form):
     s = eb.System(box_l=box)
     s.time_step = 0.01
     s.part.add(pos=pos, q=q, type=types)
+    off = 0.2 if form == "offset" else 0.0
     if form == "wca":
         pairs = {(0, 0): dict(wca_eps=1.0, wca_sig=1.0)}
         s.non_bonded_inter[0, 0].wca.set_params(epsilon=1.0, sigma=1.0)
     else:
-        off = 0.2 if form == "offset" else 0.0
         lj = dict(lj_eps=1.3, lj_sig=0.9, lj_cut=2.0, lj_shift=0.1, lj_offset=off)
         pairs = {(0, 0): dict(wca_eps=1.0, wca_sig=1.0), (0, 1): lj}  # (1, 1): none
         s.non_bonded_inter[0, 0].wca.set_params(epsilon=1.0, sigma=1.0)
@@ -113,35 +131,33 @@ def test_pair_lanes_and_types(cls, n, form):
     act = s.electrostatics.solver
     s._sync_pairs(act._handle, types)
     lib = _lib.load()
-    f = np.zeros((n, 3))
-    e, v = np.zeros(2), np.zeros(18)
-    flags = _lib.P3MX_FORCES | _lib.P3MX_ENERGY | _lib.P3MX_VIRIAL | _lib.P3MX_OVERWRITE
-    _lib.check(lib.p3mx_short_range(act._handle, n, _lib.dptr(pos), _lib.dptr(q), _lib.dptr(types),
-                                    _lib.dptr(f), e.ctypes.data_as(DP), v.ctypes.data_as(DP),
-                                    flags, None), act._handle)
     prm = O.make_params(box, [32] * 3, 3, 1.1, 2.4, 1.5)
     nt = 1 + int(types.max())
     fo, eo, vc, vn = O.short_range(prm, pos, q, types, nt, O.pair_table(nt, pairs))
     scale = np.abs(fo).max()
-    # a pair within FP32 rounding of the LJ cutoff changes two particles by the
-    # force there (0.06 at 2.0): counted apart
-    bad = np.abs(f - fo).max(1) > RTOL[cls] * scale
-    # ... and so does a pair within FP32 rounding of the Coulomb cutoff, by 7.8e-4
-    # = 1.5 (erfc(1.1 r) / r^2 + 2.2 / sqrt(pi) exp(-(1.1 r)^2) / r) at r = 2.4,
-    # above the tolerance where the largest force is below 39
-    flips = 0
+    # FP32: a pair within rounding of the LJ cutoff changes two particles by the
+    # force there (0.06 at 2.0), one at the Coulomb cutoff by 7.8e-4 = 1.5
+    # (erfc(1.1 r) / r^2 + 2.2 / sqrt(pi) exp(-(1.1 r)^2) / r) at r = 2.4; any other
+    # particle agrees
+    near = np.zeros(n, bool)
     if cls is P3MGPU:
-        tree = cKDTree(np.mod(pos, box), boxsize=box)
-        near = tree.query_pairs(2.4 + 1e-6, output_type="ndarray")
-        d = pos[near[:, 0]] - pos[near[:, 1]]
-        d -= box * np.rint(d / box)
-        flips = int((np.sqrt((d * d).sum(1)) > 2.4 - 1e-6).sum())
-        flips += 0 if form == "wca" else 1 + n // 20000
-    assert bad.sum() <= 2 * flips
-    assert np.abs(f - fo).max() <= max(RTOL[cls] * scale, 0.1 if bad.any() else 0.0)
-    np.testing.assert_allclose(e, eo, rtol=1e-9, atol=1e-9 * n)
-    np.testing.assert_allclose(v.reshape(2, 3, 3), [vc, vn], rtol=0,
-                               atol=1e-9 * max(np.abs(vc).max(), np.abs(vn).max()))
+        near = _near(pos, box, types, {None: 2.4} if form == "wca" else
+                     {None: 2.4, (0, 1): 2.0 + off})
+    # with energies and virials, and the instances without
+    for flags in (_lib.P3MX_FORCES | _lib.P3MX_ENERGY | _lib.P3MX_VIRIAL, _lib.P3MX_FORCES):
+        f = np.zeros((n, 3))
+        e, v = np.zeros(2), np.zeros(18)
+        _lib.check(lib.p3mx_short_range(act._handle, n, _lib.dptr(pos), _lib.dptr(q),
+                                        _lib.dptr(types), _lib.dptr(f), e.ctypes.data_as(DP),
+                                        v.ctypes.data_as(DP), flags | _lib.P3MX_OVERWRITE, None),
+                   act._handle)
+        d = np.abs(f - fo).max(1)
+        assert d[~near].max() <= RTOL[cls] * scale
+        assert d.max() <= max(RTOL[cls] * scale, 0.1 if near.any() else 0.0)
+        if flags & _lib.P3MX_ENERGY:
+            np.testing.assert_allclose(e, eo, rtol=1e-9, atol=1e-9 * n)
+            np.testing.assert_allclose(v.reshape(2, 3, 3), [vc, vn], rtol=0,
+                                       atol=1e-9 * max(np.abs(vc).max(), np.abs(vn).max()))
 
 
 # dipolar pair lanes: a 2x2x2 supercell (twice the mesh) gives every copy of a
@@ -160,7 +176,16 @@ def test_dipole_supercell(single, tol, n, mesh):
                          tune=False, single_precision=single)
         act._set_system([length] * 3, 0.4, (True, True, True))
         act._activate(x, m)
-        return act._compute(x, m, forces=True, energy=True)
+        f, t, e = np.zeros_like(x), np.zeros_like(x), np.zeros(2)
+        flags = _lib.P3MX_FORCES | _lib.P3MX_ENERGY | _lib.P3MX_OVERWRITE
+        act._check(_lib.load().p3mx_dp3m_compute(act._handle, len(x), _lib.dptr(x), _lib.dptr(m),
+                                                 _lib.dptr(f), _lib.dptr(t), e.ctypes.data_as(DP),
+                                                 flags, None))
+        # the instances without the energy
+        f2, t2, _ = act._compute(x, m)
+        np.testing.assert_allclose(f2, f, rtol=0, atol=tol * np.abs(f).max())
+        np.testing.assert_allclose(t2, t, rtol=0, atol=tol * np.abs(t).max())
+        return f, t, e
     f1, t1, e1 = compute(pos, mu, edge, mesh)
     shifts = np.stack(np.meshgrid(*[[0, edge]] * 3, indexing="ij"), -1).reshape(-1, 3)
     big = np.concatenate([pos + s for s in shifts])
@@ -169,6 +194,10 @@ def test_dipole_supercell(single, tol, n, mesh):
                                atol=tol * np.abs(f1).max())
     np.testing.assert_allclose(t8.reshape(8, n, 3), np.broadcast_to(t1, (8, n, 3)), rtol=0,
                                atol=tol * np.abs(t1).max())
+    # the real-space energy is the sum over the copies.  A dipole's part is of order
+    # 1 and of either sign, its error below tol and independent of the others': the
+    # sum over 8 n dipoles is of order sqrt(8 n), its error below tol 8 sqrt(8 n)
+    assert abs(e8[1] - 8 * e1[1]) <= tol * 8 * np.sqrt(8 * n)
 
 
 @pytest.mark.parametrize("cls", [P3M, P3MGPU])
@@ -298,3 +327,49 @@ def test_long_z_axis(cls, mz, energy):
     np.testing.assert_allclose(f, fo, rtol=0, atol=RTOL[cls] * np.abs(fo).max())
     if energy:
         assert abs(e[0] - eo) <= 1e-9 * (abs(eo) + (q * q).sum() * 0.9)
+
+
+@pytest.mark.parametrize("cls", [P3M, P3MGPU])
+def test_device_arrays_on_a_stream(cls):
+    """Device arrays on the caller's stream, staged by the first kernel: small
+    moves, moves beyond skin / 2, other types and other charges between calls give
+    bitwise the forces of the host-array calls."""
+    n, box = 4001, np.full(3, 20.0)
+    pos, q = _ions(n, box, seed=8)
+    q[-1] = 0.0
+    rng = np.random.default_rng(8)
+    types = (np.arange(n) % 2).astype(np.int32)
+    lib = _lib.load()
+    tab = (_lib.PairParams * 4)()
+    tab[0].wca_eps = tab[0].wca_sig = 1.0
+    tab[1].lj_eps, tab[1].lj_sig, tab[1].lj_cut = 1.0, 0.9, 2.2
+    tab[2] = tab[1]
+    acts = []
+    for _ in range(2):
+        act = _actor(cls, box, pos, q, [40] * 3, 5, alpha=1.1, r_cut=2.6)
+        _lib.check(lib.p3mx_set_pair_params(act._handle, 2, tab), act._handle)
+        acts.append(act)
+    stream = torch.cuda.Stream()
+    flags = _lib.P3MX_FORCES | _lib.P3MX_OVERWRITE
+    f_dev = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for step in range(6):
+        if step in (1, 3):
+            pos = pos + rng.uniform(-0.05, 0.05, pos.shape)
+        elif step == 2:
+            pos = pos + rng.uniform(-0.5, 0.5, pos.shape)
+        elif step == 4:
+            types = 1 - types
+        elif step == 5:
+            q = np.roll(q, 7)  # another particle is the neutral one
+        f = np.zeros((n, 3))
+        _lib.check(lib.p3mx_forces(acts[0]._handle, n, _lib.dptr(pos), _lib.dptr(q),
+                                   _lib.dptr(types), _lib.dptr(f), None, None, flags, None),
+                   acts[0]._handle)
+        with torch.cuda.stream(stream):
+            d = [torch.from_numpy(a).cuda() for a in (pos, q, types)]
+            _lib.check(lib.p3mx_forces(acts[1]._handle, n, *[_lib.dptr(a) for a in d],
+                                       _lib.dptr(f_dev), None, None,
+                                       flags | _lib.P3MX_DEVICE_PTRS,
+                                       ctypes.c_void_p(stream.cuda_stream)), acts[1]._handle)
+        np.testing.assert_array_equal(f_dev.cpu().numpy(), f)
