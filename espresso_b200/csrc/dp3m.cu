@@ -7,8 +7,8 @@
 //  2. brick binning and sort of the particles into records with the three
 //     moment components as charges, one super-brick assignment launch, one
 //     r2c z pass and one y pass over the three;
-//  3. k_fft_x_dp3m (energy sum, five spectra), the backward y and z passes to
-//     the three torque fields and the six entries of the force-field tensor,
+//  3. k_fft_x_dp3m (energy sum), k_fft_x_dp3m_inv (five spectra), the backward
+//     y and z passes to the three torque fields and the six entries of the force-field tensor,
 //     and the back-interpolation of the nine with unit-charge weights;
 //  4. k_dp3m_combine: forces and torques from the nine interpolated values;
 //  5. the real-space pair kernel over the Verlet lists of the dipoles.

@@ -6,10 +6,10 @@
 // charge path.  This file adds what is specific to point dipoles:
 //  * the dipolar influence functions G_energy (S = 2) and G_force (S = 3)
 //    on the r2c half mesh, and the aliasing sum of the energy correction;
-//  * an x pass that transforms the three components, forms
-//    mu(k) . d_op(k) once per point, accumulates the k-space energy, and
-//    emits three backward-x-transformed field spectra per launch (torque
-//    fields, or one half of the symmetric force-field tensor);
+//  * a forward x pass that forms mu(k) . d_op(k) once per point from two
+//    transforms and accumulates the k-space energy, and a backward one that
+//    emits the five spectra from which the y and z passes form the three
+//    torque fields and the six entries of the symmetric force-field tensor;
 //  * the per-particle combination of the interpolated fields into forces
 //    and torques, and the real-space pair kernel over the Verlet lists.
 #pragma once
@@ -617,9 +617,9 @@ k_dp3m_pairs(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
 // the entry's offset code, no minimum-image arithmetic): hardware reciprocal
 // square root, reciprocal and 2^x, A&S 7.1.26 or erfcf; the pairs' force and
 // torque terms and energies summed in FP64.  Bound by instruction issue: at
-// 131 072 dipoles 207 us (215 us with the six sums in pairs of FP32 values,
-// whose two-sums take more issue slots than the conversions and FP64 additions
-// and hold 48 bits), at 30 000 64 (69).
+// 131 072 dipoles 207 us for a cutoff of 4.7 (215 us with the six sums in pairs of
+// FP32 values, whose two-sums take more issue slots than the conversions and FP64
+// additions and hold 48 bits), 268 us for 5.2; at 30 000 64 (69).
 template <bool EV, int LPP>
 __global__ void __launch_bounds__(256, EV ? kDpPairBlocks32Ev : kDpPairBlocks32)
 k_dp3m_pairs_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,

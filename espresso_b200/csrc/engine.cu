@@ -424,7 +424,7 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
     m_tile_x = static_cast<int>(
         std::max<size_t>(1, std::min<size_t>(16, x_budget / (x_bufs * ldx * csz))));
     // dynamic shared memory of a block: the 227 KB limit less the kernels' static
-    // arrays
+    // arrays, 4.9 KB at most (the opt-in below fails where they do not fit)
     size_t const limit = 220 * 1024;
     size_t smem_zf = 0, smem_zi = 0;
     for (int r = 0; r < R; ++r) {
@@ -1253,7 +1253,7 @@ void Engine::launch_fft_z_inv(void *c0, long long field_stride, ZPass const &zp,
 //   ... with energies        116 / 98  118 /100  119 /102  119 /131  119 /132  121 /136
 //   FP32 ions, two types      66 / 60   74 / 67     -       88 / 84   93 / 89   96 / 97
 //   ... density 0.85         129 /102  140 /114     -      163 /143  174 /152  180 /164
-//   dipoles FP32             254 /212  263 /233  291 /261  294 /290  337 /311  340 /340
+//   dipoles FP32             245 /202  267 /217  272 /241  276 /275  309 /289  314 /317
 //   dipoles FP64             394 /314  407 /344  457 /354  458 /429  459 /455  465 /470
 // Below one wave, at 1 / 2 / 4 / 8 lanes, those chosen in brackets: FP32 23 457 ions
 // 33 / 25 / [22] / 26, 98 304 ions [37] / 39 / 41 / 53; 16 384 dipoles FP64 197 / 108

@@ -471,7 +471,8 @@ k_verlet_build(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of_
                    s_group_b + threadIdx.x * 8);
 }
 
-// FP32 exp(x) for the real-space kernel (x = -(alpha r)^2 in [-88, 0]):
+// FP32 exp(x) over the real-space kernels' range (x = -(alpha r)^2 in [-88, 0]), the
+// accurate form that p3mx_exp_check sets beside the kernels' single ex2:
 // e^x = 2^y with y = x log2(e) split error-free into y_hi + y_lo (the FMA
 // residual of the product, Dekker's TwoProduct, plus the low part of the
 // constant), then 2^y = 2^y_hi (hardware ex2.approx, ~2 ulp) * (1 + y_lo ln 2).
@@ -682,8 +683,8 @@ constexpr int kPairTail = 15, kPairTailLong = 18;
 // a group and FP64 across groups.
 // Bound by instruction issue (about 45 scalar instructions per entry and
 // three MUFU operations): the range-independent arithmetic runs on two
-// entries at a time in packed FP32, with the scalar code's roundings: 2^20 ions
-// 311 -> 241 us, 131 072 ions 57 -> 52 us.
+// entries at a time in packed FP32, with the scalar code's roundings.  The kernel
+// alone at density 0.5, cutoff 3.5: 2^20 ions 294 -> 271 us, 131 072 ions 49 -> 42 us.
 template <int MODE, int LPP>
 __global__ void __launch_bounds__(256, kPairBlocks32)
 k_pair_forces_rel(const RepGeom *__restrict__ reps, const int2 *__restrict__ blk,
