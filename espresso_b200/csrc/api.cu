@@ -771,7 +771,7 @@ int p3mx_set_bonds(p3mx_handle *h, int n_types, const p3mx_bond_params *types, s
     h->bond_types = bond_types_from_abi(n_types, types, n_bonds, bonds);
     h->bonds.assign(bonds, bonds + 3 * n_bonds);
     h->bonds_dirty = true;
-    if (h->eng && h->activated) {
+    if (h->eng && h->activated && h->eng->configured()) {
       h->eng->set_bonds(h->bond_types, h->bonds, h->eng->stream());
       h->bonds_dirty = false;
     }

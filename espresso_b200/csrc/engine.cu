@@ -1862,6 +1862,7 @@ void Engine::mark(const char *name, cudaStream_t st) {
 }
 
 std::vector<std::pair<std::string, double>> Engine::profile(int reps, cudaStream_t st) {
+  require_configured();
   std::vector<std::pair<std::string, double>> acc;
   for (int r = 0; r < reps; ++r) {
     m_marks.clear();
