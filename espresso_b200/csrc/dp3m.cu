@@ -178,10 +178,12 @@ public:
       int2 const *tab = E.m_blk_mesh.as<int2>() + E.m_sb_off[c];
       P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(E.m_sb_edge, cnt, st, geom, tab,
                                                      E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(),
-                                                     qmax3, E.m_tiles.as<Real>(), E.kerr(), 3,
+                                                     qmax3, E.m_tiles.as<Real>(), E.kerr(),
+                                                     E.m_cnt.as<int>(), E.m_clear, 3,
                                                      E.m_tiles_n, 1)));
       ++E.m_launches;
     }
+    E.m_cnt_dirty = false;
     E.launch_fft_z_fwd<Real>(E.m_tiles.as<Real>(), ck3, 3, st);
     E.mark("dp_assign_fft_z", st);
     E.launch_fft_y<Real>(ck3, E.m_cplx, y_plain(3), false, 0, st);

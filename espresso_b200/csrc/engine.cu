@@ -716,8 +716,8 @@ void Engine::sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, lon
 
 // Corner binning and brick sort of the particles into records; q holds nc (1
 // or 3) charges per particle, qmax receives nc words per replica.  The brick
-// counts are zero on entry (cleared by the sort before; by a memset after a
-// failed one).  The order inside a brick is left as the atomic slots made
+// counts are zero on entry (cleared by the sort or the assignment before; by a
+// memset after one that failed between).  The order inside a brick is left as the atomic slots made
 // it: the fixed-point assignment sums integers and the interpolation treats
 // every particle on its own, so the results do not depend on it.
 template <typename Real>
@@ -748,7 +748,7 @@ void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t 
              m_key.as<int>(), m_slot.as<int>(), m_start.as<int>(), m_dist.as<Real>(), q, m_n,
              m_rec.as<PRec<Real>>(), qmax, m_cnt.as<int>(), static_cast<int>(m_nkeys));
   ++m_launches;
-  m_cnt_dirty = false;
+  m_clear = scan ? static_cast<int>(m_nkeys) : 0;
 }
 
 namespace {
@@ -807,12 +807,12 @@ namespace {
 template <typename Real, int P>
 void launch_assign(int edge, int cnt, cudaStream_t st, RepGeom const *geom, int2 const *tab,
                    int const *start, PRec<Real> const *recs, unsigned const *qmax_bits,
-                   Real *tiles, int *err, int ncomp = 1, long long comp_tile = 0,
-                   int comp_q = 0) {
+                   Real *tiles, int *err, int *clear, int nclear, int ncomp = 1,
+                   long long comp_tile = 0, int comp_q = 0) {
   auto go = [&](auto kern, size_t smem) {
     pdl_launch(kern, dim3(static_cast<unsigned>(cnt), static_cast<unsigned>(ncomp)), 32 * kSbWarps,
                smem, st, true, geom, tab, cnt, start, recs, qmax_bits, tiles, err, comp_tile,
-               comp_q);
+               comp_q, clear, nclear);
   };
   if (edge == kSbEdgeSmall)
     go(ncomp > 1 ? k_p3m_assign_sb<Real, P, kSbEdgeSmall, true>
@@ -875,6 +875,7 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   } else {
     P3MX_CUDA(cudaMemsetAsync(m_start.p, 0, (m_nkeys + 1) * sizeof(int), st));
     P3MX_CUDA(cudaMemsetAsync(qmax_bits, 0, R * sizeof(int), st));
+    m_clear = 0;
   }
   // 2. charge assignment: one block per super-brick, its tile stored whole
   for (int c = 1; c <= 7; ++c) {
@@ -884,9 +885,11 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
     P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, geom, tab, m_start.as<int>(),
                                                    m_rec.as<PRec<Real>>(), qmax_bits,
-                                                   m_tiles.as<Real>(), kerr())));
+                                                   m_tiles.as<Real>(), kerr(), m_cnt.as<int>(),
+                                                   m_clear)));
     ++m_launches;
   }
+  m_cnt_dirty = m_cnt_dirty && m_n == 0; // cleared by the placing kernel or the assignment
   mark("p3m_assign", st);
   // 3. forward FFT z (r2c) and y
   launch_fft_z_fwd<Real>(m_tiles.as<Real>(), m_ck.p, 1, st);

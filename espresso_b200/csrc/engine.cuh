@@ -202,6 +202,7 @@ private:
   template <typename Real>
   void bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t st);
   bool m_cnt_dirty = true; // the brick counts are not known to be zero
+  int m_clear = 0;         // brick counts that the assignment behind the sort clears
   void sort_keys(int *key, int *slot, int *cnt, int *start, int *perm, long long nkeys,
                  cudaStream_t st, const int *cond = nullptr);
 

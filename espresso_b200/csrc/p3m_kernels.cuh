@@ -146,12 +146,13 @@ k_p3m_bin(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of,
 // (FP32 bits rounded up, atomic maximum: order-independent; set c at
 // qmax_bits + c * n_rep) for the fixed-point scale of the charge assignment.
 // NC charges per particle, q[NC i + c].  The brick counts `cnt` are cleared for
-// the next sort.  A particle is one full 32-byte sector (FP32) written at
-// random: the gathering weight kernel it replaces read five random sectors and
-// wrote 112 bytes.
-// SCAN (small systems, up to kPlaceScan bricks): `start` is not given but made, every block
-// scanning all counts for itself (16 KB from L2 at most) and block 0 storing the
-// result; the last block to have read the counts clears them (ticket cnt[nkeys]).
+// the next sort (without SCAN, where `start` already holds their scan).  A
+// particle is one full 32-byte sector (FP32) written at random: the gathering
+// weight kernel it replaces read five random sectors and wrote 112 bytes.
+// SCAN (small systems, up to kPlaceScan bricks): `start` is not given but made,
+// every block scanning all counts for itself (16 KB from L2 at most) and block 0 storing the
+// result; the assignment, behind this kernel, clears the counts (a last block that
+// does so here needs a ticket between two fences: 4.2 -> 5.1 us at 2000 ions).
 // A small system's pass is bound by the number of dependent launches, and this
 // is one less.
 constexpr int kPlaceScan = 4096;
@@ -183,20 +184,9 @@ k_p3m_place(const RepGeom *__restrict__ reps, const int *__restrict__ rep_of, in
           start[k0 + k] = run;
         run += v[k];
       }
-    __shared__ bool s_last;
-    if (threadIdx.x == 0) {
-      if (blockIdx.x == 0)
-        start[nkeys] = total;
-      // the block's reads of the counts (behind the scan's barrier) come before
-      // its ticket, the last ticket before the clearing
-      __threadfence();
-      s_last = atomicAdd(cnt + nkeys, 1) == static_cast<int>(gridDim.x) - 1;
-      __threadfence();
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      start[nkeys] = total;
     __syncthreads();
-    if (s_last) // every block has read the counts
-      for (int k = threadIdx.x; k <= nkeys; k += 256)
-        cnt[k] = 0;
   } else {
     for (long long k = i; k <= nkeys; k += static_cast<long long>(gridDim.x) * blockDim.x)
       cnt[k] = 0;
@@ -385,7 +375,10 @@ __global__ void __launch_bounds__(32 * kSbWarps, sizeof(Real) == 4 ? 4 : 1)
 k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, int nsb,
                 const int *__restrict__ start, const PRec<Real> *__restrict__ recs,
                 const unsigned *__restrict__ qmax_bits, Real *__restrict__ tiles,
-                int *__restrict__ err, long long comp_tile, int comp_q) {
+                int *__restrict__ err, long long comp_tile, int comp_q, int *__restrict__ clear,
+                int nclear) {
+  // clear: nclear words set to zero (the brick counts that the placing kernel
+  // before this one has scanned).
   // MC: blockIdx.y picks one of several charge sets assigned by one launch
   // (the dipole components): its tiles and |q| maxima lie comp_tile / comp_q
   // elements after the previous set's. The single-set instance leaves the
@@ -413,6 +406,8 @@ k_p3m_assign_sb(const RepGeom *__restrict__ reps, const int2 *__restrict__ sbs, 
   __shared__ int s_r0[kSbMaxRuns], s_pre[kSbMaxRuns + 1];
   __shared__ Real s_cf[8 * 8];
   pdl_enter();
+  for (int k = blockIdx.x * NT + threadIdx.x; k < nclear; k += gridDim.x * NT)
+    clear[k] = 0;
   if (static_cast<int>(blockIdx.x) >= nsb)
     return; // whole block
   Word *tile = reinterpret_cast<Word *>(smem_raw);
