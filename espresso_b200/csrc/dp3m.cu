@@ -33,7 +33,7 @@ namespace p3mx {
 
 class Dp3mEngine {
 public:
-  explicit Dp3mEngine(bool fp32) : m_eng(fp32) { m_eng.set_field_sets(3, kDipoleSpectra); }
+  explicit Dp3mEngine(bool fp32) : m_eng(fp32) {}
 
   Engine &engine() { return m_eng; }
   long long n() const { return m_eng.n_part(); }
@@ -41,10 +41,26 @@ public:
   // False until the first configuration and after one that threw.
   bool configured() const { return m_configured && m_eng.configured(); }
 
-  // One cubic replica of edge L with mesh M^3.
+  // One cubic replica of edge L with mesh M^3: with a field mesh for each of the
+  // three field sets, or, where the device memory does not hold these, with one
+  // for all (two launches more per evaluation each of the backward z pass and of
+  // the interpolation).
   void configure(double L, int M, int cao, double alpha, double r_cut, double skin,
                  const double *mesh_off, long long n) {
+    try {
+      configure_sets(3, L, M, cao, alpha, r_cut, skin, mesh_off, n);
+    } catch (Error const &e) {
+      if (e.code != 4)
+        throw;
+      configure_sets(1, L, M, cao, alpha, r_cut, skin, mesh_off, n);
+    }
+  }
+  void configure_sets(int meshes, double L, int M, int cao, double alpha, double r_cut, double skin,
+                 const double *mesh_off, long long n) {
     m_configured = false;
+    if (meshes != m_meshes)
+      m_eng.set_field_sets(3, kDipoleSpectra, meshes);
+    m_meshes = meshes;
     ReplicaConf c;
     for (int d = 0; d < 3; ++d) {
       c.box[d] = L;
@@ -170,7 +186,8 @@ public:
     E.mark("dp_sort", st);
     // 2. the three component meshes: one assignment and one z pass over all
     // three (blockIdx.y = component)
-    C *ck3 = E.m_ck.as<C>();
+    C *ck3 = static_cast<C *>(E.ck());
+    Real *tiles = static_cast<Real *>(E.tiles());
     for (int c = 1; c <= 7; ++c) {
       int const cnt = E.m_sb_off[c + 1] - E.m_sb_off[c];
       if (cnt == 0)
@@ -178,13 +195,13 @@ public:
       int2 const *tab = E.m_blk_mesh.as<int2>() + E.m_sb_off[c];
       P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(E.m_sb_edge, cnt, st, geom, tab,
                                                      E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(),
-                                                     qmax3, E.m_tiles.as<Real>(), E.kerr(),
+                                                     qmax3, tiles, E.kerr(),
                                                      E.m_cnt.as<int>(), E.m_clear, 3,
                                                      E.m_tiles_n, 1)));
       ++E.m_launches;
     }
     E.m_cnt_dirty = false;
-    E.launch_fft_z_fwd<Real>(E.m_tiles.as<Real>(), ck3, 3, st);
+    E.launch_fft_z_fwd<Real>(tiles, ck3, 3, st);
     E.mark("dp_assign_fft_z", st);
     E.launch_fft_y<Real>(ck3, E.m_cplx, y_plain(3), false, 0, st);
     E.mark("dp_fft_y", st);
@@ -216,27 +233,30 @@ public:
     if (!want_ft)
       return;
     E.launch_fft_y<Real>(E.m_field.p, E.m_cplx, dp_y_pass(), true, 0, st);
-    E.launch_fft_z_inv<Real>(E.m_field.p, E.m_cplx, dp_z_pass(), 3, 0, E.m_E.p, st);
-    E.mark("dp_inv_yz", st);
-    double *out = m_out.as<double>();
     RepGeom const *gi = m_geom_interp.as<RepGeom>();
-    for (int c = 1; n > 0 && c <= 7; ++c) {
-      int const nbr = E.m_brick_off[c + 1] - E.m_brick_off[c];
-      if (nbr == 0)
-        continue;
-      int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
-      // a third of the resident blocks per field set, rounded down: rounded up,
-      // one or two blocks had to wait for a second wave as long as the first
-      // (131 072 dipoles FP32 166 -> 113 us, 16 384 FP64 78 -> 58 us)
-      P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>,
-                                 dim3(std::max(1, interp_grid<Real, P>(3 * nbr) / 3), 3),
-                                 32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true, gi, tab,
-                                 nbr, E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(), 1,
-                                 E.m_tmap.as<CUtensorMap>(), 1, E.d_q(), E.m_dipole.as<double>(),
-                                 out, 3 * n, 1, E.kerr())));
-      ++E.m_launches;
+    for (int set = 0; set < 3; set += m_meshes) {
+      E.launch_fft_z_inv<Real>(E.m_field.p, E.m_cplx, dp_z_pass(set), m_meshes, 0, E.m_E.p, st);
+      E.mark("dp_inv_yz", st);
+      double *out = m_out.as<double>() + 3 * n * set;
+      for (int c = 1; n > 0 && c <= 7; ++c) {
+        int const nbr = E.m_brick_off[c + 1] - E.m_brick_off[c];
+        if (nbr == 0)
+          continue;
+        int2 const *tab = E.m_blk_brick.as<int2>() + E.m_brick_off[c];
+        // a third of the resident blocks per field set, rounded down: rounded up,
+        // one or two blocks had to wait for a second wave as long as the first
+        // (131 072 dipoles FP32 166 -> 113 us, 16 384 FP64 78 -> 58 us)
+        P3MX_CAO_DISPATCH_R(c, (pdl_launch(k_p3m_interp<Real, P>,
+                                   dim3(std::max(1, interp_grid<Real, P>(m_meshes * nbr) / m_meshes),
+                                        m_meshes),
+                                   32 * (1 + kInterpWarps), interp_smem<Real, P>(), st, true, gi, tab,
+                                   nbr, E.m_start.as<int>(), E.m_rec.as<PRec<Real>>(), 1,
+                                   E.m_tmap.as<CUtensorMap>(), 1, E.d_q(), E.m_dipole.as<double>(),
+                                   out, 3 * n, 1, E.kerr())));
+        ++E.m_launches;
+      }
+      E.mark("dp_interp", st);
     }
-    E.mark("dp_interp", st);
   }
 
   // Full evaluation.  f, t: device arrays (3N) or nullptr when not wanted;
@@ -421,6 +441,7 @@ private:
   DevBuf m_mu, m_out, m_smu, m_ge, m_gf, m_part, m_sums, m_flag, m_geom_interp;
   DevBuf m_qmax3;
   bool m_configured = false;
+  int m_meshes = 0; // field meshes: 3, or 1 for all sets
   bool m_g_valid = false, m_phi_valid = false, m_table_set = false;
   double m_phi = 0.0;
   int m_M = 0, m_cao = 0;

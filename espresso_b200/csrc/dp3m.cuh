@@ -398,8 +398,15 @@ inline YPass dp_y_pass() {
   return YPass{9, {0, 1, 1, 2, 3, 3, 4, 4, 4}, {0, 5, 6, 2, 7, 8, 9, 10, 11},
                {0, 1, 0, 0, 1, 0, 2, 1, 0}};
 }
-inline ZPass dp_z_pass() {
-  return ZPass{{0, 5, 6, 2, 7, 8, 9, 10, 11}, {0, 0, 1, 0, 0, 1, 0, 1, 2}};
+// (of the sets from `set` on)
+inline ZPass dp_z_pass(int set) {
+  constexpr signed char arr[9] = {0, 5, 6, 2, 7, 8, 9, 10, 11}, pw[9] = {0, 0, 1, 0, 0, 1, 0, 1, 2};
+  ZPass z{};
+  for (int k = 3 * set; k < 9; ++k) {
+    z.arr[k - 3 * set] = arr[k];
+    z.pw[k - 3 * set] = pw[k];
+  }
+  return z;
 }
 
 // Forces and torques from the interpolated fields (AoS, 3 per particle):

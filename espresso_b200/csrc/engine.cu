@@ -566,11 +566,12 @@ void Engine::configure(std::vector<ReplicaConf> const &conf, long long n_total) 
   m_scan_tiles.ensure((ceil_div(std::max(m_nkeys, m_oct_mult * m_cells) + 1, kScanTile) + 1) * sizeof(int));
   m_dist.ensure(3 * n * rsz);
   m_rec.ensure(n * (m_fp32 ? sizeof(PRec<float>) : sizeof(PRec<double>)));
-  m_tiles.ensure(m_sets * static_cast<size_t>(m_tiles_n) * rsz);
-  m_E.ensure(m_sets * 4 * m_ebins * rsz);
+  size_t const spectrum = m_cplx * csz, ntile = m_sets * static_cast<size_t>(m_tiles_n) * rsz;
+  m_ck_off = std::max((m_spectra - m_sets) * spectrum, (ntile + 255) / 256 * 256);
+  m_field.ensure(m_ck_off + m_sets * spectrum);
+  m_sorted = false;
+  m_E.ensure(m_meshes * 4 * m_ebins * rsz);
   encode_field_maps(st);
-  m_ck.ensure(m_sets * m_cplx * csz);
-  m_field.ensure(m_spectra * m_cplx * csz);
   m_ginf.ensure(m_cplx * rsz);
   m_part_x.ensure(static_cast<size_t>(m_n_blk_x) * 8 * sizeof(double));
   m_sums_x.ensure(static_cast<size_t>(R) * 8 * sizeof(double));
@@ -724,6 +725,7 @@ template <typename Real>
 void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t st) {
   int const R = n_rep();
   const int *rep_of = R > 1 ? m_rep_of.as<int>() : nullptr;
+  m_sorted = false;
   if (!m_binned) {
     if (m_cnt_dirty)
       P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
@@ -749,6 +751,7 @@ void Engine::bin_and_sort(const double *q, int nc, unsigned *qmax, cudaStream_t 
              m_rec.as<PRec<Real>>(), qmax, m_cnt.as<int>(), static_cast<int>(m_nkeys));
   ++m_launches;
   m_clear = scan ? static_cast<int>(m_nkeys) : 0;
+  m_sorted = true;
 }
 
 namespace {
@@ -770,13 +773,13 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // One tensor map per replica over its packed, ghost-padded field mesh E (4
 // values per point): dims (4 E2, E1, E0) with E = epad, box (4 Ed, Ed, Ed)
-// with Ed = brick + cao - 1 (<= epad by construction); m_sets field meshes
+// with Ed = brick + cao - 1 (<= epad by construction); m_meshes field meshes
 // m_ebins records apart.
 void Engine::encode_field_maps(cudaStream_t st) {
   auto enc = tensor_map_encoder();
   size_t const es = m_fp32 ? sizeof(float) : sizeof(double);
   size_t const R = m_geom.size();
-  std::vector<CUtensorMap> maps(m_sets * R);
+  std::vector<CUtensorMap> maps(m_meshes * R);
   for (size_t m = 0; m < maps.size(); ++m) {
     size_t const set = m / R;
     RepGeom const &G = m_geom[m - set * R];
@@ -853,6 +856,21 @@ template <typename Real, int P> int interp_grid(int nbricks) {
   case 6: { constexpr int P = 6; KERNEL_CALL; } break;                         \
   default: { constexpr int P = 7; KERNEL_CALL; } break;                        \
   }
+template <typename Real> void Engine::assign(int nclear, cudaStream_t st) {
+  unsigned const *qmax_bits = reinterpret_cast<unsigned *>(m_cnt.as<int>() + m_nkeys + 1);
+  for (int c = 1; c <= 7; ++c) {
+    int const cnt = m_sb_off[c + 1] - m_sb_off[c];
+    if (cnt == 0)
+      continue;
+    int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
+    P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, m_geom_d.as<RepGeom>(), tab,
+                                                   m_start.as<int>(), m_rec.as<PRec<Real>>(),
+                                                   qmax_bits, static_cast<Real *>(tiles()), kerr(),
+                                                   m_cnt.as<int>(), nclear)));
+    ++m_launches;
+  }
+}
+
 template <typename Real>
 void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
                           cudaStream_t st) {
@@ -876,24 +894,15 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
     P3MX_CUDA(cudaMemsetAsync(m_start.p, 0, (m_nkeys + 1) * sizeof(int), st));
     P3MX_CUDA(cudaMemsetAsync(qmax_bits, 0, R * sizeof(int), st));
     m_clear = 0;
+    m_sorted = true;
   }
   // 2. charge assignment: one block per super-brick, its tile stored whole
-  for (int c = 1; c <= 7; ++c) {
-    int const cnt = m_sb_off[c + 1] - m_sb_off[c];
-    if (cnt == 0)
-      continue;
-    int2 const *tab = m_blk_mesh.as<int2>() + m_sb_off[c];
-    P3MX_CAO_DISPATCH_R(c, (launch_assign<Real, P>(m_sb_edge, cnt, st, geom, tab, m_start.as<int>(),
-                                                   m_rec.as<PRec<Real>>(), qmax_bits,
-                                                   m_tiles.as<Real>(), kerr(), m_cnt.as<int>(),
-                                                   m_clear)));
-    ++m_launches;
-  }
+  assign<Real>(m_clear, st);
   m_cnt_dirty = m_cnt_dirty && m_n == 0; // cleared by the placing kernel or the assignment
   mark("p3m_assign", st);
   // 3. forward FFT z (r2c) and y
-  launch_fft_z_fwd<Real>(m_tiles.as<Real>(), m_ck.p, 1, st);
-  launch_fft_y<Real>(m_ck.p, 0, y_plain(1), false, 0, st);
+  launch_fft_z_fwd<Real>(static_cast<Real *>(tiles()), ck(), 1, st);
+  launch_fft_y<Real>(ck(), 0, y_plain(1), false, 0, st);
   mark("fft_fwd_zy", st);
   // 4. x pass fused with the k-space operator (+ energy/virial partials)
   bool const want_f = (f != nullptr);
@@ -901,7 +910,7 @@ void Engine::long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
   fft_pick(m_kind[0], [&](auto kind) {
     constexpr int K = decltype(kind)::value;
     pdl_launch(want_ev ? k_fft_x_kspace<Real, true, K> : k_fft_x_kspace<Real, false, K>, m_n_blk_x,
-               256, m_smem_x, st, true, geom, m_blk_x.as<Blk>(), m_ck.as<C>(), m_ginf.as<Real>(),
+               256, m_smem_x, st, true, geom, m_blk_x.as<Blk>(), static_cast<const C *>(ck()), m_ginf.as<Real>(),
                m_field.as<C>(), m_cplx, m_tile_x, want_f ? 1 : 0, m_part_x.as<double>(),
                m_tw.as<C>());
   });
@@ -1177,6 +1186,7 @@ template <typename Real> void Engine::front(ParticleArrays const &in, cudaStream
   if (m_cnt_dirty)
     P3MX_CUDA(cudaMemsetAsync(m_cnt.p, 0, (m_nkeys + 1) * sizeof(int), st));
   m_cnt_dirty = true;
+  m_sorted = false;
   int const R = n_rep();
   k_front<Real><<<ceil_div(m_n, 256), 256, 0, st>>>(
       m_geom_d.as<RepGeom>(), R > 1 ? m_rep_of.as<int>() : nullptr, m_n, in, d_pos(), d_q(),
@@ -1565,13 +1575,17 @@ std::vector<double> Engine::mesh_copy(int r, cudaStream_t st) {
   require_configured();
   auto const &G = m_geom[r];
   long long const ms = static_cast<long long>(G.mesh[0]) * G.mesh[1] * G.mesh[2];
-  std::vector<double> out(ms);
-  // the mesh is the sum of the assignment's tiles
+  std::vector<double> out(ms, 0.0);
+  if (!m_sorted)
+    return out; // nothing assigned yet
+  // the mesh is the sum of the assignment's tiles, made again from the records
+  // (the same integers): the spectra have taken the tiles' place
   auto sum = [&](auto zero) {
     using Real = decltype(zero);
     m_rho.ensure(ms * sizeof(Real));
+    assign<Real>(0, st);
     k_tiles_to_mesh<Real><<<ceil_div(ms, 256), 256, 0, st>>>(
-        m_geom_d.as<RepGeom>(), r, m_tiles.as<Real>(), m_cov.as<int>(), m_sb_edge,
+        m_geom_d.as<RepGeom>(), r, static_cast<const Real *>(tiles()), m_cov.as<int>(), m_sb_edge,
         m_rho.as<Real>());
     ++m_launches;
     std::vector<Real> t(ms);

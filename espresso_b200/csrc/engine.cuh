@@ -26,13 +26,16 @@ struct DevBuf {
     if (p)
       cudaFree(p);
   }
-  void ensure(size_t nbytes) {
-    if (nbytes <= bytes && p)
-      return;
+  void release() {
     if (p)
       cudaFree(p);
     p = nullptr;
     bytes = 0;
+  }
+  void ensure(size_t nbytes) {
+    if (nbytes <= bytes && p)
+      return;
+    release();
     size_t const want = nbytes ? nbytes : 16;
     if (cudaMalloc(&p, want) != cudaSuccess) {
       cudaGetLastError();
@@ -82,11 +85,13 @@ public:
   ReplicaConf const &conf(int r) const { return m_conf[r]; }
   cudaStream_t stream() const { return m_stream; }
 
-  // Charge sets (tiles, spectra and field meshes) and field spectra that
-  // configure() allocates: one and kChargeSpectra, or a dipolar engine's.
-  void set_field_sets(int sets, int spectra) {
+  // Charge sets (tiles and forward spectra), field spectra and field meshes that
+  // configure() allocates: one, kChargeSpectra and one, or a dipolar engine's.
+  void set_field_sets(int sets, int spectra, int meshes) {
     m_sets = sets;
     m_spectra = spectra;
+    m_meshes = meshes;
+    m_E.release();
   }
   // (Re)builds geometry, plans, block tables; allocates the buffers.
   void configure(std::vector<ReplicaConf> const &conf, long long n_total);
@@ -169,6 +174,9 @@ public:
                   const double *box, double prefactor);
 
 private:
+  // The charge assignment of the sorted records into the tiles, nclear brick
+  // counts cleared beside it.
+  template <typename Real> void assign(int nclear, cudaStream_t st);
   template <typename Real> void long_range_t(double *f, bool overwrite, bool want_e, bool want_v,
                                              cudaStream_t st);
   template <typename Real> void short_range_t(double *f, bool overwrite, bool want_ev,
@@ -213,7 +221,7 @@ private:
 
   bool m_fp32;
   bool m_configured = false;
-  int m_sets = 1, m_spectra = kChargeSpectra;
+  int m_sets = 1, m_spectra = kChargeSpectra, m_meshes = 1;
   int m_device = 0, m_sms = 148;
   cudaStream_t m_stream = nullptr;
   long long m_launches = 0;
@@ -254,7 +262,16 @@ private:
   DevBuf m_key, m_slot, m_cnt, m_start, m_scan_tiles;
   DevBuf m_dist, m_rec; // distances to the mesh points; brick-sorted records
   DevBuf m_rho; // charge mesh of one replica (mesh_copy only)
-  DevBuf m_tiles, m_ck, m_field, m_E, m_ginf;
+  // One buffer for the assignment's tiles (at its start, read by the forward z
+  // pass), the m_sets forward spectra (at m_ck_off, read by the x pass) and the
+  // m_spectra field spectra (from its start; the x pass writes none over the
+  // forward spectra, the y pass behind it may)
+  DevBuf m_field;
+  size_t m_ck_off = 0;
+  void *tiles() const { return m_field.p; }
+  void *ck() const { return m_field.as<char>() + m_ck_off; }
+  bool m_sorted = false; // records and brick starts of the last evaluation stand
+  DevBuf m_E, m_ginf;
   DevBuf m_tmap; // per replica: tensor map of its field mesh (interpolation tiles)
   DevBuf m_part_x, m_part_census, m_sums_x, m_sums_census, m_dipole;
   bool m_ginf_valid = false;

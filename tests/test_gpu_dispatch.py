@@ -373,3 +373,42 @@ def test_device_arrays_on_a_stream(cls):
                                        flags | _lib.P3MX_DEVICE_PTRS,
                                        ctypes.c_void_p(stream.cuda_stream)), acts[1]._handle)
         np.testing.assert_array_equal(f_dev.cpu().numpy(), f)
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_dipoles_with_little_memory(single):
+    """Where the device memory does not hold three field meshes, one serves the
+    three field sets in turn: the same forces and torques, bitwise."""
+    n, mesh, edge = 3000, 160, 18.0
+    pos, _ = _ions(n, [edge] * 3, seed=2)
+    mu = np.random.default_rng(2).normal(size=(n, 3))
+    lib = _lib.load()
+
+    def compute():
+        act = DipolarP3M(prefactor=1.1, accuracy=1e-4, mesh=mesh, cao=5, r_cut=3.0, alpha=1.0,
+                         tune=False, single_precision=single)
+        act._set_system([edge] * 3, 0.4, (True, True, True))
+        act._activate(pos, mu)
+        f, t, _ = act._compute(pos, mu)
+        count = ctypes.c_longlong()
+        lib.p3mx_dp3m_launch_count(act._handle, ctypes.byref(count))
+        return act, f, t, count.value
+    act = compute()[0]  # kernels loaded, caches filled
+    del act
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    act, f, t, launches = compute()
+    used = before - torch.cuda.mem_get_info()[0]
+    del act
+    # leave one field mesh less than the actor took
+    field = 4 * (4 if single else 8) * (mesh + 4) ** 3
+    ballast = torch.empty(before - used + field, dtype=torch.uint8, device="cuda")
+    try:
+        act, f1, t1, launches1 = compute()
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    assert launches1 == launches + 4
+    np.testing.assert_array_equal(f1, f)
+    np.testing.assert_array_equal(t1, t)
