@@ -172,9 +172,13 @@ void Engine::set_pair_table(int ntypes, std::vector<PairIA> const &tab) {
   if (m_configured && ntypes == m_ntypes && tab.size() == m_ia.size() &&
       std::memcmp(tab.data(), m_ia.data(), tab.size() * sizeof(PairIA)) == 0)
     return;
+  // the sorted records stand where the configuration they belong to is made again
+  bool const sorted = m_sorted && m_configured;
   store_pair_table(ntypes, tab);
-  if (!m_conf.empty())
+  if (!m_conf.empty()) {
     configure(std::vector<ReplicaConf>(m_conf), m_n);
+    m_sorted = sorted;
+  }
 }
 
 void Engine::require_configured() const {

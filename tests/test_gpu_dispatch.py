@@ -263,6 +263,19 @@ def test_observables_without_forces(cls):
         _lib.check(lib.p3mx_copy_mesh(act._handle, rho.ctypes.data_as(DP), rho.size), act._handle)
         rho_o = O.p3m_kspace(prm, x, q, want_mesh=True)[3]
         np.testing.assert_allclose(rho, rho_o, rtol=0, atol=RTOL[cls] * np.abs(rho_o).max())
+    # a mesh is copied again as it was, also after a new pair table
+    _lib.check(lib.p3mx_forces(act._handle, 1500, _lib.dptr(x), _lib.dptr(q), None, _lib.dptr(force),
+                               None, None, _lib.P3MX_OVERWRITE, None), act._handle)
+    tab = (_lib.PairParams * 1)()
+    tab[0].wca_eps = tab[0].wca_sig = 1.0
+    again = []
+    for k in range(2):
+        rho = np.zeros((32, 32, 32))
+        _lib.check(lib.p3mx_copy_mesh(act._handle, rho.ctypes.data_as(DP), rho.size), act._handle)
+        again.append(rho)
+        _lib.check(lib.p3mx_set_pair_params(act._handle, 1, tab), act._handle)
+    np.testing.assert_array_equal(again[1], again[0])
+    np.testing.assert_allclose(again[0], rho_o, rtol=0, atol=RTOL[cls] * np.abs(rho_o).max())
 
 
 def _device_call(lib, act, fn, n, pos, q, types, f):
